@@ -29,7 +29,7 @@ def mlel():
 
 @pytest.fixture(scope="session")
 def reference_root():
-    if not os.path.isdir(REFERENCE_ROOT):
+    if not os.path.isdir(os.path.join(REFERENCE_ROOT, "tests")):  # absent, or an empty mount point
         pytest.skip("reference checkout not present")
     return REFERENCE_ROOT
 
