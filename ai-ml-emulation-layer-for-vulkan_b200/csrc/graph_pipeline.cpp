@@ -1389,7 +1389,18 @@ void GraphPipeline::fuse() {
     for (int i = 0; i < n; ++i) {
         const int gi = group[size_t(i)];
         if (gi < 0) {
-            exec_.push_back(ops_[size_t(i)]);
+            // The reference's CONCAT is one pass per input: consecutive passes into one tensor run as one node, whose
+            // inputs and offsets are theirs in order.
+            OpDesc *last = exec_.empty() ? nullptr : &exec_.back();
+            const OpDesc &op = ops_[size_t(i)];
+            if (op.kind == OP_CONCAT && last != nullptr && last->kind == OP_CONCAT && last->out == op.out &&
+                last->i[0] == op.i[0] && int(last->in.size()) < kMaxConcatPasses && op.in[0] != op.out[0]) {
+                last->i[1 + last->in.size()] = op.i[1];
+                last->in.push_back(op.in[0]);
+                last->fusedOps.push_back(i);
+                continue;
+            }
+            exec_.push_back(op);
             exec_.back().fusedOps = {i};
         } else if (fused[size_t(gi)].last == i) {
             std::sort(fused[size_t(gi)].node.fusedOps.begin(), fused[size_t(gi)].node.fusedOps.end());

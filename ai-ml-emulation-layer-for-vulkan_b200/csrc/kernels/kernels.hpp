@@ -55,7 +55,7 @@ int transposeForMatmul(const int8_t *b, int8_t *bt, int32_t *corr, int batches, 
 // corr[n][w] = -za * sum_c b[n][c][w] (mod 2^32) alone, for the kernel that reads b where it lies.  W a multiple of 16.
 int columnSumsForMatmul(const int8_t *b, int32_t *corr, int batches, int C, int W, int32_t za, cudaStream_t s);
 bool maxPoolI8Eligible(const TView &in, const TView &out);
-// packed int8 NHWC tensors (same conditions as maxPoolI8Eligible) with a window of at least 16 taps
+// packed int8 NHWC tensors with a window of at least 16 taps
 bool avgPoolI8Eligible(const TView &in, const TView &out, const PoolAttr &a);
 int avgPoolI8(const TView &in, const TView &out, const PoolAttr &a, cudaStream_t s);
 int maxPoolI8(const TView &in, const TView &out, const PoolAttr &a, cudaStream_t s);
@@ -79,6 +79,16 @@ bool vecRowReduce(int32_t op, const TView &in, const TView &out, uint32_t axis, 
 bool vecTransposeRows(const TView &in, const TView &out, const uint32_t *perms, cudaStream_t s, int *rc);
 // one-byte elements, the input's last axis becomes the output's second-to-last and another axis its last
 bool vecTransposeLast2Bytes(const TView &in, const TView &out, const uint32_t *perms, cudaStream_t s, int *rc);
+
+// move_ops.cu: strided copies as runs of bytes.  As above: false when the copy does not reduce to one.
+bool moveTranspose(const TView &in, const TView &out, const uint32_t *perms, cudaStream_t s, int *rc);
+bool moveConcat(const TView *const *ins, const uint32_t *offsets, int count, const TView &out, uint32_t axis, cudaStream_t s,
+                int *rc);
+bool moveSlice(const TView &in, const TView &out, const uint32_t *start, cudaStream_t s, int *rc);
+bool moveTile(const TView &in, const TView &out, cudaStream_t s, int *rc);
+bool moveReverse(const TView &in, const TView &out, uint32_t axis, cudaStream_t s, int *rc);
+bool moveResizeNearest(const TView &in, const TView &out, const ResizeAttr &a, cudaStream_t s, int *rc);
+bool moveArgmaxLast(const TView &in, const TView &out, uint32_t axis, cudaStream_t s, int *rc);
 
 // Joins column blocks of byte rows: out[row][first[g] + j] = staging[(g * rows + row) * pitch + j], j < count[g].
 // The blocks follow one another (first[0] = 0, first[g + 1] = first[g] + count[g]); at most kMaxColumnBlocks.

@@ -333,13 +333,29 @@ int launchOp(const OpDesc &op, const TView *T, cudaStream_t s, LaunchChain *chai
         for (int k = 0; k < kMaxRank; ++k) {
             perms[k] = uint32_t(op.i[k]);
         }
-        if (vecTransposeRows(in(0), out, perms, s, &rc) || vecTransposeLast2Bytes(in(0), out, perms, s, &rc)) {
+        if (vecTransposeRows(in(0), out, perms, s, &rc) || vecTransposeLast2Bytes(in(0), out, perms, s, &rc) ||
+            moveTranspose(in(0), out, perms, s, &rc)) {
             return rc;
         }
         return genericTranspose(in(0), out, perms, s);
     }
-    case OP_CONCAT:
-        return genericConcat(in(0), out, uint32_t(op.i[0]), uint32_t(op.i[1]), s);
+    case OP_CONCAT: {
+        // one pass of the reference, or consecutive passes into one tensor (GraphPipeline::fuse)
+        const TView *ins[kMaxConcatPasses];
+        uint32_t offsets[kMaxConcatPasses];
+        const int count = int(op.in.size());
+        for (int k = 0; k < count; ++k) {
+            ins[k] = &in(size_t(k));
+            offsets[k] = uint32_t(op.i[1 + k]);
+        }
+        if (moveConcat(ins, offsets, count, out, uint32_t(op.i[0]), s, &rc)) {
+            return rc;
+        }
+        for (int k = 0; k < count && rc == MLEL_SUCCESS; ++k) {
+            rc = genericConcat(*ins[k], out, uint32_t(op.i[0]), offsets[k], s);
+        }
+        return rc;
+    }
     case OP_CLAMP:
         if (vecClampI8(in(0), out, wrapTo(out.dtype, int64_t(op.d[0])), wrapTo(out.dtype, int64_t(op.d[1])), s, &rc)) {
             return rc;
@@ -394,6 +410,9 @@ int launchOp(const OpDesc &op, const TView *T, cudaStream_t s, LaunchChain *chai
         for (int k = 0; k < kMaxRank; ++k) {
             start[k] = uint32_t(op.i[k]);
         }
+        if (moveSlice(in(0), out, start, s, &rc)) {
+            return rc;
+        }
         return genericSlice(in(0), out, start, s);
     }
     case OP_PAD:
@@ -409,14 +428,23 @@ int launchOp(const OpDesc &op, const TView *T, cudaStream_t s, LaunchChain *chai
     case OP_RFFT2D:
         return fft2d(&in(0), nullptr, out, T[op.out[1]], false, s);
     case OP_ARGMAX:
+        if (moveArgmaxLast(in(0), out, uint32_t(op.i[0]), s, &rc)) {
+            return rc;
+        }
         return indexArgmax(in(0), out, uint32_t(op.i[0]), s);
     case OP_GATHER:
         return indexGather(in(0), in(1), out, s);
     case OP_SCATTER:
         return indexScatter(in(0), in(1), in(2), out, s);
     case OP_REVERSE:
+        if (moveReverse(in(0), out, uint32_t(op.i[0]), s, &rc)) {
+            return rc;
+        }
         return indexReverse(in(0), out, uint32_t(op.i[0]), s);
     case OP_TILE:
+        if (moveTile(in(0), out, s, &rc)) {
+            return rc;
+        }
         return indexTile(in(0), out, s);
     case OP_RESIZE: {
         ResizeAttr a{};
@@ -424,6 +452,9 @@ int launchOp(const OpDesc &op, const TView *T, cudaStream_t s, LaunchChain *chai
             a.scale[k] = op.i[k];
         }
         a.offset[0] = op.i[4], a.offset[1] = op.i[5], a.border[0] = op.i[6], a.border[1] = op.i[7], a.mode = op.i[8];
+        if (moveResizeNearest(in(0), out, a, s, &rc)) {
+            return rc;
+        }
         return resizeInteger(in(0), out, a, s);
     }
     case OP_TRANSPOSE_CONV2D:

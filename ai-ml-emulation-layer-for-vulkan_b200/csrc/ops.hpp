@@ -223,6 +223,7 @@ struct RowProgram {
     int64_t rows{0};
     int32_t len{0};
 };
+constexpr int kMaxConcatPasses = 16; // consecutive CONCAT passes into one tensor that a node can hold
 constexpr int kMaxRowInsts = 40, kMaxRowValues = 16;
 
 struct OpDesc {
