@@ -1,6 +1,9 @@
 // Vectorised kernels for the packed int8 NHWC shapes that dominate real graphs.  Each has a generic
 // counterpart in generic_ops.cu that defines the result; these only change how the bytes move.
+#include <algorithm>
+
 #include "device_common.cuh"
+#include "gemm_i8_tcgen05.hpp"
 #include "kernels.hpp"
 
 namespace mlel {
@@ -156,66 +159,91 @@ __global__ void __launch_bounds__(256) columnSumKernel(const int8_t *__restrict_
     }
 }
 
-// ---- AVG_POOL2D, int8 NHWC, C % 4 == 0 (avgpool2d.comp:27-75) ---------------------------------------------
-// A 256-thread block owns one output pixel and up to 128 channels: 32 lanes hold four channels each (one
-// coalesced 128-byte read per tap), eight slices share the window's taps and add their partial sums in
-// shared memory.  Built for the global pooling at the end of a classifier, where the generic kernel's one
-// thread per output walks 49 dependent loads.
+// ---- AVG_POOL2D, int8 NHWC (avgpool2d.comp:27-75) ---------------------------------------------------------
+// One output pixel and up to 256 channel units (a unit is four channels, or one where C % 4 != 0) belong to a cluster of
+// `split` blocks.  The in-range part of a window is rows of contiguous bytes, one run when it spans whole image rows (a
+// global pool), so a thread keeps one channel unit and strides over the pixels of its block's share: consecutive threads
+// read consecutive bytes whatever the channel count.  Partial sums join in shared memory, first of the block, then of
+// the cluster's blocks in block 0 (distributed shared memory).
+// The classifier's pool has one output pixel per image: one block for each left the chip idle on small batches and large
+// windows (64 images of 112 x 112 x 64: 264 us with one block per pixel, 64 blocks, now 20.5; a channel count that is no
+// multiple of 16 took the one-thread-per-output kernel: 3 x 57 x 57 x 36, 990 us, now 9).
+template <int CH>
 __global__ void __launch_bounds__(256) avgPoolI8Kernel(const int8_t *__restrict__ in, int8_t *__restrict__ out, int H, int W,
-                                                       int C, int OH, int OW, PoolAttr a) {
-    __shared__ int32_t part[8][32][4];
-    const int lane = threadIdx.x & 31, slice = threadIdx.x >> 5;
-    const int chunks = (C + 127) / 128;
-    int64_t b = blockIdx.x;
-    const int c0 = int(b % chunks) * 128 + lane * 4;
-    b /= chunks;
-    const int ox = int(b % OW);
-    b /= OW;
-    const int oy = int(b % OH);
-    const int n = int(b / OH);
+                                                       int C, int OH, int OW, int chunks, int split, PoolAttr a) {
+    __shared__ int32_t part[256 * CH];
+    const int rank = int(blockIdx.x % unsigned(split));
+    unsigned b = blockIdx.x / unsigned(split);
+    const int units = C / CH; // per pixel
+    const int unit0 = int(b % unsigned(chunks)) * 256, unitsHere = min(units - unit0, 256);
+    b /= unsigned(chunks);
+    const int ox = int(b % unsigned(OW));
+    b /= unsigned(OW);
+    const int oy = int(b % unsigned(OH)), n = int(b / unsigned(OH));
     const int iy = oy * a.stride[0] - a.pad[0], ix = ox * a.stride[1] - a.pad[2];
-    const int taps = a.kernel[0] * a.kernel[1];
-    int32_t acc[4] = {0, 0, 0, 0};
-    // in-range taps of the whole window: (rows inside) x (columns inside)
-    const int ny = min(iy + a.kernel[0], H) - max(iy, 0), nx = min(ix + a.kernel[1], W) - max(ix, 0);
-    const int count = (ny > 0 && nx > 0) ? ny * nx : 0;
-    // eight taps of this slice at a time: all their loads are issued before the first sum
-    const int8_t *image = in + int64_t(n) * H * W * C + c0;
-    for (int t0 = slice; t0 < taps; t0 += 64) {
-        uint32_t word[8];
-        bool live[8];
+    const int y0 = max(iy, 0), x0 = max(ix, 0);
+    const int ny = max(min(iy + a.kernel[0], H) - y0, 0), nx = max(min(ix + a.kernel[1], W) - x0, 0);
+    const int count = ny * nx;
+
+    const int lanes = 256 / unitsHere; // pixels in flight per block
+    const int pixel = int(threadIdx.x) / unitsHere, unit = int(threadIdx.x) - pixel * unitsHere;
+    int32_t acc[CH];
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            const int t = t0 + 8 * i;
-            const int ky = t / a.kernel[1], kx = t - ky * a.kernel[1];
-            const int y = iy + ky, x = ix + kx;
-            live[i] = t < taps && y >= 0 && y < H && x >= 0 && x < W && c0 < C;
-            word[i] = live[i] ? __ldg(reinterpret_cast<const uint32_t *>(image + (int64_t(y) * W + x) * C)) : 0u;
-        }
+    for (int k = 0; k < CH; ++k) {
+        acc[k] = 0;
+    }
+    if (pixel < lanes) {
+        const bool joined = nx == W; // the window's rows follow one another in memory
+        const int lines = joined ? 1 : ny, length = joined ? count : nx;
+        // this block's share: lines, or a stretch of the one line
+        const int line0 = joined ? 0 : int(int64_t(lines) * rank / split), line1 = joined ? 1 : int(int64_t(lines) * (rank + 1) / split);
+        const int from = joined ? int(int64_t(length) * rank / split) : 0, to = joined ? int(int64_t(length) * (rank + 1) / split) : length;
+        const auto take = [&](const int8_t *p) {
+            if (CH == 4) {
+                const int word = __ldg(reinterpret_cast<const int *>(p));
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            if (live[i]) {
-#pragma unroll
-                for (int k = 0; k < 4; ++k) {
-                    acc[k] += int32_t(int8_t(word[i] >> (8 * k))) - a.inZp;
+                for (int k = 0; k < CH; ++k) {
+                    acc[k] = __dp4a(word, 1 << (8 * k), acc[k]);
                 }
+            } else {
+                acc[0] += int32_t(__ldg(p));
+            }
+        };
+        for (int line = line0; line < line1; ++line) {
+            const int8_t *row = in + ((int64_t(n) * H + y0 + line) * W + x0) * C + (unit0 + unit) * CH;
+#pragma unroll 8
+            for (int x = from + pixel; x < to; x += lanes) {
+                take(row + int64_t(x) * C);
             }
         }
     }
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-        part[slice][lane][k] = acc[k];
+    for (int k = 0; k < CH; ++k) {
+        part[threadIdx.x * CH + k] = acc[k];
     }
     __syncthreads();
-    if (slice == 0 && c0 < C) {
-        uint32_t word = 0;
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            int32_t v = 0;
-#pragma unroll
-            for (int sl = 0; sl < 8; ++sl) {
-                v = int32_t(uint32_t(v) + uint32_t(part[sl][lane][k]));
+    // sum over the pixels in flight: thread j holds value j of unitsHere * CH
+    for (int j = threadIdx.x; j < unitsHere * CH; j += 256) {
+        uint32_t v = 0;
+        for (int q = 0; q < lanes; ++q) {
+            v += uint32_t(part[q * unitsHere * CH + j]);
+        }
+        part[j] = int32_t(v); // slot j of lane 0 is read by this thread alone
+    }
+    if (split > 1) {
+        asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+    }
+    if (rank == 0) {
+        for (int j = threadIdx.x; j < unitsHere * CH; j += 256) {
+            uint32_t sum = uint32_t(part[j]);
+            for (int r = 1; r < split; ++r) {
+                uint32_t peer, v;
+                const uint32_t local = uint32_t(__cvta_generic_to_shared(&part[j]));
+                asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(peer) : "r"(local), "r"(r));
+                asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(v) : "r"(peer));
+                sum += v;
             }
+            int32_t v = int32_t(sum - uint32_t(a.inZp) * uint32_t(count));
             if (count == 0) {
                 v = 0;
             } else {
@@ -224,9 +252,11 @@ __global__ void __launch_bounds__(256) avgPoolI8Kernel(const int8_t *__restrict_
             }
             v = int32_t(uint32_t(v) + uint32_t(a.outZp));
             v = v < -128 ? -128 : (v > 127 ? 127 : v);
-            word |= uint32_t(uint8_t(v)) << (8 * k);
+            out[((int64_t(n) * OH + oy) * OW + ox) * C + unit0 * CH + j] = int8_t(v);
         }
-        *reinterpret_cast<uint32_t *>(out + ((int64_t(n) * OH + oy) * OW + ox) * C + c0) = word;
+    }
+    if (split > 1) { // block 0 has read the others' shared memory before they leave
+        asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
     }
 }
 
@@ -314,6 +344,44 @@ __global__ void maxPoolI8Kernel(const int8_t *__restrict__ in, int8_t *__restric
             }
         }
         reinterpret_cast<int4 *>(out + ((int64_t(n) * OH + oy) * OW + ox) * C)[g] = acc.packed();
+    }
+}
+
+// Channel counts that are no multiple of 16: a thread per output pixel and four channels (CH == 4, C % 4 == 0) or one.
+template <int CH>
+__global__ void __launch_bounds__(256) maxPoolNarrowKernel(const int8_t *__restrict__ in, int8_t *__restrict__ out,
+                                                           uint32_t total, int H, int W, int C, FastDiv groups, FastDiv divOW,
+                                                           FastDiv divOH, PoolAttr a) {
+    const uint32_t step = gridDim.x * blockDim.x;
+    for (uint64_t e64 = blockIdx.x * blockDim.x + threadIdx.x; e64 < total; e64 += step) {
+        const uint32_t e = uint32_t(e64);
+        const auto div = [](uint32_t v, const FastDiv &f) { return f.mul == 0u ? v : __umulhi(v, f.mul) >> f.shift; };
+        const uint32_t pix = div(e, groups), line = div(pix, divOW), n = div(line, divOH);
+        const int c0 = int(e - pix * groups.d) * CH;
+        const int ox = int(pix - line * divOW.d), oy = int(line - n * divOH.d);
+        const int iy0 = oy * max(a.stride[0], 1) - a.pad[0], ix0 = ox * max(a.stride[1], 1) - a.pad[2];
+        const int y0 = max(iy0, 0), y1 = min(iy0 + a.kernel[0], H), x0 = max(ix0, 0), x1 = min(ix0 + a.kernel[1], W);
+        const int8_t *image = in + int64_t(n) * H * W * C + c0;
+        uint32_t even = 0x80008000u, odd = 0x80008000u; // int8 lowest in both lanes
+        int32_t top = -128;
+        for (int y = y0; y < y1; ++y) {
+#pragma unroll 4
+            for (int x = x0; x < x1; ++x) {
+                const int8_t *p = image + (int64_t(y) * W + x) * C;
+                if (CH == 4) {
+                    const uint32_t w = __ldg(reinterpret_cast<const uint32_t *>(p));
+                    even = max3Lanes(even, evenBytesHigh(w), even);
+                    odd = max3Lanes(odd, oddBytesHigh(w), odd);
+                } else {
+                    top = max(top, int32_t(__ldg(p)));
+                }
+            }
+        }
+        if (CH == 4) {
+            reinterpret_cast<uint32_t *>(out)[e] = __byte_perm(even, odd, 0x7351);
+        } else {
+            out[e] = int8_t(top);
+        }
     }
 }
 
@@ -459,7 +527,8 @@ int columnSumsForMatmul(const int8_t *b, int32_t *corr, int batches, int C, int 
     return finish("MATMUL operand column sums");
 }
 
-bool maxPoolI8Eligible(const TView &in, const TView &out) {
+// Packed int8 NHWC tensors; the kernels look at the channel count and the addresses themselves.
+bool poolI8Eligible(const TView &in, const TView &out) {
     const auto packed = [](const TView &t) {
         int64_t s = 1;
         for (int i = t.rank - 1; i >= 0; --i) {
@@ -468,30 +537,74 @@ bool maxPoolI8Eligible(const TView &in, const TView &out) {
             }
             s *= t.dims[i];
         }
-        return true;
+        return s > 0 && s < (int64_t(1) << 40);
     };
-    return in.dtype == MLEL_I8 && out.dtype == MLEL_I8 && in.rank == 4 && out.rank == 4 && in.dims[3] % 16 == 0 &&
-           in.dims[3] == out.dims[3] && in.dims[0] == out.dims[0] && packed(in) && packed(out) &&
-           ((reinterpret_cast<uintptr_t>(in.ptr) | reinterpret_cast<uintptr_t>(out.ptr)) & 15u) == 0;
+    return in.dtype == MLEL_I8 && out.dtype == MLEL_I8 && in.rank == 4 && out.rank == 4 && in.dims[3] == out.dims[3] &&
+           in.dims[0] == out.dims[0] && packed(in) && packed(out);
+}
+
+namespace {
+// Widest access (16, 4 or 1 bytes) that the channel count and both addresses allow.
+int poolUnit(const TView &in, const TView &out) {
+    const uintptr_t bits =
+        uintptr_t(in.dims[3]) | reinterpret_cast<uintptr_t>(in.ptr) | reinterpret_cast<uintptr_t>(out.ptr);
+    return (bits & 15u) == 0 ? 16 : ((bits & 3u) == 0 ? 4 : 1);
+}
+} // namespace
+
+bool maxPoolI8Eligible(const TView &in, const TView &out) {
+    int64_t n = 1;
+    for (int i = 0; i < out.rank; ++i) {
+        n *= out.dims[i];
+    }
+    return poolI8Eligible(in, out) && (poolUnit(in, out) == 16 || n / poolUnit(in, out) < (int64_t(1) << 31));
 }
 
 bool avgPoolI8Eligible(const TView &in, const TView &out, const PoolAttr &a) {
-    // one block per output pixel and 128 channels: worthwhile when the window is large
-    return maxPoolI8Eligible(in, out) && a.kernel[0] > 0 && a.kernel[1] > 0 && a.kernel[0] * a.kernel[1] >= 16 &&
-           a.stride[0] > 0 && a.stride[1] > 0 &&
-           int64_t(out.dims[0]) * out.dims[1] * out.dims[2] * ((out.dims[3] + 127) / 128) < (int64_t(1) << 30);
+    // one block or more per output pixel and 256 channel units: worthwhile when the window is large
+    return poolI8Eligible(in, out) && a.kernel[0] > 0 && a.kernel[1] > 0 && int64_t(a.kernel[0]) * a.kernel[1] >= 16 &&
+           int64_t(a.kernel[0]) * a.kernel[1] < (int64_t(1) << 24) && a.stride[0] > 0 && a.stride[1] > 0 &&
+           int64_t(out.dims[0]) * out.dims[1] * out.dims[2] * ((int64_t(out.dims[3]) + 255) / 256) < (int64_t(1) << 27);
 }
 
 int avgPoolI8(const TView &in, const TView &out, const PoolAttr &a, cudaStream_t s) {
     const int C = int(in.dims[3]);
-    const int64_t blocks = int64_t(out.dims[0]) * out.dims[1] * out.dims[2] * ((C + 127) / 128);
-    avgPoolI8Kernel<<<unsigned(blocks), 256, 0, s>>>(reinterpret_cast<const int8_t *>(in.ptr),
-                                                    reinterpret_cast<int8_t *>(out.ptr), int(in.dims[1]), int(in.dims[2]), C,
-                                                    int(out.dims[1]), int(out.dims[2]), a);
+    const int ch = poolUnit(in, out) == 1 ? 1 : 4, units = C / ch, chunks = (units + 255) / 256;
+    const int64_t groups = int64_t(out.dims[0]) * out.dims[1] * out.dims[2] * chunks;
+    // Blocks per group: as long as the SMs are not filled twice over and a block's share stays at a few kilobytes
+    // (below that the cluster's two barriers cost more than the shorter walk gives).
+    const int64_t bytes = int64_t(std::min(a.kernel[0], int(in.dims[1]))) * std::min(a.kernel[1], int(in.dims[2])) *
+                          std::min(units, 256) * ch;
+    int split = 1;
+    while (split < 8 && groups * split < 4 * kNumSMs && bytes / (2 * split) >= 2048) {
+        split *= 2;
+    }
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(unsigned(groups * split));
+    cfg.blockDim = dim3(256);
+    cfg.stream = s;
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = unsigned(split);
+    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, ch == 4 ? avgPoolI8Kernel<4> : avgPoolI8Kernel<1>, reinterpret_cast<const int8_t *>(in.ptr),
+                       reinterpret_cast<int8_t *>(out.ptr), int(in.dims[1]), int(in.dims[2]), C, int(out.dims[1]),
+                       int(out.dims[2]), chunks, split, a);
     return finish("AVG_POOL2D");
 }
 
 int maxPoolI8(const TView &in, const TView &out, const PoolAttr &a, cudaStream_t s) {
+    if (const int unit = poolUnit(in, out); unit < 16) {
+        const int64_t words = int64_t(out.dims[0]) * out.dims[1] * out.dims[2] * (out.dims[3] / unsigned(unit));
+        const auto kernel = unit == 4 ? maxPoolNarrowKernel<4> : maxPoolNarrowKernel<1>;
+        kernel<<<gridFor(words, kThreads, 16), kThreads, 0, s>>>(
+            reinterpret_cast<const int8_t *>(in.ptr), reinterpret_cast<int8_t *>(out.ptr), uint32_t(words), int(in.dims[1]),
+            int(in.dims[2]), int(in.dims[3]), makeFastDiv(out.dims[3] / unsigned(unit)), makeFastDiv(out.dims[2]),
+            makeFastDiv(out.dims[1]), a);
+        return finish("MAX_POOL2D");
+    }
     const int64_t total = int64_t(out.dims[0]) * out.dims[1] * out.dims[2] * (out.dims[3] >> 4);
     const auto launch = [&](auto kernel) {
         kernel<<<gridFor(total, kThreads, 16), kThreads, 0, s>>>(
