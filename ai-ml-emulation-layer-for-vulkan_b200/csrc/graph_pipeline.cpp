@@ -34,6 +34,7 @@
 //   CONV3D                    i[0..5] pad i[6..8] stride i[9..11] dilation i[12] inputZeroPoint
 //                             i[13] weightZeroPoint i[14] accType      in = {input, weights, biases}
 #include "graph_pipeline.hpp"
+#include "kernels/attention_i8.hpp"
 #include "kernels/device_common.cuh"
 #include "kernels/gemm_i8_tcgen05.hpp"
 
@@ -1051,6 +1052,278 @@ void GraphPipeline::fuseRowRuns(std::vector<int> &group, const std::vector<UseIn
     }
 }
 
+// MATMUL(Q, K^T) -> row-wise softmax -> MATMUL(P, V) -> RESCALE -> OP_FUSED_ATTENTION (kernels/attention_i8.cu), with the
+// transposes that split Q, K and V into heads and merge the context again taken in as strides where nothing else reads
+// them.  Conditions beyond the pattern itself:
+//   * a row of scores fits the kernel (at most kAttentionMaxKeys keys), head dimension a multiple of 32 up to 128: 32 is
+//     the tensor core's K step, below it the score product would be mostly padding;
+//   * at least 32 keys: shorter rows would leave most of a tile's columns empty, and the separate kernels are short;
+//   * zero points 0 on Q, K and V, and 0 or -128 on the probabilities (signed or unsigned operand bytes);
+//   * shifts and bounds for which both element-wise RESCALEs fit 32-bit words (scaleHigh32), from the constant tables;
+//   * operands in session memory or constants: their addresses are 16-byte aligned by construction.
+void GraphPipeline::fuseAttention(std::vector<int> &group, const std::vector<UseInfo> &uses, const std::vector<int> &producer,
+                                  const std::function<void(OpDesc, const std::vector<int> &)> &emit) {
+    const int n = int(ops_.size());
+    // The single reader of an elidable tensor, or -1 (also when that reader is already part of a node).
+    const auto soleConsumer = [&](int32_t t) -> int {
+        const auto &td = tensor(t);
+        const auto &u = uses[size_t(t)];
+        if (td.cls != TensorClass::Session || td.isGraphOutput || td.isGraphInput || !td.packed() || u.producers != 1 ||
+            u.consumers.size() != 1 || group[size_t(u.consumers[0])] >= 0) {
+            return -1;
+        }
+        return u.consumers[0];
+    };
+    struct Scale {
+        int32_t mult, shift, inZp, outZp;
+        bool doubleRound;
+    };
+    // A per-tensor RESCALE with constant parameters between the given types.
+    const auto scaleOf = [&](int k, int32_t inDtype, int32_t outDtype, Scale *sc) {
+        if (k < 0 || ops_[size_t(k)].kind != OP_RESCALE) {
+            return false;
+        }
+        const OpDesc &r = ops_[size_t(k)];
+        const TensorDescriptor &m = tensor(r.in[1]), &sh = tensor(r.in[2]);
+        if (tensor(r.in[0]).dtype != inDtype || tensor(r.out[0]).dtype != outDtype || !r.i[2] || r.i[4] || r.i[5] || r.i[6] ||
+            m.cls != TensorClass::Constant || sh.cls != TensorClass::Constant || m.dtype != MLEL_I32 || elemSize(sh.dtype) != 1 ||
+            m.hostData.size() < 4 || sh.hostData.empty()) {
+            return false;
+        }
+        std::memcpy(&sc->mult, m.hostData.data(), 4);
+        sc->shift = int32_t(int8_t(sh.hostData[0]));
+        sc->inZp = int32_t(wrapTo(inDtype, r.i[0])), sc->outZp = int32_t(wrapTo(outDtype, r.i[1]));
+        sc->doubleRound = r.i[3] != 0;
+        return sc->shift >= 0 && sc->shift <= 62;
+    };
+    const auto tableOf = [&](int k) -> const int16_t * { // int16 -> int32 TABLE with a constant table
+        if (k < 0 || ops_[size_t(k)].kind != OP_TABLE) {
+            return nullptr;
+        }
+        const TensorDescriptor &t = tensor(ops_[size_t(k)].in[1]);
+        const bool ok = t.cls == TensorClass::Constant && t.dtype == MLEL_I16 && t.numel() == 513 && t.packed() &&
+                        tensor(ops_[size_t(k)].out[0]).dtype == MLEL_I32;
+        return ok ? reinterpret_cast<const int16_t *>(t.hostData.data()) : nullptr;
+    };
+    // The value step of a 32-bit-word RESCALE: mult, rounding constant for a known sign of x, remaining shift.
+    const auto words = [](const Scale &sc, bool negative, int32_t *round, int32_t *shift) {
+        *round = (int32_t(1) << (sc.shift - 31)) + (sc.doubleRound ? (negative ? -1 : 1) : 0);
+        *shift = sc.shift - 30;
+        return sc.shift >= 32 && sc.shift <= 60;
+    };
+    // Where a rank-3 operand [B, rows, columns] lies: through RESHAPE and TRANSPOSE of a [N, heads, rows, columns] tensor
+    // when nothing else reads the two, else the operand itself.
+    struct View {
+        int32_t tensor = -1;
+        int64_t heads = 0; // 0: the operand itself, any split of B works
+        int64_t stride[4]; // sequence, head, row, column
+        std::vector<int> ops;
+    };
+    const auto viewOf = [&](int32_t t, int reader) {
+        View v;
+        const TensorDescriptor &td = tensor(t);
+        const int re = producer[size_t(t)];
+        if (re >= 0 && ops_[size_t(re)].kind == OP_RESHAPE && soleConsumer(t) == reader && group[size_t(re)] < 0) {
+            const int32_t u = ops_[size_t(re)].in[0];
+            const TensorDescriptor &ud = tensor(u);
+            const int tr = producer[size_t(u)];
+            if (ud.rank() == 4 && ud.dims[0] * ud.dims[1] == td.dims[0] && ud.dims[2] == td.dims[1] && ud.dims[3] == td.dims[2] &&
+                tr >= 0 && ops_[size_t(tr)].kind == OP_TRANSPOSE && soleConsumer(u) == re && group[size_t(tr)] < 0) {
+                const int32_t w = ops_[size_t(tr)].in[0];
+                const TensorDescriptor &wd = tensor(w);
+                if (wd.rank() == 4 && wd.packed() && wd.cls != TensorClass::External) {
+                    v.tensor = w, v.heads = ud.dims[1], v.ops = {tr, re};
+                    for (int k = 0; k < 4; ++k) {
+                        v.stride[k] = wd.strides[size_t(ops_[size_t(tr)].i[k])];
+                    }
+                    return v;
+                }
+            }
+        }
+        if (td.packed() && td.cls != TensorClass::External) {
+            v.tensor = t;
+            v.stride[2] = td.strides[1], v.stride[3] = td.strides[2];
+            v.stride[0] = v.stride[1] = td.strides[0]; // the sequence stride follows once the number of heads is known
+        }
+        return v;
+    };
+
+    for (int i = 0; i < n; ++i) {
+        const OpDesc &mm = ops_[size_t(i)];
+        if (group[size_t(i)] >= 0 || mm.kind != OP_MATMUL || mm.i[0] != 0 || mm.i[1] != 0) {
+            continue;
+        }
+        const int32_t scores = mm.out[0];
+        const TensorDescriptor &sd = tensor(scores), &qd = tensor(mm.in[0]), &kd = tensor(mm.in[1]);
+        if (sd.dtype != MLEL_I32 || qd.dtype != MLEL_I8 || kd.dtype != MLEL_I8 || sd.rank() != 3 || qd.rank() != 3 ||
+            kd.rank() != 3 || sd.cls != TensorClass::Session || sd.isGraphOutput || sd.isGraphInput ||
+            uses[size_t(scores)].producers != 1 || uses[size_t(scores)].consumers.size() != 2) {
+            continue;
+        }
+        const int64_t B = sd.dims[0], Sq = sd.dims[1], Sk = sd.dims[2], d = qd.dims[2];
+        if (qd.dims[0] != B || kd.dims[0] != B || kd.dims[1] != d || Sk < 32 || Sk > kAttentionMaxKeys || d % 32 != 0 || d > 128 ||
+            B * ((Sq + 127) / 128) >= (int64_t(1) << 31)) {
+            continue;
+        }
+        // ---- softmax
+        int mx = -1, sb = -1;
+        for (int c : uses[size_t(scores)].consumers) {
+            (ops_[size_t(c)].kind == OP_REDUCE ? mx : sb) = c;
+        }
+        if (mx < 0 || sb < 0 || group[size_t(mx)] >= 0 || group[size_t(sb)] >= 0 || ops_[size_t(mx)].sub != RED_MAX ||
+            ops_[size_t(mx)].i[0] != 2 || soleConsumer(ops_[size_t(mx)].out[0]) != sb || ops_[size_t(sb)].kind != OP_BINARY ||
+            ops_[size_t(sb)].sub != BIN_SUB || ops_[size_t(sb)].in[0] != scores || ops_[size_t(sb)].in[1] != ops_[size_t(mx)].out[0] ||
+            tensor(ops_[size_t(sb)].out[0]).dims != sd.dims) {
+            continue;
+        }
+        Scale diff{}, den{}, prob{}, ctx{};
+        const int rsDiff = soleConsumer(ops_[size_t(sb)].out[0]);
+        if (!scaleOf(rsDiff, MLEL_I32, MLEL_I16, &diff)) {
+            continue;
+        }
+        const int tbExp = soleConsumer(ops_[size_t(rsDiff)].out[0]);
+        const int16_t *expLut = tableOf(tbExp);
+        if (expLut == nullptr || ops_[size_t(tbExp)].in[0] != ops_[size_t(rsDiff)].out[0]) {
+            continue;
+        }
+        const int32_t e = ops_[size_t(tbExp)].out[0];
+        const auto &eUses = uses[size_t(e)];
+        if (tensor(e).cls != TensorClass::Session || tensor(e).isGraphOutput || eUses.producers != 1 || eUses.consumers.size() != 2) {
+            continue;
+        }
+        int sum = -1, mul = -1;
+        for (int c : eUses.consumers) {
+            (ops_[size_t(c)].kind == OP_REDUCE ? sum : mul) = c;
+        }
+        if (sum < 0 || mul < 0 || group[size_t(sum)] >= 0 || group[size_t(mul)] >= 0 || ops_[size_t(sum)].sub != RED_SUM ||
+            ops_[size_t(sum)].i[0] != 2 || ops_[size_t(mul)].kind != OP_MUL) {
+            continue;
+        }
+        const int rsDen = soleConsumer(ops_[size_t(sum)].out[0]);
+        if (!scaleOf(rsDen, MLEL_I32, MLEL_I16, &den)) {
+            continue;
+        }
+        const int tbRecip = soleConsumer(ops_[size_t(rsDen)].out[0]);
+        const int16_t *recipLut = tableOf(tbRecip);
+        if (recipLut == nullptr || ops_[size_t(tbRecip)].in[0] != ops_[size_t(rsDen)].out[0] ||
+            soleConsumer(ops_[size_t(tbRecip)].out[0]) != mul || ops_[size_t(mul)].in[0] != e ||
+            ops_[size_t(mul)].in[1] != ops_[size_t(tbRecip)].out[0] || tensor(ops_[size_t(mul)].out[0]).dims != sd.dims ||
+            tensor(ops_[size_t(mul)].out[0]).dtype != MLEL_I32) {
+            continue;
+        }
+        const int rsProb = soleConsumer(ops_[size_t(mul)].out[0]);
+        if (!scaleOf(rsProb, MLEL_I32, MLEL_I8, &prob)) {
+            continue;
+        }
+        // ---- context
+        const int pv = soleConsumer(ops_[size_t(rsProb)].out[0]);
+        if (pv < 0 || ops_[size_t(pv)].kind != OP_MATMUL || ops_[size_t(pv)].in[0] != ops_[size_t(rsProb)].out[0] ||
+            ops_[size_t(pv)].in[1] == ops_[size_t(pv)].in[0] || ops_[size_t(pv)].i[1] != 0 ||
+            (ops_[size_t(pv)].i[0] != 0 && ops_[size_t(pv)].i[0] != -128)) {
+            continue;
+        }
+        const TensorDescriptor &vd = tensor(ops_[size_t(pv)].in[1]);
+        if (vd.dtype != MLEL_I8 || vd.rank() != 3 || vd.dims[0] != B || vd.dims[1] != Sk || vd.dims[2] != d ||
+            tensor(ops_[size_t(pv)].out[0]).dtype != MLEL_I32) {
+            continue;
+        }
+        const int rsCtx = soleConsumer(ops_[size_t(pv)].out[0]);
+        if (!scaleOf(rsCtx, MLEL_I32, MLEL_I8, &ctx)) {
+            continue;
+        }
+        // ---- the arithmetic's bounds
+        auto plan = std::make_shared<AttentionPlan>();
+        int64_t expMax = 0, recipMax = 0;
+        bool steps = true, nonNegative = true;
+        for (int k = 0; k < 513; ++k) {
+            expMax = std::max<int64_t>(expMax, std::abs(int(expLut[k])));
+            recipMax = std::max<int64_t>(recipMax, std::abs(int(recipLut[k])));
+            nonNegative = nonNegative && expLut[k] >= 0 && recipLut[k] >= 0;
+            const int step = k < 512 ? int(expLut[k + 1]) - int(expLut[k]) : 0;
+            steps = steps && step >= -32768 && step <= 32767;
+        }
+        const int64_t mulShift = ops_[size_t(mul)].i[0];
+        if (!steps || mulShift < 1 || mulShift > 31 || (((expMax * recipMax) << 14) >> mulShift) + 1 >= (int64_t(1) << 29) ||
+            (prob.doubleRound && !nonNegative) || diff.inZp != 0 || prob.inZp != 0 || (int64_t(1) << 15) * d >= (int64_t(1) << 29)) {
+            continue;
+        }
+        if (!words(diff, true, &plan->diffRound, &plan->diffShift) || !words(prob, false, &plan->probRound, &plan->probShift)) {
+            continue;
+        }
+        plan->diffMult = diff.mult, plan->diffAdd = diff.outZp + 32768, plan->diffLo = 0, plan->diffHi = 65535;
+        const int32_t probZp = ops_[size_t(pv)].i[0];
+        const int64_t folded = plan->probRound + (int64_t(prob.outZp - probZp) << plan->probShift);
+        if (folded < -(int64_t(1) << 29) || folded > (int64_t(1) << 29) || prob.mult < 0 || diff.mult < 0) {
+            continue; // (|mulhi(4x, mult)| < 2^30 leaves room for a rounding constant of 2^29)
+        }
+        plan->probMult = prob.mult, plan->probRound = int32_t(folded), plan->unsignedProb = probZp == -128;
+        plan->denom = makeFastRescale(den.mult, den.shift, den.inZp, den.doubleRound);
+        plan->denomOutZp = den.outZp;
+        plan->mulShift = int32_t(mulShift), plan->mulRound = int64_t(1) << (mulShift - 1);
+        plan->context = makeFastRescale(ctx.mult, ctx.shift, ctx.inZp, ctx.doubleRound);
+        plan->contextOutZp = ctx.outZp, plan->contextLo = -128, plan->contextHi = 127;
+
+        // ---- operands
+        const int32_t vT = ops_[size_t(pv)].in[1];
+        if (mm.in[0] == mm.in[1] || mm.in[0] == vT || mm.in[1] == vT) {
+            continue;
+        }
+        View q = viewOf(mm.in[0], i), k = viewOf(mm.in[1], i), v = viewOf(vT, pv);
+        int32_t outT = ops_[size_t(rsCtx)].out[0];
+        View o;
+        o.tensor = outT;
+        o.stride[2] = d, o.stride[3] = 1, o.stride[0] = o.stride[1] = Sq * d;
+        const int re = soleConsumer(outT), tr = re >= 0 && ops_[size_t(re)].kind == OP_RESHAPE ? soleConsumer(ops_[size_t(re)].out[0]) : -1;
+        if (tr >= 0 && ops_[size_t(tr)].kind == OP_TRANSPOSE) {
+            const TensorDescriptor &ud = tensor(ops_[size_t(re)].out[0]), &od = tensor(ops_[size_t(tr)].out[0]);
+            if (ud.rank() == 4 && ud.dims[0] * ud.dims[1] == B && ud.dims[2] == Sq && ud.dims[3] == d && od.rank() == 4 &&
+                od.packed() && od.cls == TensorClass::Session) {
+                o.tensor = ops_[size_t(tr)].out[0], o.heads = ud.dims[1], o.ops = {re, tr};
+                for (int k2 = 0; k2 < 4; ++k2) {
+                    o.stride[ops_[size_t(tr)].i[k2]] = od.strides[size_t(k2)];
+                }
+            }
+        }
+        int64_t heads = 0;
+        bool ok = q.tensor >= 0 && k.tensor >= 0 && v.tensor >= 0 && tensor(o.tensor).cls == TensorClass::Session &&
+                  tensor(o.tensor).packed();
+        for (const View *w : {&q, &k, &v, &o}) {
+            ok = ok && (w->heads == 0 || heads == 0 || heads == w->heads);
+            heads = w->heads != 0 ? w->heads : heads;
+        }
+        heads = heads == 0 ? 1 : heads;
+        ok = ok && B % heads == 0;
+        std::swap(k.stride[2], k.stride[3]); // K arrives transposed: its columns are the tokens
+        for (View *w : {&q, &k, &v, &o}) {
+            if (w->heads == 0) {
+                w->stride[0] = w->stride[1] * heads;
+            }
+            ok = ok && w->stride[3] == 1 && w->stride[0] % 16 == 0 && w->stride[1] % 16 == 0 && w->stride[2] % 16 == 0;
+        }
+        if (!ok) {
+            continue;
+        }
+        plan->batches = int32_t(B), plan->heads = int32_t(heads);
+        plan->queries = int32_t(Sq), plan->keys = int32_t(Sk), plan->headDim = int32_t(d);
+        for (int s = 0; s < 3; ++s) {
+            plan->qStride[s] = q.stride[s], plan->kStride[s] = k.stride[s];
+            plan->vStride[s] = v.stride[s], plan->oStride[s] = o.stride[s];
+        }
+        std::vector<int> members{i, mx, sb, rsDiff, tbExp, sum, rsDen, tbRecip, mul, rsProb, pv, rsCtx};
+        for (const View *w : {&q, &k, &v, &o}) {
+            members.insert(members.end(), w->ops.begin(), w->ops.end());
+        }
+        std::sort(members.begin(), members.end());
+        OpDesc node;
+        node.kind = OP_FUSED_ATTENTION;
+        node.name = "ATTENTION(MATMUL+SOFTMAX+MATMUL+RESCALE)";
+        node.in = {q.tensor, k.tensor, v.tensor, ops_[size_t(tbExp)].in[1], ops_[size_t(tbRecip)].in[1]};
+        node.out = {o.tensor};
+        node.attention = plan;
+        emit(std::move(node), members);
+    }
+}
+
 // Fusion keeps the arithmetic of every absorbed operator unchanged (the same integer steps run
 // back to back in registers), so results stay bit-identical to the one-kernel-per-op list; it only
 // removes the round trips of intermediates through memory.  A tensor may be elided when it lives
@@ -1127,19 +1400,21 @@ void GraphPipeline::fuse() {
 
     // Phase 0: contractions with their RESCALE and the quantised residual add.  Between the phases: contiguous runs of
     // row-wise operators (fuseRowRuns).  Phase 1: the two smaller row patterns, for what the runs left over.
+    const auto emit = [&](OpDesc node, const std::vector<int> &members) {
+        Group g;
+        g.node = std::move(node);
+        g.node.fusedOps.clear();
+        g.last = members.back();
+        const int gi = int(fused.size());
+        for (int k : members) {
+            absorb(g, gi, k);
+        }
+        fused.push_back(std::move(g));
+    };
+    fuseAttention(group, uses, producer, emit);
     for (int phase = 0; phase < 2; ++phase) {
     if (phase == 1) {
-        fuseRowRuns(group, uses, [&](OpDesc node, const std::vector<int> &members) {
-            Group g;
-            g.node = std::move(node);
-            g.node.fusedOps.clear();
-            g.last = members.back();
-            const int gi = int(fused.size());
-            for (int k : members) {
-                absorb(g, gi, k);
-            }
-            fused.push_back(std::move(g));
-        });
+        fuseRowRuns(group, uses, emit);
     }
     for (int i = 0; i < n; ++i) {
         if (group[size_t(i)] >= 0) {

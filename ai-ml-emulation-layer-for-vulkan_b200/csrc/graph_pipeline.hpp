@@ -156,6 +156,8 @@ class GraphPipeline {
     OpDesc &pushOp(OpKind kind, const std::string &name, std::vector<int32_t> in, std::vector<int32_t> out);
     void requireMutable() const;
     void fuse();
+    void fuseAttention(std::vector<int> &group, const std::vector<UseInfo> &uses, const std::vector<int> &producer,
+                       const std::function<void(OpDesc, const std::vector<int> &)> &emit);
     void fuseRowRuns(std::vector<int> &group, const std::vector<UseInfo> &uses,
                      const std::function<void(OpDesc, const std::vector<int> &)> &emit);
     void prepareTensorCore();

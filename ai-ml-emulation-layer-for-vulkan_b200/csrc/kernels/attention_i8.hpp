@@ -1,0 +1,34 @@
+// Host description of a fused quantised attention (attention_i8.cu).
+#pragma once
+
+#include "device_common.cuh"
+
+namespace mlel {
+
+// Everything about the node that its graph fixes: shapes, strides and the RESCALE constants in the kernel's forms.
+struct AttentionPlan {
+    int32_t batches, heads; // batches = sequences x heads
+    int32_t queries, keys, headDim;
+    int64_t qStride[3], kStride[3], vStride[3], oStride[3]; // bytes: sequence, head, token (the head dimension is contiguous)
+    // first RESCALE (score differences, int32 -> int16): min(max((mulhi(4x, mult) + round >> shift) + add, lo), hi), all
+    // of the result 32768 higher
+    int32_t diffMult, diffRound, diffShift, diffAdd, diffLo, diffHi;
+    FastRescale denom; // row sums -> int16
+    int32_t denomOutZp;
+    int64_t mulRound; // MUL: (e * r + round) >> shift
+    int32_t mulShift;
+    int32_t probMult, probRound, probShift; // last RESCALE minus the product's zero point, before saturation
+    bool unsignedProb;                      // zero point -128: probabilities are stored as unsigned bytes
+    FastRescale context;
+    int32_t contextOutZp, contextLo, contextHi;
+};
+
+// Limits of the kernel: a row of scores fits tensor memory (512 columns) and, with the operands, shared memory; below
+// the second limit two blocks share an SM.
+constexpr int kAttentionMaxKeys = 512, kAttentionTwoBlockKeys = 192;
+
+int attentionFused(const AttentionPlan &plan, const TView &q, const TView &k, const TView &v, const TView &expTable,
+                   const TView &recipTable, const TView &out, cudaStream_t s);
+int attentionErrorWord();
+
+} // namespace mlel

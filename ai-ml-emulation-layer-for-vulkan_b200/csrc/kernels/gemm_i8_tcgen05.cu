@@ -44,6 +44,7 @@
 #include <mutex>
 
 #include "gemm_i8_tcgen05.hpp"
+#include "attention_i8.hpp"
 #include "tcgen05_common.cuh"
 
 namespace mlel {
@@ -948,7 +949,8 @@ int tcgen05ErrorFlag() {
         return v;
     }
     const int w = ocMajorErrorWord();
-    return w != 0 ? w : pairErrorWord();
+    const int x = w != 0 ? w : pairErrorWord();
+    return x != 0 ? x : attentionErrorWord();
 }
 
 } // namespace mlel

@@ -7,6 +7,7 @@
 #include <cstdlib>
 #include <string>
 
+#include "kernels/attention_i8.hpp"
 #include "kernels/device_common.cuh"
 #include "kernels/gemm_i8_tcgen05.hpp"
 #include "kernels/kernels.hpp"
@@ -492,6 +493,8 @@ int launchOp(const OpDesc &op, const TView *T, cudaStream_t s, LaunchChain *chai
         return rowExpFused(in(0), in(1), T[op.out[0]], T[op.out[1]], devRescale(op.epi.main, T), s);
     case OP_FUSED_MUL_RESCALE:
         return mulRescaleFused(in(0), in(1), out, uint32_t(op.i[0]), devRescale(op.epi.main, T), s);
+    case OP_FUSED_ATTENTION:
+        return attentionFused(*op.attention, in(0), in(1), in(2), in(3), in(4), out, s);
     case OP_FUSED_ADD:
         return fusedAdd(reinterpret_cast<const int8_t *>(in(0).ptr), reinterpret_cast<const int8_t *>(in(1).ptr),
                         reinterpret_cast<int8_t *>(out.ptr), numelOf(out), devEpilogue(op.epi, T), s);

@@ -74,6 +74,9 @@ enum OpKind : int32_t {
     // A contiguous run of row-wise integer operators (RESCALE, TABLE, ADD, SUB, MUL, last-axis REDUCE, CLAMP) as one
     // kernel: see RowProgram.  in = every tensor read from memory (tables included), out = every tensor written.
     OP_FUSED_ROWS,
+    // Score MATMUL, row-wise softmax and context MATMUL of a quantised attention, head split and merge included.
+    // in = {q, k, v, exponential table, reciprocal table}, out = {context}: see AttentionPlan.
+    OP_FUSED_ATTENTION,
     OP_KIND_COUNT
 };
 
@@ -223,6 +226,7 @@ struct RowProgram {
     int64_t rows{0};
     int32_t len{0};
 };
+struct AttentionPlan; // kernels/attention_i8.hpp
 constexpr int kMaxConcatPasses = 16; // consecutive CONCAT passes into one tensor that a node can hold
 constexpr int kMaxRowInsts = 40, kMaxRowValues = 16;
 
@@ -237,6 +241,7 @@ struct OpDesc {
     FusedEpilogue epi;              // fused kinds only
     std::vector<int32_t> fusedOps;  // indices of the logical ops an exec node stands for
     std::shared_ptr<RowProgram> rows; // OP_FUSED_ROWS only
+    std::shared_ptr<AttentionPlan> attention; // OP_FUSED_ATTENTION only
     // Tensor-core path (set by GraphPipeline::prepareTensorCore when the node qualifies):
     //   CONV2D kinds: aux[0] correction table int32 [classes][OC], aux[1] row classes u8 [OH],
     //                 aux[2] column classes u8 [OW]; auxi[0] = number of column classes, auxi[1] = classes,
