@@ -1059,7 +1059,8 @@ void GraphPipeline::fuseRowRuns(std::vector<int> &group, const std::vector<UseIn
 //     the tensor core's K step, below it the score product would be mostly padding;
 //   * at least 32 keys: shorter rows would leave most of a tile's columns empty, and the separate kernels are short;
 //   * zero points 0 on Q, K and V, and 0 or -128 on the probabilities (signed or unsigned operand bytes);
-//   * shifts and bounds for which both element-wise RESCALEs fit 32-bit words (scaleHigh32), from the constant tables;
+//   * shifts and bounds, from the constant tables, for which both element-wise RESCALEs are the high word of one 64-bit
+//     multiply-add;
 //   * operands in session memory or constants: their addresses are 16-byte aligned by construction.
 void GraphPipeline::fuseAttention(std::vector<int> &group, const std::vector<UseInfo> &uses, const std::vector<int> &producer,
                                   const std::function<void(OpDesc, const std::vector<int> &)> &emit) {
@@ -1105,11 +1106,10 @@ void GraphPipeline::fuseAttention(std::vector<int> &group, const std::vector<Use
                         tensor(ops_[size_t(k)].out[0]).dtype == MLEL_I32;
         return ok ? reinterpret_cast<const int16_t *>(t.hostData.data()) : nullptr;
     };
-    // The value step of a 32-bit-word RESCALE: mult, rounding constant for a known sign of x, remaining shift.
-    const auto words = [](const Scale &sc, bool negative, int32_t *round, int32_t *shift) {
-        *round = (int32_t(1) << (sc.shift - 31)) + (sc.doubleRound ? (negative ? -1 : 1) : 0);
-        *shift = sc.shift - 30;
-        return sc.shift >= 32 && sc.shift <= 60;
+    // Rounding constant of a RESCALE whose operand's sign is known, plus a whole number added to its result.
+    const auto addendOf = [](const Scale &sc, bool negative, int64_t add) {
+        return (int64_t(1) << (sc.shift - 1)) + (sc.doubleRound ? (negative ? -1 : 1) * (int64_t(1) << 30) : 0) +
+               add * (int64_t(1) << sc.shift);
     };
     // Where a rank-3 operand [B, rows, columns] lies: through RESHAPE and TRANSPOSE of a [N, heads, rows, columns] tensor
     // when nothing else reads the two, else the operand itself.
@@ -1247,16 +1247,41 @@ void GraphPipeline::fuseAttention(std::vector<int> &group, const std::vector<Use
             (prob.doubleRound && !nonNegative) || diff.inZp != 0 || prob.inZp != 0 || (int64_t(1) << 15) * d >= (int64_t(1) << 29)) {
             continue;
         }
-        if (!words(diff, true, &plan->diffRound, &plan->diffShift) || !words(prob, false, &plan->probRound, &plan->probShift)) {
+        // Shifts of at least 32 see only the high word of the 64-bit sum; up to 44, 2^16 << shift and a product below
+        // 2^60 stay inside it.  A difference is never positive and its multiplier not negative, so the int16 result is
+        // at most its zero point and only the lower clamp is left.
+        const int32_t probZp = ops_[size_t(pv)].i[0];
+        if (diff.shift < 32 || diff.shift > 44 || prob.shift < 32 || prob.shift > 52 || diff.mult < 0 || prob.mult < 0) {
             continue;
         }
-        plan->diffMult = diff.mult, plan->diffAdd = diff.outZp + 32768, plan->diffLo = 0, plan->diffHi = 65535;
-        const int32_t probZp = ops_[size_t(pv)].i[0];
-        const int64_t folded = plan->probRound + (int64_t(prob.outZp - probZp) << plan->probShift);
-        if (folded < -(int64_t(1) << 29) || folded > (int64_t(1) << 29) || prob.mult < 0 || diff.mult < 0) {
-            continue; // (|mulhi(4x, mult)| < 2^30 leaves room for a rounding constant of 2^29)
+        plan->diffMult = diff.mult, plan->diffShift = diff.shift - 32;
+        plan->diffAddend = addendOf(diff, true, int64_t(diff.outZp) + 32768);
+        plan->entryBytes = 4, plan->unitByte = 0x8000;
+        plan->probMult = prob.mult, plan->probShift = prob.shift - 32, plan->unsignedProb = probZp == -128;
+        plan->probAddend = addendOf(prob, false, int64_t(prob.outZp) - probZp);
+        // Both again without the power of two that multiplier and addend share: floor(a * 2^k / 2^(s)) = floor(a / 2^(s-k)).
+        const auto narrowed = [](int64_t xMax, const Scale &sc, int32_t *mult, int64_t *addend, int32_t *shift) {
+            int k = 0;
+            while (k < sc.shift && k < 31 && ((int64_t(sc.mult) >> k) & 1) == 0 && ((*addend >> k) & 1) == 0) {
+                ++k;
+            }
+            const int64_t m = sc.mult >> k, add = *addend >> k;
+            if (sc.shift - k > 31 || xMax * m + std::abs(add) >= (int64_t(1) << 31)) {
+                return false;
+            }
+            *mult = int32_t(m), *addend = add, *shift = sc.shift - k;
+            return true;
+        };
+        {
+            AttentionPlan slim = *plan;
+            // a score and the row maximum are both at most d * 2^14 in size
+            slim.narrow = narrowed((int64_t(1) << 16) * d, diff, &slim.diffMult, &slim.diffAddend, &slim.diffShift) &&
+                          narrowed((((expMax * recipMax) << 14) >> mulShift) + 1, prob, &slim.probMult, &slim.probAddend,
+                                   &slim.probShift);
+            if (slim.narrow) {
+                *plan = slim;
+            }
         }
-        plan->probMult = prob.mult, plan->probRound = int32_t(folded), plan->unsignedProb = probZp == -128;
         plan->denom = makeFastRescale(den.mult, den.shift, den.inZp, den.doubleRound);
         plan->denomOutZp = den.outZp;
         plan->mulShift = int32_t(mulShift), plan->mulRound = int64_t(1) << (mulShift - 1);

@@ -13,21 +13,29 @@
 // Why.  As kernels of their own the steps move the int32 score tensor five times: at 32 sequences of 384 tokens and 12
 // heads that is 226 MB a pass and 294 us of a 525 us layer.  Here a block takes 128 queries of one head: the scores of
 // up to 512 keys fit its tensor memory (a lane per query, a column per key), the exponentials replace them there, the
-// probabilities go to shared memory as the next product's A operand, and only Q, K, V and C touch memory: 107 us, and no
-// row length, odd ones included, leaves the tensor cores (3 sequences of 197 tokens: 750 -> 87 us a layer).
+// probabilities go to shared memory as the next product's A operand, and only Q, K, V and C touch memory: 57 us, and no
+// row length, odd ones included, leaves the tensor cores (3 sequences of 197 tokens: 640 -> 12 us a layer).
 //
-// What bounds it: the integer arithmetic of the softmax, about 20 instructions per score (two RESCALEs, a table
+// What bounds it: the integer arithmetic of the softmax, about 15 instructions per score (two RESCALEs, a table
 // look-up with interpolation, a 64-bit product); the two products take under a tenth of that.  Hence
-//   * both RESCALEs from 32-bit words (scaleHigh32); the first one's operand is never positive and the second one's never
-//     negative, so their double-rounding terms are constants;
+//   * each element-wise RESCALE is one 32 x 32 + 64 bit multiply-add, whose high word is shifted: the operands' signs are
+//     known, so the double-rounding terms are constants, and the row maximum and both zero points are part of the addend;
 //   * a table entry holds (value, step to the next value) as two int16, so that one look-up and one two-way dot product
 //     give value * 128 + step * fraction;
 //   * P is stored minus its zero point, as unsigned bytes, so that the second product needs no correction row;
 //   * packing saturates (cvt.pack.sat), which is the clamp of the last RESCALE.
-// Sixteen warps share the 128 x keys scores (four per quarter of the tensor-memory lanes, 16-column slices in turn) and
-// exchange row maxima and row sums through shared memory.  Up to 192 keys a block has eight warps, so that two blocks
-// fit an SM and one's products run under the other's softmax.  The next tile's Q and K are fetched as soon as the score
-// product is done with them, V after the context product.
+// Sixteen warps share the 128 x keys scores (four per quarter of the tensor-memory lanes, 32-column slices in turn) and
+// exchange row maxima and row sums through shared memory.  Up to 192 keys a block has eight of them, so that two blocks
+// fit an SM and one's products run under the other's softmax.  One more warp feeds them: its first lane issues the TMA
+// loads and the MMAs.  Where scores and context fit tensor memory side by side it issues the next tile's score product
+// as soon as the probabilities of this one are out; while that runs the softmax warps store the previous tile's context
+// rows, and this tile's context product follows under the next softmax.  Otherwise the two products take turns.
+// Clock stamps of a tile of 384 keys, 15 200 cycles before this order: 1200 waiting for scores, 700 row maximum, 2400
+// context rows (most of it waiting for their product), 6200 exponentials, 400 at the barrier, 4000 probabilities.
+//
+// Of the integer pipes the multiply-add one counts: a 32 x 32 -> 64 bit product takes it four cycles a warp, a 32-bit one
+// two.  A RESCALE whose multiplier is a small number times a power of two (powers of two are the usual scales inside a
+// quantised softmax) has its constants divided by that power on the host where everything then fits 32 bits (NARROW).
 #include <algorithm>
 
 #include "attention_i8.hpp"
@@ -39,23 +47,25 @@ namespace {
 
 using namespace tc;
 
+constexpr int kTokenBox = 32;  // tokens per TMA load
 constexpr int kRowBytes = 128; // a SWIZZLE_128B row: one query or key, up to 128 bytes of head dimension
 
 struct AttentionParams {
-    const int8_t *q, *k, *v;
     int8_t *out;
     int32_t Sq, Sk, d, keysPad; // keysPad: keys rounded up to the 32 of an MMA's K step
     uint32_t tiles;
     FastDiv queryTiles, heads;
-    int64_t qStride[3], kStride[3], vStride[3], oStride[3]; // bytes: sequence batch, head, token
+    int32_t contextColumn; // first tensor-memory column of the context; 0: it takes the columns of the scores
+    int64_t oStride[3];    // bytes: sequence, head, token
     const int16_t *expTable, *recipTable;
     AttentionPlan plan;
 };
 
 struct AttentionShared {
-    uint64_t scoresDone, contextDone;
+    uint64_t loadedQK, loadedV;        // TMA
+    uint64_t scoresDone, contextDone;  // MMA
+    uint64_t probsReady, contextRead;  // softmax warps
     uint32_t tmemBase;
-    int32_t failed;
 };
 
 // dp2a: c + lo16(a) * byte0(b) + hi16(a) * byte1(b), a signed, b unsigned
@@ -74,34 +84,67 @@ template <bool UNSIGNED> __device__ __forceinline__ uint32_t packSat(int32_t y1,
     }
     return r;
 }
-__device__ __forceinline__ void tmemStore16(uint32_t taddr, const uint32_t (&r)[16]) {
-    asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], "
-                 "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};" ::"r"(taddr),
-                 "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]),
-                 "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
+__device__ __forceinline__ uint32_t ldsU32(uint32_t addr) {
+    uint32_t v;
+    asm("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(addr)); // written before the first tile, never again
+    return v;
+}
+constexpr int kSlice = 32; // score columns a warp takes at a time
+// (load and wait in one statement: the registers reach no other instruction in between)
+__device__ __forceinline__ void tmemRead32(uint32_t taddr, uint32_t (&r)[32]) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x32.b32 "
+                 "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
+                 "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];\n\t"
+                 "tcgen05.wait::ld.sync.aligned;"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+                   "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]),
+                   "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]),
+                   "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+                 : "r"(taddr)
+                 : "memory");
+}
+__device__ __forceinline__ void tmemStore32(uint32_t taddr, const uint32_t (&r)[32]) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
+                 "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, "
+                 "%17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31, %32};" ::"r"(taddr),
+                 "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]),
+                 "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]),
+                 "r"(r[16]), "r"(r[17]), "r"(r[18]), "r"(r[19]), "r"(r[20]), "r"(r[21]), "r"(r[22]), "r"(r[23]),
+                 "r"(r[24]), "r"(r[25]), "r"(r[26]), "r"(r[27]), "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31])
                  : "memory");
 }
 
-// Rows of `d` bytes into SWIZZLE_128B rows (16-byte piece j of row r at piece j ^ (r & 7)), as asynchronous copies;
-// rows past `rows` and pieces past d (up to the 32 bytes of an MMA's K step) are zero-filled.
-__device__ __forceinline__ void loadRows(uint8_t *dst, const int8_t *src, int64_t stride, int rows, int rowsPad, int d,
-                                         int threads) {
-    const int pieces = (d + 31) / 32 * 2;
-    const uint32_t base = smemAddr(dst);
-    for (int i = threadIdx.x; i < rowsPad * pieces; i += threads) {
-        const int r = i / pieces, j = i - r * pieces;
-        const bool live = r < rows && 16 * j < d;
-        const int8_t *from = live ? src + int64_t(r) * stride + 16 * j : src;
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(base + uint32_t(r * kRowBytes + ((j ^ (r & 7)) << 4))),
-                     "l"(from), "r"(live ? 16u : 0u)
-                     : "memory");
+// 4-D tensor map {head dimension, token, head, sequence} over an int8 operand with a box of 32 tokens by one 128-byte
+// SWIZZLE_128B row: bytes past the head dimension and tokens past the last arrive as zeros.
+__device__ __forceinline__ void tmaLoad4d(const CUtensorMap *map, void *dst, uint64_t *bar, int c1, int c2, int c3) {
+    asm volatile(
+        "cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6}], [%2];" ::"r"(
+            smemAddr(dst)),
+        "l"(reinterpret_cast<uint64_t>(map)), "r"(smemAddr(bar)), "r"(0), "r"(c1), "r"(c2), "r"(c3)
+        : "memory");
+}
+__device__ __forceinline__ void loadTokens(const CUtensorMap *map, uint8_t *dst, uint64_t *bar, int first, int count, int head,
+                                           int sequence) {
+    for (int r = 0; r < count; r += kTokenBox) {
+        tmaLoad4d(map, dst + r * kRowBytes, bar, first + r, head, sequence);
     }
 }
 
-template <int WARPS, bool UNSIGNED_P>
-__global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? 2 : 1) attentionI8Kernel(const __grid_constant__ AttentionParams p) {
-    constexpr int kThreads = WARPS * 32;
-    constexpr int kGroups = WARPS / 4; // warps per quarter of the tensor-memory lanes
+// (x * mult + addend) >> 32 + shift from the 64-bit product, or >> shift from the 32-bit one.
+template <bool NARROW>
+__device__ __forceinline__ int32_t scaleKnownSign(int32_t x, int32_t mult, int64_t addend, int32_t shift) {
+    if (NARROW) {
+        return (x * mult + int32_t(addend)) >> shift;
+    }
+    return int32_t((int64_t(x) * int64_t(mult) + addend) >> 32) >> shift;
+}
+
+template <int WARPS, bool UNSIGNED_P, bool NARROW>
+__global__ void __launch_bounds__(WARPS * 32 + 32, WARPS == 8 ? 2 : 1)
+attentionI8Kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant__ CUtensorMap mapK,
+                  const __grid_constant__ CUtensorMap mapV, const __grid_constant__ AttentionParams p) {
+    constexpr int kThreads = WARPS * 32 + 32;
+    constexpr int kGroups = WARPS / 4; // softmax warps per quarter of the tensor-memory lanes
     extern __shared__ uint8_t rawSmem[];
     uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(rawSmem) + 1023) & ~uintptr_t(1023));
     uint8_t *tileQ = smem;
@@ -117,22 +160,26 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? 2 : 1) attentionI8Ker
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int quarter = warp & 3, columnGroup = warp >> 2;
     const int row = quarter * 32 + lane; // query inside the tile = tensor-memory lane
+    const bool sideBySide = p.contextColumn != 0;
     uint32_t columns = 32;
-    while (columns < uint32_t(p.keysPad) || columns < uint32_t(p.d)) {
+    while (columns < uint32_t(max(p.keysPad, p.contextColumn + p.d))) {
         columns *= 2;
     }
 
     if (threadIdx.x == 0) {
+        mbarInit(&shared->loadedQK, 1);
+        mbarInit(&shared->loadedV, 1);
         mbarInit(&shared->scoresDone, 1);
         mbarInit(&shared->contextDone, 1);
-        shared->failed = 0;
+        mbarInit(&shared->probsReady, WARPS);
+        mbarInit(&shared->contextRead, WARPS);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     for (int i = threadIdx.x; i < 512; i += kThreads) {
         const int32_t value = p.expTable[i], next = p.expTable[i + 1];
         expLut[i] = (uint32_t(value) << 16) | (uint32_t(next - value) & 0xffffu); // the step fits int16 (fuseAttention)
     }
-    if (warp == 0) {
+    if (warp == WARPS) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smemAddr(&shared->tmemBase)),
                      "r"(columns)
                      : "memory");
@@ -152,82 +199,148 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? 2 : 1) attentionI8Ker
         const uint32_t b = fastDiv(t, p.queryTiles), n = fastDiv(b, p.heads);
         return Tile{n, b - n * p.heads.d, int(t - b * p.queryTiles.d) * BM};
     };
-    const auto loadQK = [&](const Tile &t) {
-        loadRows(tileQ, p.q + t.n * p.qStride[0] + t.h * p.qStride[1] + t.q0 * p.qStride[2], p.qStride[2], p.Sq - t.q0, BM, p.d,
-                 kThreads);
-        loadRows(tileK, p.k + t.n * p.kStride[0] + t.h * p.kStride[1], p.kStride[2], p.Sk, p.keysPad, p.d, kThreads);
-    };
-    const auto loadV = [&](const Tile &t) {
-        loadRows(tileV, p.v + t.n * p.vStride[0] + t.h * p.vStride[1], p.vStride[2], p.Sk, p.keysPad, p.d, kThreads);
-    };
-    const auto commitCopies = [] { asm volatile("cp.async.commit_group;" ::: "memory"); };
-    const auto waitAllButLastCopies = [] {
-        asm volatile("cp.async.wait_group 1;" ::: "memory");
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); // the tensor core reads what the copies wrote
-    };
-    // the warps of one quarter, i.e. of the same 32 rows
-    const auto quarterSync = [&] { asm volatile("bar.sync %0, %1;" ::"r"(1 + quarter), "n"(kGroups * 32) : "memory"); };
 
-    const AttentionPlan &a = p.plan;
-    const int slices = p.keysPad / 16;
-    const uint32_t laneAddr = tmemBase + (uint32_t(quarter * 32) << 16);
-    uint32_t parity = 0;
-
-    uint32_t t = blockIdx.x;
-    if (t < p.tiles) {
-        const Tile first = tileOf(t);
-        loadQK(first);
-        commitCopies();
-        loadV(first);
-        commitCopies();
-    }
-    for (; t < p.tiles; t += gridDim.x, parity ^= 1u) {
-        const Tile tile = tileOf(t);
-        const bool more = t + gridDim.x < p.tiles;
-        waitAllButLastCopies(); // Q and K; V may still be under way
-        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-        __syncthreads();
-        if (shared->failed != 0) {
-            break;
-        }
-        if (threadIdx.x == 0) {
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    if (warp == WARPS) {
+        if (lane == 0) {
+            // ---------------- loads and MMAs ----------------
+            const auto loadQK = [&](const Tile &t) {
+                mbarArriveExpectTx(&shared->loadedQK, uint32_t((BM + p.keysPad) * kRowBytes));
+                loadTokens(&mapQ, tileQ, &shared->loadedQK, t.q0, BM, int(t.h), int(t.n));
+                loadTokens(&mapK, tileK, &shared->loadedQK, 0, p.keysPad, int(t.h), int(t.n));
+            };
+            const auto loadV = [&](const Tile &t) {
+                mbarArriveExpectTx(&shared->loadedV, uint32_t(p.keysPad * kRowBytes));
+                loadTokens(&mapV, tileV, &shared->loadedV, 0, p.keysPad, int(t.h), int(t.n));
+            };
             const uint64_t descQ = smemDesc(smemAddr(tileQ), 16, 1024), descK = smemDesc(smemAddr(tileK), 16, 1024);
-            for (int n0 = 0; n0 < p.keysPad; n0 += 256) {
-                const int n = min(256, p.keysPad - n0);
-                for (int ks = 0; ks * UMMA_K < p.d; ++ks) {
-                    umma(tmemBase + uint32_t(n0), descQ + uint64_t(2 * ks), descK + uint64_t(n0 * (kRowBytes >> 4) + 2 * ks),
-                         instrDesc(n, false), ks > 0 ? 1u : 0u);
+            const uint64_t descP = smemDesc(smemAddr(tileP), 16, 1024), descV = smemDesc(smemAddr(tileV), BK * 128, 1024);
+            const auto scoreProduct = [&] {
+                for (int n0 = 0; n0 < p.keysPad; n0 += 256) {
+                    const int n = min(256, p.keysPad - n0);
+                    for (int ks = 0; ks * UMMA_K < p.d; ++ks) {
+                        umma(tmemBase + uint32_t(n0), descQ + uint64_t(2 * ks),
+                             descK + uint64_t(n0 * (kRowBytes >> 4) + 2 * ks), instrDesc(n, false), ks > 0 ? 1u : 0u);
+                    }
+                }
+                ummaCommit(&shared->scoresDone);
+            };
+            const auto contextProduct = [&] {
+                // A format 0: unsigned 8-bit
+                const uint32_t idesc = instrDesc(p.d, true) & (UNSIGNED_P ? ~(7u << 7) : ~0u);
+                for (int ks = 0; ks * UMMA_K < p.keysPad; ++ks) {
+                    umma(tmemBase + uint32_t(p.contextColumn), descP + uint64_t((ks >> 2) * ((BM * BK) >> 4) + 2 * (ks & 3)),
+                         descV + uint64_t(ks * ((UMMA_K * kRowBytes) >> 4)), idesc, ks > 0 ? 1u : 0u);
+                }
+                ummaCommit(&shared->contextDone);
+            };
+            uint32_t t = blockIdx.x;
+            bool ok = true;
+            if (t < p.tiles) {
+                loadQK(tileOf(t));
+                loadV(tileOf(t));
+                ok = mbarWait(&shared->loadedQK, 0, 71);
+                if (ok) {
+                    scoreProduct();
                 }
             }
-            ummaCommit(&shared->scoresDone);
+            for (uint32_t i = 0; t < p.tiles && ok; ++i, t += gridDim.x) {
+                const uint32_t parity = i & 1u;
+                const uint32_t next = t + gridDim.x;
+                const bool more = next < p.tiles;
+                ok = mbarWait(&shared->scoresDone, parity, 72); // Q and K have been read
+                if (ok && more) {
+                    loadQK(tileOf(next));
+                }
+                ok = ok && mbarWait(&shared->probsReady, parity, 73) && mbarWait(&shared->loadedV, parity, 74) &&
+                     (!more || mbarWait(&shared->loadedQK, parity ^ 1u, 71));
+                if (!ok) {
+                    break;
+                }
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                if (sideBySide && more) {
+                    scoreProduct();
+                }
+                if (sideBySide && i > 0) { // the previous tile's context has been stored
+                    ok = mbarWait(&shared->contextRead, parity ^ 1u, 76);
+                    if (!ok) {
+                        break;
+                    }
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                }
+                contextProduct();
+                ok = mbarWait(&shared->contextDone, parity, 75); // V and the probabilities have been read
+                if (ok && more) {
+                    loadV(tileOf(next));
+                }
+                if (!sideBySide && more) {
+                    ok = ok && mbarWait(&shared->contextRead, parity, 76);
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                    if (ok) {
+                        scoreProduct();
+                    }
+                }
+            }
         }
-        if (!mbarWait(&shared->scoresDone, parity, 71)) {
-            shared->failed = 1;
+        __syncwarp();
+    } else {
+    // ---------------- softmax and context rows ----------------
+    // the warps of one quarter, i.e. of the same 32 rows
+    const auto quarterSync = [&] { asm volatile("bar.sync %0, %1;" ::"r"(1 + quarter), "n"(kGroups * 32) : "memory"); };
+    const AttentionPlan &a = p.plan;
+    const int slices = p.keysPad / kSlice;
+    const uint32_t lutAddr = smemAddr(expLut);
+    const uint32_t laneAddr = tmemBase + (uint32_t(quarter * 32) << 16);
+    const auto contextRows = [&](const Tile &tile) {
+        int8_t *dst = p.out + tile.n * p.oStride[0] + tile.h * p.oStride[1] + int64_t(tile.q0 + row) * p.oStride[2];
+        for (int c = columnGroup; 16 * c < p.d; c += kGroups) {
+            uint32_t s[16];
+            tmemLoad16(laneAddr + uint32_t(p.contextColumn + 16 * c), s);
+            tmemWait16(s);
+            uint32_t packed[4];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                uint32_t w = 0;
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    w |= uint32_t(uint8_t(fastRescale(a.context, int32_t(s[4 * q + j]), a.contextOutZp, a.contextLo, a.contextHi)))
+                         << (8 * j);
+                }
+                packed[q] = w;
+            }
+            if (tile.q0 + row < p.Sq) {
+                *reinterpret_cast<uint4 *>(dst + 16 * c) = make_uint4(packed[0], packed[1], packed[2], packed[3]);
+            }
         }
+    };
+
+    // Waits as a warp.  After a wait that ran out the warp keeps to the barriers of its quarter and does nothing else.
+    const auto waitAll = [](uint64_t *bar, uint32_t phase, int code) {
+        const bool done = __all_sync(0xffffffffu, mbarWait(bar, phase, code));
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        if (more) {
-            loadQK(tileOf(t + gridDim.x));
-        }
-        commitCopies();
+        return done;
+    };
+    bool ok = true;
+    uint32_t i = 0;
+    Tile last{};
+    for (uint32_t t = blockIdx.x; t < p.tiles; t += gridDim.x, ++i) {
+        const uint32_t parity = i & 1u;
+        ok = ok && waitAll(&shared->scoresDone, parity, 77);
 
         // ---- row maximum
         int32_t top = int32_t(0x80000000u);
-        for (int c = columnGroup; c < slices; c += kGroups) {
-            uint32_t s[16];
-            tmemLoad16(laneAddr + uint32_t(16 * c), s);
-            tmemWait16(s);
-            const int live = p.Sk - 16 * c; // columns of real keys in this slice
-            if (live >= 16) {
+        for (int c = ok ? columnGroup : slices; c < slices; c += kGroups) {
+            uint32_t s[kSlice];
+            tmemRead32(laneAddr + uint32_t(kSlice * c), s);
+            const int live = p.Sk - kSlice * c; // columns of real keys in this slice
+            if (live < kSlice) {
 #pragma unroll
-                for (int j = 0; j < 16; j += 2) {
-                    top = __vimax3_s32(top, int32_t(s[j]), int32_t(s[j + 1]));
+                for (int j = 0; j < kSlice; ++j) {
+                    s[j] = j < live ? s[j] : 0x80000000u;
                 }
-            } else {
+            }
 #pragma unroll
-                for (int j = 0; j < 16; ++j) {
-                    top = j < live ? max(top, int32_t(s[j])) : top;
-                }
+            for (int j = 0; j < kSlice; j += 2) {
+                top = __vimax3_s32(top, int32_t(s[j]), int32_t(s[j + 1]));
             }
         }
         partMax[columnGroup * BM + row] = top;
@@ -238,34 +351,36 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? 2 : 1) attentionI8Ker
         }
 
         // ---- exponentials, in place; row sum
-        const int32_t top4 = int32_t(uint32_t(top) * 4u);
+        // (s - top) * mult + addend as s * mult + (addend - top * mult)
+        const int64_t diffAddend = a.diffAddend - int64_t(top) * int64_t(a.diffMult); // NARROW: inside 32 bits
         uint32_t sum = 0;
-        for (int c = columnGroup; c < slices; c += kGroups) {
-            uint32_t s[16];
-            tmemLoad16(laneAddr + uint32_t(16 * c), s);
-            tmemWait16(s);
-            const int live = p.Sk - 16 * c;
+        for (int c = ok ? columnGroup : slices; c < slices; c += kGroups) {
+            uint32_t s[kSlice];
+            tmemRead32(laneAddr + uint32_t(kSlice * c), s);
+            const int live = p.Sk - kSlice * c;
+            if (live < kSlice) { // columns of padding: any score up to the maximum
 #pragma unroll
-            for (int j = 0; j < 16; ++j) {
-                const int32_t x4 = int32_t(s[j] * 4u) - top4;
-                const int32_t scaled = scaleHigh32<false>(x4, a.diffMult, a.diffRound) >> a.diffShift;
-                const uint32_t u = uint32_t(min(__viaddmax_s32(scaled, a.diffAdd, a.diffLo), a.diffHi)); // int16 + 32768
-                const uint32_t entry = *reinterpret_cast<const uint32_t *>(reinterpret_cast<const uint8_t *>(expLut) + ((u >> 5) & ~3u));
-                s[j] = uint32_t(dp2aLow(entry, (u & 0x7fu) | 0x8000u, 0));
-            }
-            if (live >= 16) {
-#pragma unroll
-                for (int j = 0; j < 16; j += 2) {
-                    sum += s[j] + s[j + 1];
+                for (int j = 0; j < kSlice; ++j) {
+                    s[j] = j < live ? s[j] : uint32_t(top);
                 }
-            } else {
+            }
 #pragma unroll
-                for (int j = 0; j < 16; ++j) {
+            for (int j = 0; j < kSlice; ++j) {
+                // int16 result + 32768
+                const uint32_t u = uint32_t(max(scaleKnownSign<NARROW>(int32_t(s[j]), a.diffMult, diffAddend, a.diffShift), 0));
+                s[j] = uint32_t(dp2aLow(ldsU32(lutAddr + (u >> 7) * a.entryBytes), (u & 0x7fu) | a.unitByte, 0));
+            }
+            if (live < kSlice) {
+#pragma unroll
+                for (int j = 0; j < kSlice; ++j) {
                     s[j] = j < live ? s[j] : 0u;
-                    sum += s[j];
                 }
             }
-            tmemStore16(laneAddr + uint32_t(16 * c), s);
+#pragma unroll
+            for (int j = 0; j < kSlice; j += 2) {
+                sum += s[j] + s[j + 1];
+            }
+            tmemStore32(laneAddr + uint32_t(kSlice * c), s);
         }
         partSum[columnGroup * BM + row] = int32_t(sum);
         asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
@@ -283,75 +398,65 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? 2 : 1) attentionI8Ker
         }
 
         // ---- probabilities minus their zero point, into the A operand of the context product
-        for (int c = columnGroup; c < slices; c += kGroups) {
-            uint32_t s[16];
-            tmemLoad16(laneAddr + uint32_t(16 * c), s);
-            tmemWait16(s);
-            uint32_t packed[4];
+        if (sideBySide && i > 0) { // which the previous tile's product has read
+            ok = ok && waitAll(&shared->contextDone, parity ^ 1u, 78);
+        }
+        for (int c = ok ? columnGroup : slices; c < slices; c += kGroups) {
+            uint32_t s[kSlice];
+            tmemRead32(laneAddr + uint32_t(kSlice * c), s);
+            uint32_t packed[kSlice / 4];
 #pragma unroll
-            for (int q = 0; q < 4; ++q) {
+            for (int q = 0; q < kSlice / 4; ++q) {
                 int32_t y[4];
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
                     const uint64_t prod = uint64_t(int64_t(int32_t(s[4 * q + j])) * int64_t(recip)) + uint64_t(a.mulRound);
-                    const uint32_t x = __funnelshift_r(uint32_t(prod), uint32_t(prod >> 32), uint32_t(a.mulShift));
-                    y[j] = scaleHigh32<false>(int32_t(x * 4u), a.probMult, a.probRound) >> a.probShift;
+                    const int32_t x = int32_t(__funnelshift_r(uint32_t(prod), uint32_t(prod >> 32), uint32_t(a.mulShift)));
+                    y[j] = scaleKnownSign<NARROW>(x, a.probMult, a.probAddend, a.probShift);
                 }
                 packed[q] = packSat<UNSIGNED_P>(y[1], y[0], packSat<UNSIGNED_P>(y[3], y[2], 0u));
             }
-            // 16-byte piece c & 7 of this row in the 128-key block c >> 3
-            *reinterpret_cast<uint4 *>(tileP + (c >> 3) * (BM * BK) + row * BK + (((c & 7) ^ (row & 7)) << 4)) =
-                make_uint4(packed[0], packed[1], packed[2], packed[3]);
+            // 16-byte pieces 2 (c & 3) and the next of this row in the 128-key block c >> 2
+            const uint32_t dst = smemAddr(tileP) + uint32_t((c >> 2) * (BM * BK) + row * BK);
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(dst + uint32_t(((2 * (c & 3) + h) ^ (row & 7)) << 4)),
+                             "r"(packed[4 * h]), "r"(packed[4 * h + 1]), "r"(packed[4 * h + 2]), "r"(packed[4 * h + 3])
+                             : "memory");
+            }
         }
-        waitAllButLastCopies(); // V; the next tile's Q and K may still be under way.  The fence also covers P
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); // the tensor core reads the probabilities
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            // the context takes the first d columns: every score has been read
-            const uint32_t idesc = instrDesc(p.d, true) & (UNSIGNED_P ? ~(7u << 7) : ~0u); // A format 0: unsigned 8-bit
-            const uint64_t descP = smemDesc(smemAddr(tileP), 16, 1024), descV = smemDesc(smemAddr(tileV), BK * 128, 1024);
-            for (int ks = 0; ks * UMMA_K < p.keysPad; ++ks) {
-                umma(tmemBase, descP + uint64_t((ks >> 2) * ((BM * BK) >> 4) + 2 * (ks & 3)),
-                     descV + uint64_t(ks * ((UMMA_K * kRowBytes) >> 4)), idesc, ks > 0 ? 1u : 0u);
+        __syncwarp();
+        if (lane == 0 && ok) {
+            mbarArrive(&shared->probsReady);
+        }
+        // The context in tensor memory: the previous tile's while the next scores are made, or, where it takes columns
+        // of the scores, this tile's before they are.
+        const Tile tile = tileOf(t);
+        if (!sideBySide) {
+            last = tile;
+            ok = ok && waitAll(&shared->contextDone, parity, 79);
+        }
+        if (!sideBySide || i > 0) {
+            if (ok) {
+                contextRows(last);
             }
-            ummaCommit(&shared->contextDone);
-        }
-        if (!mbarWait(&shared->contextDone, parity, 72)) {
-            shared->failed = 1;
-        }
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        if (more) {
-            loadV(tileOf(t + gridDim.x));
-        }
-        commitCopies();
-
-        // ---- context rows
-        int8_t *dst = p.out + tile.n * p.oStride[0] + tile.h * p.oStride[1] + int64_t(tile.q0 + row) * p.oStride[2];
-        for (int c = columnGroup; 16 * c < p.d; c += kGroups) {
-            uint32_t s[16];
-            tmemLoad16(laneAddr + uint32_t(16 * c), s);
-            tmemWait16(s);
-            uint32_t packed[4];
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                uint32_t w = 0;
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    w |= uint32_t(uint8_t(fastRescale(a.context, int32_t(s[4 * q + j]), a.contextOutZp, a.contextLo, a.contextHi)))
-                         << (8 * j);
-                }
-                packed[q] = w;
-            }
-            if (tile.q0 + row < p.Sq) {
-                *reinterpret_cast<uint4 *>(dst + 16 * c) = make_uint4(packed[0], packed[1], packed[2], packed[3]);
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            __syncwarp();
+            if (lane == 0 && ok) {
+                mbarArrive(&shared->contextRead);
             }
         }
+        last = tile;
     }
-    asm volatile("cp.async.wait_all;" ::: "memory");
+    if (sideBySide && i > 0 && ok && waitAll(&shared->contextDone, (i - 1u) & 1u, 78)) {
+        contextRows(last);
+    }
+    }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
-    if (warp == 0) {
+    if (warp == WARPS) {
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmemBase), "r"(columns) : "memory");
     }
@@ -362,15 +467,41 @@ size_t attentionSmem(int keysPad, int warps) {
            2 * size_t(warps / 4) * BM * 4 + sizeof(AttentionShared);
 }
 
+bool makeTokenMap(CUtensorMap *map, const void *base, int d, int tokens, int heads, int sequences, const int64_t (&stride)[3]) {
+    EncodeTiledFn fn = encodeTiled();
+    if (fn == nullptr) {
+        setLastError("cuTensorMapEncodeTiled is not available from the driver");
+        return false;
+    }
+    const cuuint64_t dims[4] = {cuuint64_t(d), cuuint64_t(tokens), cuuint64_t(heads), cuuint64_t(sequences)};
+    const cuuint64_t strides[3] = {cuuint64_t(stride[2]), cuuint64_t(stride[1]), cuuint64_t(stride[0])};
+    const cuuint32_t box[4] = {kRowBytes, kTokenBox, 1, 1};
+    const cuuint32_t elemStrides[4] = {1, 1, 1, 1};
+    const CUresult rc = fn(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 4, const_cast<void *>(base), dims, strides, box, elemStrides,
+                           CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                           CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (rc != CUDA_SUCCESS) {
+        setLastError("attention: cuTensorMapEncodeTiled failed with code " + std::to_string(int(rc)));
+        return false;
+    }
+    return true;
+}
+
 template <int WARPS>
-int launchAttention(const AttentionParams &p, bool unsignedP, cudaStream_t s) {
+int launchAttention(const CUtensorMap (&maps)[3], AttentionParams p, cudaStream_t s) {
     const size_t smem = attentionSmem(p.keysPad, WARPS);
-    auto kernel = unsignedP ? attentionI8Kernel<WARPS, true> : attentionI8Kernel<WARPS, false>;
-    if (!allowDynamicSmem(reinterpret_cast<const void *>(kernel), attentionSmem(WARPS == 8 ? kAttentionTwoBlockKeys : kAttentionMaxKeys, WARPS))) {
+    const bool narrow = p.plan.narrow;
+    auto kernel = p.plan.unsignedProb
+                      ? (narrow ? attentionI8Kernel<WARPS, true, true> : attentionI8Kernel<WARPS, true, false>)
+                      : (narrow ? attentionI8Kernel<WARPS, false, true> : attentionI8Kernel<WARPS, false, false>);
+    if (!allowDynamicSmem(reinterpret_cast<const void *>(kernel),
+                          attentionSmem(WARPS == 8 ? kAttentionTwoBlockKeys : kAttentionMaxKeys, WARPS))) {
         return MLEL_ERROR_DEVICE;
     }
-    const int grid = int(std::min<int64_t>(p.tiles, int64_t(smCount()) * (WARPS == 8 ? 2 : 1)));
-    if (launchDependent(kernel, grid, WARPS * 32, smem, s, p) != cudaSuccess) {
+    const int blocksPerSm = WARPS == 8 ? 2 : 1;
+    p.contextColumn = p.keysPad + p.d <= 512 / blocksPerSm ? p.keysPad : 0;
+    const int grid = int(std::min<int64_t>(p.tiles, int64_t(smCount()) * blocksPerSm));
+    if (launchDependent(kernel, grid, WARPS * 32 + 32, smem, s, maps[0], maps[1], maps[2], p) != cudaSuccess) {
         setLastError(std::string("attention: ") + cudaGetErrorString(cudaGetLastError()));
         return MLEL_ERROR_DEVICE;
     }
@@ -383,11 +514,13 @@ int attentionErrorWord() { return readErrorWord(); }
 
 int attentionFused(const AttentionPlan &plan, const TView &q, const TView &k, const TView &v, const TView &expTable,
                    const TView &recipTable, const TView &out, cudaStream_t s) {
+    if (((reinterpret_cast<uintptr_t>(q.ptr) | reinterpret_cast<uintptr_t>(k.ptr) | reinterpret_cast<uintptr_t>(v.ptr) |
+          reinterpret_cast<uintptr_t>(out.ptr)) & 15u) != 0) {
+        setLastError("attention: operands must be 16-byte aligned");
+        return MLEL_ERROR_UNKNOWN;
+    }
     AttentionParams p{};
     p.plan = plan;
-    p.q = reinterpret_cast<const int8_t *>(q.ptr);
-    p.k = reinterpret_cast<const int8_t *>(k.ptr);
-    p.v = reinterpret_cast<const int8_t *>(v.ptr);
     p.out = reinterpret_cast<int8_t *>(out.ptr);
     p.expTable = reinterpret_cast<const int16_t *>(expTable.ptr);
     p.recipTable = reinterpret_cast<const int16_t *>(recipTable.ptr);
@@ -398,16 +531,17 @@ int attentionFused(const AttentionPlan &plan, const TView &q, const TView &k, co
     p.queryTiles = makeFastDiv(queryTiles);
     p.heads = makeFastDiv(plan.heads);
     for (int i = 0; i < 3; ++i) {
-        p.qStride[i] = plan.qStride[i], p.kStride[i] = plan.kStride[i];
-        p.vStride[i] = plan.vStride[i], p.oStride[i] = plan.oStride[i];
+        p.oStride[i] = plan.oStride[i];
     }
-    if (((reinterpret_cast<uintptr_t>(p.q) | reinterpret_cast<uintptr_t>(p.k) | reinterpret_cast<uintptr_t>(p.v) |
-          reinterpret_cast<uintptr_t>(p.out)) & 15u) != 0) {
-        setLastError("attention: operands must be 16-byte aligned");
-        return MLEL_ERROR_UNKNOWN;
+    CUtensorMap maps[3];
+    const int sequences = plan.batches / plan.heads;
+    if (!makeTokenMap(&maps[0], q.ptr, p.d, p.Sq, plan.heads, sequences, plan.qStride) ||
+        !makeTokenMap(&maps[1], k.ptr, p.d, p.Sk, plan.heads, sequences, plan.kStride) ||
+        !makeTokenMap(&maps[2], v.ptr, p.d, p.Sk, plan.heads, sequences, plan.vStride)) {
+        return MLEL_ERROR_DEVICE;
     }
-    return p.keysPad <= kAttentionTwoBlockKeys ? launchAttention<8>(p, plan.unsignedProb, s)
-                                              : launchAttention<16>(p, plan.unsignedProb, s);
+    return p.keysPad <= kAttentionTwoBlockKeys ? launchAttention<8>(maps, p, s)
+                                              : launchAttention<16>(maps, p, s);
 }
 
 } // namespace mlel

@@ -10,14 +10,19 @@ struct AttentionPlan {
     int32_t batches, heads; // batches = sequences x heads
     int32_t queries, keys, headDim;
     int64_t qStride[3], kStride[3], vStride[3], oStride[3]; // bytes: sequence, head, token (the head dimension is contiguous)
-    // first RESCALE (score differences, int32 -> int16): min(max((mulhi(4x, mult) + round >> shift) + add, lo), hi), all
-    // of the result 32768 higher
-    int32_t diffMult, diffRound, diffShift, diffAdd, diffLo, diffHi;
+    // first RESCALE (score differences, int32 -> int16), its result 32768 higher: max((x * mult + addend) >> 32 + shift, 0)
+    int32_t diffMult, diffShift;
+    int64_t diffAddend;
+    // 4 and 0x8000, from the parameter block so that they stay operands of one multiply-add and one logic operation
+    uint32_t entryBytes, unitByte;
     FastRescale denom; // row sums -> int16
     int32_t denomOutZp;
     int64_t mulRound; // MUL: (e * r + round) >> shift
     int32_t mulShift;
-    int32_t probMult, probRound, probShift; // last RESCALE minus the product's zero point, before saturation
+    // last RESCALE, minus the product's zero point, before saturation: (x * mult + addend) >> 32 + shift
+    int32_t probMult, probShift;
+    int64_t probAddend;
+    bool narrow;       // both RESCALEs divided by a power of two of their multipliers: (x * mult + addend) >> shift in 32 bits
     bool unsignedProb;                      // zero point -128: probabilities are stored as unsigned bytes
     FastRescale context;
     int32_t contextOutZp, contextLo, contextHi;

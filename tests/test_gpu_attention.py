@@ -14,7 +14,7 @@ pytestmark = pytest.mark.gpu
 ATTENTION = "ATTENTION(MATMUL+SOFTMAX+MATMUL+RESCALE)"
 
 
-def attention_graph(n, heads, sq, sk, d, prob_zp=-128, double_round=False, merge=True, seed=0):
+def attention_graph(n, heads, sq, sk, d, prob_zp=-128, double_round=False, merge=True, pow2=False, seed=0):
     rng = np.random.Generator(np.random.PCG64(seed))
     x = (np.arange(513, dtype=np.float64) - 256.0) * 128.0
     exp_lut = np.round(32767.0 * np.exp(np.minimum(x, 0.0) / 4096.0)).astype(np.int16)
@@ -28,12 +28,12 @@ def attention_graph(n, heads, sq, sk, d, prob_zp=-128, double_round=False, merge
     v = g.reshape(g.transpose(v, (0, 2, 1, 3)), (n * heads, sk, d))
     s = g.matmul(q, k, 0, 0)
     diff = g.sub(s, g.reduce("REDUCE_MAX", s, 2))
-    e = g.table(g.rescale(diff, [int(rng.integers(1 << 30, 1 << 31))], [30 + max(2, int(math.log2(d)) - 2)], 0, 0, np.int16,
+    e = g.table(g.rescale(diff, [1 << 30 if pow2 else int(rng.integers(1 << 30, 1 << 31))], [30 + max(2, int(math.log2(d)) - 2)], 0, 0, np.int16,
                           double_round=double_round), exp_lut)
     log_keys = max(1, math.ceil(math.log2(sk)))
     denom = g.rescale(g.reduce("REDUCE_SUM", e, 2), [1 << 30], [37 + log_keys], 0, -32768, np.int16)
     r = g.table(denom, recip_lut)
-    p = g.rescale(g.mul(e, r, 22), [1 << 30], [37 + log_keys - (0 if prob_zp else 1)], 0, prob_zp, np.int8,
+    p = g.rescale(g.mul(e, r, 22), [1 << 30 if pow2 else (1 << 30) + 12345], [37 + log_keys - (0 if prob_zp else 1)], 0, prob_zp, np.int8,
                   double_round=double_round)
     c = g.rescale(g.matmul(p, v, prob_zp, 0), [int(rng.integers(1 << 30, 1 << 31))], [38], 0, 3, np.int8, double_round=True)
     if merge:
@@ -47,10 +47,10 @@ def attention_graph(n, heads, sq, sk, d, prob_zp=-128, double_round=False, merge
     (3, 2, 129, 191, 96), (1, 4, 192, 192, 64), (1, 2, 100, 193, 64), (1, 1, 300, 384, 64), (1, 2, 65, 256, 32),
     (2, 1, 511, 511, 128), (20, 12, 257, 65, 64),
 ])
-@pytest.mark.parametrize("prob_zp,double_round", [(-128, False), (0, True)])
-def test_attention_matches_the_operators(mlel, n, heads, sq, sk, d, prob_zp, double_round):
+@pytest.mark.parametrize("prob_zp,double_round,pow2", [(-128, False, False), (0, True, False), (-128, True, True), (0, False, True)])
+def test_attention_matches_the_operators(mlel, n, heads, sq, sk, d, prob_zp, double_round, pow2):
     from mlel_b200.runtime import GraphRunner
-    g, data = attention_graph(n, heads, sq, sk, d, prob_zp, double_round, merge=(sq % 2 == 0 or n > 1), seed=sk)
+    g, data = attention_graph(n, heads, sq, sk, d, prob_zp, double_round, merge=(sq % 2 == 0 or n > 1), pow2=pow2, seed=sk)
     runner = GraphRunner(g)
     assert ATTENTION in runner.pipeline.exec_names(), runner.pipeline.exec_names()
     want = evaluate(g, data)[0]
