@@ -70,6 +70,9 @@ bool vecTable(const TView &in, const TView &out, const TView &table, cudaStream_
 // hold at once for `slots` full-shaped values of `len` elements (0: the run cannot be fused).
 int rowMachineWarps(int slots, int len);
 int rowMachine(const RowProgram &program, const TView *tensors, cudaStream_t s);
+// row_norm.cu: the program of a residual add with layer norm, in registers
+bool rowNormMatch(const RowProgram &program);
+int rowNorm(const RowProgram &program, const TView *tensors, cudaStream_t s);
 // Fused nodes of the fusion pass (OP_FUSED_ROW_EXP, OP_FUSED_MUL_RESCALE): see vector_ops.cu.
 int rowExpFused(const TView &x, const TView &table, const TView &e, const TView &sums, const DevRescale &r, cudaStream_t s);
 int mulRescaleFused(const TView &a, const TView &b, const TView &out, uint32_t shift, const DevRescale &r, cudaStream_t s);

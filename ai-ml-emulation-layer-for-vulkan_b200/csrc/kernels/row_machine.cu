@@ -311,6 +311,9 @@ int rowMachine(const RowProgram &program, const TView *T, cudaStream_t s) {
         setLastError("fused rows: program out of range");
         return MLEL_ERROR_UNKNOWN;
     }
+    if (rowNormMatch(program)) {
+        return rowNorm(program, T, s);
+    }
     prog.count = int32_t(program.insts.size());
     prog.len = program.len;
     prog.slots = program.slots;

@@ -1,0 +1,35 @@
+"""GPU parity of the register-resident residual add + layer norm: rows at and beside its 128-element groups, scales that
+the 32-bit forms take (powers of two) and scales that they do not, double rounding and zero points.  Bit-exact against
+the CPU oracle, operator by operator."""
+import numpy as np
+import pytest
+
+from mlel_b200.graph_builder import GraphBuilder
+from tests.test_gpu_vector_ops import check_fused, full_range, rng
+
+pytestmark = pytest.mark.gpu
+
+NORM = "ROWS(RESCALE+RESCALE+ADD+REDUCE_SUM+MUL+SUB+MUL+REDUCE_SUM+MUL+RESCALE+TABLE+MUL+RESCALE)"
+
+
+@pytest.mark.parametrize("rows,length", [(1, 4), (3, 128), (37, 132), (5, 508), (2, 768), (9, 772), (3, 1024), (2, 2048), (2, 2052)])
+@pytest.mark.parametrize("mult,shift,out_shift,in_zp,double_round", [
+    (1 << 30, 24, 45, 0, True),            # 32-bit forms
+    (3 << 28, 26, 44, -7, False),
+    ((1 << 30) + 12345, 25, 46, 5, True),  # 64-bit forms
+    (1 << 30, 33, 40, 0, True),            # double rounding on the inputs: 64-bit forms
+])
+def test_residual_layer_norm(mlel, rows, length, mult, shift, out_shift, in_zp, double_round):
+    r = rng(length + shift)
+    g = GraphBuilder()
+    a, b = g.input(np.int8, (1, rows, length)), g.input(np.int8, (1, rows, length))
+    t = g.add(g.rescale(a, [mult], [shift], in_zp, 0, np.int32, double_round=shift > 31),
+              g.rescale(b, [1 << 30], [24], 0, 3, np.int32))
+    inv = g.inline(np.asarray([(1 << 20) // length], np.int32).reshape(1, 1, 1))
+    cen = g.sub(t, g.mul(g.reduce("REDUCE_SUM", t, 2), inv, 20))
+    var = g.mul(g.reduce("REDUCE_SUM", g.mul(cen, cen, 8), 2), inv, 20)
+    var16 = g.rescale(var, [1 << 30], [34], 0, -32768, np.int16)
+    x = (np.arange(513, dtype=np.float64) - 256.0) * 128.0
+    rsqrt = np.clip(np.round(32767.0 * 16.0 / np.sqrt(x + 32768.0 + 256.0)), 0, 32767).astype(np.int16)
+    g.output(g.rescale(g.mul(cen, g.table(var16, rsqrt), 12), [mult], [out_shift], 0, -3, np.int8, double_round=double_round))
+    check_fused(mlel, g, [full_range(r, np.int8, a.shape), full_range(r, np.int8, b.shape)], [NORM])
