@@ -109,6 +109,8 @@ int mlel_set_tuning(const char *key, int value) {
         const bool width = value == 0 || value == 128 || value == 192 || value == 256;
         if (k == "pair_kernel" && value >= 0 && value <= 2) {
             t.pairKernel = value;
+        } else if (k == "small_kernel" && value >= 0) {
+            t.smallKernel = value;
         } else if (k == "tile_progress" && value >= 0 && value <= 7) {
             t.tileProgress = value;
         } else if (k == "oc_tile_rule" && value >= 0 && value <= 8) {
@@ -128,7 +130,7 @@ int mlel_set_tuning(const char *key, int value) {
 }
 
 long long mlel_tensor_core_launches(int kernel) {
-    return kernel >= 0 && kernel < 3 ? g_tensorCoreLaunches[kernel].load(std::memory_order_relaxed) : -1;
+    return kernel >= 0 && kernel < 4 ? g_tensorCoreLaunches[kernel].load(std::memory_order_relaxed) : -1;
 }
 
 int mlel_selftest_wait_timeout(void *cuda_stream, int *recorded_code) {

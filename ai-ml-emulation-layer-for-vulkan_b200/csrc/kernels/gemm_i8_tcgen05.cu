@@ -838,7 +838,7 @@ int launchVariant(const CUtensorMap &mapA, const CUtensorMap &mapB, const GemmI8
 
 } // namespace
 
-std::atomic<long long> g_tensorCoreLaunches[3];
+std::atomic<long long> g_tensorCoreLaunches[4];
 
 TensorCoreTuning &tensorCoreTuning() {
     static TensorCoreTuning t;
@@ -950,7 +950,8 @@ int tcgen05ErrorFlag() {
     }
     const int w = ocMajorErrorWord();
     const int x = w != 0 ? w : pairErrorWord();
-    return x != 0 ? x : attentionErrorWord();
+    const int y = x != 0 ? x : attentionErrorWord();
+    return y != 0 ? y : smallErrorWord();
 }
 
 } // namespace mlel

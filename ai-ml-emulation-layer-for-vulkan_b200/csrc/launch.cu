@@ -43,6 +43,17 @@ bool tryPairKernel(const GemmI8Problem &q, bool convolution, cudaStream_t s, int
     return taken || *rc != MLEL_SUCCESS;
 }
 
+// The same for the small-problem kernel.
+bool trySmallKernel(const GemmI8Problem &q, cudaStream_t s, int *rc) {
+    int pixels = 0, split = 0;
+    if (!gemmI8SmallApplies(q, &pixels, &split)) {
+        return false;
+    }
+    bool taken = false;
+    *rc = gemmI8SmallLaunch(q, pixels, split, s, &taken);
+    return taken || *rc != MLEL_SUCCESS;
+}
+
 PoolAttr poolAttr(const OpDesc &op) {
     PoolAttr a{};
     a.kernel[0] = op.i[0], a.kernel[1] = op.i[1], a.stride[0] = op.i[2], a.stride[1] = op.i[3];
@@ -164,6 +175,10 @@ int launchConvTensorCore(const OpDesc &op, const TView *T, cudaStream_t s, Launc
             q.bRowBytes = uint64_t(p.K);
             q.bBatchBytes = 0;
             q.bMnMajor = false;
+            int smallRc = MLEL_SUCCESS;
+            if (trySmallKernel(q, s, &smallRc)) {
+                return smallRc;
+            }
             return gemmI8OcMajorApplies(q) ? gemmI8OcMajorLaunch(q, s) : gemmI8Launch(q, s);
         }
         p.chunkBytes = op.auxi[2];
@@ -187,7 +202,7 @@ int launchConvTensorCore(const OpDesc &op, const TView *T, cudaStream_t s, Launc
     q.bBatchBytes = 0;
     q.bMnMajor = false;
     int rc = MLEL_SUCCESS;
-    if (tryPairKernel(q, true, s, &rc)) {
+    if (tryPairKernel(q, true, s, &rc) || trySmallKernel(q, s, &rc)) {
         return rc;
     }
     return gemmI8OcMajorApplies(q) ? gemmI8OcMajorLaunch(q, s, chain, consumed) : gemmI8Launch(q, s);
@@ -264,7 +279,9 @@ int launchMatmulTensorCore(const OpDesc &op, const TView *T, cudaStream_t s) {
     q.bBatchBytes = uint64_t(p.K) * uint64_t(p.N);
     q.bMnMajor = false;
     int rc = MLEL_SUCCESS;
-    if (tryPairKernel(q, false, s, &rc)) {
+    // ("pair_kernel" 2 asks for the paired kernel wherever it applies)
+    const bool pairFirst = tensorCoreTuning().pairKernel.load(std::memory_order_relaxed) == 2;
+    if ((pairFirst && tryPairKernel(q, false, s, &rc)) || trySmallKernel(q, s, &rc) || tryPairKernel(q, false, s, &rc)) {
         return rc;
     }
     return gemmI8Launch(q, s);

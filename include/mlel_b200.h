@@ -311,6 +311,8 @@ int mlel_measure_int8_mma_peak(int batches, void *cuda_stream, float *ms, double
  *                       rounds of 192-pixel tiles per SM takes 256-pixel tiles.  0: 192 pixels for every layer above
  *                       128 pixels;
  *   "dependent_launch"  1 (default) launches the tensor-core kernels with programmatic dependent launch;
+ *   "small_kernel"      1 (default): fused int8 problems that would leave most SMs idle run on the kernel that splits the
+ *                       contraction of narrow tiles over a cluster; 0: never;
  *   "tile_progress"     7 (default): a convolution whose input the convolution before it wrote starts on that launch's
  *                       finished pixel tiles; bit 0 read by tiles, bit 1 publish, bit 2 channel tiles first; 0 off.
  * Another key or value: MLEL_ERROR_UNKNOWN. */
@@ -325,7 +327,7 @@ int mlel_selftest_wait_timeout(void *cuda_stream, int *recorded_code);
 
 /* Diagnostic (no counterpart in the reference): how often the library has enqueued tensor-core kernel
  * `kernel` since it was loaded -- 0 the pixel-major tcgen05 kernel, 1 the channel-major one, 2 the paired
- * (two-CTA) one; -1 for another index.  Tests use it to see which kernel took a case. */
+ * (two-CTA) one, 3 the small-problem one; -1 for another index.  Tests use it to see which kernel took a case. */
 long long mlel_tensor_core_launches(int kernel);
 
 /* Number of kernels one dispatch launches. */
