@@ -15,6 +15,7 @@
 
 #include "device_common.cuh"
 #include "kernels.hpp"
+#include "launch_overlapped.cuh"
 
 namespace mlel {
 
@@ -182,6 +183,7 @@ __device__ __forceinline__ int32_t elementAny(int op, int32_t x, int32_t y, cons
 }
 
 __global__ void __launch_bounds__(256) rowMachineKernel(const __grid_constant__ DevRowProgram prog, int64_t rows) {
+    dependencySync();
     extern __shared__ int32_t rowSmem[];
     const int lane = threadIdx.x & 31, warpInBlock = threadIdx.x >> 5;
     const int len = prog.len;
@@ -360,7 +362,7 @@ int rowMachine(const RowProgram &program, const TView *T, cudaStream_t s) {
     const int64_t blocksWanted = (program.rows + prog.warps - 1) / prog.warps;
     const int64_t cap = int64_t(kNumSMs) * 8;
     const int grid = int(blocksWanted < cap ? (blocksWanted < 1 ? 1 : blocksWanted) : cap);
-    rowMachineKernel<<<grid, prog.warps * 32, smemBytes, s>>>(prog, program.rows);
+    launchOverlapped(rowMachineKernel, grid, prog.warps * 32, smemBytes, s, prog, program.rows);
     const cudaError_t err = cudaGetLastError();
     if (err != cudaSuccess) {
         setLastError(std::string("fused rows: ") + cudaGetErrorString(err));

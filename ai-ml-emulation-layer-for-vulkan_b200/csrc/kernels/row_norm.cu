@@ -15,6 +15,7 @@
 
 #include "device_common.cuh"
 #include "kernels.hpp"
+#include "launch_overlapped.cuh"
 
 namespace mlel {
 
@@ -60,6 +61,7 @@ template <bool NARROW, bool SIGNED> __device__ __forceinline__ int32_t scaled(co
 // GROUPS x 128 elements a row at most.
 template <int GROUPS, bool NARROW>
 __global__ void __launch_bounds__(256) rowNormKernel(const __grid_constant__ NormParams p) {
+    dependencySync();
     const int lane = threadIdx.x & 31;
     const int64_t warps = (int64_t(gridDim.x) * blockDim.x) >> 5;
     for (int64_t row = (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5; row < p.rows; row += warps) {
@@ -234,7 +236,7 @@ int rowNorm(const RowProgram &program, const TView *T, cudaStream_t s) {
 
     const int groups = (p.len + 127) / 128;
     const int grid = gridFor(p.rows * 32, 256, 16);
-    const auto launch = [&](auto slim, auto full) { (narrow ? slim : full)<<<grid, 256, 0, s>>>(p); };
+    const auto launch = [&](auto slim, auto full) { launchOverlapped((narrow ? slim : full), grid, 256, 0, s, p); };
     if (groups <= 2) {
         launch(rowNormKernel<2, true>, rowNormKernel<2, false>);
     } else if (groups <= 4) {

@@ -14,6 +14,7 @@
 #include "device_common.cuh"
 #include "gemm_i8_tcgen05.hpp"
 #include "kernels.hpp"
+#include "launch_overlapped.cuh"
 
 namespace mlel {
 
@@ -204,6 +205,7 @@ void launchRescale(const TView &in, const TView &out, const TView &mult, const T
 // ---- TABLE (table.comp:17-52) -------------------------------------------------------------------------------
 __global__ void tableI8Kernel(const int8_t *__restrict__ in, int8_t *__restrict__ out, int64_t groups, int rest,
                               const int8_t *__restrict__ table) {
+    dependencySync();
     __shared__ int8_t lut[256];
     for (int i = threadIdx.x; i < 256; i += blockDim.x) {
         lut[i] = table[i];
@@ -659,9 +661,10 @@ bool vecTable(const TView &in, const TView &out, const TView &table, cudaStream_
         return false;
     }
     if (in.dtype == MLEL_I8 && out.dtype == MLEL_I8 && table.dtype == MLEL_I8 && packedNumel(table) == 256) {
-        tableI8Kernel<<<gridFor(n / 16 + n % 16, kThreads, 16), kThreads, 0, s>>>(reinterpret_cast<const int8_t *>(in.ptr),
-                                                                         reinterpret_cast<int8_t *>(out.ptr), n / 16, int(n % 16),
-                                                                         reinterpret_cast<const int8_t *>(table.ptr));
+        // (the GELU between two projections: its blocks are scheduled while the product before it drains)
+        launchOverlapped(tableI8Kernel, gridFor(n / 16 + n % 16, kThreads, 16), kThreads, 0, s,
+                         reinterpret_cast<const int8_t *>(in.ptr), reinterpret_cast<int8_t *>(out.ptr), n / 16, int(n % 16),
+                         reinterpret_cast<const int8_t *>(table.ptr));
         *rc = finish("TABLE");
         return true;
     }
