@@ -296,4 +296,53 @@ template <bool SIGNED> __device__ __forceinline__ int32_t scaleHigh32(int32_t x4
     return t;
 }
 
+// ---- RESCALE as one multiply-add -----------------------------------------------------------------------------------
+// A shift s of 32 to 50 only sees the high word of the 64-bit sum, and there everything constant -- correction times
+// multiplier, rounding, output zero point times 2^s -- fits the multiply-add's 64-bit addend:
+//   ((v * mult + addend) >> 32) >> (s - 32).
+// On this machine an ordinary integer instruction holds a scheduler's pipe for two cycles and a 32 x 32 -> 64 bit product
+// for four, and the pipes add up: fastRescale with its bounds takes about 22 cycles a warp, this 8 (6 and the bounds).
+// Conditions: v + offset - input zero point stays inside int32, and double rounding either does not have to look at its
+// sign (wordsScaleSignFree: every negative value ends at the lower bound whichever way it is rounded) or takes the signed
+// form; then the result is the same bits.
+//
+// The signed form: the addend rounds as for a negative x, W = x * mult + 2^(s-1) - 2^30, and x >= 0 adds 2^31, i.e. the
+// low word's top bit as a carry.  The sign may be taken from W (mult >= 0): for x >= 0 it is not negative, and where x < 0
+// but W >= 0, W and W + 2^31 both lie in [0, 2^s), the same result.  The output zero point is added afterwards.
+struct WordsScale {
+    int32_t mult, shift; // shift of the high word
+    uint32_t low, high;  // addend
+};
+__device__ __forceinline__ bool wordsScaleApplies(int32_t mult, int32_t shift, bool doubleRound) {
+    return shift >= 32 && shift <= 50 && (!doubleRound || mult >= 0);
+}
+__device__ __forceinline__ bool wordsScaleSignFree(bool doubleRound, int32_t outZp, int32_t lo) { return !doubleRound || lo >= outZp; }
+// x0 = offset - input zero point, whole = what is added to the result (the output zero point)
+template <bool SIGNED>
+__device__ __forceinline__ WordsScale makeWordsScale(int32_t mult, int32_t shift, bool doubleRound, int32_t x0, int32_t whole) {
+    const int64_t bump = doubleRound ? int64_t(1) << 30 : 0;
+    const int64_t addend = int64_t(x0) * int64_t(mult) + (int64_t(1) << (shift - 1)) +
+                           (SIGNED ? -bump : bump + int64_t(whole) * (int64_t(1) << shift));
+    return WordsScale{mult, shift - 32, uint32_t(uint64_t(addend)), uint32_t(uint64_t(addend) >> 32)};
+}
+template <bool SIGNED> __device__ __forceinline__ int32_t wordsScale(const WordsScale &w, int32_t v) {
+    const uint64_t addend = (uint64_t(w.high) << 32) | uint64_t(w.low);
+    const uint64_t sum = uint64_t(int64_t(v) * int64_t(w.mult)) + addend;
+    uint32_t high = uint32_t(sum >> 32);
+    if (SIGNED) {
+        high += (uint32_t(sum) & ~high) >> 31;
+    }
+    return int32_t(high) >> w.shift;
+}
+// Four results as bytes, saturated to int8 (value 0 in the lowest byte).
+__device__ __forceinline__ uint32_t packSatS8(int32_t y0, int32_t y1, int32_t y2, int32_t y3) {
+    uint32_t r;
+    asm("{\n\t.reg .b32 t;\n\t"
+        "cvt.pack.sat.s8.s32.b32 t, %4, %3, 0;\n\t"
+        "cvt.pack.sat.s8.s32.b32 %0, %2, %1, t;\n\t}"
+        : "=r"(r)
+        : "r"(y0), "r"(y1), "r"(y2), "r"(y3));
+    return r;
+}
+
 } // namespace mlel

@@ -5,6 +5,7 @@
 //
 // Arithmetic: conv2d.comp:59-112 / depthwise_conv2d.comp:47-75 / matmul.comp:42-69 followed per
 // element by rescale.comp:27-72 and clamp.comp:24-53.
+#include <type_traits>
 #include <utility>
 
 #include "device_common.cuh"
@@ -225,10 +226,11 @@ __device__ __forceinline__ void transpose4x4Bytes(uint32_t a, uint32_t b, uint32
 }
 
 template <int R, int SX, bool OUT8>
-__global__ void __launch_bounds__(128) depthwise3x3RowsKernel(const int8_t *__restrict__ in, const int8_t *__restrict__ w,
+__global__ void __launch_bounds__(128, 4) depthwise3x3RowsKernel(const int8_t *__restrict__ in, const int8_t *__restrict__ w,
                                                               const int32_t *__restrict__ bias, int biasCount,
                                                               void *__restrict__ out, int N, int H, int W, int C, int OH,
-                                                              int OW, ConvAttr a, DevEpilogue epi) {
+                                                              int OW, FastDiv divC, FastDiv divX, FastDiv divY, ConvAttr a,
+                                                              DevEpilogue epi) {
     constexpr int PX = 4;
     constexpr int COLS = (PX - 1) * SX + 3; // input pixels under the four windows of a row: 6 or 9
     constexpr int NT = SX == 1 ? 2 : 4;     // transposed groups of four pixels per input row
@@ -241,13 +243,11 @@ __global__ void __launch_bounds__(128) depthwise3x3RowsKernel(const int8_t *__re
     const int64_t total = int64_t(N) * groupsY * groupsX * cw;
     const uint32_t zword = uint32_t(uint8_t(a.inZp)) * 0x01010101u;
     GRID_STRIDE(e, total) {
-        int64_t t = e;
-        const int c0 = int(t % cw) * 4;
-        t /= cw;
-        const int ox0 = int(t % groupsX) * PX;
-        t /= groupsX;
-        const int oy0 = int(t % groupsY) * R;
-        const int n = int(t / groupsY);
+        // (four 64-bit divisions here were a tenth of the kernel's instructions)
+        const auto div = [](uint32_t v, const FastDiv &f) { return f.mul == 0u ? v : __umulhi(v, f.mul) >> f.shift; };
+        const uint32_t tx = div(uint32_t(e), divC), ty = div(tx, divX), tn = div(ty, divY);
+        const int c0 = int(uint32_t(e) - tx * divC.d) * 4, ox0 = int(tx - ty * divX.d) * PX, oy0 = int(ty - tn * divY.d) * R;
+        const int n = int(tn);
         // the three weights of a window row of one channel at byte offsets 0 and 1, and their sum
         uint32_t wa[3][4], wb[3][4];
         int32_t wsum[4] = {0, 0, 0, 0};
@@ -279,49 +279,109 @@ __global__ void __launch_bounds__(128) depthwise3x3RowsKernel(const int8_t *__re
         const int x0 = ox0 * SX - a.pad[2];
         const int yFirst = oy0 * SX - a.pad[0];
         constexpr int ROWS = (R - 1) * SX + 3; // input rows under the R windows of a column (y stride = x stride)
+        // Offsets in 32 bits (the launcher refuses 2^31 elements), and no range tests where all windows lie inside: with
+        // a 64-bit address and two tests per word an output took 30 instructions, twice its arithmetic.
+        const auto convolve = [&](auto insideTag) {
+            constexpr bool INSIDE = decltype(insideTag)::value;
+            int32_t rowOffset = ((n * H + yFirst) * W + x0) * C + c0;
 #pragma unroll
-        for (int iy = 0; iy < ROWS; ++iy) {
-            const int y = yFirst + iy;
-            const bool rowOk = y >= 0 && y < H;
-            const int8_t *row = in + ((int64_t(n) * H + (rowOk ? y : 0)) * W) * C + c0;
-            uint32_t cols[COLS];
+            for (int iy = 0; iy < ROWS; ++iy) {
+                const bool rowOk = INSIDE || (yFirst + iy >= 0 && yFirst + iy < H);
+                uint32_t cols[COLS];
+                uint32_t offset = uint32_t(rowOffset);
 #pragma unroll
-            for (int i = 0; i < COLS; ++i) {
-                const int x = x0 + i;
-                cols[i] = (rowOk && x >= 0 && x < W) ? __ldg(reinterpret_cast<const uint32_t *>(row + int64_t(x) * C)) : zword;
-            }
-            // tr[g][k]: four consecutive pixels of channel k.  Stride 1: pixels 0-3 and 2-5; window px starts at byte
-            // px & 1 of group px >> 1.  Stride 2: pixels 0-3, 2-5, 4-7, 5-8; windows start at bytes 0, 0, 0, 1.
-            uint32_t tr[NT][4];
-            transpose4x4Bytes(cols[0], cols[1], cols[2], cols[3], tr[0]);
-            transpose4x4Bytes(cols[2], cols[3], cols[4], cols[5], tr[1]);
-            if (SX == 2) {
-                transpose4x4Bytes(cols[4], cols[5], cols[6], cols[7], tr[2]);
-                transpose4x4Bytes(cols[5], cols[6], cols[7], cols[8], tr[3]);
-            }
+                for (int i = 0; i < COLS; ++i) {
+                    const bool ok = INSIDE || (rowOk && x0 + i >= 0 && x0 + i < W);
+                    cols[i] = ok ? __ldg(reinterpret_cast<const uint32_t *>(in + offset)) : zword;
+                    offset += uint32_t(C);
+                }
+                rowOffset += W * C;
+                // tr[g][k]: four consecutive pixels of channel k.  Stride 1: pixels 0-3 and 2-5; window px starts at byte
+                // px & 1 of group px >> 1.  Stride 2: pixels 0-3, 2-5, 4-7, 5-8; windows start at bytes 0, 0, 0, 1.
+                uint32_t tr[NT][4];
+                transpose4x4Bytes(cols[0], cols[1], cols[2], cols[3], tr[0]);
+                transpose4x4Bytes(cols[2], cols[3], cols[4], cols[5], tr[1]);
+                if (SX == 2) {
+                    transpose4x4Bytes(cols[4], cols[5], cols[6], cols[7], tr[2]);
+                    transpose4x4Bytes(cols[5], cols[6], cols[7], cols[8], tr[3]);
+                }
 #pragma unroll
-            for (int r = 0; r < R; ++r) {
-                const int ky = iy - r * SX; // this input row as a row of output row r's window (a compile-time value)
-                if (ky >= 0 && ky < 3) {
+                for (int r = 0; r < R; ++r) {
+                    const int ky = iy - r * SX; // this input row as a row of output row r's window (a compile-time value)
+                    if (ky >= 0 && ky < 3) {
 #pragma unroll
-                    for (int px = 0; px < PX; ++px) {
-                        const int g = SX == 1 ? px >> 1 : px;
-                        const bool second = SX == 1 ? (px & 1) != 0 : px == 3;
+                        for (int px = 0; px < PX; ++px) {
+                            const int g = SX == 1 ? px >> 1 : px;
+                            const bool second = SX == 1 ? (px & 1) != 0 : px == 3;
 #pragma unroll
-                        for (int k = 0; k < 4; ++k) {
-                            const uint32_t wsel = second ? wb[ky][k] : wa[ky][k];
-                            acc[r][px][k] = __dp4a(int32_t(tr[g][k]), int32_t(wsel), acc[r][px][k]);
+                            for (int k = 0; k < 4; ++k) {
+                                const uint32_t wsel = second ? wb[ky][k] : wa[ky][k];
+                                acc[r][px][k] = __dp4a(int32_t(tr[g][k]), int32_t(wsel), acc[r][px][k]);
+                            }
                         }
                     }
                 }
             }
+        };
+        // (R == 2 is for small images, where most warps would run both forms one after the other)
+        if (R == 4 && x0 >= 0 && x0 + COLS <= W && yFirst >= 0 && yFirst + ROWS <= H) {
+            convolve(std::true_type{});
+        } else {
+            convolve(std::false_type{});
         }
         int32_t add[4];
-        FastRescale fr[4]; // the fused RESCALE of this thread's four channels (OUT8 only)
+        bool words = OUT8; // the four channels' RESCALEs are one multiply-add each (WordsScale)
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
             const int32_t b = __ldg(bias + (biasCount == 1 ? 0 : c0 + k));
             add[k] = int32_t(uint32_t(b) - uint32_t(a.inZp) * uint32_t(wsum[k]));
+            if (OUT8) {
+                const int ci = epi.main.perChannel ? c0 + k : 0;
+                // |sum of nine products| <= 9 * 2^14: with this bound sum + add - zero point stays inside int32
+                words = words && abs(int64_t(add[k])) < (int64_t(1) << 30) &&
+                        wordsScaleApplies(__ldg(epi.main.mult + ci), int32_t(__ldg(epi.main.shift + ci)), epi.main.doubleRound != 0);
+            }
+        }
+        if (OUT8 && words) {
+            const auto finish = [&](auto signedTag) {
+                constexpr bool SIGNED = decltype(signedTag)::value;
+                WordsScale ws[4];
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    const int ci = epi.main.perChannel ? c0 + k : 0;
+                    ws[k] = makeWordsScale<SIGNED>(__ldg(epi.main.mult + ci), int32_t(__ldg(epi.main.shift + ci)),
+                                                   epi.main.doubleRound != 0, add[k] - epi.main.inZp, epi.main.outZp);
+                }
+                const bool full = oy0 + R <= OH && ox0 + PX <= OW;
+#pragma unroll
+                for (int r = 0; r < R; ++r) {
+                    const uint32_t rowOut = uint32_t(((n * OH + oy0 + r) * OW + ox0) * C + c0);
+#pragma unroll
+                    for (int px = 0; px < PX; ++px) {
+                        if (full || (oy0 + r < OH && ox0 + px < OW)) {
+                            int32_t y[4];
+#pragma unroll
+                            for (int k = 0; k < 4; ++k) {
+                                y[k] = wordsScale<SIGNED>(ws[k], acc[r][px][k]);
+                                y[k] = SIGNED ? __viaddmax_s32(y[k], epi.main.outZp, epi.main.lo) : max(y[k], epi.main.lo);
+                                y[k] = min(y[k], epi.main.hi);
+                            }
+                            *reinterpret_cast<uint32_t *>(static_cast<int8_t *>(out) + (rowOut + uint32_t(px) * uint32_t(C))) =
+                                packSatS8(y[0], y[1], y[2], y[3]);
+                        }
+                    }
+                }
+            };
+            if (wordsScaleSignFree(epi.main.doubleRound != 0, epi.main.outZp, epi.main.lo)) {
+                finish(std::false_type{});
+            } else {
+                finish(std::true_type{});
+            }
+            continue;
+        }
+        FastRescale fr[4]; // any RESCALE (OUT8 only)
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
             if (OUT8) {
                 const int ci = epi.main.perChannel ? c0 + k : 0;
                 fr[k] = makeFastRescale(__ldg(epi.main.mult + ci), int32_t(__ldg(epi.main.shift + ci)), epi.main.inZp,
@@ -330,17 +390,12 @@ __global__ void __launch_bounds__(128) depthwise3x3RowsKernel(const int8_t *__re
         }
 #pragma unroll
         for (int r = 0; r < R; ++r) {
-            const int oy = oy0 + r;
-            if (oy >= OH) {
-                break;
-            }
 #pragma unroll
             for (int px = 0; px < PX; ++px) {
-                const int ox = ox0 + px;
-                if (ox >= OW) {
-                    break;
+                if (oy0 + r >= OH || ox0 + px >= OW) {
+                    continue;
                 }
-                const int64_t flat = ((int64_t(n) * OH + oy) * OW + ox) * C + c0;
+                const int64_t flat = ((int64_t(n) * OH + oy0 + r) * OW + ox0 + px) * C + c0;
                 if (OUT8) {
                     uint32_t word = 0;
 #pragma unroll
@@ -501,7 +556,8 @@ int depthwise3x3(const TView &in, const TView &w, const TView &bias, const TView
         const int64_t total = int64_t(N) * ((OH + R - 1) / R) * ((OW + PX - 1) / PX) * (C / 4);
         const int grid = gridFor(total, 128, 16);
 #define MLEL_LAUNCH_ROWS(RR, SS, O8) \
-    launchOverlapping(depthwise3x3RowsKernel<RR, SS, O8>, grid, 128, s, pi, pw, pb, nb, out.ptr, N, H, W, C, OH, OW, a, e)
+    launchOverlapping(depthwise3x3RowsKernel<RR, SS, O8>, grid, 128, s, pi, pw, pb, nb, out.ptr, N, H, W, C, OH, OW, makeFastDiv(C / 4), \
+                      makeFastDiv((OW + PX - 1) / PX), makeFastDiv((OH + R - 1) / R), a, e)
         if (epi != nullptr) {
             if (a.stride[1] == 1) {
                 if (four) { MLEL_LAUNCH_ROWS(4, 1, true); } else { MLEL_LAUNCH_ROWS(2, 1, true); }
