@@ -160,7 +160,7 @@ __global__ void __launch_bounds__(256) columnSumKernel(const int8_t *__restrict_
 }
 
 // ---- AVG_POOL2D, int8 NHWC (avgpool2d.comp:27-75) ---------------------------------------------------------
-// One output pixel and up to 256 channel units (a unit is four channels, or one where C % 4 != 0) belong to a cluster of
+// One output pixel and up to `width` channel units (a unit is four channels, or one where C % 4 != 0) belong to a cluster of
 // `split` blocks.  The in-range part of a window is rows of contiguous bytes, one run when it spans whole image rows (a
 // global pool), so a thread keeps one channel unit and strides over the pixels of its block's share: consecutive threads
 // read consecutive bytes whatever the channel count.  Partial sums join in shared memory, first of the block, then of
@@ -170,12 +170,12 @@ __global__ void __launch_bounds__(256) columnSumKernel(const int8_t *__restrict_
 // multiple of 16 took the one-thread-per-output kernel: 3 x 57 x 57 x 36, 990 us, now 9).
 template <int CH>
 __global__ void __launch_bounds__(256) avgPoolI8Kernel(const int8_t *__restrict__ in, int8_t *__restrict__ out, int H, int W,
-                                                       int C, int OH, int OW, int chunks, int split, PoolAttr a) {
+                                                       int C, int OH, int OW, int chunks, int width, int split, PoolAttr a) {
     __shared__ int32_t part[256 * CH];
     const int rank = int(blockIdx.x % unsigned(split));
     unsigned b = blockIdx.x / unsigned(split);
     const int units = C / CH; // per pixel
-    const int unit0 = int(b % unsigned(chunks)) * 256, unitsHere = min(units - unit0, 256);
+    const int unit0 = int(b % unsigned(chunks)) * width, unitsHere = min(units - unit0, width);
     b /= unsigned(chunks);
     const int ox = int(b % unsigned(OW));
     b /= unsigned(OW);
@@ -564,19 +564,27 @@ bool avgPoolI8Eligible(const TView &in, const TView &out, const PoolAttr &a) {
     // one block or more per output pixel and 256 channel units: worthwhile when the window is large
     return poolI8Eligible(in, out) && a.kernel[0] > 0 && a.kernel[1] > 0 && int64_t(a.kernel[0]) * a.kernel[1] >= 16 &&
            int64_t(a.kernel[0]) * a.kernel[1] < (int64_t(1) << 24) && a.stride[0] > 0 && a.stride[1] > 0 &&
-           int64_t(out.dims[0]) * out.dims[1] * out.dims[2] * ((int64_t(out.dims[3]) + 255) / 256) < (int64_t(1) << 27);
+           int64_t(out.dims[0]) * out.dims[1] * out.dims[2] * ((int64_t(out.dims[3]) + 31) / 32) < (int64_t(1) << 27);
 }
 
 int avgPoolI8(const TView &in, const TView &out, const PoolAttr &a, cudaStream_t s) {
     const int C = int(in.dims[3]);
-    const int ch = poolUnit(in, out) == 1 ? 1 : 4, units = C / ch, chunks = (units + 255) / 256;
-    const int64_t groups = int64_t(out.dims[0]) * out.dims[1] * out.dims[2] * chunks;
-    // Blocks per group: as long as the SMs are not filled twice over and a block's share stays at a few kilobytes
-    // (below that the cluster's two barriers cost more than the shorter walk gives).
+    const int ch = poolUnit(in, out) == 1 ? 1 : 4, units = C / ch;
+    const int64_t pixels = int64_t(out.dims[0]) * out.dims[1] * out.dims[2];
+    // More blocks while the SMs are not filled four times over: first of fewer channels, down to 32 units (full 32-byte
+    // sectors), so that a block has more pixels in flight; then a cluster per group while a block's share is no less than
+    // the 256 threads fetch in one go of eight words (below that the cluster's barriers cost more than the shorter walk
+    // gives: 64 images of 7 x 7 x 2048 took 20.4 us as clusters of eight blocks of 256 units).
+    int width = 256;
+    while (width > 32 && pixels * ((units + width - 1) / width) < 4 * kNumSMs) {
+        width /= 2;
+    }
+    const int chunks = (units + width - 1) / width;
+    const int64_t groups = pixels * chunks;
     const int64_t bytes = int64_t(std::min(a.kernel[0], int(in.dims[1]))) * std::min(a.kernel[1], int(in.dims[2])) *
-                          std::min(units, 256) * ch;
+                          std::min(units, width) * ch;
     int split = 1;
-    while (split < 8 && groups * split < 4 * kNumSMs && bytes / (2 * split) >= 2048) {
+    while (split < 8 && groups * split < 4 * kNumSMs && bytes / (2 * split) >= 256 * 8 * ch) {
         split *= 2;
     }
     cudaLaunchConfig_t cfg{};
@@ -591,7 +599,7 @@ int avgPoolI8(const TView &in, const TView &out, const PoolAttr &a, cudaStream_t
     cfg.numAttrs = 1;
     cudaLaunchKernelEx(&cfg, ch == 4 ? avgPoolI8Kernel<4> : avgPoolI8Kernel<1>, reinterpret_cast<const int8_t *>(in.ptr),
                        reinterpret_cast<int8_t *>(out.ptr), int(in.dims[1]), int(in.dims[2]), C, int(out.dims[1]),
-                       int(out.dims[2]), chunks, split, a);
+                       int(out.dims[2]), chunks, width, split, a);
     return finish("AVG_POOL2D");
 }
 
