@@ -477,14 +477,18 @@ bool makeTokenMap(CUtensorMap *map, const void *base, int d, int tokens, int hea
     const cuuint64_t strides[3] = {cuuint64_t(stride[2]), cuuint64_t(stride[1]), cuuint64_t(stride[0])};
     const cuuint32_t box[4] = {kRowBytes, kTokenBox, 1, 1};
     const cuuint32_t elemStrides[4] = {1, 1, 1, 1};
-    const CUresult rc = fn(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 4, const_cast<void *>(base), dims, strides, box, elemStrides,
-                           CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-                           CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (rc != CUDA_SUCCESS) {
-        setLastError("attention: cuTensorMapEncodeTiled failed with code " + std::to_string(int(rc)));
-        return false;
-    }
-    return true;
+    const MapKey key{{4, reinterpret_cast<uint64_t>(base), uint64_t(d), uint64_t(tokens), uint64_t(heads), uint64_t(sequences),
+                      uint64_t(stride[0]), uint64_t(stride[1]), uint64_t(stride[2])}};
+    return rememberedMap(map, key, [&](CUtensorMap *m) {
+        const CUresult rc = fn(m, CU_TENSOR_MAP_DATA_TYPE_UINT8, 4, const_cast<void *>(base), dims, strides, box, elemStrides,
+                               CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+        if (rc != CUDA_SUCCESS) {
+            setLastError("attention: cuTensorMapEncodeTiled failed with code " + std::to_string(int(rc)));
+            return false;
+        }
+        return true;
+    });
 }
 
 template <int WARPS>

@@ -7,11 +7,13 @@
 
 #include <cstdint>
 #include <cstdlib>
+#include <cstring>
 #include <atomic>
 #include <mutex>
 #include <set>
 #include <string>
 #include <utility>
+#include <vector>
 
 #include "device_common.cuh"
 #include "gemm_i8_tcgen05.hpp"
@@ -372,6 +374,36 @@ __device__ __forceinline__ void gatherBlock(const GatherRow (&rows)[ROWS], const
 
 
 // ---- host side ----
+// Encoded tensor maps by their description.  A map is a function of its arguments alone (the address among them), and the
+// driver takes about half a microsecond to encode one: three of them were a third of what enqueueing a convolution costs
+// the host.  A session that enqueues the same launches again finds them here; one table of fixed size per host thread.
+struct MapKey {
+    uint64_t v[16] = {};
+};
+template <class Encode> inline bool rememberedMap(CUtensorMap *map, const MapKey &key, Encode &&encode) {
+    struct Entry {
+        MapKey key;
+        CUtensorMap map;
+        bool valid = false;
+    };
+    static thread_local std::vector<Entry> table(512);
+    uint64_t h = 0xcbf29ce484222325ull;
+    for (const uint64_t v : key.v) {
+        h = (h ^ v) * 0x9e3779b97f4a7c15ull;
+        h ^= h >> 29;
+    }
+    Entry &e = table[h % table.size()];
+    if (e.valid && std::memcmp(&e.key, &key, sizeof(MapKey)) == 0) {
+        *map = e.map;
+        return true;
+    }
+    if (!encode(map)) {
+        return false;
+    }
+    e.key = key, e.map = *map, e.valid = true;
+    return true;
+}
+
 using EncodeTiledFn = CUresult (*)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *,
                                    const cuuint64_t *, const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave,
                                    CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
@@ -402,15 +434,18 @@ inline bool makeMap(CUtensorMap *map, const void *base, uint64_t d0, uint64_t d1
     const cuuint64_t strides[2] = {stride1, stride2}; // bytes, for dims 1 and 2
     const cuuint32_t box[3] = {b0, b1, 1};
     const cuuint32_t elemStrides[3] = {1, 1, 1};
-    const CUresult rc = fn(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, const_cast<void *>(base), dims, strides, box,
-                           elemStrides, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                           swizzle128 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE,
-                           CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (rc != CUDA_SUCCESS) {
-        setLastError("cuTensorMapEncodeTiled failed with code " + std::to_string(int(rc)));
-        return false;
-    }
-    return true;
+    const MapKey key{{1, reinterpret_cast<uint64_t>(base), d0, d1, d2, stride1, stride2, b0, b1, swizzle128 ? 1u : 0u}};
+    return rememberedMap(map, key, [&](CUtensorMap *m) {
+        const CUresult rc = fn(m, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, const_cast<void *>(base), dims, strides, box,
+                               elemStrides, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                               swizzle128 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE,
+                               CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+        if (rc != CUDA_SUCCESS) {
+            setLastError("cuTensorMapEncodeTiled failed with code " + std::to_string(int(rc)));
+            return false;
+        }
+        return true;
+    });
 }
 
 // Weights [OC][taps][IC] (OHWI) as a 3-D map {IC, taps, OC} with a {128, 1, rows} box: one load brings 128
@@ -425,9 +460,12 @@ inline bool makeWeightTapMap(CUtensorMap *map, const void *base, int IC, int tap
     const cuuint64_t strides[2] = {cuuint64_t(IC), cuuint64_t(IC) * taps};
     const cuuint32_t box[3] = {128, 1, rows};
     const cuuint32_t elemStrides[3] = {1, 1, 1};
-    return fn(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, const_cast<void *>(base), dims, strides, box, elemStrides,
-              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+    const MapKey key{{2, reinterpret_cast<uint64_t>(base), uint64_t(IC), uint64_t(taps), uint64_t(OC), rows}};
+    return rememberedMap(map, key, [&](CUtensorMap *m) {
+        return fn(m, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, const_cast<void *>(base), dims, strides, box, elemStrides,
+                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+    });
 }
 
 using EncodeIm2colFn = CUresult (*)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *,
@@ -473,10 +511,14 @@ inline bool makeIm2colMap(CUtensorMap *map, const void *base, int N, int H, int 
         return false;
     }
     const cuuint32_t elemStrides[4] = {1, cuuint32_t(strideX), cuuint32_t(strideY), 1};
-    const CUresult rc = fn(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 4, const_cast<void *>(base), dims, strides, lower, upper, 128,
-                           pixels, elemStrides, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
-                           CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    return rc == CUDA_SUCCESS;
+    const auto pair = [](int64_t a, int64_t b) { return (uint64_t(uint32_t(int32_t(a))) << 32) | uint64_t(uint32_t(int32_t(b))); };
+    const MapKey key{{3, reinterpret_cast<uint64_t>(base), pair(N, C), pair(H, W), pair(KH, KW), pair(padTop, padLeft), pair(OH, OW),
+                      pair(strideY, strideX), pair(dilY, dilX), pixels}};
+    return rememberedMap(map, key, [&](CUtensorMap *m) {
+        return fn(m, CU_TENSOR_MAP_DATA_TYPE_UINT8, 4, const_cast<void *>(base), dims, strides, lower, upper, 128, pixels,
+                  elemStrides, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+    });
 }
 
 // Launches `kernel` so that it may overlap the end of its predecessor in the stream (see gridDependencySync).

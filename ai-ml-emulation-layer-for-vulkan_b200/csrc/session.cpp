@@ -465,6 +465,12 @@ int Session::dispatchGraph(cudaStream_t stream) {
     if (rc != MLEL_SUCCESS) {
         return rc;
     }
+    // One kernel is enqueued quicker than a graph of one node is launched: back to back 6.6 against 10.3 us for a small
+    // convolution, the host having 5.3 and 1.8 us to do.
+    const auto &exec = pipeline_->getExecList();
+    if (exec.size() == 1 && exec[0].scratch < 0) {
+        return dispatch(stream);
+    }
     // A captured graph holds the addresses that were bound when it was taken: one graph per set of bindings.
     constexpr size_t kMaxCapturedGraphs = 64;
     const std::vector<const void *> key = bindingKey();
