@@ -1057,7 +1057,6 @@ void GraphPipeline::fuseRowRuns(std::vector<int> &group, const std::vector<UseIn
 // them.  Conditions beyond the pattern itself:
 //   * a row of scores fits the kernel (at most kAttentionMaxKeys keys), head dimension a multiple of 32 up to 128: 32 is
 //     the tensor core's K step, below it the score product would be mostly padding;
-//   * at least 32 keys: shorter rows would leave most of a tile's columns empty, and the separate kernels are short;
 //   * zero points 0 on Q, K and V, and 0 or -128 on the probabilities (signed or unsigned operand bytes);
 //   * shifts and bounds, from the constant tables, for which both element-wise RESCALEs are the high word of one 64-bit
 //     multiply-add;
@@ -1161,7 +1160,7 @@ void GraphPipeline::fuseAttention(std::vector<int> &group, const std::vector<Use
             continue;
         }
         const int64_t B = sd.dims[0], Sq = sd.dims[1], Sk = sd.dims[2], d = qd.dims[2];
-        if (qd.dims[0] != B || kd.dims[0] != B || kd.dims[1] != d || Sk < 32 || Sk > kAttentionMaxKeys || d % 32 != 0 || d > 128 ||
+        if (qd.dims[0] != B || kd.dims[0] != B || kd.dims[1] != d || Sk > kAttentionMaxKeys || d % 32 != 0 || d > 128 ||
             B * ((Sq + 127) / 128) >= (int64_t(1) << 31)) {
             continue;
         }
@@ -1982,25 +1981,31 @@ void GraphPipeline::prepareTensorCore() {
                 continue;
             }
             const int64_t Nb = b.dims[0], C = b.dims[1], W = b.dims[2];
-            if (in.dims[0] != Nb || in.dims[2] != C || C % 16 != 0 || C > 65536 ||
-                out.numel() >= (int64_t(1) << 31) || in.numel() >= (int64_t(1) << 31)) {
+            // Both operands are read with K contiguous and rows on 16-byte boundaries: where C is no multiple of 16 the
+            // first input goes through a copy with rows of Cp bytes, and the second is laid out that way.
+            const int64_t Cp = (C + 15) / 16 * 16, aBytes = C == Cp ? 0 : (Nb * in.dims[1] * Cp + 255) / 256 * 256;
+            if (in.dims[0] != Nb || in.dims[2] != C || C > 65536 || out.numel() >= (int64_t(1) << 31) ||
+                in.numel() >= (int64_t(1) << 31) || aBytes >= (int64_t(1) << 31)) {
                 continue;
             }
             if (b.cls != TensorClass::Constant) {
                 // Second input produced at run time (tc == 3): a kernel in front of the product transposes it to
                 // the K-contiguous form the tensor core reads and sums its columns for the zero-point
-                // correction; both land in one scratch tensor: [Nb][W][C] bytes, then [Nb][W] int32.
-                if (W % 16 != 0 || b.numel() >= (int64_t(1) << 31)) {
+                // correction; all land in one scratch tensor: the copy of the first input (if any), [Nb][W][Cp] bytes,
+                // then [Nb][W] int32.
+                const int64_t btBytes = (Nb * W * Cp + 255) / 256 * 256;
+                // (Copy, transpose and product are three launches, about 8 us for the smallest sizes; one thread per
+                // output is quicker while its chain of C products and the total are short.)
+                if (aBytes + btBytes + Nb * W * 4 >= (int64_t(1) << 31)) {
                     continue;
                 }
-                const int64_t btBytes = (Nb * W * C + 255) / 256 * 256;
-                op.scratch = addScratchTensor(MLEL_I8, {btBytes + Nb * W * 4});
-                op.auxi[2] = int32_t(btBytes);
+                op.scratch = addScratchTensor(MLEL_I8, {aBytes + btBytes + Nb * W * 4});
+                op.auxi[0] = int32_t(aBytes), op.auxi[2] = int32_t(aBytes + btBytes);
                 op.tc = 3;
                 continue;
             }
             const auto *bdata = reinterpret_cast<const int8_t *>(b.hostData.data());
-            std::vector<int8_t> bt(size_t(Nb * W * C));
+            std::vector<int8_t> bt(size_t(Nb * W * Cp), 0);
             std::vector<int32_t> corr(size_t(Nb * W));
             const int64_t za = op.i[0];
             for (int64_t n = 0; n < Nb; ++n) {
@@ -2008,14 +2013,17 @@ void GraphPipeline::prepareTensorCore() {
                     int64_t sum = 0;
                     for (int64_t c = 0; c < C; ++c) {
                         const int8_t v = bdata[(n * C + c) * W + w];
-                        bt[size_t((n * W + w) * C + c)] = v;
+                        bt[size_t((n * W + w) * Cp + c)] = v;
                         sum += v;
                     }
                     corr[size_t(n * W + w)] = int32_t(uint32_t(uint64_t(-za * sum)));
                 }
             }
             op.aux[0] = addDerivedConstant(MLEL_I32, {Nb * W}, corr.data());
-            op.aux[3] = addDerivedConstant(MLEL_I8, {Nb, W, C}, bt.data());
+            op.aux[3] = addDerivedConstant(MLEL_I8, {Nb, W, Cp}, bt.data());
+            if (aBytes != 0) {
+                op.scratch = addScratchTensor(MLEL_I8, {aBytes});
+            }
             op.tc = 1;
         }
     }

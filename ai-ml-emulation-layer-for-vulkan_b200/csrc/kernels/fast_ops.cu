@@ -38,6 +38,48 @@ __global__ void padImageKernel(const int8_t *__restrict__ in, int8_t *__restrict
     }
 }
 
+// 16 bytes from any address, of which the first `valid` (1 to 16) exist; the others are zero.  Only aligned words that hold
+// one of those bytes are read.
+__device__ __forceinline__ int4 loadRagged16(const int8_t *p, int valid) {
+    const uint32_t skip = uint32_t(reinterpret_cast<uintptr_t>(p)) & 3u;
+    const uint32_t *words = reinterpret_cast<const uint32_t *>(p - skip);
+    const int bytes = int(skip) + valid;
+    uint32_t w[5], v[4];
+#pragma unroll
+    for (int k = 0; k < 5; ++k) {
+        w[k] = 4 * k < bytes ? __ldg(words + k) : 0u;
+    }
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        v[k] = __funnelshift_r(w[k], w[k + 1], 8 * skip);
+        const int left = valid - 4 * k;
+        v[k] = left >= 4 ? v[k] : (left <= 0 ? 0u : v[k] & ((1u << (8 * left)) - 1u));
+    }
+    return make_int4(int(v[0]), int(v[1]), int(v[2]), int(v[3]));
+}
+
+// The same copy for channels padded to a multiple of 16: a thread makes 16 bytes of one pixel, from whole words.  BORDER:
+// the copy has pixels that the image has not (false: rows of C bytes become rows of Cp).  Bound by its bytes.
+template <bool BORDER>
+__global__ void __launch_bounds__(256) padPixels16Kernel(const int8_t *__restrict__ in, int4 *__restrict__ out, uint32_t units, int H,
+                                                         int W, int C, FastDiv perPixel, FastDiv divWp, FastDiv divHp, int padTop,
+                                                         int padLeft) {
+    const auto div = [](uint32_t v, const FastDiv &f) { return f.mul == 0u ? v : __umulhi(v, f.mul) >> f.shift; };
+    for (uint32_t e = blockIdx.x * blockDim.x + threadIdx.x; e < units; e += gridDim.x * blockDim.x) {
+        const uint32_t pix = div(e, perPixel);
+        const int c0 = int(e - pix * perPixel.d) * 16;
+        int64_t from = pix;
+        bool live = c0 < C;
+        if (BORDER) {
+            const uint32_t line = div(pix, divWp), n = div(line, divHp);
+            const int x = int(pix - line * divWp.d) - padLeft, y = int(line - n * divHp.d) - padTop;
+            live = live && unsigned(x) < unsigned(W) && unsigned(y) < unsigned(H);
+            from = (int64_t(n) * H + y) * W + x;
+        }
+        out[e] = live ? loadRagged16(in + from * C + c0, min(16, C - c0)) : make_int4(0, 0, 0, 0);
+    }
+}
+
 // The same copy for Cp == 4 and an even Wp (the RGB stem): one block per row of the copy, two pixels (one 8-byte
 // store) per thread, no divisions in the element loop.
 __global__ void __launch_bounds__(128) padImageRows4Kernel(const int8_t *__restrict__ in, int8_t *__restrict__ out, int H,
@@ -66,27 +108,38 @@ __global__ void __launch_bounds__(128) padImageRows4Kernel(const int8_t *__restr
     }
 }
 
-// ---- transpose of MATMUL's second input [N][C][W] -> [N][W][C] with column sums ---------------------------
-// A block owns 64 columns (w) of one batch and walks the rows (c) in tiles of 64: 16-byte loads of the
-// tile, byte transposition through shared memory, 16-byte stores; each thread keeps the running sum of the
-// bytes it moved, and four neighbouring lanes combine them into the column sum at the end.
+// ---- transpose of MATMUL's second input [N][C][W] -> [N][W][Cp] with column sums ---------------------------
+// Cp: C rounded up to a multiple of 16, the tail zero.  64 columns (w) of one batch belong to a cluster of `split` blocks
+// that share the rows (c) and walk them in tiles of 64: 16-byte loads of the tile (the next tile's while this one is
+// turned), byte transposition through shared memory, 16-byte stores; each thread keeps the running sum of the bytes it
+// moved, four neighbouring lanes and then the cluster's blocks combine them into the column sum at the end.
+// Latency bounds it where there are few columns: a tile is a chain of load, turn and store.
+// ALIGNED: rows of B start on 16-byte boundaries.
+template <bool ALIGNED>
 __global__ void __launch_bounds__(256) transposeColsumKernel(const int8_t *__restrict__ b, int8_t *__restrict__ bt,
-                                                             int32_t *__restrict__ corr, int C, int W, int32_t za) {
+                                                             int32_t *__restrict__ corr, int C, int W, int Cp, int32_t za, int split) {
     __shared__ int8_t tile[64][64 + 16]; // [c][w], rows padded to spread the banks of the column reads
+    __shared__ int32_t part[64];
     const int n = blockIdx.y;
-    const int w0 = blockIdx.x * 64;
+    const int rank = int(blockIdx.x % unsigned(split)), w0 = int(blockIdx.x / unsigned(split)) * 64;
     const int t = threadIdx.x;
     const int8_t *src = b + int64_t(n) * C * W;
-    int8_t *dst = bt + int64_t(n) * W * C;
+    int8_t *dst = bt + int64_t(n) * W * Cp;
     // load role: row (c) t / 4, 16-byte segment (w) t % 4; store role: column (w) t / 4, segment (c) t % 4
     const int lr = t >> 2, ls = (t & 3) * 16;
     int32_t sum = 0;
-    for (int c0 = 0; c0 < C; c0 += 64) {
-        int4 v = make_int4(0, 0, 0, 0);
-        if (c0 + lr < C && w0 + ls < W) {
-            v = __ldg(reinterpret_cast<const int4 *>(src + int64_t(c0 + lr) * W + w0 + ls));
+    const int tiles = (C + 63) / 64, first = tiles * rank / split * 64, last = tiles * (rank + 1) / split * 64;
+    const auto fetch = [&](int c0) {
+        if (c0 + lr >= C || w0 + ls >= W || c0 >= last) {
+            return make_int4(0, 0, 0, 0);
         }
-        *reinterpret_cast<int4 *>(&tile[lr][ls]) = v;
+        const int8_t *p = src + int64_t(c0 + lr) * W + w0 + ls;
+        return ALIGNED ? __ldg(reinterpret_cast<const int4 *>(p)) : loadRagged16(p, min(16, W - (w0 + ls)));
+    };
+    int4 next = fetch(first);
+    for (int c0 = first; c0 < last; c0 += 64) {
+        *reinterpret_cast<int4 *>(&tile[lr][ls]) = next;
+        next = fetch(c0 + 64);
         __syncthreads();
         uint32_t words[4] = {0, 0, 0, 0};
 #pragma unroll
@@ -95,15 +148,32 @@ __global__ void __launch_bounds__(256) transposeColsumKernel(const int8_t *__res
             sum += x;
             words[i >> 2] |= uint32_t(uint8_t(x)) << (8 * (i & 3));
         }
-        if (w0 + lr < W && c0 + ls < C) {
-            *reinterpret_cast<int4 *>(dst + int64_t(w0 + lr) * C + c0 + ls) =
+        if (w0 + lr < W && c0 + ls < Cp) {
+            *reinterpret_cast<int4 *>(dst + int64_t(w0 + lr) * Cp + c0 + ls) =
                 make_int4(int(words[0]), int(words[1]), int(words[2]), int(words[3]));
         }
         __syncthreads();
     }
     sum += __shfl_xor_sync(0xffffffffu, sum, 1);
     sum += __shfl_xor_sync(0xffffffffu, sum, 2);
-    if ((t & 3) == 0 && w0 + lr < W) {
+    if (split > 1) {
+        if ((t & 3) == 0) {
+            part[lr] = sum;
+        }
+        asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+        if (rank == 0) {
+            for (int r = 1; r < split; ++r) {
+                uint32_t peer, v;
+                const uint32_t local = uint32_t(__cvta_generic_to_shared(&part[lr]));
+                asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(peer) : "r"(local), "r"(r));
+                asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(v) : "r"(peer));
+                sum += int32_t(v);
+            }
+        }
+        // block 0 has read the others' shared memory before they leave
+        asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+    }
+    if (rank == 0 && (t & 3) == 0 && w0 + lr < W) {
         corr[int64_t(n) * W + w0 + lr] = int32_t(uint32_t(0) - uint32_t(za) * uint32_t(sum));
     }
 }
@@ -510,14 +580,38 @@ int padImageI8(const int8_t *in, int8_t *out, int N, int H, int W, int C, int Hp
         padImageRows4Kernel<<<unsigned(N * Hp), 128, 0, s>>>(in, out, H, W, C, Hp, Wp, padTop, padLeft);
         return finish("padded copy");
     }
+    const int64_t pixels = int64_t(N) * Hp * Wp, units = pixels * (Cp >> 4);
+    if (Cp % 16 == 0 && units < (int64_t(1) << 30) && (reinterpret_cast<uintptr_t>(out) & 15u) == 0) {
+        const bool border = Hp != H || Wp != W || padTop != 0 || padLeft != 0;
+        (border ? padPixels16Kernel<true> : padPixels16Kernel<false>)<<<gridFor(units, 256, 8), 256, 0, s>>>(
+            in, reinterpret_cast<int4 *>(out), uint32_t(units), H, W, C, makeFastDiv(Cp >> 4), makeFastDiv(Wp), makeFastDiv(Hp), padTop,
+            padLeft);
+        return finish("padded copy");
+    }
     const int64_t words = int64_t(N) * Hp * Wp * (Cp >> 2);
     padImageKernel<<<gridFor(words, kThreads, 8), kThreads, 0, s>>>(in, out, words, H, W, C, Hp, Wp, Cp, padTop, padLeft);
     return finish("padded copy");
 }
 
 int transposeForMatmul(const int8_t *b, int8_t *bt, int32_t *corr, int batches, int C, int W, int32_t za, cudaStream_t s) {
-    const dim3 grid(unsigned((W + 63) / 64), unsigned(batches));
-    transposeColsumKernel<<<grid, 256, 0, s>>>(b, bt, corr, C, W, za);
+    // more blocks per 64 columns while the SMs are not filled twice over and each keeps two tiles of rows
+    const int columns = (W + 63) / 64, tiles = (C + 63) / 64;
+    int split = 1;
+    while (split < 8 && int64_t(columns) * batches * split < 2 * kNumSMs && tiles >= 4 * split) {
+        split *= 2;
+    }
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(unsigned(columns * split), unsigned(batches));
+    cfg.blockDim = dim3(256);
+    cfg.stream = s;
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = unsigned(split);
+    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, W % 16 == 0 ? transposeColsumKernel<true> : transposeColsumKernel<false>, b, bt, corr, C, W,
+                       (C + 15) / 16 * 16, za, split);
     return finish("MATMUL operand transpose");
 }
 

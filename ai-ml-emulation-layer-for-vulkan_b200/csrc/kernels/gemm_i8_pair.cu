@@ -496,7 +496,7 @@ bool gemmI8PairApplies(const GemmI8Problem &q) {
     if (p.out8 == nullptr || !p.epi.hasMain || p.N <= kOcTile || p.gatherTable != nullptr) {
         return false;
     }
-    if (p.N % 16 != 0 || p.ldOut % 16 != 0 || p.K % 16 != 0 || (reinterpret_cast<uintptr_t>(p.out8) & 15u) != 0 ||
+    if (p.N % 16 != 0 || p.ldOut % 16 != 0 || q.bRowBytes % 16 != 0 || (reinterpret_cast<uintptr_t>(p.out8) & 15u) != 0 ||
         (reinterpret_cast<uintptr_t>(q.bMatrix) & 15u) != 0) {
         return false;
     }

@@ -15,8 +15,8 @@
 //     Integer sums wrap, so the order does not change the result;
 //   * sixteen epilogue warps: a thread has BNP / SPLIT / 4 results (a residual tail is three RESCALEs more, and 32 results
 //     a thread took 3.5 us);
-//   * weights and the epilogue's constants do not depend on the launch before: they are fetched ahead of
-//     griddepcontrol.wait, and a CTA is small enough (about 100 KB, 32 or 64 columns of tensor memory) to be resident
+//   * weights and the epilogue's constants do not depend on the launch before (unless it made them: a product of two
+//     activations): they are fetched ahead of griddepcontrol.wait, and a CTA is small enough (about 100 KB, 32 or 64 columns of tensor memory) to be resident
 //     beside the CTAs of the launches around it;
 //   * results go from registers to memory: 32 lanes hold 32 neighbouring channels of a pixel.
 // The arithmetic is the other kernels' (fastRescale); a residual tail evaluates its three RESCALEs.
@@ -151,6 +151,9 @@ gemmI8Small(const __grid_constant__ CUtensorMap mapX, const __grid_constant__ CU
                 }
             };
             const int ahead = min(kbCount, kStages);
+            if (p.lateOperand != 0) {
+                asm volatile("griddepcontrol.wait;" ::: "memory");
+            }
             for (int i = 0; i < ahead; ++i) {
                 loadW(i);
             }
@@ -195,6 +198,9 @@ gemmI8Small(const __grid_constant__ CUtensorMap mapX, const __grid_constant__ CU
         const int ci = p.epi.main.perChannel && ocValid ? oc : 0;
         main = makeFastRescale(__ldg(p.epi.main.mult + ci), int32_t(__ldg(p.epi.main.shift + ci)), p.epi.main.inZp,
                                p.epi.main.doubleRound != 0);
+        if (p.lateOperand != 0) {
+            asm volatile("griddepcontrol.wait;" ::: "memory");
+        }
 #pragma unroll
         for (int j = 0; j < kMine; ++j) {
             int cls = p.baseClass;

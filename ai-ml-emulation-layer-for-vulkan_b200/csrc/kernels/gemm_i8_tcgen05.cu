@@ -136,15 +136,50 @@ __device__ __forceinline__ void rescale16Words32(const uint32_t (&acc)[16], uint
     }
 }
 
-template <int BN, int NSTAGE, bool RESIDUAL>
+// Int8 rows at odd addresses: the 32 rows of a quarter of the tile are put together in shared memory by the four warps that
+// compute them, and leave as runs of aligned words -- a run per row, or one run for all of them where a row is one tile
+// wide.  Stored byte by byte a step was 16 store instructions, each to 32 lines (1 x 270 x 480 pixels of 21 channels: 18.5
+// us; 16 products of 1024 x 1024 x 1023: see launchMatmulTensorCore).
+template <int BN> constexpr int kRowPitchWords = BN / 4 + 1; // no bank conflicts
+template <int BN> constexpr int kStageBytesRows8 = 4 * 32 * kRowPitchWords<BN> * 4;
+
+__device__ __forceinline__ void quarterSync(int quarter) { // the 128 threads of a quarter's four warps
+    asm volatile("bar.sync %0, 128;" ::"r"(2 + quarter) : "memory");
+}
+
+// `length` bytes from shared memory (a word boundary) to any address: lanes first, first + step, ... take a word each.
+__device__ __forceinline__ void storeRun(int8_t *to, const uint32_t *words, int length, int first, int step) {
+    const int skip = int(reinterpret_cast<uintptr_t>(to) & 3u);
+    const int count = (skip + length + 3) >> 2;
+    for (int k = first; k < count; k += step) {
+        const int at = 4 * k - skip; // first byte of the word
+        const uint32_t here = words[k];
+        const uint32_t v = skip == 0 ? here : __funnelshift_r(k > 0 ? words[k - 1] : 0u, here, 32 - 8 * skip);
+        if (at >= 0 && at + 4 <= length) {
+            *reinterpret_cast<uint32_t *>(to + at) = v;
+        } else {
+#pragma unroll
+            for (int b = 0; b < 4; ++b) {
+                if (at + b >= 0 && at + b < length) {
+                    to[at + b] = int8_t(v >> (8 * b));
+                }
+            }
+        }
+    }
+}
+
+// ROWS16: every row of the output starts on a 16-byte boundary, a thread stores its own row's 16 columns at once.
+template <int BN, int NSTAGE, bool RESIDUAL, bool ROWS16>
 __device__ __forceinline__ void epilogueInt8(const GemmI8Params &p, PipeBarriers *bars, ColConst *colTab,
                                              uint32_t tmemBase, int warp, int lane, int64_t numTiles, int mTiles,
-                                             int nTiles) {
+                                             int nTiles, uint32_t *rows8) {
     const int quarter = warp & 3; // TMEM lanes [32 * quarter, 32 * quarter + 32)
     const int half = warp >> 2;   // which half of the tile's columns
     constexpr int kColsPerWarp = BN / (kEpilogueWarps / 4);
     constexpr int kSteps = kColsPerWarp / 16;
     const int row = quarter * 32 + lane;
+    bool failed = false;
+    uint32_t *rows = rows8 + quarter * (32 * kRowPitchWords<BN>); // !ROWS16: this quarter's rows
     FastRescale fa{}, fb{}, fo{};
     if (RESIDUAL) {
         fa = makeFastRescale(__ldg(p.epi.a.mult), int32_t(__ldg(p.epi.a.shift)), p.epi.a.inZp, p.epi.a.doubleRound != 0);
@@ -233,8 +268,12 @@ __device__ __forceinline__ void epilogueInt8(const GemmI8Params &p, PipeBarriers
         }
         const int64_t outRow = (int64_t(batch) * p.M + m) * p.ldOut;
 
-        if (!mbarWait(&bars->accFull[buf], (tileCount >> 1) & 1u, 4)) {
-            break;
+        if (ROWS16) {
+            if (!mbarWait(&bars->accFull[buf], (tileCount >> 1) & 1u, 4)) {
+                break;
+            }
+        } else { // after a wait that ran out the warp still meets the others of its quarter
+            failed = failed || !mbarWait(&bars->accFull[buf], (tileCount >> 1) & 1u, 4);
         }
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const uint32_t taddr = tmemBase + buf * uint32_t(BN) + (uint32_t(quarter * 32) << 16);
@@ -255,9 +294,8 @@ __device__ __forceinline__ void epilogueInt8(const GemmI8Params &p, PipeBarriers
             if (!rowValid || col0 >= p.N) {
                 continue;
             }
-            const int ncols = min(16, p.N - col0);
+            const int ncols = ROWS16 ? 16 : min(16, p.N - col0);
             int8_t *dst = p.out8 + outRow + col0;
-            const bool vec = ncols == 16 && (reinterpret_cast<uintptr_t>(dst) & 15u) == 0;
             if (cls != p.baseClass) {
                 // a pixel whose window crosses the border: swap the table's correction for its own class's
                 const int32_t *own = corrBatch + int64_t(cls) * p.N + col0;
@@ -271,7 +309,7 @@ __device__ __forceinline__ void epilogueInt8(const GemmI8Params &p, PipeBarriers
             uint32_t sc[4] = {0, 0, 0, 0}; // 16 shortcut bytes of this row
             if (RESIDUAL) {
                 const int8_t *scp = p.epi.shortcut + outRow + col0;
-                if (vec) {
+                if (ROWS16) {
                     const int4 s0 = __ldg(reinterpret_cast<const int4 *>(scp));
                     sc[0] = uint32_t(s0.x), sc[1] = uint32_t(s0.y), sc[2] = uint32_t(s0.z), sc[3] = uint32_t(s0.w);
                 } else {
@@ -342,16 +380,35 @@ __device__ __forceinline__ void epilogueInt8(const GemmI8Params &p, PipeBarriers
                     packed[q] = pack4(y[0], y[1], y[2], y[3]);
                 }
             }
-            if (vec) {
+            if (ROWS16) {
                 *reinterpret_cast<int4 *>(dst) = make_int4(int(packed[0]), int(packed[1]), int(packed[2]), int(packed[3]));
-            } else {
+            } else if (nTiles == 1) {
+                int8_t *mine = reinterpret_cast<int8_t *>(rows) + lane * p.N + cl;
 #pragma unroll
                 for (int j = 0; j < 16; ++j) {
                     if (j < ncols) {
-                        dst[j] = int8_t(packed[j >> 2] >> (8 * (j & 3)));
+                        mine[j] = int8_t(packed[j >> 2] >> (8 * (j & 3)));
                     }
                 }
+            } else {
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    rows[lane * kRowPitchWords<BN> + (cl >> 2) + q] = packed[q];
+                }
             }
+        }
+        if (!ROWS16) {
+            quarterSync(quarter);
+            const int firstRow = m0 + quarter * 32, rowsHere = min(32, p.M - firstRow);
+            int8_t *to = p.out8 + (int64_t(batch) * p.M + firstRow) * p.ldOut + n0;
+            if (nTiles == 1) {
+                storeRun(to, rows, rowsHere * p.N, half * 32 + lane, 128);
+            } else {
+                for (int r = half; r < rowsHere; r += 4) {
+                    storeRun(to + int64_t(r) * p.ldOut, rows + r * kRowPitchWords<BN>, min(BN, p.N - n0), lane, 32);
+                }
+            }
+            quarterSync(quarter); // before the next tile's rows
         }
     }
 }
@@ -467,18 +524,20 @@ __device__ __forceinline__ void epilogueInt32(const GemmI8Params &p, PipeBarrier
     }
 }
 
-template <int BN, int NSTAGE>
+template <int BN, int NSTAGE, bool ROWS16>
 __device__ __forceinline__ void epilogueWarps(const GemmI8Params &p, PipeBarriers *bars, ColConst *colTab,
                                               uint32_t tmemBase, int warp, int lane, int64_t numTiles, int mTiles,
-                                              int nTiles, int32_t *staging) {
+                                              int nTiles, int32_t *staging, uint32_t *rows8) {
     if (p.out32 != nullptr) {
         // the staged stores need 16-byte aligned rows
         const bool staged = staging != nullptr && p.ldOut % 4 == 0 && (reinterpret_cast<uintptr_t>(p.out32) & 15u) == 0;
         epilogueInt32<BN, NSTAGE>(p, bars, tmemBase, warp, lane, numTiles, mTiles, nTiles, staged ? staging : nullptr);
-    } else if (p.epi.hasResidual) {
-        epilogueInt8<BN, NSTAGE, true>(p, bars, colTab, tmemBase, warp, lane, numTiles, mTiles, nTiles);
+        return;
+    }
+    if (p.epi.hasResidual) {
+        epilogueInt8<BN, NSTAGE, true, ROWS16>(p, bars, colTab, tmemBase, warp, lane, numTiles, mTiles, nTiles, rows8);
     } else {
-        epilogueInt8<BN, NSTAGE, false>(p, bars, colTab, tmemBase, warp, lane, numTiles, mTiles, nTiles);
+        epilogueInt8<BN, NSTAGE, false, ROWS16>(p, bars, colTab, tmemBase, warp, lane, numTiles, mTiles, nTiles, rows8);
     }
 }
 
@@ -516,7 +575,9 @@ __device__ __forceinline__ void gatherPieces(const int8_t *origin, const int32_t
 // tmapA is a plain matrix, kAIm2col = tmapA is an im2col map of the NHWC input and tmapB a {IC, taps, OC} map.
 // B_MN : B is an N-contiguous [K][N] matrix (MN-major operand), otherwise a K-contiguous [N][K] matrix.
 // STAGE32: shared memory for the staged int32 stores of epilogueInt32 is set aside (see there).
-template <int BN, int NSTAGE, int A_MODE, bool B_MN, bool STAGE32 = false>
+// ROWS16: see epilogueInt8 (a kernel of its own: in one kernel the two forms' registers spilled, 64 images of the
+// ResNet-50 shape 970 -> 1003 us).
+template <int BN, int NSTAGE, int A_MODE, bool B_MN, bool STAGE32 = false, bool ROWS16 = true>
 __global__ void __launch_bounds__(A_MODE != kAGather ? kThreadsTma : kThreadsGather, 1)
 gemmI8Tcgen05(const __grid_constant__ CUtensorMap tmapA, const __grid_constant__ CUtensorMap tmapB, const GemmI8Params p) {
     constexpr bool A_TMA = A_MODE != kAGather;
@@ -535,6 +596,9 @@ gemmI8Tcgen05(const __grid_constant__ CUtensorMap tmapA, const __grid_constant__
     int32_t *tapTab = gatherTab + kMaxGatherPieces; // tap offsets of the segment gather
     // STAGE32 (TMA variants only: no gather tables): the epilogue warps' staging blocks follow the barriers
     int32_t *staging = STAGE32 ? gatherTab : nullptr;
+    // the int8 epilogue's staging comes last
+    uint32_t *rows8 = reinterpret_cast<uint32_t *>(gatherTab) +
+                      (A_TMA ? (STAGE32 ? kEpilogueWarps * kStageBytesPerWarp / 4 : 0) : kMaxGatherPieces + kTapTabEntries);
     const bool fastGather = !A_TMA && fastGatherApplies(p);
 
     const int warp = threadIdx.x >> 5;
@@ -793,7 +857,7 @@ gemmI8Tcgen05(const __grid_constant__ CUtensorMap tmapA, const __grid_constant__
         }
     } else {
         // ---------------- epilogue: warps 0-15 ----------------
-        epilogueWarps<BN, NSTAGE>(p, bars, colTab, tmemBase, warp, lane, numTiles, mTiles, nTiles, staging);
+        epilogueWarps<BN, NSTAGE, ROWS16>(p, bars, colTab, tmemBase, warp, lane, numTiles, mTiles, nTiles, staging, rows8);
     }
 
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -807,7 +871,7 @@ gemmI8Tcgen05(const __grid_constant__ CUtensorMap tmapA, const __grid_constant__
 
 // ---- host side --------------------------------------------------------------------------------------------
 
-template <int BN, int NSTAGE, int A_MODE, bool B_MN, bool STAGE32 = false>
+template <int BN, int NSTAGE, int A_MODE, bool B_MN, bool STAGE32 = false, bool ROWS16 = true>
 int launchVariant(const CUtensorMap &mapA, const CUtensorMap &mapB, const GemmI8Params &params, cudaStream_t s) {
     static_assert(!STAGE32 || A_MODE != kAGather, "the staging blocks take the place of the gather tables");
     GemmI8Params p = params;
@@ -815,10 +879,10 @@ int launchVariant(const CUtensorMap &mapA, const CUtensorMap &mapB, const GemmI8
     p.divTiles0 = makeFastDiv((p.N + BN - 1) / BN), p.divTiles1 = makeFastDiv((p.M + BM - 1) / BM);
     constexpr size_t smemBytes =
         size_t(NSTAGE) * (BM * BK + BN * BK) + BN * sizeof(ColConst) + sizeof(PipeBarriers) + 1024 +
-        (A_MODE != kAGather ? 0 : (kMaxGatherPieces + kTapTabEntries) * sizeof(int32_t) + 16) +
-        (STAGE32 ? size_t(kEpilogueWarps) * kStageBytesPerWarp + 16 : 0);
+        (A_MODE != kAGather ? 0 : (kMaxGatherPieces + kTapTabEntries) * sizeof(int32_t)) + 16 +
+        (STAGE32 ? size_t(kEpilogueWarps) * kStageBytesPerWarp : 0) + (ROWS16 ? 0 : kStageBytesRows8<BN>);
     static_assert(smemBytes <= 232448, "shared memory per CTA");
-    auto kernel = gemmI8Tcgen05<BN, NSTAGE, A_MODE, B_MN, STAGE32>;
+    auto kernel = gemmI8Tcgen05<BN, NSTAGE, A_MODE, B_MN, STAGE32, ROWS16>;
     if (!allowDynamicSmem(reinterpret_cast<const void *>(kernel), smemBytes)) {
         return MLEL_ERROR_DEVICE;
     }
@@ -890,6 +954,17 @@ int gemmI8Launch(const GemmI8Problem &q, cudaStream_t s) {
     if (q.bMnMajor) {
         return aMode == kATiled ? launchVariant<128, 6, kATiled, true>(mapA, mapB, p, s)
                                 : launchVariant<128, 6, kAGather, true>(mapA, mapB, p, s);
+    }
+    const bool rows16 = p.out8 == nullptr || (p.ldOut % 16 == 0 && (reinterpret_cast<uintptr_t>(p.out8) & 15u) == 0);
+    if (!rows16) {
+        if (bn == 64) {
+            return aMode == kATiled    ? launchVariant<64, 8, kATiled, false, false, false>(mapA, mapB, p, s)
+                   : aMode == kAIm2col ? launchVariant<64, 8, kAIm2col, false, false, false>(mapA, mapB, p, s)
+                                       : launchVariant<64, 8, kAGather, false, false, false>(mapA, mapB, p, s);
+        }
+        return aMode == kATiled    ? launchVariant<128, 6, kATiled, false, false, false>(mapA, mapB, p, s)
+               : aMode == kAIm2col ? launchVariant<128, 6, kAIm2col, false, false, false>(mapA, mapB, p, s)
+                                   : launchVariant<128, 6, kAGather, false, false, false>(mapA, mapB, p, s);
     }
     if (bn == 64) {
         return aMode == kATiled    ? launchVariant<64, 8, kATiled, false>(mapA, mapB, p, s)

@@ -57,6 +57,7 @@ struct GemmI8Params {
     const uint8_t *rowClass; // [OH] border class of an output row, or null (single class)
     const uint8_t *colClass; // [OW]
     int32_t numColClasses, numClasses, batchedCorr;
+    int32_t lateOperand;     // 1: the weight operand and the corrections are results of a launch before this one
     int32_t baseClass;       // the most common class: its correction row is staged in shared memory
     int32_t corrSmall;       // 1: every |corr| <= 2^30 - 256: accumulator + correction - zero point stays inside int32;
                              // 2: it even stays below 2^29 in size

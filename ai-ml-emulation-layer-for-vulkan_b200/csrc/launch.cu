@@ -233,17 +233,28 @@ int launchMatmulTensorCore(const OpDesc &op, const TView *T, cudaStream_t s) {
         p.out32 = reinterpret_cast<int32_t *>(out.ptr);
     }
     q.batches = int32_t(a.dims[0]);
+    const int Cp = (p.K + 15) / 16 * 16; // row pitch of what is read with K contiguous
     q.aMatrix = a.ptr;
-    q.aRowBytes = uint64_t(p.K);
-    q.aBatchBytes = uint64_t(p.K) * uint64_t(p.M);
+    q.aRowBytes = uint64_t(Cp);
+    q.aBatchBytes = uint64_t(Cp) * uint64_t(p.M);
+    if (Cp != p.K) {
+        int8_t *copy = reinterpret_cast<int8_t *>(T[op.scratch].ptr);
+        const int rows = int(a.dims[0]) * p.M;
+        const int rc = padImageI8(reinterpret_cast<const int8_t *>(a.ptr), copy, 1, 1, rows, p.K, 1, rows, Cp, 0, 0, s);
+        if (rc != MLEL_SUCCESS) {
+            return rc;
+        }
+        q.aMatrix = copy;
+    }
     const void *bt = nullptr;
     if (op.tc == 3) {
         const TView &b = T[op.in[1]];
         p.N = int32_t(b.dims[2]);
         p.ldOut = p.N;
-        int8_t *scratch = reinterpret_cast<int8_t *>(T[op.scratch].ptr);
-        int32_t *corr = reinterpret_cast<int32_t *>(scratch + op.auxi[2]);
+        int8_t *scratch = reinterpret_cast<int8_t *>(T[op.scratch].ptr) + op.auxi[0];
+        int32_t *corr = reinterpret_cast<int32_t *>(reinterpret_cast<int8_t *>(T[op.scratch].ptr) + op.auxi[2]);
         p.corr = corr;
+        p.lateOperand = 1;
         // The paired kernel reads the run-time operand where it lies ([C][W], the output column contiguous: an
         // MN-major tensor-core operand) and only needs the column sums; the single-CTA kernel takes a transposed
         // copy, made together with the sums.
@@ -275,8 +286,8 @@ int launchMatmulTensorCore(const OpDesc &op, const TView *T, cudaStream_t s) {
         p.corr = reinterpret_cast<const int32_t *>(T[op.aux[0]].ptr);
     }
     q.bMatrix = bt;
-    q.bRowBytes = uint64_t(p.K);
-    q.bBatchBytes = uint64_t(p.K) * uint64_t(p.N);
+    q.bRowBytes = uint64_t(Cp);
+    q.bBatchBytes = uint64_t(Cp) * uint64_t(p.N);
     q.bMnMajor = false;
     int rc = MLEL_SUCCESS;
     // ("pair_kernel" 2 asks for the paired kernel wherever it applies)

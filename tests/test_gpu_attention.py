@@ -45,7 +45,7 @@ def attention_graph(n, heads, sq, sk, d, prob_zp=-128, double_round=False, merge
 @pytest.mark.parametrize("n,heads,sq,sk,d", [
     (1, 1, 128, 128, 64), (1, 2, 32, 32, 32), (2, 3, 197, 197, 64), (1, 1, 130, 33, 128), (1, 2, 1, 512, 64),
     (3, 2, 129, 191, 96), (1, 4, 192, 192, 64), (1, 2, 100, 193, 64), (1, 1, 300, 384, 64), (1, 2, 65, 256, 32),
-    (2, 1, 511, 511, 128), (20, 12, 257, 65, 64),
+    (2, 1, 511, 511, 128), (20, 12, 257, 65, 64), (1, 1, 40, 16, 64), (3, 2, 19, 19, 64), (1, 2, 7, 1, 32),
 ])
 @pytest.mark.parametrize("prob_zp,double_round,pow2", [(-128, False, False), (0, True, False), (-128, True, True), (0, False, True)])
 def test_attention_matches_the_operators(mlel, n, heads, sq, sk, d, prob_zp, double_round, pow2):
@@ -61,7 +61,7 @@ def test_attention_matches_the_operators(mlel, n, heads, sq, sk, d, prob_zp, dou
         assert len(bad) == 0, (len(bad), got.size, bad[:4].tolist())
 
 
-@pytest.mark.parametrize("n,heads,sq,sk,d", [(1, 1, 40, 16, 64), (1, 1, 16, 513, 32), (1, 2, 48, 48, 16)])
+@pytest.mark.parametrize("n,heads,sq,sk,d", [(1, 1, 16, 513, 32), (1, 2, 48, 48, 16)])
 def test_attention_outside_the_kernel_stays_with_the_operators(mlel, n, heads, sq, sk, d):
     from mlel_b200.runtime import GraphRunner
     g, data = attention_graph(n, heads, sq, sk, d, seed=7)

@@ -1,0 +1,40 @@
+"""GPU parity of int8 products whose row lengths are no multiple of 16: copies with padded rows, transposes by a cluster,
+rows of output at odd addresses.  Bit-exact against the CPU oracle."""
+import numpy as np
+import pytest
+
+from mlel_b200.graph_builder import GraphBuilder
+from tests.test_gpu_small import conv
+from tests.test_gpu_vector_ops import check
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("batch,rows,k,n", [
+    (1, 1, 1, 1), (1, 17, 33, 15), (3, 64, 100, 48), (2, 130, 197, 197), (5, 197, 64, 197), (1, 128, 127, 256), (2, 200, 1023, 272),
+    (2, 129, 640, 129), (1, 31, 4100, 50), (3, 257, 144, 301),
+])
+@pytest.mark.parametrize("constant", [False, True])
+def test_products_of_every_row_length(mlel, batch, rows, k, n, constant):
+    r = np.random.Generator(np.random.PCG64(rows * k + n))
+    a8, b8 = (r.integers(-128, 128, s, dtype=np.int8) for s in ((batch, rows, k), (batch, k, n)))
+    g = GraphBuilder()
+    a = g.input(np.int8, a8.shape)
+    b = g.constant(b8) if constant else g.input(np.int8, b8.shape)
+    g.output(g.matmul(a, b, -20, 0))
+    for shift in (34, 40):
+        g.output(g.rescale(g.matmul(a, b, 3, 0), [1 << 30 | 12345], [shift], 0, 1, np.int8, double_round=True))
+    check(g, [a8] if constant else [a8, b8])
+
+
+@pytest.mark.parametrize("channels", [5, 21, 34, 150])
+def test_rows_at_odd_addresses_with_residual_tail(mlel, channels):
+    r = np.random.Generator(np.random.PCG64(channels))
+    g = GraphBuilder()
+    x = g.input(np.int8, (2, 40, 41, channels))
+    y = conv(g, r, x, channels, 1, 1, 0, 4, True)
+    a = g.rescale(y, [int(r.integers(1 << 30, 1 << 31))], [23], 4, 0, np.int32)
+    b = g.rescale(x, [int(r.integers(1 << 30, 1 << 31))], [23], -3, 0, np.int32)
+    g.output(g.rescale(g.add(a, b), [int(r.integers(1 << 30, 1 << 31))], [40], 0, -20, np.int8, double_round=True))
+    g.output(conv(g, r, x, channels, 3, 1, 1, 4, True))
+    check(g, [r.integers(-128, 128, x.shape, dtype=np.int8)])
