@@ -111,6 +111,8 @@ int mlel_set_tuning(const char *key, int value) {
             t.pairKernel = value;
         } else if (k == "small_kernel" && value >= 0) {
             t.smallKernel = value;
+        } else if (k == "window_kernel" && value >= 0 && value <= 1) {
+            t.windowKernel = value;
         } else if (k == "tile_progress" && value >= 0 && value <= 7) {
             t.tileProgress = value;
         } else if (k == "oc_tile_rule" && value >= 0 && value <= 8) {
@@ -130,7 +132,7 @@ int mlel_set_tuning(const char *key, int value) {
 }
 
 long long mlel_tensor_core_launches(int kernel) {
-    return kernel >= 0 && kernel < 4 ? g_tensorCoreLaunches[kernel].load(std::memory_order_relaxed) : -1;
+    return kernel >= 0 && kernel < 5 ? g_tensorCoreLaunches[kernel].load(std::memory_order_relaxed) : -1;
 }
 
 int mlel_selftest_wait_timeout(void *cuda_stream, int *recorded_code) {

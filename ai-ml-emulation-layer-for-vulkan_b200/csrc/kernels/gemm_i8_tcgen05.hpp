@@ -141,10 +141,17 @@ bool gemmI8SmallApplies(const GemmI8Problem &problem, int *pixels, int *split);
 int gemmI8SmallLaunch(const GemmI8Problem &problem, int pixels, int split, cudaStream_t stream, bool *taken);
 int smallErrorWord();
 
+// Window variant (gemm_i8_window.cu): stride-1 windows over at most 128 channels from one resident input tile.  Launch sets
+// *taken as the paired variant does.
+bool gemmI8WindowApplies(const GemmI8Problem &problem);
+int gemmI8WindowLaunch(const GemmI8Problem &problem, cudaStream_t stream, bool *taken);
+int windowErrorWord();
+
 // Kernel-selection knobs of the tensor-core launchers (mlel_set_tuning): 0 = the library's own choice.
 struct TensorCoreTuning {
     std::atomic<int> pairKernel{1};        // paired kernel for: 0 nothing, 1 matrix products, 2 convolutions too
     std::atomic<int> smallKernel{1};       // small-problem kernel: 0 never, 1 by its rule, p * 100 + s: forced (32 p pixels, s CTAs)
+    std::atomic<int> windowKernel{1};      // window kernel: 0 never, 1 where it applies
     std::atomic<int> pairTilePixels{0};    // 128, 192 or 256: pixels per tile of the paired kernel
     std::atomic<int> ocTilePixels{0};      // 128, 192 or 256: pixels per tile of the channel-major kernel
     std::atomic<int> ocTileRule{3};        // >= 1: narrow tiles for layers that would leave a quarter of the SMs idle;
@@ -154,10 +161,10 @@ struct TensorCoreTuning {
 };
 TensorCoreTuning &tensorCoreTuning();
 
-// Launches of the four tensor-core kernels since the library was loaded: 0 pixel-major (gemm_i8_tcgen05.cu),
-// 1 channel-major (gemm_i8_ocmajor.cu), 2 paired (gemm_i8_pair.cu), 3 small (gemm_i8_small.cu).  Tests use them to see
-// which kernel took a case.
-extern std::atomic<long long> g_tensorCoreLaunches[4];
+// Launches of the five tensor-core kernels since the library was loaded: 0 pixel-major (gemm_i8_tcgen05.cu),
+// 1 channel-major (gemm_i8_ocmajor.cu), 2 paired (gemm_i8_pair.cu), 3 small (gemm_i8_small.cu), 4 window
+// (gemm_i8_window.cu).  Tests use them to see which kernel took a case.
+extern std::atomic<long long> g_tensorCoreLaunches[5];
 
 // Value of the device-side error word written by a bounded wait that ran out (0 = none).
 int tcgen05ErrorFlag();

@@ -1,0 +1,499 @@
+// int8 convolution windows on the tcgen05 tensor cores from one resident input tile (stride 1, at most 128 input channels).
+//
+// Why.  The im2col kernels fetch every tap of a tile's windows on its own: a 3x3 window moves each input pixel nine times
+// from L2 into shared memory, and with few channels the copies, not the products, take the time: per 128 pixels of a
+// 64-channel layer 9 x 192 rows of 128 bytes for 18 MMAs of some 50 cycles each.  Here a tile's input -- its pixels and
+// the border its windows reach, zero-filled outside the image -- is fetched once, by one TMA box, and every tap's MMA reads
+// it from another start address:
+//
+//   D[pixel, oc] = sum over taps (ky, kx) of X[pixel + ky * pitch + kx, :] * W[tap][oc, :]
+//
+// Pixels lie in shared memory `pitch` to an image row, a pixel's channels in 32, 64 or 128 bytes (the swizzle of that
+// width).  A tensor-core operand is groups of eight consecutive rows a fixed stride apart, so two tile shapes work:
+//   rows   - whole stretches of tileW pixels, the border columns included: operand row r is pixel r of the box (stride
+//            8 pixels), rows that fall on border columns are computed and dropped;
+//   blocks - 8 pixels wide and 16 high: group g is image row g (stride: one pitch).
+// The host takes the shape with the least time by its count of tiles, copied rows and MMAs.
+//
+// The weights of a CTA's output channels (all taps) stay in shared memory for its lifetime; CTAs are persistent and take
+// every (CTAs / channel tiles)-th pixel tile.  Warps 0-15 epilogue, 16 TMA, 17 MMA; accumulators alternate.
+//
+// Measured (3x3, im2col kernels before): 64 x 56 x 56, 64 -> 64 channels 37.2 -> 19.1 us, 32 -> 64 37.8 -> 15.5; 270 x 480,
+// 96 -> 32 32.4 -> 11.9; 64 x 28 x 28, 128 -> 128 15.4 -> 13.8.  Bound now by the epilogue's RESCALEs and, with 128
+// channels, by the MMAs.
+#include <cuda.h>
+#include <cuda_runtime.h>
+
+#include <algorithm>
+#include <cstdint>
+#include <type_traits>
+
+#include "gemm_i8_tcgen05.hpp"
+#include "pixel_epilogue.cuh"
+#include "tcgen05_common.cuh"
+
+namespace mlel {
+namespace {
+
+using namespace tc;
+
+constexpr int kWindowMaxStages = 4;
+constexpr size_t kWindowSmemLimit = 232448; // shared memory per CTA
+
+// Geometry of a launch (see the head of the file).
+struct WindowTiling {
+    int32_t pixelBytes;   // bytes of one pixel in shared memory: 32, 64 or 128
+    int32_t boxW, boxH;   // pixels of the box; boxW is the pitch
+    int32_t tileW, tileH; // output pixels of a tile
+    int32_t blocks;       // 1: 8 x 16 blocks, 0: rows
+    int32_t stages, stageBytes;
+    int32_t tilesX, tilesY, pixelTiles, channelTiles;
+    FastDiv divTilesX, divTilesY, divPitch;
+};
+
+struct __align__(8) WindowBarriers {
+    uint64_t full[kWindowMaxStages], empty[kWindowMaxStages];
+    uint64_t accFull[2], accEmpty[2];
+    uint64_t weights;
+    uint32_t tmemBase, forms;
+};
+
+__device__ __forceinline__ void tmaLoad4d(const CUtensorMap *map, void *dst, uint64_t *bar, int c0, int c1, int c2, int c3) {
+    asm volatile(
+        "cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6}], [%2];"
+        ::"r"(smemAddr(dst)), "l"(reinterpret_cast<uint64_t>(map)), "r"(smemAddr(bar)), "r"(c0), "r"(c1), "r"(c2), "r"(c3)
+        : "memory");
+}
+
+// Descriptor of a K-major operand whose rows are `rowBytes` long in the swizzle of that width.
+__device__ __forceinline__ uint64_t rowDesc(uint32_t addr, uint32_t rowBytes, uint32_t groupBytes) {
+    const uint64_t layout = rowBytes == 128 ? 2 : (rowBytes == 64 ? 4 : 6);
+    return (smemDesc(addr, 16, groupBytes) & ~(uint64_t(7) << 61)) | (layout << 61);
+}
+
+// One MMA by the leading lane of a warp that executes this as a whole (see the MMA warp).  The descriptors come as low words
+// (address; no sum of these carries) and constant high words.
+__device__ __forceinline__ void ummaLed(uint32_t leader, uint32_t tmemD, uint32_t lowA, uint32_t highA, uint32_t lowB, uint32_t highB,
+                                        uint32_t idesc, uint32_t accumulate) {
+    asm volatile("{\n\t.reg .pred p, l;\n\t.reg .b64 a, b;\n\t"
+                 "setp.ne.b32 l, %8, 0;\n\t"
+                 "setp.ne.b32 p, %6, 0;\n\t"
+                 "mov.b64 a, {%1, %2};\n\t"
+                 "mov.b64 b, {%3, %4};\n\t"
+                 "@l tcgen05.mma.cta_group::1.kind::i8 [%0], a, b, %5, {%7, %7, %7, %7}, p;\n\t}"
+                 ::"r"(tmemD), "r"(lowA), "r"(highA), "r"(lowB), "r"(highB), "r"(idesc), "r"(accumulate), "r"(0u), "r"(leader)
+                 : "memory");
+}
+
+// BN: output channels of a tile (32, 64 or 128).
+template <int BN>
+__global__ void __launch_bounds__(kThreadsTma, 1)
+gemmI8Window(const __grid_constant__ CUtensorMap mapX, const __grid_constant__ CUtensorMap mapW, const GemmI8Params p,
+             const WindowTiling g) {
+    extern __shared__ uint8_t rawSmem[];
+    uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(rawSmem) + 1023) & ~uintptr_t(1023));
+    const int taps = p.KH * p.KW, tapBytes = BN * g.pixelBytes;
+    uint8_t *weights = smem;
+    uint8_t *stages = smem + taps * tapBytes;
+    ColConst *colTab = reinterpret_cast<ColConst *>(stages + g.stages * g.stageBytes);
+    WindowBarriers *bars = reinterpret_cast<WindowBarriers *>(colTab + BN);
+
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int c0 = int(blockIdx.x % unsigned(g.channelTiles)) * BN;
+    const int firstTile = int(blockIdx.x / unsigned(g.channelTiles)), tileStep = int(gridDim.x / unsigned(g.channelTiles));
+    // warps that drain one accumulator: four per 16 columns; with 32 columns half of the warps take every other tile
+    constexpr int kSets = BN == 32 ? 2 : 1, kGroups = 4 / kSets, kSteps = BN / 16 / kGroups;
+
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < g.stages; ++s) {
+            mbarInit(&bars->full[s], 1u);
+            mbarInit(&bars->empty[s], 1u);
+        }
+        for (int b = 0; b < 2; ++b) {
+            mbarInit(&bars->accFull[b], 1u);
+            mbarInit(&bars->accEmpty[b], uint32_t(kEpilogueWarps / kSets));
+        }
+        mbarInit(&bars->weights, 1u);
+        bars->forms = 7;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == kMmaWarp) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smemAddr(&bars->tmemBase)),
+                     "r"(uint32_t(2 * BN))
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const uint32_t tmemBase = bars->tmemBase;
+
+    if (warp == kTmaWarp) {
+        if (lane == 0) {
+            // the weights are constants of the pipeline: before the launch ahead has finished
+            mbarArriveExpectTx(&bars->weights, uint32_t(taps * tapBytes));
+            for (int t = 0; t < taps; ++t) {
+                tmaLoad3d(&mapW, weights + t * tapBytes, &bars->weights, 0, t, c0);
+            }
+            gridDependencySync();
+            int s = 0;
+            uint32_t phase = 0;
+            for (int tile = firstTile; tile < g.pixelTiles; tile += tileStep) {
+                const uint32_t ty = fastDiv(uint32_t(tile), g.divTilesX), n = fastDiv(ty, g.divTilesY);
+                const int x0 = (tile - int(ty) * g.tilesX) * g.tileW, y0 = int(ty - n * uint32_t(g.tilesY)) * g.tileH;
+                if (!mbarWait(&bars->empty[s], phase ^ 1u, 91)) {
+                    break;
+                }
+                mbarArriveExpectTx(&bars->full[s], uint32_t(g.boxW * g.boxH * g.pixelBytes));
+                tmaLoad4d(&mapX, stages + s * g.stageBytes, &bars->full[s], 0, x0 - p.padLeft, y0 - p.padTop, int(n));
+                if (++s == g.stages) {
+                    s = 0;
+                    phase ^= 1u;
+                }
+            }
+        }
+        __syncwarp();
+    } else if (warp == kMmaWarp) {
+        // The whole warp runs the loop and one lane issues: with nothing divergent around them the descriptors stay in uniform
+        // registers.  (With the loop inside `if (lane == 0)` every MMA cost the thread some 200 cycles of moves and waits behind
+        // the epilogue warps of its scheduler, 4000 of a 64-channel tile's 4600.)  A wait that runs out only ends the waiting:
+        // the later MMAs read old bytes, the recorded error tells.
+        gridDependencySync();
+        constexpr uint32_t idesc = instrDesc(BN, false);
+        const uint32_t groupBytes = uint32_t((g.blocks ? g.boxW : 8) * g.pixelBytes), leader = lane == 0 ? 1u : 0u;
+        const uint64_t descX = rowDesc(smemAddr(stages), uint32_t(g.pixelBytes), groupBytes);
+        const uint64_t descW = rowDesc(smemAddr(weights), uint32_t(g.pixelBytes), uint32_t(8 * g.pixelBytes));
+        const uint32_t lowX = uint32_t(descX), highX = uint32_t(descX >> 32), lowW = uint32_t(descW), highW = uint32_t(descW >> 32);
+        const uint32_t tapStep = uint32_t(p.dilX * g.pixelBytes) >> 4, rowStep = uint32_t(p.dilY * g.boxW * g.pixelBytes) >> 4,
+                       weightStep = uint32_t(tapBytes) >> 4, stageStep = uint32_t(g.stageBytes) >> 4;
+        const int windowH = p.KH, windowW = p.KW, pixelTiles = g.pixelTiles, stageCount = g.stages;
+        // slices: MMAs per tap, 32 channels each; three: a 3x3 window, unrolled
+        const auto tiles = [&](auto sliceCount, auto three) {
+            constexpr int kSlices = decltype(sliceCount)::value;
+            constexpr bool kThree = decltype(three)::value;
+            bool failed = !mbarWait(&bars->weights, 0u, 92);
+            int s = 0;
+            uint32_t phase = 0, tileCount = 0, stageX = lowX;
+            for (int tile = firstTile; tile < pixelTiles; tile += tileStep, ++tileCount) {
+                const uint32_t buf = tileCount & 1u;
+                failed = failed || !mbarWait(&bars->accEmpty[buf], ((tileCount >> 1) & 1u) ^ 1u, 93) || !mbarWait(&bars->full[s], phase, 94);
+                __syncwarp();
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                const uint32_t tmemD = tmemBase + buf * uint32_t(BN);
+                const auto tap = [&](uint32_t x, uint32_t w, bool first) {
+#pragma unroll
+                    for (int u = 0; u < kSlices; ++u) {
+                        ummaLed(leader, tmemD, x + uint32_t(2 * u), highX, w + uint32_t(2 * u), highW, idesc, first && u == 0 ? 0u : 1u);
+                    }
+                };
+                if (kThree) {
+#pragma unroll
+                    for (int t = 0; t < 9; ++t) {
+                        tap(stageX + uint32_t(t / 3) * rowStep + uint32_t(t % 3) * tapStep, lowW + uint32_t(t) * weightStep, t == 0);
+                    }
+                } else {
+                    uint32_t w = lowW, rowX = stageX;
+                    for (int ky = 0; ky < windowH; ++ky, rowX += rowStep) {
+                        uint32_t x = rowX;
+                        for (int kx = 0; kx < windowW; ++kx, x += tapStep, w += weightStep) {
+                            tap(x, w, ky + kx == 0);
+                        }
+                    }
+                }
+                if (lane == 0) {
+                    ummaCommit(&bars->empty[s]);
+                    ummaCommit(&bars->accFull[buf]);
+                }
+                __syncwarp();
+                stageX += stageStep;
+                if (++s == stageCount) {
+                    s = 0;
+                    stageX = lowX;
+                    phase ^= 1u;
+                }
+            }
+        };
+        const bool three = windowH == 3 && windowW == 3;
+        using Three = std::true_type;
+        using Any = std::false_type;
+        switch ((p.IC + UMMA_K - 1) / UMMA_K) {
+        case 1:
+            three ? tiles(std::integral_constant<int, 1>{}, Three{}) : tiles(std::integral_constant<int, 1>{}, Any{});
+            break;
+        case 2:
+            three ? tiles(std::integral_constant<int, 2>{}, Three{}) : tiles(std::integral_constant<int, 2>{}, Any{});
+            break;
+        case 3:
+            three ? tiles(std::integral_constant<int, 3>{}, Three{}) : tiles(std::integral_constant<int, 3>{}, Any{});
+            break;
+        default:
+            three ? tiles(std::integral_constant<int, 4>{}, Three{}) : tiles(std::integral_constant<int, 4>{}, Any{});
+        }
+    } else {
+        // ---- epilogue: the table of this CTA's channels, then a tile row (pixel) per lane, 16 columns per step
+        const int32_t zpMain = p.epi.main.inZp, outZp = p.epi.main.outZp, lo = p.epi.main.lo, hi = p.epi.main.hi;
+        const bool twoRounds = p.epi.main.doubleRound != 0;
+        FastRescale f{};
+        int32_t corr0 = 0;
+        if (threadIdx.x < BN) {
+            const int col = c0 + int(threadIdx.x), ci = (p.epi.main.perChannel && col < p.N) ? col : 0;
+            f = makeFastRescale(__ldg(p.epi.main.mult + ci), int32_t(__ldg(p.epi.main.shift + ci)), zpMain, twoRounds);
+            const int shift = f.s1 + f.s2;
+            const uint32_t fails = (f.s1 != 32 ? 1u : 0u) | ((shift < 32 || shift > 60) ? 2u : 0u) | (f.mult < 0 ? 4u : 0u);
+            if (fails != 0) {
+                atomicAnd(&bars->forms, ~fails);
+            }
+            corr0 = col < p.N ? __ldg(p.corr + int64_t(p.baseClass) * p.N + col) : 0;
+        }
+        epilogueSync();
+        const uint32_t holds = *const_cast<volatile uint32_t *>(&bars->forms);
+        const bool words32 = (holds & 1u) != 0 && p.corrSmall >= 2 && (holds & 2u) != 0;
+        const bool signFree = !twoRounds || (lo >= outZp && (holds & 4u) != 0);
+        if (threadIdx.x < BN) { // general or 32-bit form: see ColConst
+            ColConst c;
+            c.mult = f.mult, c.s1 = f.s1, c.s2 = f.s2, c.corr0 = corr0;
+            c.bump = f.rpLo - f.rnLo;
+            if (words32) {
+                const int shift = f.s1 + f.s2;
+                c.corr = int32_t((uint32_t(corr0) - uint32_t(f.zpIn)) * 4u);
+                c.rnLo = (1u << ((shift - 31) & 31)) + (twoRounds ? 1u : 0u);
+                c.rnHi = uint32_t(shift - 30);
+            } else {
+                c.corr = corr0, c.rnLo = f.rnLo, c.rnHi = f.rnHi;
+            }
+            colTab[threadIdx.x] = c;
+        }
+        epilogueSync();
+        gridDependencySync();
+
+        const int quarter = warp & 3, part = warp >> 2, set = part / kGroups, group = part - set * kGroups;
+        const int row = quarter * 32 + lane;
+        const int yy = g.blocks ? row >> 3 : int(fastDiv(uint32_t(row), g.divPitch)), xx = g.blocks ? row & 7 : row - yy * g.boxW;
+        const bool rowInTile = yy < g.tileH && xx < g.tileW;
+        const uint32_t tabAddr = smemAddr(colTab);
+        uint32_t tileCount = 0;
+        for (int tile = firstTile; tile < g.pixelTiles; tile += tileStep, ++tileCount) {
+            const uint32_t buf = tileCount & 1u;
+            if (kSets == 2 && int(buf) != set) {
+                continue;
+            }
+            const uint32_t ty = fastDiv(uint32_t(tile), g.divTilesX), n = fastDiv(ty, g.divTilesY);
+            const int x = (tile - int(ty) * g.tilesX) * g.tileW + xx, y = int(ty - n * uint32_t(g.tilesY)) * g.tileH + yy;
+            const bool valid = rowInTile && x < p.OW && y < p.OH;
+            int cls = p.baseClass;
+            if (p.rowClass != nullptr && valid) {
+                cls = int(__ldg(p.rowClass + y)) * p.numColClasses + int(__ldg(p.colClass + x));
+            }
+            int8_t *dst = p.out8 + ((int64_t(n) * p.OH + y) * p.OW + x) * p.ldOut + c0;
+            if (!mbarWait(&bars->accFull[buf], (tileCount >> 1) & 1u, 95)) {
+                break;
+            }
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const uint32_t taddr = tmemBase + buf * uint32_t(BN) + (uint32_t(quarter * 32) << 16);
+#pragma unroll 1
+            for (int st = 0; st < kSteps; ++st) {
+                const int cl = (group * kSteps + st) * 16;
+                uint32_t acc[16];
+                tmemLoad16(taddr + uint32_t(cl), acc);
+                tmemWait16(acc);
+                if (st == kSteps - 1) {
+                    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                    if (lane == 0) {
+                        mbarArrive(&bars->accEmpty[buf]);
+                    }
+                }
+                if (!valid || c0 + cl >= p.N) {
+                    continue;
+                }
+                if (cls != p.baseClass) {
+                    // a pixel whose window crosses the border: swap the table's correction for its own class's
+                    const int4 *own = reinterpret_cast<const int4 *>(p.corr + int64_t(cls) * p.N + c0 + cl);
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) {
+                        const int4 v = __ldg(own + q);
+                        acc[4 * q] += uint32_t(v.x) - uint32_t(colTab[cl + 4 * q].corr0);
+                        acc[4 * q + 1] += uint32_t(v.y) - uint32_t(colTab[cl + 4 * q + 1].corr0);
+                        acc[4 * q + 2] += uint32_t(v.z) - uint32_t(colTab[cl + 4 * q + 2].corr0);
+                        acc[4 * q + 3] += uint32_t(v.w) - uint32_t(colTab[cl + 4 * q + 3].corr0);
+                    }
+                }
+                uint32_t packed[4];
+                const uint32_t tab = tabAddr + uint32_t(cl) * 32u;
+                if (words32) {
+                    if (signFree) {
+                        rescale16Words32<false>(acc, tab, outZp, lo, hi, packed);
+                    } else {
+                        rescale16Words32<true>(acc, tab, outZp, lo, hi, packed);
+                    }
+                } else {
+                    rescale16General(acc, tab, zpMain, outZp, lo, hi, packed);
+                }
+                *reinterpret_cast<int4 *>(dst + cl) = make_int4(int(packed[0]), int(packed[1]), int(packed[2]), int(packed[3]));
+            }
+        }
+    }
+    __syncthreads();
+    if (warp == kMmaWarp) {
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmemBase), "r"(uint32_t(2 * BN)) : "memory");
+    }
+}
+
+// ---- host side --------------------------------------------------------------------------------------------
+
+template <int BN>
+int launchWindow(const CUtensorMap &mapX, const CUtensorMap &mapW, const GemmI8Params &p, const WindowTiling &g, size_t smem,
+                 cudaStream_t s) {
+    auto kernel = gemmI8Window<BN>;
+    if (!allowDynamicSmem(reinterpret_cast<const void *>(kernel), kWindowSmemLimit)) {
+        return MLEL_ERROR_DEVICE;
+    }
+    const int perChannelTile = std::max(1, std::min(smCount() / g.channelTiles, g.pixelTiles));
+    const cudaError_t err = launchDependent(kernel, perChannelTile * g.channelTiles, kThreadsTma, smem, s, mapX, mapW, p, g);
+    if (err != cudaSuccess) {
+        setLastError(std::string("int8 window launch: ") + cudaGetErrorString(err));
+        return MLEL_ERROR_DEVICE;
+    }
+    return MLEL_SUCCESS;
+}
+
+size_t windowSmem(const GemmI8Params &p, const WindowTiling &g, int bn) {
+    return 1024 + size_t(p.KH) * p.KW * bn * g.pixelBytes + size_t(g.stages) * g.stageBytes + size_t(bn) * sizeof(ColConst) +
+           sizeof(WindowBarriers);
+}
+
+// Tiling of p with output tiles of bn channels; false: it does not fit.  *cost: estimated cycles of a CTA (the slowest of
+// MMAs, copies and epilogue per tile, times the tiles of the busiest CTA).
+bool windowTiling(const GemmI8Params &p, int bn, WindowTiling *best, double *cost) {
+    const int reachX = (p.KW - 1) * p.dilX, reachY = (p.KH - 1) * p.dilY, images = p.M / (p.OH * p.OW);
+    bool found = false;
+    const auto consider = [&](bool blocks, int tileW, int tileH) {
+        WindowTiling g{};
+        g.pixelBytes = p.IC <= 32 ? 32 : (p.IC <= 64 ? 64 : 128);
+        g.blocks = blocks ? 1 : 0;
+        g.tileW = tileW, g.tileH = tileH;
+        g.boxW = tileW + reachX, g.boxH = tileH + reachY;
+        if (g.boxW > 256 || g.boxH > 256) {
+            return;
+        }
+        // pixels that the MMAs of the last tap read (rows of the operand past the box hold old bytes; their results are dropped)
+        const int reach = reachY * g.boxW + reachX + (blocks ? 15 * g.boxW + 8 : 128);
+        g.stageBytes = (std::max(reach, g.boxW * g.boxH) * g.pixelBytes + 1023) / 1024 * 1024;
+        g.stages = kWindowMaxStages;
+        while (g.stages > 1 && windowSmem(p, g, bn) > kWindowSmemLimit) {
+            --g.stages;
+        }
+        if (g.stages < 2) {
+            return;
+        }
+        g.tilesX = (p.OW + tileW - 1) / tileW, g.tilesY = (p.OH + tileH - 1) / tileH;
+        const int64_t tiles = int64_t(images) * g.tilesX * g.tilesY;
+        if (tiles >= (int64_t(1) << 30)) {
+            return;
+        }
+        g.pixelTiles = int(tiles);
+        g.channelTiles = (p.N + bn - 1) / bn;
+        const int ctas = smCount() / g.channelTiles;
+        if (ctas < 1) {
+            return;
+        }
+        const double mma = double(p.KH * p.KW) * ((p.IC + 31) / 32) * (32 + bn / 4), copy = double(g.boxW) * g.boxH * g.pixelBytes / 50,
+                     epilogue = 13.0 * std::min(bn, p.N);
+        const double cycles = (std::max(mma, std::max(copy, epilogue)) + 150) * double((g.pixelTiles + ctas - 1) / ctas);
+        if (!found || cycles < *cost) {
+            found = true;
+            *cost = cycles;
+            *best = g;
+        }
+    };
+    consider(true, 8, 16);
+    for (int pieces = 1; pieces <= 16; ++pieces) { // rows: the image row in equal pieces, as many of them as 128 operand rows hold
+        const int tileW = (p.OW + pieces - 1) / pieces;
+        if (tileW > 128) {
+            continue;
+        }
+        const int tileH = std::min(p.OH, (128 - tileW) / (tileW + reachX) + 1);
+        consider(false, tileW, tileH);
+        if (tileW < 16) {
+            break;
+        }
+    }
+    return found;
+}
+
+template <int RANK>
+bool makeWindowMap(CUtensorMap *map, uint64_t kind, const void *base, const cuuint64_t (&dims)[RANK], const cuuint32_t (&box)[RANK]) {
+    EncodeTiledFn fn = encodeTiled();
+    if (fn == nullptr) {
+        return false;
+    }
+    cuuint64_t strides[RANK - 1];
+    cuuint32_t elemStrides[RANK];
+    MapKey key{{kind, reinterpret_cast<uint64_t>(base)}};
+    for (int i = 0; i < RANK; ++i) {
+        if (i + 1 < RANK) {
+            strides[i] = (i == 0 ? 1 : strides[i - 1]) * dims[i];
+        }
+        elemStrides[i] = 1;
+        key.v[2 + i] = dims[i], key.v[8 + i] = box[i];
+    }
+    const CUtensorMapSwizzle swizzle =
+        box[0] == 128 ? CU_TENSOR_MAP_SWIZZLE_128B : (box[0] == 64 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_32B);
+    return rememberedMap(map, key, [&](CUtensorMap *m) {
+        return fn(m, CU_TENSOR_MAP_DATA_TYPE_UINT8, RANK, const_cast<void *>(base), dims, strides, box, elemStrides,
+                  CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+    });
+}
+
+} // namespace
+
+// Stride 1 because the tensor core walks pixels at a constant distance; at most 128 channels because a CTA keeps the weights
+// of all taps (and a pixel is one swizzled row); more than one tap because a 1x1 window is fetched once anyway.
+bool gemmI8WindowApplies(const GemmI8Problem &q) {
+    const GemmI8Params &p = q.params;
+    const int mode = tensorCoreTuning().windowKernel.load(std::memory_order_relaxed);
+    return mode != 0 && p.out8 != nullptr && p.epi.hasMain && !p.epi.hasResidual && q.aMatrix == nullptr && !q.bMnMajor && q.batches == 1 &&
+           p.gatherTable == nullptr && p.strideX == 1 && p.strideY == 1 && p.IC % 16 == 0 && p.IC <= 128 && p.N % 16 == 0 &&
+           p.ldOut % 16 == 0 && p.KH * p.KW > 1 && p.padLeft >= 0 && p.padTop >= 0 &&
+           ((reinterpret_cast<uintptr_t>(p.in) | reinterpret_cast<uintptr_t>(p.out8) | reinterpret_cast<uintptr_t>(q.bMatrix) |
+             reinterpret_cast<uintptr_t>(p.corr)) & 15u) == 0;
+}
+
+int gemmI8WindowLaunch(const GemmI8Problem &q, cudaStream_t s, bool *taken) {
+    GemmI8Params p = q.params;
+    *taken = false;
+    WindowTiling g{};
+    int bn = 0;
+    double cost = 0;
+    for (const int width : {32, 64, 128}) {
+        WindowTiling t{};
+        double c = 0;
+        if ((width == 32 || width < 2 * p.N) && windowTiling(p, width, &t, &c) && (bn == 0 || c < cost)) {
+            bn = width, g = t, cost = c;
+        }
+    }
+    if (bn == 0) {
+        return MLEL_SUCCESS;
+    }
+    const int images = p.M / (p.OH * p.OW);
+    CUtensorMap mapX{}, mapW{};
+    const cuuint64_t xDims[4] = {cuuint64_t(p.IC), cuuint64_t(p.W), cuuint64_t(p.H), cuuint64_t(images)};
+    const cuuint32_t xBox[4] = {cuuint32_t(g.pixelBytes), cuuint32_t(g.boxW), cuuint32_t(g.boxH), 1};
+    const cuuint64_t wDims[3] = {cuuint64_t(p.IC), cuuint64_t(p.KH * p.KW), cuuint64_t(p.N)};
+    const cuuint32_t wBox[3] = {cuuint32_t(g.pixelBytes), 1, cuuint32_t(bn)};
+    if (!makeWindowMap(&mapX, 5, p.in, xDims, xBox) || !makeWindowMap(&mapW, 6, q.bMatrix, wDims, wBox)) {
+        return MLEL_SUCCESS; // another kernel fetches the taps one by one
+    }
+    *taken = true;
+    g_tensorCoreLaunches[4].fetch_add(1, std::memory_order_relaxed);
+    g.divTilesX = makeFastDiv(g.tilesX), g.divTilesY = makeFastDiv(g.tilesY), g.divPitch = makeFastDiv(g.boxW);
+    const size_t smem = windowSmem(p, g, bn);
+    return bn == 32   ? launchWindow<32>(mapX, mapW, p, g, smem, s)
+           : bn == 64 ? launchWindow<64>(mapX, mapW, p, g, smem, s)
+                      : launchWindow<128>(mapX, mapW, p, g, smem, s);
+}
+
+int windowErrorWord() { return readErrorWord(); }
+
+} // namespace mlel

@@ -54,6 +54,16 @@ bool trySmallKernel(const GemmI8Problem &q, cudaStream_t s, int *rc) {
     return taken || *rc != MLEL_SUCCESS;
 }
 
+// The same for the window kernel.
+bool tryWindowKernel(const GemmI8Problem &q, cudaStream_t s, int *rc) {
+    if (!gemmI8WindowApplies(q)) {
+        return false;
+    }
+    bool taken = false;
+    *rc = gemmI8WindowLaunch(q, s, &taken);
+    return taken || *rc != MLEL_SUCCESS;
+}
+
 PoolAttr poolAttr(const OpDesc &op) {
     PoolAttr a{};
     a.kernel[0] = op.i[0], a.kernel[1] = op.i[1], a.stride[0] = op.i[2], a.stride[1] = op.i[3];
@@ -202,7 +212,7 @@ int launchConvTensorCore(const OpDesc &op, const TView *T, cudaStream_t s, Launc
     q.bBatchBytes = 0;
     q.bMnMajor = false;
     int rc = MLEL_SUCCESS;
-    if (tryPairKernel(q, true, s, &rc) || trySmallKernel(q, s, &rc)) {
+    if (tryPairKernel(q, true, s, &rc) || trySmallKernel(q, s, &rc) || tryWindowKernel(q, s, &rc)) {
         return rc;
     }
     return gemmI8OcMajorApplies(q) ? gemmI8OcMajorLaunch(q, s, chain, consumed) : gemmI8Launch(q, s);

@@ -312,7 +312,11 @@ int mlel_measure_int8_mma_peak(int batches, void *cuda_stream, float *ms, double
  *                       128 pixels;
  *   "dependent_launch"  1 (default) launches the tensor-core kernels with programmatic dependent launch;
  *   "small_kernel"      1 (default): fused int8 problems that would leave most SMs idle run on the kernel that splits the
- *                       contraction of narrow tiles over a cluster; 0: never;
+ *                       contraction of narrow tiles over a cluster; 0: never; 100 * p + s: every problem that the kernel can
+ *                       take, in tiles of 32 * p pixels (p 1 or 2) over s CTAs (1, 2, 4 or 8, at most what the contraction
+ *                       length gives);
+ *   "window_kernel"     1 (default): fused int8 convolution windows of stride 1 over at most 128 channels run on the kernel
+ *                       that reads every tap from one resident input tile; 0: never;
  *   "tile_progress"     7 (default): a convolution whose input the convolution before it wrote starts on that launch's
  *                       finished pixel tiles; bit 0 read by tiles, bit 1 publish, bit 2 channel tiles first; 0 off.
  * Another key or value: MLEL_ERROR_UNKNOWN. */

@@ -1,0 +1,43 @@
+"""GPU parity of the window kernel: both tile shapes, image sizes at and beside their edges, every pixel width (32, 64 and
+128 bytes, whole and padded), one to several channel tiles, windows of other sizes and dilations, border classes, shifts
+on both sides of 32.  Bit-exact against the CPU oracle; a counter tells that the kernel took the case."""
+import ctypes
+
+import numpy as np
+import pytest
+
+from mlel_b200.graph_builder import GraphBuilder
+from tests.graph_eval import evaluate
+from tests.test_gpu_small import conv
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("n,h,w,ic,oc,k,pad,dil,shift", [
+    (2, 56, 56, 64, 64, 3, 1, 1, 37), (1, 16, 8, 128, 128, 3, 1, 1, 38), (3, 28, 28, 128, 128, 3, 1, 1, 38), (1, 45, 131, 96, 32, 3, 1, 1, 37),
+    (1, 17, 9, 64, 64, 3, 1, 1, 37), (2, 40, 130, 32, 48, 3, 0, 1, 35), (1, 33, 257, 16, 16, 3, 1, 1, 34), (2, 23, 61, 48, 160, 3, 1, 1, 37),
+    (1, 64, 70, 80, 96, 3, 1, 2, 37), (1, 30, 41, 32, 32, 5, 2, 1, 36), (2, 20, 120, 112, 16, 2, 0, 1, 30), (1, 50, 50, 16, 64, 7, 3, 1, 36),
+    (5, 14, 14, 64, 256, 3, 1, 1, 29), (1, 3, 400, 32, 64, 3, 1, 1, 36), (1, 300, 2, 64, 16, 3, 1, 1, 36),
+])
+def test_windows(mlel, n, h, w, ic, oc, k, pad, dil, shift):
+    from mlel_b200.runtime import GraphRunner
+    r = np.random.Generator(np.random.PCG64(h * 1000 + w))
+    g = GraphBuilder()
+    x = g.input(np.int8, (n, h, w, ic))
+    g.output(conv(g, r, x, oc, k, 1, pad, -7, False, shift, dil))
+    g.output(conv(g, r, x, oc, k, 1, pad, 5, True, shift, dil))
+    data = r.integers(-128, 128, x.shape, dtype=np.int8)
+    want = evaluate(g, [data])
+    lib = mlel.lib()
+    lib.mlel_tensor_core_launches.restype = ctypes.c_longlong
+    try:
+        assert lib.mlel_set_tuning(b"small_kernel", 0) == 0
+        before = lib.mlel_tensor_core_launches(4)
+        runner = GraphRunner(g)
+        for use_cuda_graph in (False, True):
+            for a, b in zip(runner.run([data], use_cuda_graph=use_cuda_graph), want):
+                bad = np.argwhere(a != b)
+                assert len(bad) == 0, (len(bad), a.size, bad[0].tolist(), bad[-1].tolist())
+        assert lib.mlel_tensor_core_launches(4) > before
+    finally:
+        assert lib.mlel_set_tuning(b"small_kernel", 1) == 0
