@@ -215,51 +215,47 @@ gemmI8OcMajor(const __grid_constant__ CUtensorMap tmapX, const __grid_constant__
             }
         }
     } else if (warp == kOcMmaWarp) {
-        // ---------------- MMA issuer ----------------
-        if (lane == 0) {
-            constexpr uint32_t idesc = instrDesc(BNP, false);
-            static_assert(BK / UMMA_K == 4, "ummaBlockPeek issues the four MMAs of a K block");
-            const uint64_t descW0 = smemDesc(smemAddr(tilesW), 16, 1024), descX0 = smemDesc(smemAddr(tilesX), 16, 1024);
-            uint32_t it = 0, tileCount = 0;
-            uint32_t ready = 0; // 1: the stage of the coming K block is known to be full (see ummaBlockPeek)
-            int s = 0;
-            uint32_t phase = 0;
-            bool ok = true;
-            for (int64_t t = blockIdx.x; t < numTiles && ok; t += gridDim.x, ++tileCount) {
-                const uint32_t buf = tileCount & 1u;
-                ok = mbarWait(&bars->accEmpty[buf], ((tileCount >> 1) & 1u) ^ 1u, 15);
-                if (!ok) {
-                    break;
+        // ---------------- MMA issuer (the whole warp: see ummaBlockPeek) ----------------
+        constexpr uint32_t idesc = instrDesc(BNP, false);
+        static_assert(BK / UMMA_K == 4, "ummaBlockPeek issues the four MMAs of a K block");
+        const uint32_t leader = lane == 0 ? 1u : 0u;
+        const DescWords descW0 = descWords(smemDesc(smemAddr(tilesW), 16, 1024)), descX0 = descWords(smemDesc(smemAddr(tilesX), 16, 1024));
+        uint32_t tileCount = 0;
+        uint32_t ready = 0; // 1: the stage of the coming K block is known to be full (see ummaBlockPeek)
+        int s = 0;
+        uint32_t phase = 0;
+        bool failed = false; // a wait ran out: no more waits, the later MMAs read old bytes, the recorded error tells
+        for (int64_t t = blockIdx.x; t < numTiles; t += gridDim.x, ++tileCount) {
+            const uint32_t buf = tileCount & 1u;
+            failed = failed || !mbarWait(&bars->accEmpty[buf], ((tileCount >> 1) & 1u) ^ 1u, 15);
+            __syncwarp();
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const uint32_t tmemD = tmemBase + buf * uint32_t(BNP);
+            int kLeft = X_MODE == kXIm2col ? p.IC : p.K;
+            for (int kb = 0; kb < numKb; ++kb) {
+                if (ready == 0) {
+                    failed = failed || !mbarWait(&bars->full[s], phase, 12);
                 }
+                __syncwarp();
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const uint32_t tmemD = tmemBase + buf * uint32_t(BNP);
-                int kLeft = X_MODE == kXIm2col ? p.IC : p.K;
-                for (int kb = 0; kb < numKb; ++kb, ++it) {
-                    if (ready == 0) {
-                        ok = mbarWait(&bars->full[s], phase, 12);
-                        if (!ok) {
-                            break;
-                        }
-                    }
-                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                    // the ring runs on across tiles: the next K block's stage follows this one whatever tile it is in
-                    const int sNext = s + 1 == NSTAGE ? 0 : s + 1;
-                    const uint32_t phaseNext = sNext == 0 ? phase ^ 1u : phase;
-                    ready = ummaBlockPeek(tmemD, descW0 + uint64_t(uint32_t(s) * uint32_t(kTileW >> 4)), 2,
-                                          descX0 + uint64_t(uint32_t(s) * uint32_t(kTileX >> 4)), 2, idesc, kb != 0 ? 1u : 0u,
-                                          ummaCountFor(kLeft), &bars->empty[s], &bars->full[sNext], phaseNext);
-                    // bytes of K in the next block: the rest of the tap's channels (im2col) or of the whole K axis
-                    kLeft -= BK;
-                    if (kLeft <= 0) {
-                        kLeft = X_MODE == kXIm2col ? p.IC : 0;
-                    }
-                    s = sNext;
-                    phase = phaseNext;
+                // the ring runs on across tiles: the next K block's stage follows this one whatever tile it is in
+                const int sNext = s + 1 == NSTAGE ? 0 : s + 1;
+                const uint32_t phaseNext = sNext == 0 ? phase ^ 1u : phase;
+                ready = ummaBlockPeek(leader, tmemD, {descW0.low + uint32_t(s) * uint32_t(kTileW >> 4), descW0.high}, 2,
+                                      {descX0.low + uint32_t(s) * uint32_t(kTileX >> 4), descX0.high}, 2, idesc, kb != 0 ? 1u : 0u,
+                                      ummaCountFor(kLeft), &bars->empty[s], &bars->full[sNext], phaseNext);
+                // bytes of K in the next block: the rest of the tap's channels (im2col) or of the whole K axis
+                kLeft -= BK;
+                if (kLeft <= 0) {
+                    kLeft = X_MODE == kXIm2col ? p.IC : 0;
                 }
-                if (ok) {
-                    ummaCommit(&bars->accFull[buf]);
-                }
+                s = sNext;
+                phase = phaseNext;
             }
+            if (lane == 0) {
+                ummaCommit(&bars->accFull[buf]);
+            }
+            __syncwarp();
         }
     } else if (warp >= kOcGatherWarp0) {
         if (X_TMA) {

@@ -650,54 +650,50 @@ gemmI8Tcgen05(const __grid_constant__ CUtensorMap tmapA, const __grid_constant__
             }
         }
     } else if (warp == kMmaWarp) {
-        // ---------------- MMA issuer ----------------
-        if (lane == 0) {
-            constexpr uint32_t idesc = instrDesc(BN, B_MN);
-            static_assert(BK / UMMA_K == 4, "ummaBlockPeek issues the four MMAs of a K block");
-            // K-major: step 32 bytes inside the 128-byte swizzle row; MN-major: step 32 K-rows of 128 bytes
-            const uint64_t descA0 = smemDesc(smemAddr(tilesA), 16, 1024);
-            const uint64_t descB0 = B_MN ? smemDesc(smemAddr(tilesB), BK * 128, 1024) : smemDesc(smemAddr(tilesB), 16, 1024);
-            constexpr uint64_t kStepB = B_MN ? uint64_t(UMMA_K * 128) >> 4 : 2;
-            uint32_t tileCount = 0;
-            uint32_t ready = 0; // 1: the stage of the coming K block is known to be full (see ummaBlockPeek)
-            int s = 0;
-            uint32_t phase = 0;
-            bool ok = true;
-            for (int64_t t = blockIdx.x; t < numTiles && ok; t += gridDim.x, ++tileCount) {
-                const uint32_t buf = tileCount & 1u;
-                // wait until the epilogue has drained this accumulator (passes at once for the first two tiles)
-                ok = mbarWait(&bars->accEmpty[buf], ((tileCount >> 1) & 1u) ^ 1u, 5);
-                if (!ok) {
-                    break;
+        // ---------------- MMA issuer (the whole warp: see ummaBlockPeek) ----------------
+        constexpr uint32_t idesc = instrDesc(BN, B_MN);
+        static_assert(BK / UMMA_K == 4, "ummaBlockPeek issues the four MMAs of a K block");
+        const uint32_t leader = lane == 0 ? 1u : 0u;
+        // K-major: step 32 bytes inside the 128-byte swizzle row; MN-major: step 32 K-rows of 128 bytes
+        const DescWords descA0 = descWords(smemDesc(smemAddr(tilesA), 16, 1024));
+        const DescWords descB0 = descWords(B_MN ? smemDesc(smemAddr(tilesB), BK * 128, 1024) : smemDesc(smemAddr(tilesB), 16, 1024));
+        constexpr uint32_t kStepB = B_MN ? uint32_t(UMMA_K * 128) >> 4 : 2;
+        uint32_t tileCount = 0;
+        uint32_t ready = 0; // 1: the stage of the coming K block is known to be full (see ummaBlockPeek)
+        int s = 0;
+        uint32_t phase = 0;
+        bool failed = false; // a wait ran out: no more waits, the later MMAs read old bytes, the recorded error tells
+        for (int64_t t = blockIdx.x; t < numTiles; t += gridDim.x, ++tileCount) {
+            const uint32_t buf = tileCount & 1u;
+            // wait until the epilogue has drained this accumulator (passes at once for the first two tiles)
+            failed = failed || !mbarWait(&bars->accEmpty[buf], ((tileCount >> 1) & 1u) ^ 1u, 5);
+            __syncwarp();
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const uint32_t tmemD = tmemBase + buf * uint32_t(BN);
+            int kLeft = A_MODE == kAIm2col ? p.IC : p.K; // bytes of K in the coming block's tap or K axis
+            for (int kb = 0; kb < numKb; ++kb) {
+                if (ready == 0) {
+                    failed = failed || !mbarWait(&bars->full[s], phase, 2);
                 }
+                __syncwarp();
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const uint32_t tmemD = tmemBase + buf * uint32_t(BN);
-                int kLeft = A_MODE == kAIm2col ? p.IC : p.K; // bytes of K in the coming block's tap or K axis
-                for (int kb = 0; kb < numKb; ++kb) {
-                    if (ready == 0) {
-                        ok = mbarWait(&bars->full[s], phase, 2);
-                        if (!ok) {
-                            break;
-                        }
-                    }
-                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                    // the ring runs on across tiles: the next K block's stage follows this one whatever tile it is in
-                    const int sNext = s + 1 == NSTAGE ? 0 : s + 1;
-                    const uint32_t phaseNext = sNext == 0 ? phase ^ 1u : phase;
-                    ready = ummaBlockPeek(tmemD, descA0 + uint64_t(uint32_t(s) * uint32_t(kTileA >> 4)), 2,
-                                          descB0 + uint64_t(uint32_t(s) * uint32_t(kTileB >> 4)), kStepB, idesc,
-                                          kb != 0 ? 1u : 0u, ummaCountFor(kLeft), &bars->empty[s], &bars->full[sNext], phaseNext);
-                    kLeft -= BK;
-                    if (kLeft <= 0) {
-                        kLeft = A_MODE == kAIm2col ? p.IC : 0;
-                    }
-                    s = sNext;
-                    phase = phaseNext;
+                // the ring runs on across tiles: the next K block's stage follows this one whatever tile it is in
+                const int sNext = s + 1 == NSTAGE ? 0 : s + 1;
+                const uint32_t phaseNext = sNext == 0 ? phase ^ 1u : phase;
+                ready = ummaBlockPeek(leader, tmemD, {descA0.low + uint32_t(s) * uint32_t(kTileA >> 4), descA0.high}, 2,
+                                      {descB0.low + uint32_t(s) * uint32_t(kTileB >> 4), descB0.high}, kStepB, idesc,
+                                      kb != 0 ? 1u : 0u, ummaCountFor(kLeft), &bars->empty[s], &bars->full[sNext], phaseNext);
+                kLeft -= BK;
+                if (kLeft <= 0) {
+                    kLeft = A_MODE == kAIm2col ? p.IC : 0;
                 }
-                if (ok) {
-                    ummaCommit(&bars->accFull[buf]);
-                }
+                s = sNext;
+                phase = phaseNext;
             }
+            if (lane == 0) {
+                ummaCommit(&bars->accFull[buf]);
+            }
+            __syncwarp();
         }
     } else if (warp >= kGatherWarp0) {
         // ---------------- A gather (implicit GEMM): one tile row per thread ----------------

@@ -197,36 +197,48 @@ __device__ __forceinline__ void ummaCommit(uint64_t *bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smemAddr(bar))
                  : "memory");
 }
+// The warp that issues MMAs runs its loops as a whole, one lane (`leader`) issues: with nothing divergent around them the
+// operands of tcgen05.mma stay in uniform registers.  From inside `if (lane == 0)` every MMA took the thread a dozen moves
+// and waits behind the epilogue warps that share its scheduler (3x3 windows over 64 channels: some 200 cycles per MMA that
+// the pipe does in 50).  Descriptors are given as low words (address; no sum of these carries) and constant high words.
+//
 // One 128-byte K block: up to four MMAs of 32 bytes of K each (`count` of them: the tail of a K block that only
 // holds zero fill is skipped; descriptors advance by stepA / stepB units of 16 bytes, 2 for a K-major SWIZZLE_128B
 // tile), the commit that hands the stage back, and -- issued AHEAD of them -- a non-blocking test of the barrier the
 // next K block will wait for.  Why in one statement: an mbarrier test issued after MMAs and a commit takes about 185
-// cycles to answer even when the phase has long completed (it queues behind them), and the thread that needs the
-// answer stalls for it; measured on a loop of this shape, 626 cycles per K block whatever N is, against 384 for the
-// four MMAs of N = 192 alone.  Asked before the MMAs are issued, the answer arrives while they and the commit go out
-// (463 cycles per K block; 513 = the pipe's own time at N = 256).  Returns 1 when the next barrier's phase
-// `peekParity` is complete; 0 means "not yet known": wait for it in the ordinary way.
-__device__ __forceinline__ uint32_t ummaBlockPeek(uint32_t tmemD, uint64_t descA, uint64_t stepA, uint64_t descB,
-                                                  uint64_t stepB, uint32_t idesc, uint32_t accumulateFirst, int count,
+// cycles to answer even when the phase has long completed (it queues behind them), and the warp that needs the
+// answer stalls for it.  Returns 1 when the next barrier's phase `peekParity` is complete; 0 means "not yet known":
+// wait for it in the ordinary way.
+struct DescWords {
+    uint32_t low, high;
+};
+__device__ __forceinline__ DescWords descWords(uint64_t d) { return {uint32_t(d), uint32_t(d >> 32)}; }
+__device__ __forceinline__ uint32_t ummaBlockPeek(uint32_t leader, uint32_t tmemD, DescWords a, uint32_t stepA, DescWords b,
+                                                  uint32_t stepB, uint32_t idesc, uint32_t accumulateFirst, int count,
                                                   uint64_t *commitBar, uint64_t *peekBar, uint32_t peekParity) {
     uint32_t ready;
-    asm volatile("{\n\t.reg .pred q, a0, a1, g1, g2, g3;\n\t"
+    asm volatile("{\n\t.reg .pred q, l, a0, a1, g1, g2, g3;\n\t"
+                 ".reg .b32 la, lb;\n\t.reg .b64 da, db;\n\t"
                  "mbarrier.test_wait.parity.shared::cta.b64 q, [%1], %2;\n\t"
+                 "setp.ne.b32 l, %15, 0;\n\t"
                  "setp.ne.b32 a0, %9, 0;\n\t"
-                 "setp.ne.b32 a1, %10, 0;\n\t"
-                 "setp.gt.s32 g1, %17, 1;\n\t"
-                 "setp.gt.s32 g2, %17, 2;\n\t"
-                 "setp.gt.s32 g3, %17, 3;\n\t"
-                 "tcgen05.mma.cta_group::1.kind::i8 [%3], %4, %5, %8, {%11, %11, %11, %11}, a0;\n\t"
-                 "@g1 tcgen05.mma.cta_group::1.kind::i8 [%3], %6, %7, %8, {%11, %11, %11, %11}, a1;\n\t"
-                 "@g2 tcgen05.mma.cta_group::1.kind::i8 [%3], %12, %13, %8, {%11, %11, %11, %11}, a1;\n\t"
-                 "@g3 tcgen05.mma.cta_group::1.kind::i8 [%3], %14, %15, %8, {%11, %11, %11, %11}, a1;\n\t"
-                 "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%16];\n\t"
+                 "setp.ne.b32 a1, %15, %10;\n\t"
+                 "setp.gt.and.s32 g1, %11, 1, l;\n\t"
+                 "setp.gt.and.s32 g2, %11, 2, l;\n\t"
+                 "setp.gt.and.s32 g3, %11, 3, l;\n\t"
+                 "mov.b64 da, {%4, %5};\n\tmov.b64 db, {%6, %7};\n\t"
+                 "@l tcgen05.mma.cta_group::1.kind::i8 [%3], da, db, %8, {%10, %10, %10, %10}, a0;\n\t"
+                 "add.u32 la, %4, %13;\n\tadd.u32 lb, %6, %14;\n\tmov.b64 da, {la, %5};\n\tmov.b64 db, {lb, %7};\n\t"
+                 "@g1 tcgen05.mma.cta_group::1.kind::i8 [%3], da, db, %8, {%10, %10, %10, %10}, a1;\n\t"
+                 "add.u32 la, la, %13;\n\tadd.u32 lb, lb, %14;\n\tmov.b64 da, {la, %5};\n\tmov.b64 db, {lb, %7};\n\t"
+                 "@g2 tcgen05.mma.cta_group::1.kind::i8 [%3], da, db, %8, {%10, %10, %10, %10}, a1;\n\t"
+                 "add.u32 la, la, %13;\n\tadd.u32 lb, lb, %14;\n\tmov.b64 da, {la, %5};\n\tmov.b64 db, {lb, %7};\n\t"
+                 "@g3 tcgen05.mma.cta_group::1.kind::i8 [%3], da, db, %8, {%10, %10, %10, %10}, a1;\n\t"
+                 "@l tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%12];\n\t"
                  "selp.u32 %0, 1, 0, q;\n\t}"
                  : "=r"(ready)
-                 : "r"(smemAddr(peekBar)), "r"(peekParity), "r"(tmemD), "l"(descA), "l"(descB), "l"(descA + stepA),
-                   "l"(descB + stepB), "r"(idesc), "r"(accumulateFirst), "r"(1u), "r"(0u), "l"(descA + 2 * stepA),
-                   "l"(descB + 2 * stepB), "l"(descA + 3 * stepA), "l"(descB + 3 * stepB), "r"(smemAddr(commitBar)), "r"(count)
+                 : "r"(smemAddr(peekBar)), "r"(peekParity), "r"(tmemD), "r"(a.low), "r"(a.high), "r"(b.low), "r"(b.high), "r"(idesc),
+                   "r"(accumulateFirst), "r"(0u), "r"(count), "r"(smemAddr(commitBar)), "r"(stepA), "r"(stepB), "r"(leader)
                  : "memory");
     return ready;
 }
