@@ -1940,6 +1940,34 @@ void GraphPipeline::prepareTensorCore() {
             if (!padChannels && op.kind == OP_FUSED_CONV2D && op.epi.hasResidual) {
                 buildResidualTable(op);
             }
+            // At most four channels, stride 1 or 2 (an RGB stem, tc == 4): the input is copied into 16-byte units of four
+            // pixels, of which a window is a whole number, and runs on the window kernel.  Up to sixteen units (7x7 at
+            // stride 2) and whole 16-byte rows of output; other windows take the table gather below.
+            {
+                const int64_t perUnitX = sx == 1 ? 4 : 2, perUnitY = sx == 1 ? 1 : 2;
+                const int64_t unitsX = (KW + perUnitX - 1) / perUnitX, unitRows = (KH + perUnitY - 1) / perUnitY;
+                const int64_t units = (unitsX * unitRows + 1) / 2 * 2;
+                const int64_t remX = sx == 1 ? padLeft : padLeft & 1, remY = sx == 1 ? 0 : padTop & 1;
+                const int64_t Wu = sx == 1 ? W + padLeft : (W + remX + 1) / 2, Hu = sx == 1 ? H : (H + remY + 1) / 2;
+                if (IC <= 4 && sx == sy && sx <= 2 && dx == 1 && dy == 1 && padLeft >= 0 && padTop >= 0 && units <= 16 && OC % 16 == 0 &&
+                    OC <= 4096 && op.kind == OP_FUSED_CONV2D && op.epi.hasMain && !op.epi.hasResidual &&
+                    in.dims[0] * Hu * Wu < (int64_t(1) << 27)) {
+                    std::vector<int8_t> wUnits(size_t(units * OC * 16), 0);
+                    for (int64_t oc = 0; oc < OC; ++oc) {
+                        for (int64_t ky = 0; ky < KH; ++ky) {
+                            for (int64_t kx = 0; kx < KW; ++kx) {
+                                const int64_t unit = ky / perUnitY * unitsX + kx / perUnitX;
+                                const int64_t pixel = ky % perUnitY * perUnitX + kx % perUnitX;
+                                std::memcpy(&wUnits[size_t((unit * OC + oc) * 16 + pixel * 4)], wd + ((oc * KH + ky) * KW + kx) * IC, size_t(IC));
+                            }
+                        }
+                    }
+                    op.aux[3] = addDerivedConstant(MLEL_I8, {units, OC, 16}, wUnits.data());
+                    op.scratch = addScratchTensor(MLEL_I8, {in.dims[0], Hu, Wu, 16});
+                    op.tc = 4;
+                    continue;
+                }
+            }
             if (padChannels) {
                 // geometry of the padded copy: rows and columns that any window can touch
                 const int64_t Hp = std::max<int64_t>(H + padTop, (OH - 1) * sy + (KH - 1) * dy + 1);

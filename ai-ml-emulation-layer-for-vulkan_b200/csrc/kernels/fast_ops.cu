@@ -4,6 +4,7 @@
 
 #include "device_common.cuh"
 #include "gemm_i8_tcgen05.hpp"
+#include "launch_overlapped.cuh"
 #include "kernels.hpp"
 
 namespace mlel {
@@ -77,6 +78,34 @@ __global__ void __launch_bounds__(256) padPixels16Kernel(const int8_t *__restric
             from = (int64_t(n) * H + y) * W + x;
         }
         out[e] = live ? loadRagged16(in + from * C + c0, min(16, C - c0)) : make_int4(0, 0, 0, 0);
+    }
+}
+
+// ---- 16-byte units of four pixels for windows over at most four channels (gemm_i8_window.cu) --------------------
+// Unit (y, x) of [N][Hu][Wu]: at stride 1 the pixels x - padLeft + 0..3 of row y, at stride 2 the pixels 2 x - padLeft + {0, 1}
+// of the rows 2 y - padTop + {0, 1} (there padLeft and padTop are the paddings' remainders); four channels each, the
+// missing ones and pixels outside the image zero.  Reads whole aligned words that hold a byte of the pixel.
+template <int STRIDE>
+__global__ void __launch_bounds__(256) gatherUnitsKernel(const int8_t *__restrict__ in, int4 *__restrict__ out, uint32_t units, int H,
+                                                         int W, int C, FastDiv divWu, FastDiv divHu, int padTop, int padLeft) {
+    dependencySync();
+    const auto div = [](uint32_t v, const FastDiv &f) { return f.mul == 0u ? v : __umulhi(v, f.mul) >> f.shift; };
+    const uint32_t mask = C == 4 ? 0xffffffffu : (1u << (8 * C)) - 1u;
+    const uint32_t *words = reinterpret_cast<const uint32_t *>(in);
+    for (uint32_t e = blockIdx.x * blockDim.x + threadIdx.x; e < units; e += gridDim.x * blockDim.x) {
+        const uint32_t line = div(e, divWu), n = div(line, divHu);
+        const int x0 = int(e - line * divWu.d) * STRIDE - padLeft, y0 = int(line - n * divHu.d) * STRIDE - padTop;
+        uint32_t px[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const int x = x0 + (STRIDE == 1 ? k : k & 1), y = y0 + (STRIDE == 1 ? 0 : k >> 1);
+            px[k] = 0;
+            if (unsigned(x) < unsigned(W) && unsigned(y) < unsigned(H)) {
+                const int64_t at = ((int64_t(n) * H + y) * W + x) * C;
+                px[k] = __funnelshift_r(__ldg(words + (at >> 2)), __ldg(words + ((at + C - 1) >> 2)), 8 * (uint32_t(at) & 3u)) & mask;
+            }
+        }
+        out[e] = make_int4(int(px[0]), int(px[1]), int(px[2]), int(px[3]));
     }
 }
 
@@ -591,6 +620,14 @@ int padImageI8(const int8_t *in, int8_t *out, int N, int H, int W, int C, int Hp
     const int64_t words = int64_t(N) * Hp * Wp * (Cp >> 2);
     padImageKernel<<<gridFor(words, kThreads, 8), kThreads, 0, s>>>(in, out, words, H, W, C, Hp, Wp, Cp, padTop, padLeft);
     return finish("padded copy");
+}
+
+int gatherUnitsI8(const int8_t *in, void *out, int N, int H, int W, int C, int Hu, int Wu, int stride, int padTop, int padLeft,
+                  cudaStream_t s) {
+    const int64_t units = int64_t(N) * Hu * Wu;
+    launchOverlapped(stride == 1 ? gatherUnitsKernel<1> : gatherUnitsKernel<2>, dim3(gridFor(units, 256, 8)), 256, 0, s, in,
+                     reinterpret_cast<int4 *>(out), uint32_t(units), H, W, C, makeFastDiv(Wu), makeFastDiv(Hu), padTop, padLeft);
+    return finish("units of four pixels");
 }
 
 int transposeForMatmul(const int8_t *b, int8_t *bt, int32_t *corr, int batches, int C, int W, int32_t za, cudaStream_t s) {

@@ -145,6 +145,16 @@ int smallErrorWord();
 // *taken as the paired variant does.
 bool gemmI8WindowApplies(const GemmI8Problem &problem);
 int gemmI8WindowLaunch(const GemmI8Problem &problem, cudaStream_t stream, bool *taken);
+// The same kernel over 16-byte units of an input of at most four channels (see gatherUnitsI8); q.bMatrix: weights
+// [units of a window, rounded up to even][N][16], zero where a unit's pixels lie outside the window.
+struct UnitWindow {
+    const void *units;        // [images][height][width][16]
+    int32_t width, height;
+    int32_t unitsX, unitRows; // units of a window: per row, rows
+    int32_t unitStep;         // distance of a row's units
+    int32_t originX, originY; // a window's first unit minus the output pixel's own position
+};
+int gemmI8UnitsLaunch(const GemmI8Problem &q, const UnitWindow &u, cudaStream_t stream);
 int windowErrorWord();
 
 // Kernel-selection knobs of the tensor-core launchers (mlel_set_tuning): 0 = the library's own choice.

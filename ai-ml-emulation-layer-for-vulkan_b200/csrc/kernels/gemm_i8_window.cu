@@ -15,6 +15,12 @@
 //   blocks - 8 pixels wide and 16 high: group g is image row g (stride: one pitch).
 // The host takes the shape with the least time by its count of tiles, copied rows and MMAs.
 //
+// Few channels (an RGB stem; stride 1 or 2).  A pixel of at most four channels is too small for an operand row (16 bytes at
+// least).  A copy of the input gathers 16-byte units first -- four pixels of four (zero-padded) channels: at stride 1 the
+// pixels x to x + 3 of a row, at stride 2 the 2 x 2 pixels under one output pixel -- so that an output pixel's window is
+// whole units at constant distances and output pixels are one unit apart.  Rows of 16 bytes need no swizzle; an MMA takes
+// two units per row, the second at its own distance (the descriptor's leading offset).  The loops are the same.
+//
 // The weights of a CTA's output channels (all taps) stay in shared memory for its lifetime; CTAs are persistent and take
 // every (CTAs / channel tiles)-th pixel tile.  Warps 0-15 epilogue, 16 TMA, 17 MMA; accumulators alternate.
 //
@@ -38,16 +44,20 @@ namespace {
 using namespace tc;
 
 constexpr int kWindowMaxStages = 4;
+constexpr int kMaxUnitPairs = 8; // 32 bytes of window each: 7x7 at stride 2 has sixteen units, at stride 1 fourteen
 constexpr size_t kWindowSmemLimit = 232448; // shared memory per CTA
 
 // Geometry of a launch (see the head of the file).
 struct WindowTiling {
-    int32_t pixelBytes;   // bytes of one pixel in shared memory: 32, 64 or 128
+    int32_t pixelBytes;   // bytes of one pixel in shared memory: 32, 64 or 128; of one unit: 16
     int32_t boxW, boxH;   // pixels of the box; boxW is the pitch
     int32_t tileW, tileH; // output pixels of a tile
     int32_t blocks;       // 1: 8 x 16 blocks, 0: rows
     int32_t stages, stageBytes;
     int32_t tilesX, tilesY, pixelTiles, channelTiles;
+    int32_t originX, originY; // a window's first pixel (unit) minus the output pixel's own position
+    int32_t weightBytes;      // of one channel tile
+    int32_t unitsX, unitStep, unitPairs; // units: per window row, distance in a row, pairs of a window
     FastDiv divTilesX, divTilesY, divPitch;
 };
 
@@ -71,6 +81,11 @@ __device__ __forceinline__ uint64_t rowDesc(uint32_t addr, uint32_t rowBytes, ui
     return (smemDesc(addr, 16, groupBytes) & ~(uint64_t(7) << 61)) | (layout << 61);
 }
 
+// Descriptor of a K-major operand without a swizzle: groups of eight 16-byte rows.
+__device__ __forceinline__ uint64_t smemDescPlain(uint32_t addr, uint32_t leadingBytes, uint32_t groupBytes) {
+    return smemDesc(addr, leadingBytes, groupBytes) & ~(uint64_t(7) << 61);
+}
+
 // One MMA by the leading lane of a warp that executes this as a whole (see the MMA warp).  The descriptors come as low words
 // (address; no sum of these carries) and constant high words.
 __device__ __forceinline__ void ummaLed(uint32_t leader, uint32_t tmemD, uint32_t lowA, uint32_t highA, uint32_t lowB, uint32_t highB,
@@ -85,8 +100,8 @@ __device__ __forceinline__ void ummaLed(uint32_t leader, uint32_t tmemD, uint32_
                  : "memory");
 }
 
-// BN: output channels of a tile (32, 64 or 128).
-template <int BN>
+// BN: output channels of a tile (32, 64 or 128).  UNITS: the input is 16-byte units (see the head of the file).
+template <int BN, bool UNITS>
 __global__ void __launch_bounds__(kThreadsTma, 1)
 gemmI8Window(const __grid_constant__ CUtensorMap mapX, const __grid_constant__ CUtensorMap mapW, const GemmI8Params p,
              const WindowTiling g) {
@@ -94,7 +109,7 @@ gemmI8Window(const __grid_constant__ CUtensorMap mapX, const __grid_constant__ C
     uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(rawSmem) + 1023) & ~uintptr_t(1023));
     const int taps = p.KH * p.KW, tapBytes = BN * g.pixelBytes;
     uint8_t *weights = smem;
-    uint8_t *stages = smem + taps * tapBytes;
+    uint8_t *stages = smem + g.weightBytes;
     ColConst *colTab = reinterpret_cast<ColConst *>(stages + g.stages * g.stageBytes);
     WindowBarriers *bars = reinterpret_cast<WindowBarriers *>(colTab + BN);
 
@@ -131,9 +146,13 @@ gemmI8Window(const __grid_constant__ CUtensorMap mapX, const __grid_constant__ C
     if (warp == kTmaWarp) {
         if (lane == 0) {
             // the weights are constants of the pipeline: before the launch ahead has finished
-            mbarArriveExpectTx(&bars->weights, uint32_t(taps * tapBytes));
-            for (int t = 0; t < taps; ++t) {
-                tmaLoad3d(&mapW, weights + t * tapBytes, &bars->weights, 0, t, c0);
+            mbarArriveExpectTx(&bars->weights, uint32_t(g.weightBytes));
+            if (UNITS) {
+                tmaLoad3d(&mapW, weights, &bars->weights, 0, c0, 0);
+            } else {
+                for (int t = 0; t < taps; ++t) {
+                    tmaLoad3d(&mapW, weights + t * tapBytes, &bars->weights, 0, t, c0);
+                }
             }
             gridDependencySync();
             int s = 0;
@@ -145,7 +164,11 @@ gemmI8Window(const __grid_constant__ CUtensorMap mapX, const __grid_constant__ C
                     break;
                 }
                 mbarArriveExpectTx(&bars->full[s], uint32_t(g.boxW * g.boxH * g.pixelBytes));
-                tmaLoad4d(&mapX, stages + s * g.stageBytes, &bars->full[s], 0, x0 - p.padLeft, y0 - p.padTop, int(n));
+                if (UNITS) { // (a unit is two elements of the map)
+                    tmaLoad3d(&mapX, stages + s * g.stageBytes, &bars->full[s], 2 * (x0 + g.originX), y0 + g.originY, int(n));
+                } else {
+                    tmaLoad4d(&mapX, stages + s * g.stageBytes, &bars->full[s], 0, x0 + g.originX, y0 + g.originY, int(n));
+                }
                 if (++s == g.stages) {
                     s = 0;
                     phase ^= 1u;
@@ -167,6 +190,17 @@ gemmI8Window(const __grid_constant__ CUtensorMap mapX, const __grid_constant__ C
         const uint32_t tapStep = uint32_t(p.dilX * g.pixelBytes) >> 4, rowStep = uint32_t(p.dilY * g.boxW * g.pixelBytes) >> 4,
                        weightStep = uint32_t(tapBytes) >> 4, stageStep = uint32_t(g.stageBytes) >> 4;
         const int windowH = p.KH, windowW = p.KW, pixelTiles = g.pixelTiles, stageCount = g.stages;
+        // UNITS: first words of the descriptors of every pair's MMA, from the stage's and the weights' start
+        uint32_t pairX[kMaxUnitPairs], pairHigh = 0, weightHigh = 0;
+        if (UNITS) {
+            const auto unitAt = [&](int u) { return uint32_t(u / g.unitsX * g.boxW + u % g.unitsX * g.unitStep); };
+#pragma unroll
+            for (int m = 0; m < kMaxUnitPairs; ++m) {
+                const bool last = 2 * m + 1 >= g.unitsX * windowH; // an odd unit out: any second one, its weights are zero
+                pairX[m] = unitAt(2 * m) + ((last ? 1u : unitAt(2 * m + 1) - unitAt(2 * m)) << 16);
+            }
+            pairHigh = uint32_t(smemDescPlain(0, 0, groupBytes) >> 32), weightHigh = uint32_t(smemDescPlain(0, 0, 128) >> 32);
+        }
         // slices: MMAs per tap, 32 channels each; three: a 3x3 window, unrolled
         const auto tiles = [&](auto sliceCount, auto three) {
             constexpr int kSlices = decltype(sliceCount)::value;
@@ -186,7 +220,15 @@ gemmI8Window(const __grid_constant__ CUtensorMap mapX, const __grid_constant__ C
                         ummaLed(leader, tmemD, x + uint32_t(2 * u), highX, w + uint32_t(2 * u), highW, idesc, first && u == 0 ? 0u : 1u);
                     }
                 };
-                if (kThree) {
+                if (UNITS) {
+                    const uint32_t stage = smemAddr(stages + s * g.stageBytes) >> 4, w = (smemAddr(weights) >> 4) + (uint32_t(BN) << 16);
+#pragma unroll
+                    for (int m = 0; m < kMaxUnitPairs; ++m) {
+                        if (m < g.unitPairs) {
+                            ummaLed(leader, tmemD, stage + pairX[m], pairHigh, w + uint32_t(2 * m * BN), weightHigh, idesc, m == 0 ? 0u : 1u);
+                        }
+                    }
+                } else if (kThree) {
 #pragma unroll
                     for (int t = 0; t < 9; ++t) {
                         tap(stageX + uint32_t(t / 3) * rowStep + uint32_t(t % 3) * tapStep, lowW + uint32_t(t) * weightStep, t == 0);
@@ -214,6 +256,9 @@ gemmI8Window(const __grid_constant__ CUtensorMap mapX, const __grid_constant__ C
             }
         };
         const bool three = windowH == 3 && windowW == 3;
+        if (UNITS) {
+            tiles(std::integral_constant<int, 1>{}, std::false_type{});
+        } else {
         using Three = std::true_type;
         using Any = std::false_type;
         switch ((p.IC + UMMA_K - 1) / UMMA_K) {
@@ -228,6 +273,7 @@ gemmI8Window(const __grid_constant__ CUtensorMap mapX, const __grid_constant__ C
             break;
         default:
             three ? tiles(std::integral_constant<int, 4>{}, Three{}) : tiles(std::integral_constant<int, 4>{}, Any{});
+        }
         }
     } else {
         // ---- epilogue: the table of this CTA's channels, then a tile row (pixel) per lane, 16 columns per step
@@ -341,10 +387,10 @@ gemmI8Window(const __grid_constant__ CUtensorMap mapX, const __grid_constant__ C
 
 // ---- host side --------------------------------------------------------------------------------------------
 
-template <int BN>
+template <int BN, bool UNITS>
 int launchWindow(const CUtensorMap &mapX, const CUtensorMap &mapW, const GemmI8Params &p, const WindowTiling &g, size_t smem,
                  cudaStream_t s) {
-    auto kernel = gemmI8Window<BN>;
+    auto kernel = gemmI8Window<BN, UNITS>;
     if (!allowDynamicSmem(reinterpret_cast<const void *>(kernel), kWindowSmemLimit)) {
         return MLEL_ERROR_DEVICE;
     }
@@ -357,30 +403,39 @@ int launchWindow(const CUtensorMap &mapX, const CUtensorMap &mapW, const GemmI8P
     return MLEL_SUCCESS;
 }
 
-size_t windowSmem(const GemmI8Params &p, const WindowTiling &g, int bn) {
-    return 1024 + size_t(p.KH) * p.KW * bn * g.pixelBytes + size_t(g.stages) * g.stageBytes + size_t(bn) * sizeof(ColConst) +
-           sizeof(WindowBarriers);
+size_t windowSmem(const WindowTiling &g, int bn) {
+    return 1024 + size_t(g.weightBytes) + size_t(g.stages) * g.stageBytes + size_t(bn) * sizeof(ColConst) + sizeof(WindowBarriers);
 }
+
+// What a tiling is chosen for: the reach of a window past its first pixel (unit) and the work of a tile.
+struct WindowShape {
+    int reachX, reachY;
+    int pixelBytes;
+    int weightRowBytes; // weights of one output channel
+    int mmas;           // per tile
+    int boxLimitW;
+};
 
 // Tiling of p with output tiles of bn channels; false: it does not fit.  *cost: estimated cycles of a CTA (the slowest of
 // MMAs, copies and epilogue per tile, times the tiles of the busiest CTA).
-bool windowTiling(const GemmI8Params &p, int bn, WindowTiling *best, double *cost) {
-    const int reachX = (p.KW - 1) * p.dilX, reachY = (p.KH - 1) * p.dilY, images = p.M / (p.OH * p.OW);
+bool windowTiling(const GemmI8Params &p, const WindowShape &w, int bn, WindowTiling *best, double *cost) {
+    const int images = p.M / (p.OH * p.OW);
     bool found = false;
     const auto consider = [&](bool blocks, int tileW, int tileH) {
         WindowTiling g{};
-        g.pixelBytes = p.IC <= 32 ? 32 : (p.IC <= 64 ? 64 : 128);
+        g.pixelBytes = w.pixelBytes;
+        g.weightBytes = w.weightRowBytes * bn;
         g.blocks = blocks ? 1 : 0;
         g.tileW = tileW, g.tileH = tileH;
-        g.boxW = tileW + reachX, g.boxH = tileH + reachY;
-        if (g.boxW > 256 || g.boxH > 256) {
+        g.boxW = tileW + w.reachX, g.boxH = tileH + w.reachY;
+        if (g.boxW > w.boxLimitW || g.boxH > 256) {
             return;
         }
         // pixels that the MMAs of the last tap read (rows of the operand past the box hold old bytes; their results are dropped)
-        const int reach = reachY * g.boxW + reachX + (blocks ? 15 * g.boxW + 8 : 128);
+        const int reach = w.reachY * g.boxW + w.reachX + (blocks ? 15 * g.boxW + 8 : 128) + (w.pixelBytes == 16 ? 1 : 0);
         g.stageBytes = (std::max(reach, g.boxW * g.boxH) * g.pixelBytes + 1023) / 1024 * 1024;
         g.stages = kWindowMaxStages;
-        while (g.stages > 1 && windowSmem(p, g, bn) > kWindowSmemLimit) {
+        while (g.stages > 1 && windowSmem(g, bn) > kWindowSmemLimit) {
             --g.stages;
         }
         if (g.stages < 2) {
@@ -397,7 +452,7 @@ bool windowTiling(const GemmI8Params &p, int bn, WindowTiling *best, double *cos
         if (ctas < 1) {
             return;
         }
-        const double mma = double(p.KH * p.KW) * ((p.IC + 31) / 32) * (32 + bn / 4), copy = double(g.boxW) * g.boxH * g.pixelBytes / 50,
+        const double mma = double(w.mmas) * (32 + bn / 4), copy = double(g.boxW) * g.boxH * g.pixelBytes / 50,
                      epilogue = 13.0 * std::min(bn, p.N);
         const double cycles = (std::max(mma, std::max(copy, epilogue)) + 150) * double((g.pixelTiles + ctas - 1) / ctas);
         if (!found || cycles < *cost) {
@@ -412,7 +467,7 @@ bool windowTiling(const GemmI8Params &p, int bn, WindowTiling *best, double *cos
         if (tileW > 128) {
             continue;
         }
-        const int tileH = std::min(p.OH, (128 - tileW) / (tileW + reachX) + 1);
+        const int tileH = std::min(p.OH, (128 - tileW) / (tileW + w.reachX) + 1);
         consider(false, tileW, tileH);
         if (tileW < 16) {
             break;
@@ -421,8 +476,25 @@ bool windowTiling(const GemmI8Params &p, int bn, WindowTiling *best, double *cos
     return found;
 }
 
+// The tile width and tiling of least estimated time; 0: none fits.
+int chooseTiling(const GemmI8Params &p, const WindowShape &w, WindowTiling *g) {
+    int bn = 0;
+    double cost = 0;
+    for (const int width : {32, 64, 128}) {
+        WindowTiling t{};
+        double c = 0;
+        if ((width == 32 || width < 2 * p.N) && windowTiling(p, w, width, &t, &c) && (bn == 0 || c < cost)) {
+            bn = width, *g = t, cost = c;
+        }
+    }
+    g->divTilesX = makeFastDiv(g->tilesX), g->divTilesY = makeFastDiv(g->tilesY), g->divPitch = makeFastDiv(g->boxW);
+    return bn;
+}
+
+// Packed tensor (dims[0] fastest), elements of one byte or of eight.
 template <int RANK>
-bool makeWindowMap(CUtensorMap *map, uint64_t kind, const void *base, const cuuint64_t (&dims)[RANK], const cuuint32_t (&box)[RANK]) {
+bool makeWindowMap(CUtensorMap *map, uint64_t kind, const void *base, const cuuint64_t (&dims)[RANK], const cuuint32_t (&box)[RANK],
+                   bool wide = false) {
     EncodeTiledFn fn = encodeTiled();
     if (fn == nullptr) {
         return false;
@@ -432,15 +504,16 @@ bool makeWindowMap(CUtensorMap *map, uint64_t kind, const void *base, const cuui
     MapKey key{{kind, reinterpret_cast<uint64_t>(base)}};
     for (int i = 0; i < RANK; ++i) {
         if (i + 1 < RANK) {
-            strides[i] = (i == 0 ? 1 : strides[i - 1]) * dims[i];
+            strides[i] = (i == 0 ? (wide ? 8 : 1) : strides[i - 1]) * dims[i];
         }
         elemStrides[i] = 1;
         key.v[2 + i] = dims[i], key.v[8 + i] = box[i];
     }
     const CUtensorMapSwizzle swizzle =
-        box[0] == 128 ? CU_TENSOR_MAP_SWIZZLE_128B : (box[0] == 64 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_32B);
+        wide || box[0] < 32 ? CU_TENSOR_MAP_SWIZZLE_NONE
+        : box[0] == 128 ? CU_TENSOR_MAP_SWIZZLE_128B : (box[0] == 64 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_32B);
     return rememberedMap(map, key, [&](CUtensorMap *m) {
-        return fn(m, CU_TENSOR_MAP_DATA_TYPE_UINT8, RANK, const_cast<void *>(base), dims, strides, box, elemStrides,
+        return fn(m, wide ? CU_TENSOR_MAP_DATA_TYPE_UINT64 : CU_TENSOR_MAP_DATA_TYPE_UINT8, RANK, const_cast<void *>(base), dims, strides, box, elemStrides,
                   CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
     });
@@ -463,35 +536,58 @@ bool gemmI8WindowApplies(const GemmI8Problem &q) {
 int gemmI8WindowLaunch(const GemmI8Problem &q, cudaStream_t s, bool *taken) {
     GemmI8Params p = q.params;
     *taken = false;
+    const int taps = p.KH * p.KW, pixelBytes = p.IC <= 32 ? 32 : (p.IC <= 64 ? 64 : 128);
+    const WindowShape w{(p.KW - 1) * p.dilX, (p.KH - 1) * p.dilY, pixelBytes, taps * pixelBytes, taps * ((p.IC + 31) / 32), 256};
     WindowTiling g{};
-    int bn = 0;
-    double cost = 0;
-    for (const int width : {32, 64, 128}) {
-        WindowTiling t{};
-        double c = 0;
-        if ((width == 32 || width < 2 * p.N) && windowTiling(p, width, &t, &c) && (bn == 0 || c < cost)) {
-            bn = width, g = t, cost = c;
-        }
-    }
+    const int bn = chooseTiling(p, w, &g);
     if (bn == 0) {
         return MLEL_SUCCESS;
     }
+    g.originX = -p.padLeft, g.originY = -p.padTop;
     const int images = p.M / (p.OH * p.OW);
     CUtensorMap mapX{}, mapW{};
     const cuuint64_t xDims[4] = {cuuint64_t(p.IC), cuuint64_t(p.W), cuuint64_t(p.H), cuuint64_t(images)};
     const cuuint32_t xBox[4] = {cuuint32_t(g.pixelBytes), cuuint32_t(g.boxW), cuuint32_t(g.boxH), 1};
-    const cuuint64_t wDims[3] = {cuuint64_t(p.IC), cuuint64_t(p.KH * p.KW), cuuint64_t(p.N)};
+    const cuuint64_t wDims[3] = {cuuint64_t(p.IC), cuuint64_t(taps), cuuint64_t(p.N)};
     const cuuint32_t wBox[3] = {cuuint32_t(g.pixelBytes), 1, cuuint32_t(bn)};
     if (!makeWindowMap(&mapX, 5, p.in, xDims, xBox) || !makeWindowMap(&mapW, 6, q.bMatrix, wDims, wBox)) {
         return MLEL_SUCCESS; // another kernel fetches the taps one by one
     }
     *taken = true;
     g_tensorCoreLaunches[4].fetch_add(1, std::memory_order_relaxed);
-    g.divTilesX = makeFastDiv(g.tilesX), g.divTilesY = makeFastDiv(g.tilesY), g.divPitch = makeFastDiv(g.boxW);
-    const size_t smem = windowSmem(p, g, bn);
-    return bn == 32   ? launchWindow<32>(mapX, mapW, p, g, smem, s)
-           : bn == 64 ? launchWindow<64>(mapX, mapW, p, g, smem, s)
-                      : launchWindow<128>(mapX, mapW, p, g, smem, s);
+    const size_t smem = windowSmem(g, bn);
+    return bn == 32   ? launchWindow<32, false>(mapX, mapW, p, g, smem, s)
+           : bn == 64 ? launchWindow<64, false>(mapX, mapW, p, g, smem, s)
+                      : launchWindow<128, false>(mapX, mapW, p, g, smem, s);
+}
+
+int gemmI8UnitsLaunch(const GemmI8Problem &q, const UnitWindow &u, cudaStream_t s) {
+    GemmI8Params p = q.params;
+    p.KH = u.unitRows; // (rows of units)
+    const int units = (u.unitsX * u.unitRows + 1) / 2 * 2;
+    const WindowShape w{(u.unitsX - 1) * u.unitStep, u.unitRows - 1, 16, units * 16, units / 2, 128};
+    WindowTiling g{};
+    const int bn = chooseTiling(p, w, &g);
+    if (bn == 0 || units > 2 * kMaxUnitPairs) {
+        setLastError("int8 window of few channels: no tiling");
+        return MLEL_ERROR_UNKNOWN;
+    }
+    g.originX = u.originX, g.originY = u.originY;
+    g.unitsX = u.unitsX, g.unitStep = u.unitStep, g.unitPairs = units / 2;
+    CUtensorMap mapX{}, mapW{};
+    const cuuint64_t xDims[3] = {cuuint64_t(2) * u.width, cuuint64_t(u.height), cuuint64_t(p.M / (p.OH * p.OW))};
+    const cuuint32_t xBox[3] = {cuuint32_t(2 * g.boxW), cuuint32_t(g.boxH), 1};
+    const cuuint64_t wDims[3] = {16, cuuint64_t(p.N), cuuint64_t(units)};
+    const cuuint32_t wBox[3] = {16, cuuint32_t(bn), cuuint32_t(units)};
+    if (!makeWindowMap(&mapX, 7, u.units, xDims, xBox, true) || !makeWindowMap(&mapW, 8, q.bMatrix, wDims, wBox)) {
+        setLastError("int8 window of few channels: no tensor map");
+        return MLEL_ERROR_DEVICE;
+    }
+    g_tensorCoreLaunches[4].fetch_add(1, std::memory_order_relaxed);
+    const size_t smem = windowSmem(g, bn);
+    return bn == 32   ? launchWindow<32, true>(mapX, mapW, p, g, smem, s)
+           : bn == 64 ? launchWindow<64, true>(mapX, mapW, p, g, smem, s)
+                      : launchWindow<128, true>(mapX, mapW, p, g, smem, s);
 }
 
 int windowErrorWord() { return readErrorWord(); }

@@ -50,7 +50,10 @@ int fusedAdd(const int8_t *x, const int8_t *y, int8_t *out, int64_t n, const Dev
 // fast_ops.cu: vectorised kernels for packed int8 NHWC tensors
 int padImageI8(const int8_t *in, int8_t *out, int N, int H, int W, int C, int Hp, int Wp, int Cp, int padTop, int padLeft,
                cudaStream_t s);
-// bt[n][w][c] = b[n][c][w]; corr[n][w] = -za * sum_c b[n][c][w] (mod 2^32).  C and W multiples of 16.
+int gatherUnitsI8(const int8_t *in, void *out, int N, int H, int W, int C, int Hu, int Wu, int stride, int padTop, int padLeft,
+                  cudaStream_t s);
+// bt[n][w][c] = b[n][c][w]; corr[n][w] = -za * sum_c b[n][c][w] (mod 2^32); rows of bt are
+// C rounded up to a multiple of 16 long, the tail zero.
 int transposeForMatmul(const int8_t *b, int8_t *bt, int32_t *corr, int batches, int C, int W, int32_t za, cudaStream_t s);
 // corr[n][w] = -za * sum_c b[n][c][w] (mod 2^32) alone, for the kernel that reads b where it lies.  W a multiple of 16.
 int columnSumsForMatmul(const int8_t *b, int32_t *corr, int batches, int C, int W, int32_t za, cudaStream_t s);

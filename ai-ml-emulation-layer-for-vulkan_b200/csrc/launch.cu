@@ -160,6 +160,23 @@ int launchConvTensorCore(const OpDesc &op, const TView *T, cudaStream_t s, Launc
         p.out32 = reinterpret_cast<int32_t *>(out.ptr);
     }
     q.batches = 1;
+    if (op.tc == 4) {
+        // At most four channels: windows over 16-byte units of four pixels (GraphPipeline::prepareTensorCore)
+        const TView &copy = T[op.scratch];
+        const int stride = p.strideX, remX = stride == 1 ? p.padLeft : p.padLeft & 1, remY = stride == 1 ? 0 : p.padTop & 1;
+        UnitWindow u{};
+        u.units = copy.ptr;
+        u.height = int32_t(copy.dims[1]), u.width = int32_t(copy.dims[2]);
+        u.unitsX = stride == 1 ? (p.KW + 3) / 4 : (p.KW + 1) / 2, u.unitRows = stride == 1 ? p.KH : (p.KH + 1) / 2;
+        u.unitStep = stride == 1 ? 4 : 1;
+        u.originX = stride == 1 ? 0 : -((p.padLeft - remX) / 2), u.originY = stride == 1 ? -p.padTop : -((p.padTop - remY) / 2);
+        const int rc = gatherUnitsI8(p.in, copy.ptr, int(in.dims[0]), p.H, p.W, p.IC, u.height, u.width, stride, remY, remX, s);
+        if (rc != MLEL_SUCCESS) {
+            return rc;
+        }
+        q.bMatrix = T[op.aux[3]].ptr;
+        return gemmI8UnitsLaunch(q, u, s);
+    }
     if (op.tc == 2) {
         // Channel count not a multiple of 16: gather, by a table of offsets, from a copy of the input with
         // zero-padded channels and borders.

@@ -254,6 +254,8 @@ struct OpDesc {
     //                 [N][Hp][Wp][ICp], a copy of the input with zero-padded channels and borders;
     //                 aux[3] weights re-laid to the gather's K order [OC][kPad]; aux[4] int32 byte offset
     //                 of every gathered piece from a pixel's window origin; auxi[2] = bytes per piece
+    //   CONV2D kinds with tc == 4 (at most four channels): scratch = session tensor [N][Hu][Wu][16], units of four
+    //                 pixels; aux[3] weights per unit [units][OC][16]
     int32_t tc{0};
     int32_t scratch{-1};
     int32_t aux[5]{-1, -1, -1, -1, -1};

@@ -41,3 +41,28 @@ def test_windows(mlel, n, h, w, ic, oc, k, pad, dil, shift):
         assert lib.mlel_tensor_core_launches(4) > before
     finally:
         assert lib.mlel_set_tuning(b"small_kernel", 1) == 0
+
+
+@pytest.mark.parametrize("n,h,w,ic,oc,k,stride,pad,shift", [
+    (2, 56, 56, 3, 64, 7, 2, 3, 36), (1, 45, 131, 3, 32, 3, 1, 1, 33), (3, 33, 47, 3, 32, 3, 2, 1, 33), (1, 16, 8, 4, 16, 3, 1, 0, 33),
+    (1, 20, 120, 1, 48, 5, 1, 2, 31), (2, 21, 257, 2, 16, 3, 2, 0, 32), (1, 40, 40, 3, 160, 7, 1, 3, 36), (1, 9, 300, 3, 64, 5, 2, 2, 29),
+    (1, 5, 5, 4, 32, 2, 2, 0, 31), (2, 7, 7, 3, 16, 1, 2, 0, 30), (1, 70, 3, 3, 64, 3, 2, 2, 33),
+])
+def test_windows_of_few_channels(mlel, n, h, w, ic, oc, k, stride, pad, shift):
+    from mlel_b200.runtime import GraphRunner
+    r = np.random.Generator(np.random.PCG64(h * 1000 + w))
+    g = GraphBuilder()
+    x = g.input(np.int8, (n, h, w, ic))
+    g.output(conv(g, r, x, oc, k, stride, pad, -7, False, shift))
+    g.output(conv(g, r, x, oc, k, stride, pad, 5, True, shift))
+    data = r.integers(-128, 128, x.shape, dtype=np.int8)
+    want = evaluate(g, [data])
+    lib = mlel.lib()
+    lib.mlel_tensor_core_launches.restype = ctypes.c_longlong
+    before = lib.mlel_tensor_core_launches(4)
+    runner = GraphRunner(g)
+    for use_cuda_graph in (False, True):
+        for a, b in zip(runner.run([data], use_cuda_graph=use_cuda_graph), want):
+            bad = np.argwhere(a != b)
+            assert len(bad) == 0, (len(bad), a.size, bad[0].tolist(), bad[-1].tolist())
+    assert lib.mlel_tensor_core_launches(4) > before
