@@ -139,29 +139,20 @@ __device__ __forceinline__ void stsU8(uint32_t addr, int32_t v) {
     asm volatile("st.shared.u8 [%0], %1;" ::"r"(addr), "r"(v) : "memory");
 }
 
-// The rest of such a RESCALE: remaining shift, output zero point (wrapping add), clamp.
-__device__ __forceinline__ int32_t finishHigh(int32_t high, int32_t s2, int32_t outZp, int32_t lo, int32_t hi) {
-    return min(__viaddmax_s32(high >> s2, outZp, lo), hi);
-}
-
 // Constants of one epilogue thread (one output channel) and of the per-tensor output stage.
 struct EpiConsts {
     FastRescale fm;
-    uint64_t rnM;    // scaleHigh: rounding constant without the zero-point fold, for x < 0
-    uint32_t bumpM;  // scaleHigh: 2^31 with double rounding, else 0
     int32_t corr0;   // correction of the most common border class
-    int32_t corrX;   // corr0 - input zero point: accumulator + corrX is x of scaleHigh
     int32_t outZpMain, loMain, hiMain;
-    bool fast; // the shift is at least 32 and the corrections are small: see scaleHigh
-    // 0: the 64-bit forms above; 1: scaleHigh32 with the sign of x; 2: scaleHigh32 without it
-    int words32;
-    int32_t corrX4, c32, shift32; // scaleHigh32: 4 * corrX, rounding units, shift - 30
+    // 0: fastRescale; 1: wordsScale with the sign of x; 2: wordsScale without it
+    int words;
+    WordsScale scale;
 };
 
 // 16 pixels of one channel: accumulator slice -> bytes in the C/D tile (column `cd`, rows 128 bytes apart).
 // All shortcut bytes are read before the first result is written: the compiler must assume that a byte store
 // may alias any later load, and 16 load-compute-store chains in a row would run one after the other.
-template <bool RESIDUAL, bool FAST, int WORDS32 = 0>
+template <bool RESIDUAL, int WORDS>
 __device__ __forceinline__ void rescaleSliceImpl(const uint32_t (&acc)[16], const EpiConsts &k, uint32_t tab128,
                                                  uint32_t cd) {
     constexpr int CH = 8; // pixels per group: enough independent chains, few enough live registers
@@ -177,24 +168,13 @@ __device__ __forceinline__ void rescaleSliceImpl(const uint32_t (&acc)[16], cons
         int32_t r[CH];
 #pragma unroll
         for (int j = 0; j < CH; ++j) {
-            if (WORDS32 != 0) {
-                const int32_t x4 = int32_t(acc[g + j] * 4u + uint32_t(k.corrX4));
-                const int32_t q = scaleHigh32<WORDS32 == 1>(x4, k.fm.mult, k.c32) >> k.shift32;
-                if (RESIDUAL) {
-                    r[j] = __viaddmin_s32_relu(q, k.outZpMain - k.loMain, k.hiMain - k.loMain);
-                } else {
-                    r[j] = min(__viaddmax_s32(q, k.outZpMain, k.loMain), k.hiMain);
-                }
-            } else if (FAST) {
-                const int32_t x = int32_t(acc[g + j] + uint32_t(k.corrX));
-                const int32_t high = scaleHigh(x, k.fm.mult, k.rnM, k.bumpM);
-                if (RESIDUAL) {
-                    // the value is only used as a row number of the residual table: clamp(q + zp, lo, hi) - lo is one
-                    // add-min-relu, and the table's base address takes the - lo
-                    r[j] = __viaddmin_s32_relu(high >> k.fm.s2, k.outZpMain - k.loMain, k.hiMain - k.loMain);
-                } else {
-                    r[j] = finishHigh(high, k.fm.s2, k.outZpMain, k.loMain, k.hiMain);
-                }
+            if (WORDS == 2) { // (with the output zero point, for the residual table less the lower bound)
+                const int32_t q = wordsScale<false>(k.scale, int32_t(acc[g + j]));
+                r[j] = RESIDUAL ? __vimin_s32_relu(q, k.hiMain - k.loMain) : min(max(q, k.loMain), k.hiMain);
+            } else if (WORDS == 1) {
+                const int32_t q = wordsScale<true>(k.scale, int32_t(acc[g + j]));
+                r[j] = RESIDUAL ? __viaddmin_s32_relu(q, k.outZpMain - k.loMain, k.hiMain - k.loMain)
+                                : min(__viaddmax_s32(q, k.outZpMain, k.loMain), k.hiMain);
             } else {
                 const int32_t v = int32_t(acc[g + j] + uint32_t(k.corr0));
                 r[j] = fastRescale(k.fm, v, k.outZpMain, k.loMain, k.hiMain) - (RESIDUAL ? k.loMain : 0);
@@ -219,17 +199,14 @@ __device__ __forceinline__ void rescaleSliceImpl(const uint32_t (&acc)[16], cons
 // of the residual table's row for the lowest main-stage value.
 template <bool RESIDUAL>
 __device__ __forceinline__ void rescaleSlice(const uint32_t (&acc)[16], const EpiConsts &k, uint32_t tab128, uint32_t cd) {
-    if (k.words32 == 2) {
-        rescaleSliceImpl<RESIDUAL, true, 2>(acc, k, tab128, cd);
-    } else if (k.words32 == 1) {
-        rescaleSliceImpl<RESIDUAL, true, 1>(acc, k, tab128, cd);
-    } else if (k.fast) {
-        rescaleSliceImpl<RESIDUAL, true>(acc, k, tab128, cd);
+    if (k.words == 2) {
+        rescaleSliceImpl<RESIDUAL, 2>(acc, k, tab128, cd);
+    } else if (k.words == 1) {
+        rescaleSliceImpl<RESIDUAL, 1>(acc, k, tab128, cd);
     } else {
-        rescaleSliceImpl<RESIDUAL, false>(acc, k, tab128, cd);
+        rescaleSliceImpl<RESIDUAL, 0>(acc, k, tab128, cd);
     }
 }
-
 
 // Which tiles the epilogue warps of one CTA walk, and where they hand a drained accumulator back.  A CTA that
 // works alone walks tiles blockIdx.x, blockIdx.x + gridDim.x, ... and arrives on its own barriers; the two CTAs
@@ -307,23 +284,19 @@ __device__ __forceinline__ void epilogueOcMajor(const CUtensorMap *tmapD, const 
             k.fm = makeFastRescale(__ldg(p.epi.main.mult + ci), int32_t(__ldg(p.epi.main.shift + ci)), p.epi.main.inZp,
                                    p.epi.main.doubleRound != 0);
             k.corr0 = ocValid ? __ldg(corrBatch + int64_t(baseClass) * p.N + oc) : 0;
-            k.corrX = int32_t(uint32_t(k.corr0) - uint32_t(k.fm.zpIn));
-            // shift >= 32 here whenever the constants below are used
+            const int32_t x0 = int32_t(uint32_t(k.corr0) - uint32_t(k.fm.zpIn));
             const bool twoRounds = p.epi.main.doubleRound != 0;
             const int shiftM = k.fm.s1 + k.fm.s2;
-            k.rnM = (uint64_t(1) << ((shiftM > 0 ? shiftM : 1) - 1)) - (twoRounds ? (uint64_t(1) << 30) : 0);
-            k.bumpM = twoRounds ? 0x80000000u : 0u;
-            k.fast = __all_sync(0xffffffffu, k.fm.s1 == 32) && p.corrSmall != 0;
-            // 32-bit words only: every lane's shift is 32..60 and the host has bounded |x| below 2^29.  The sign of x is
-            // left out without double rounding, and where every x < 0 ends at the lower clamp bound whichever way it was
-            // rounded (no negative multiplier, bound not below the output zero point).
-            k.words32 = 0;
-            if (p.corrSmall >= 2 && __all_sync(0xffffffffu, shiftM >= 32 && shiftM <= 60)) {
-                const bool signFree = !twoRounds || (k.loMain >= k.outZpMain && __all_sync(0xffffffffu, k.fm.mult >= 0));
-                k.words32 = signFree ? 2 : 1;
-                k.corrX4 = int32_t(uint32_t(k.corrX) * 4u);
-                k.c32 = (shiftM >= 32 ? int32_t(1) << ((shiftM - 31) & 31) : 0) + (twoRounds ? 1 : 0);
-                k.shift32 = shiftM - 30;
+            // One multiply-add (see WordsScale): the forms fit every lane and the host has bounded |x| below 2^29.
+            k.words = 0;
+            if (p.corrSmall >= 2 && __all_sync(0xffffffffu, wordsScaleApplies(k.fm.mult, shiftM, twoRounds))) {
+                if (wordsScaleSignFree(twoRounds, k.outZpMain, k.loMain)) {
+                    k.words = 2;
+                    k.scale = makeWordsScale<false>(k.fm.mult, shiftM, twoRounds, x0, k.outZpMain - (RESIDUAL ? k.loMain : 0));
+                } else {
+                    k.words = 1;
+                    k.scale = makeWordsScale<true>(k.fm.mult, shiftM, twoRounds, x0, 0);
+                }
             }
             curC0 = c0;
             curBatch = batch;
