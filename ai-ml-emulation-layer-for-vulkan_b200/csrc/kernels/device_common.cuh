@@ -262,40 +262,6 @@ __device__ __forceinline__ int32_t fastRescale(const FastRescale &f, int32_t v, 
     return min(max(r, lo), hi);
 }
 
-// High 32 bits of x * mult + round(x), x = value - input zero point: product and rounding of a RESCALE whose shift
-// is at least 32, where the result only depends on the high word of the sum.  Double rounding adds 2^30 for x >= 0 and
-// subtracts it for x < 0: that is rn = 2^(shift-1) - 2^30 plus 2^31 when the sign bit of x is clear, one logic
-// operation on x (bumpMask = 2^31, or 0 without double rounding) feeding the third input of the 64-bit addition.
-// (Measured and not kept: the same value as acc * mult + (corrX * mult + rn) with the bump and the remaining shift
-// as multiply-high-adds.  It moves instructions from the general integer pipe to the multiply-add pipe, 56 % -> 43 %
-// and 14 % -> 19 % of their peaks, and ran 10 % slower: this epilogue issues one instruction every other cycle
-// whatever the mix.)
-__device__ __forceinline__ int32_t scaleHigh(int32_t x, int32_t mult, uint64_t rn, uint32_t bumpMask) {
-    const uint64_t prod = uint64_t(int64_t(x) * int64_t(mult));
-    const uint32_t extra = ~uint32_t(x) & bumpMask;
-    const uint64_t sum = prod + rn + uint64_t(extra);
-    return int32_t(uint32_t(sum >> 32));
-}
-
-// The same RESCALE from 32-bit words only, for shifts of 32 to 60 and |x| < 2^29 (x = value - input zero point).
-// Four times the sum is (4x) * mult + 2^(shift+1) +- 2^32: both rounding terms are whole units of the product's high
-// word, and what the low word holds cannot change floor(sum / 2^shift) = (high + 2^(shift-31) +- 1) >> (shift - 30).
-// x4 = 4x; c32 = 2^(shift-31), plus 1 with double rounding.  SIGNED: double rounding with the sign of x looked at
-// (-1 instead of +1 for x < 0); callers leave it out where every x < 0 ends at the lower clamp bound either way.
-template <bool SIGNED> __device__ __forceinline__ int32_t scaleHigh32(int32_t x4, int32_t mult, int32_t c32) {
-    // (written out: from __mulhi(x4, mult) + c32 and + ((x4 >> 31) << 1) the compiler made a multiply-high, two
-    // additions, a shift and a logic operation; counted over a ResNet-50 dispatch this form is 4 % fewer instructions)
-    int32_t t;
-    asm("mad.hi.s32 %0, %1, %2, %3;" : "=r"(t) : "r"(x4), "r"(mult), "r"(c32));
-    if (SIGNED) {
-        int32_t sign, u;
-        asm("shr.s32 %0, %1, 31;" : "=r"(sign) : "r"(x4));
-        asm("{\n\t.reg .s32 a;\n\tadd.s32 a, %1, %2;\n\tadd.s32 %0, a, %2;\n\t}" : "=r"(u) : "r"(t), "r"(sign));
-        t = u;
-    }
-    return t;
-}
-
 // ---- RESCALE as one multiply-add -----------------------------------------------------------------------------------
 // A shift s of 32 to 50 only sees the high word of the 64-bit sum, and there everything constant -- correction times
 // multiplier, rounding, output zero point times 2^s -- fits the multiply-add's 64-bit addend:

@@ -125,11 +125,10 @@ __device__ __forceinline__ void epilogueInt8(const GemmI8Params &p, PipeBarriers
     }
     const int32_t zpMain = p.epi.main.inZp, outZpMain = p.epi.main.outZp;
     const uint32_t tabAddr = smemAddr(colTab);
-    // what holds for every column of the table -- bit 0: a shift of at least 32; bit 1: a shift of 32..60; bit 2: no
-    // negative multiplier
+    // what holds for every column of the table -- bit 0: a shift of at least 32; bit 1: wordsScaleApplies
     volatile uint32_t *fastFlag = &bars->pad;
-    bool fast = false, high = false, words32 = false, signFree = false; // forms of the table: see ColConst
-    const uint32_t bumpMask = p.epi.main.doubleRound != 0 ? 0x80000000u : 0u;
+    bool fast = false;
+    int form = kGeneralForm; // of the table
     const int32_t loMain = p.epi.main.lo, hiMain = p.epi.main.hi;
     uint32_t tileCount = 0;
     int tabN0 = -1, tabBatch = -1; // what the shared constants table was built for
@@ -146,7 +145,7 @@ __device__ __forceinline__ void epilogueInt8(const GemmI8Params &p, PipeBarriers
         if (n0 != tabN0 || (p.batchedCorr && batch != tabBatch)) {
             epilogueSync(); // everyone is done with the previous table
             if (threadIdx.x == 0) {
-                *fastFlag = 7;
+                *fastFlag = 3;
             }
             epilogueSync();
             FastRescale f{};
@@ -157,8 +156,8 @@ __device__ __forceinline__ void epilogueInt8(const GemmI8Params &p, PipeBarriers
                 f = makeFastRescale(__ldg(p.epi.main.mult + ci), int32_t(__ldg(p.epi.main.shift + ci)), zpMain,
                                     p.epi.main.doubleRound != 0);
                 const int shift = f.s1 + f.s2;
-                // (a shift below 32 in this tile: the low word of the product matters)
-                const uint32_t fails = (f.s1 != 32 ? 1u : 0u) | ((shift < 32 || shift > 60) ? 2u : 0u) | (f.mult < 0 ? 4u : 0u);
+                const uint32_t fails =
+                    (f.s1 != 32 ? 1u : 0u) | (wordsScaleApplies(f.mult, shift, p.epi.main.doubleRound != 0) ? 0u : 2u);
                 if (fails != 0) {
                     atomicAnd(const_cast<uint32_t *>(fastFlag), ~fails);
                 }
@@ -167,28 +166,10 @@ __device__ __forceinline__ void epilogueInt8(const GemmI8Params &p, PipeBarriers
             epilogueSync();
             const uint32_t holds = *fastFlag;
             fast = (holds & 1u) != 0;
-            high = fast && p.corrSmall != 0 && !RESIDUAL;
-            words32 = high && p.corrSmall >= 2 && (holds & 2u) != 0;
-            // the sign of x only matters to double rounding, and not where every x < 0 ends at the lower clamp bound
-            signFree = p.epi.main.doubleRound == 0 || (loMain >= outZpMain && (holds & 4u) != 0);
+            // (with the residual tail, whose three RESCALEs follow in registers, one form of the loop)
+            form = !RESIDUAL && p.corrSmall != 0 && (holds & 2u) != 0 ? wordsForm(p.epi.main) : kGeneralForm;
             if (threadIdx.x < BN) {
-                ColConst c;
-                c.mult = f.mult, c.s1 = f.s1, c.s2 = f.s2, c.corr0 = corr0;
-                c.bump = f.rpLo - f.rnLo; // (rp - rn) mod 2^32: 0 or 2^31
-                if (words32) {
-                    const int shift = f.s1 + f.s2;
-                    c.corr = int32_t((uint32_t(corr0) - uint32_t(f.zpIn)) * 4u);
-                    c.rnLo = (1u << ((shift - 31) & 31)) + (p.epi.main.doubleRound != 0 ? 1u : 0u);
-                    c.rnHi = uint32_t(shift - 30);
-                } else if (high) {
-                    const bool twoRounds = p.epi.main.doubleRound != 0;
-                    const uint64_t rn = (uint64_t(1) << (f.s1 + f.s2 - 1)) - (twoRounds ? (uint64_t(1) << 30) : 0);
-                    c.corr = int32_t(uint32_t(corr0) - uint32_t(f.zpIn));
-                    c.rnLo = uint32_t(rn), c.rnHi = uint32_t(rn >> 32);
-                } else {
-                    c.corr = corr0, c.rnLo = f.rnLo, c.rnHi = f.rnHi;
-                }
-                colTab[threadIdx.x] = c;
+                colTab[threadIdx.x] = makeColConst(f, corr0, p.epi.main, form);
             }
             epilogueSync();
             tabN0 = n0;
@@ -258,30 +239,10 @@ __device__ __forceinline__ void epilogueInt8(const GemmI8Params &p, PipeBarriers
                 }
             }
             uint32_t packed[4];
-            if (!RESIDUAL && words32) {
-                // (two copies of the loop behind one branch: as a select per element the compiler computed the sign
-                // term for every element and dropped it afterwards)
-                if (signFree) {
-                    rescale16Words32<false>(acc, tabAddr + uint32_t(cl) * 32u, outZpMain, loMain, hiMain, packed);
-                } else {
-                    rescale16Words32<true>(acc, tabAddr + uint32_t(cl) * 32u, outZpMain, loMain, hiMain, packed);
-                }
-            } else if (!RESIDUAL && high) {
-#pragma unroll
-                for (int q = 0; q < 4; ++q) {
-                    int32_t y[4];
-#pragma unroll
-                    for (int e = 0; e < 4; ++e) {
-                        const int j = 4 * q + e;
-                        uint32_t mult, corrX, rnLo, rnHi;
-                        ldsV4(tabAddr + uint32_t(cl + j) * 32u, mult, corrX, rnLo, rnHi);
-                        const int32_t s2 = ldsS32(tabAddr + uint32_t(cl + j) * 32u + 16u);
-                        const int32_t h = tc::scaleHigh(int32_t(acc[j] + corrX), int32_t(mult), (uint64_t(rnHi) << 32) | rnLo,
-                                                    bumpMask);
-                        y[e] = min(__viaddmax_s32(h >> s2, outZpMain, loMain), hiMain);
-                    }
-                    packed[q] = pack4(y[0], y[1], y[2], y[3]);
-                }
+            if (!RESIDUAL && form == kWords) {
+                rescale16Words<false>(acc, tabAddr + uint32_t(cl) * 32u, outZpMain, loMain, hiMain, packed);
+            } else if (!RESIDUAL && form == kSignedWords) {
+                rescale16Words<true>(acc, tabAddr + uint32_t(cl) * 32u, outZpMain, loMain, hiMain, packed);
             } else {
 #pragma unroll
                 for (int q = 0; q < 4; ++q) {
@@ -313,7 +274,7 @@ __device__ __forceinline__ void epilogueInt8(const GemmI8Params &p, PipeBarriers
                         }
                         y[e] = r;
                     }
-                    packed[q] = pack4(y[0], y[1], y[2], y[3]);
+                    packed[q] = packSatS8(y[0], y[1], y[2], y[3]);
                 }
             }
             if (ROWS16) {

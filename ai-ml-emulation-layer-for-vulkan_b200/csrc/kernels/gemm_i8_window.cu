@@ -129,7 +129,7 @@ gemmI8Window(const __grid_constant__ CUtensorMap mapX, const __grid_constant__ C
             mbarInit(&bars->accEmpty[b], uint32_t(kEpilogueWarps / kSets));
         }
         mbarInit(&bars->weights, 1u);
-        bars->forms = 7;
+        bars->forms = 1; // wordsScaleApplies to every column
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == kMmaWarp) {
@@ -284,30 +284,16 @@ gemmI8Window(const __grid_constant__ CUtensorMap mapX, const __grid_constant__ C
         if (threadIdx.x < BN) {
             const int col = c0 + int(threadIdx.x), ci = (p.epi.main.perChannel && col < p.N) ? col : 0;
             f = makeFastRescale(__ldg(p.epi.main.mult + ci), int32_t(__ldg(p.epi.main.shift + ci)), zpMain, twoRounds);
-            const int shift = f.s1 + f.s2;
-            const uint32_t fails = (f.s1 != 32 ? 1u : 0u) | ((shift < 32 || shift > 60) ? 2u : 0u) | (f.mult < 0 ? 4u : 0u);
-            if (fails != 0) {
-                atomicAnd(&bars->forms, ~fails);
+            if (!wordsScaleApplies(f.mult, f.s1 + f.s2, twoRounds)) {
+                atomicAnd(&bars->forms, 0u);
             }
             corr0 = col < p.N ? __ldg(p.corr + int64_t(p.baseClass) * p.N + col) : 0;
         }
         epilogueSync();
         const uint32_t holds = *const_cast<volatile uint32_t *>(&bars->forms);
-        const bool words32 = (holds & 1u) != 0 && p.corrSmall >= 2 && (holds & 2u) != 0;
-        const bool signFree = !twoRounds || (lo >= outZp && (holds & 4u) != 0);
-        if (threadIdx.x < BN) { // general or 32-bit form: see ColConst
-            ColConst c;
-            c.mult = f.mult, c.s1 = f.s1, c.s2 = f.s2, c.corr0 = corr0;
-            c.bump = f.rpLo - f.rnLo;
-            if (words32) {
-                const int shift = f.s1 + f.s2;
-                c.corr = int32_t((uint32_t(corr0) - uint32_t(f.zpIn)) * 4u);
-                c.rnLo = (1u << ((shift - 31) & 31)) + (twoRounds ? 1u : 0u);
-                c.rnHi = uint32_t(shift - 30);
-            } else {
-                c.corr = corr0, c.rnLo = f.rnLo, c.rnHi = f.rnHi;
-            }
-            colTab[threadIdx.x] = c;
+        const int form = holds != 0 && p.corrSmall != 0 ? wordsForm(p.epi.main) : kGeneralForm;
+        if (threadIdx.x < BN) {
+            colTab[threadIdx.x] = makeColConst(f, corr0, p.epi.main, form);
         }
         epilogueSync();
         gridDependencySync();
@@ -365,12 +351,10 @@ gemmI8Window(const __grid_constant__ CUtensorMap mapX, const __grid_constant__ C
                 }
                 uint32_t packed[4];
                 const uint32_t tab = tabAddr + uint32_t(cl) * 32u;
-                if (words32) {
-                    if (signFree) {
-                        rescale16Words32<false>(acc, tab, outZp, lo, hi, packed);
-                    } else {
-                        rescale16Words32<true>(acc, tab, outZp, lo, hi, packed);
-                    }
+                if (form == kWords) {
+                    rescale16Words<false>(acc, tab, outZp, lo, hi, packed);
+                } else if (form == kSignedWords) {
+                    rescale16Words<true>(acc, tab, outZp, lo, hi, packed);
                 } else {
                     rescale16General(acc, tab, zpMain, outZp, lo, hi, packed);
                 }

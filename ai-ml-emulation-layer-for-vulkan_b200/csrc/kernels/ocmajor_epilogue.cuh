@@ -287,9 +287,9 @@ __device__ __forceinline__ void epilogueOcMajor(const CUtensorMap *tmapD, const 
             const int32_t x0 = int32_t(uint32_t(k.corr0) - uint32_t(k.fm.zpIn));
             const bool twoRounds = p.epi.main.doubleRound != 0;
             const int shiftM = k.fm.s1 + k.fm.s2;
-            // One multiply-add (see WordsScale): the forms fit every lane and the host has bounded |x| below 2^29.
+            // One multiply-add (see WordsScale): the forms fit every lane and the host has bounded the corrections.
             k.words = 0;
-            if (p.corrSmall >= 2 && __all_sync(0xffffffffu, wordsScaleApplies(k.fm.mult, shiftM, twoRounds))) {
+            if (p.corrSmall != 0 && __all_sync(0xffffffffu, wordsScaleApplies(k.fm.mult, shiftM, twoRounds))) {
                 if (wordsScaleSignFree(twoRounds, k.outZpMain, k.loMain)) {
                     k.words = 2;
                     k.scale = makeWordsScale<false>(k.fm.mult, shiftM, twoRounds, x0, k.outZpMain - (RESIDUAL ? k.loMain : 0));

@@ -250,8 +250,7 @@ int launchMatmulTensorCore(const OpDesc &op, const TView *T, cudaStream_t s) {
     // whenever that bound is (see GemmI8Params::corrSmall)
     {
         const int64_t corrBound = int64_t(op.i[0] < 0 ? -op.i[0] : op.i[0]) * p.K * 128;
-        const bool tiny = corrBound + int64_t(p.K) * (int64_t(1) << 14) + 256 < (int64_t(1) << 29);
-        p.corrSmall = tiny ? 2 : (corrBound <= (int64_t(1) << 30) - 256 ? 1 : 0);
+        p.corrSmall = corrBound <= (int64_t(1) << 30) - 256 ? 1 : 0;
     }
     if (op.kind == OP_FUSED_MATMUL) {
         p.out8 = reinterpret_cast<int8_t *>(out.ptr);
