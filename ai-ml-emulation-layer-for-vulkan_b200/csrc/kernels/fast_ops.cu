@@ -210,11 +210,14 @@ __global__ void __launch_bounds__(256) transposeColsumKernel(const int8_t *__res
 // ---- column sums of MATMUL's second input [N][C][W]: corr[n][w] = -za * sum_c b[n][c][w] --------------------
 // For the tensor-core path that reads the operand where it lies (no transposed copy).  A block owns 64 columns
 // of one batch: 4 lanes hold 16 columns each (one 16-byte load per row), 64 slices share the rows, eight rows in
-// flight per thread, and add their partial sums in shared memory.  Each byte goes through one dp4a against a
-// one-hot selector, which sign-extends and accumulates it.
+// flight per thread.  Each byte goes through one dp4a against a one-hot selector, which sign-extends and accumulates it.
+// A warp's eight slices join by shuffles, the eight warps in shared memory.
+// The product is let in at once and waits for the sums only before its epilogue (kLateCorrections): 1024^3 14.5 -> 12.4 us.
 __global__ void __launch_bounds__(256) columnSumKernel(const int8_t *__restrict__ b, int32_t *__restrict__ corr, int C, int W,
                                                        int32_t za) {
-    __shared__ int32_t part[64][64 + 1];
+    __shared__ int32_t part[8][64];
+    asm volatile("griddepcontrol.wait;" ::: "memory"); // first: the launch after this one relies on it
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const int n = blockIdx.y;
     const int w0 = blockIdx.x * 64;
     const int seg = threadIdx.x & 3, slice = threadIdx.x >> 2;
@@ -243,16 +246,27 @@ __global__ void __launch_bounds__(256) columnSumKernel(const int8_t *__restrict_
             }
         }
     }
+    // lanes 4 apart hold the same columns: halve the columns a lane keeps with each exchange
+    const int lane = threadIdx.x & 31;
+    int first = 0;
 #pragma unroll
-    for (int i = 0; i < 16; ++i) {
-        part[slice][seg * 16 + i] = acc[i];
+    for (int half = 8, bit = 4; half >= 2; half >>= 1, bit <<= 1) {
+        const bool upper = (lane & bit) != 0;
+#pragma unroll
+        for (int i = 0; i < half; ++i) {
+            const int32_t give = upper ? acc[i] : acc[i + half], keep = upper ? acc[i + half] : acc[i];
+            acc[i] = keep + __shfl_xor_sync(0xffffffffu, give, bit);
+        }
+        first += upper ? half : 0;
     }
+    part[threadIdx.x >> 5][seg * 16 + first] = acc[0];
+    part[threadIdx.x >> 5][seg * 16 + first + 1] = acc[1];
     __syncthreads();
     if (threadIdx.x < 64 && w0 + threadIdx.x < W) {
         int32_t sum = 0;
-#pragma unroll 8
-        for (int sl = 0; sl < 64; ++sl) {
-            sum += part[sl][threadIdx.x];
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+            sum += part[q][threadIdx.x];
         }
         corr[int64_t(n) * W + w0 + threadIdx.x] = int32_t(uint32_t(0) - uint32_t(za) * uint32_t(sum));
     }
@@ -654,7 +668,7 @@ int transposeForMatmul(const int8_t *b, int8_t *bt, int32_t *corr, int batches, 
 
 int columnSumsForMatmul(const int8_t *b, int32_t *corr, int batches, int C, int W, int32_t za, cudaStream_t s) {
     const dim3 grid(unsigned((W + 63) / 64), unsigned(batches));
-    columnSumKernel<<<grid, 256, 0, s>>>(b, corr, C, W, za);
+    launchOverlapped(columnSumKernel, grid, 256, 0, s, b, corr, C, W, za);
     return finish("MATMUL operand column sums");
 }
 

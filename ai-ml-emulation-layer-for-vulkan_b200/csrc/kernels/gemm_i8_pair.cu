@@ -265,7 +265,12 @@ gemmI8Pair(const __grid_constant__ CUtensorMap tmapX, const __grid_constant__ CU
         mbarArriveExpectTx(&bars->tabFull, uint32_t(kResidualTableBytes));
         bulkLoad(resTab, p.residualTable, uint32_t(kResidualTableBytes), &bars->tabFull);
     }
-    gridDependencySync(); // from here on activations are read and written
+    // From here on activations are read and written.  With kLateCorrections the operands are complete already (the launch
+    // before, which makes the corrections, itself started after everything older had ended): copies and MMAs begin at once.
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    if (p.lateOperand != kLateCorrections || warp >= kStoreWarpP) {
+        asm volatile("griddepcontrol.wait;" ::: "memory");
+    }
 
     if (warp == kTmaWarpP) {
         // ---------------- TMA producer (both CTAs) ----------------

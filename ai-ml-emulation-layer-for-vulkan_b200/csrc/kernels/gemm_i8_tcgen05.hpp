@@ -32,6 +32,8 @@ inline FastDiv makeFastDiv(int64_t divisor) {
     return f;
 }
 
+enum : int32_t { kLateOperand = 1, kLateCorrections = 2 };
+
 // Device-side parameters (passed by value to the kernel).
 struct GemmI8Params {
     int32_t M, N, K;     // per batch: rows, columns (output channels), contraction length in bytes
@@ -57,7 +59,9 @@ struct GemmI8Params {
     const uint8_t *rowClass; // [OH] border class of an output row, or null (single class)
     const uint8_t *colClass; // [OW]
     int32_t numColClasses, numClasses, batchedCorr;
-    int32_t lateOperand;     // 1: the weight operand and the corrections are results of a launch before this one
+    int32_t lateOperand;     // kLateOperand: the weight operand and the corrections are results of the launch before this
+                             // one; kLateCorrections: only the corrections, and that launch waits for all older ones
+                             // before it lets this one start
     int32_t baseClass;       // the most common class: its correction row is staged in shared memory
     int32_t corrSmall;       // 1: every |corr| <= 2^30 - 256: accumulator + correction - zero point stays inside int32
     // outputs: exactly one of out32 / out8 is set

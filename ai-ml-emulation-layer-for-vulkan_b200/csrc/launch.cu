@@ -280,7 +280,7 @@ int launchMatmulTensorCore(const OpDesc &op, const TView *T, cudaStream_t s) {
         int8_t *scratch = reinterpret_cast<int8_t *>(T[op.scratch].ptr) + op.auxi[0];
         int32_t *corr = reinterpret_cast<int32_t *>(reinterpret_cast<int8_t *>(T[op.scratch].ptr) + op.auxi[2]);
         p.corr = corr;
-        p.lateOperand = 1;
+        p.lateOperand = kLateCorrections;
         // The paired kernel reads the run-time operand where it lies ([C][W], the output column contiguous: an
         // MN-major tensor-core operand) and only needs the column sums; the single-CTA kernel takes a transposed
         // copy, made together with the sums.
@@ -299,6 +299,7 @@ int launchMatmulTensorCore(const OpDesc &op, const TView *T, cudaStream_t s) {
                 return rc;
             }
         }
+        p.lateOperand = kLateOperand;
         const int rc = transposeForMatmul(reinterpret_cast<const int8_t *>(b.ptr), scratch, corr, int(b.dims[0]), p.K, p.N,
                                           op.i[0], s);
         if (rc != MLEL_SUCCESS) {
