@@ -185,7 +185,7 @@ __device__ __forceinline__ uint32_t tmaStagePeekIm2colPair(uint64_t *fullOwn, ui
 // X_MODE: kXTiled = tmapX is a K-major matrix {K, M, batches}; kXIm2col = tmapX is an im2col map of the NHWC input
 //         and tmapW the {IC, taps, OC} weight map.
 // W_MN  : tmapW is {N, K, batches}, N contiguous (kXTiled only).
-template <int BNP, int NSTAGE, int EW, int X_MODE, bool W_MN, bool RESIDUAL>
+template <int BNP, int NSTAGE, int EW, int X_MODE, bool W_MN, bool RESIDUAL, bool TABLE = false>
 __global__ void __launch_bounds__((EW + 4) * 32, 1)
 gemmI8Pair(const __grid_constant__ CUtensorMap tmapX, const __grid_constant__ CUtensorMap tmapW,
            const __grid_constant__ CUtensorMap tmapC, const __grid_constant__ CUtensorMap tmapD, const GemmI8Params p) {
@@ -200,7 +200,7 @@ gemmI8Pair(const __grid_constant__ CUtensorMap tmapX, const __grid_constant__ CU
     uint8_t *tilesX = smem + NSTAGE * kTileW;
     uint8_t *cdTiles = smem + NSTAGE * (kTileW + kTileX);
     uint8_t *resTab = cdTiles + 2 * kTileCd;
-    OcBarriers *bars = reinterpret_cast<OcBarriers *>(resTab + (RESIDUAL ? kResidualTableBytes : 0));
+    OcBarriers *bars = reinterpret_cast<OcBarriers *>(resTab + (RESIDUAL ? kResidualTableBytes : (TABLE ? 256 : 0)));
 
     static_assert(NSTAGE <= 6, "OcBarriers holds six stages");
     static_assert(BK / UMMA_K == 4, "the MMA loop issues four instructions per K block");
@@ -261,9 +261,10 @@ gemmI8Pair(const __grid_constant__ CUtensorMap tmapX, const __grid_constant__ CU
             atomicCAS(&g_tcgen05Error, 0, 29);
         }
     }
-    if (RESIDUAL && warp == kTmaWarpP && lane == 0) {
-        mbarArriveExpectTx(&bars->tabFull, uint32_t(kResidualTableBytes));
-        bulkLoad(resTab, p.residualTable, uint32_t(kResidualTableBytes), &bars->tabFull);
+    if ((RESIDUAL || TABLE) && warp == kTmaWarpP && lane == 0) {
+        constexpr uint32_t kTableBytes = RESIDUAL ? uint32_t(kResidualTableBytes) : 256u;
+        mbarArriveExpectTx(&bars->tabFull, kTableBytes);
+        bulkLoad(resTab, RESIDUAL ? static_cast<const void *>(p.residualTable) : p.epi.table, kTableBytes, &bars->tabFull);
     }
     // From here on activations are read and written.  With kLateCorrections the operands are complete already (the launch
     // before, which makes the corrections, itself started after everything older had ended): copies and MMAs begin at once.
@@ -424,7 +425,7 @@ gemmI8Pair(const __grid_constant__ CUtensorMap tmapX, const __grid_constant__ CU
         walk.cOffset = int(rank) * kOcTile;
         walk.accEmpty[0] = mapToCta(smemAddr(&bars->accEmpty[0]), 0u);
         walk.accEmpty[1] = mapToCta(smemAddr(&bars->accEmpty[1]), 0u);
-        epilogueOcMajor<BNP, EW, RESIDUAL, kPairChannels, true>(&tmapD, p, bars, resTab, cdTiles, tmemBase,
+        epilogueOcMajor<BNP, EW, RESIDUAL, kPairChannels, true, TABLE>(&tmapD, p, bars, resTab, cdTiles, tmemBase,
                                                                 warp - kFirstEpiWarp, lane, numTiles, pTiles, cTiles, walk);
     }
 
@@ -442,15 +443,15 @@ struct PairMaps {
     CUtensorMap x, w, c, d;
 };
 
-template <int BNP, int NSTAGE, int EW, int X_MODE, bool W_MN, bool RESIDUAL>
+template <int BNP, int NSTAGE, int EW, int X_MODE, bool W_MN, bool RESIDUAL, bool TABLE = false>
 int launchPair(const PairMaps &maps, const GemmI8Params &params, cudaStream_t s) {
     GemmI8Params p = params;
     p.divPlane = makeFastDiv(int64_t(p.OH) * p.OW), p.divOW = makeFastDiv(p.OW);
     p.divTiles0 = makeFastDiv((p.M + BNP - 1) / BNP), p.divTiles1 = makeFastDiv((p.N + kPairChannels - 1) / kPairChannels);
     constexpr size_t smemBytes = size_t(NSTAGE) * (kOcTile * BK + (BNP / 2) * BK) + 2 * size_t(BNP) * 128 +
-                                 (RESIDUAL ? size_t(kResidualTableBytes) : 0) + sizeof(OcBarriers) + 1024;
+                                 (RESIDUAL ? size_t(kResidualTableBytes) : (TABLE ? 256 : 0)) + sizeof(OcBarriers) + 1024;
     static_assert(smemBytes <= 232448, "shared memory per CTA");
-    auto kernel = gemmI8Pair<BNP, NSTAGE, EW, X_MODE, W_MN, RESIDUAL>;
+    auto kernel = gemmI8Pair<BNP, NSTAGE, EW, X_MODE, W_MN, RESIDUAL, TABLE>;
     if (!allowDynamicSmem(reinterpret_cast<const void *>(kernel), smemBytes)) {
         return MLEL_ERROR_DEVICE;
     }
@@ -489,6 +490,9 @@ int launchPairShape(const PairMaps &maps, const GemmI8Params &p, int xMode, bool
     }
     if (xMode == kXIm2col) {
         return launchPair<BNP, NSTAGE, EW, kXIm2col, false, false>(maps, p, s);
+    }
+    if (p.epi.table != nullptr && !wMn) {
+        return launchPair<BNP, NSTAGE, EW, kXTiled, false, false, true>(maps, p, s);
     }
     return wMn ? launchPair<BNP, NSTAGE, EW, kXTiled, true, false>(maps, p, s)
                : launchPair<BNP, NSTAGE, EW, kXTiled, false, false>(maps, p, s);

@@ -62,7 +62,7 @@ __device__ __forceinline__ void prefetchMap(const CUtensorMap *map) {
 }
 
 // IM2COL: mapX is an im2col map of the NHWC input and mapW a {IC, taps, OC} map; else mapX is a plain pixel matrix.
-template <int BNP, int SPLIT, bool IM2COL, bool RESIDUAL>
+template <int BNP, int SPLIT, bool IM2COL, bool RESIDUAL, bool TABLE = false>
 __global__ void __launch_bounds__(kSmallThreads, 2)
 gemmI8Small(const __grid_constant__ CUtensorMap mapX, const __grid_constant__ CUtensorMap mapW, const __grid_constant__ GemmI8Params p) {
     constexpr int kStages = smallStages(BNP);
@@ -292,6 +292,9 @@ gemmI8Small(const __grid_constant__ CUtensorMap mapX, const __grid_constant__ CU
                 const int32_t tb = fastRescale(fb, int32_t(shortcut[j]), p.epi.b.outZp, p.epi.b.lo, p.epi.b.hi);
                 v = fastRescale(fo, int32_t(uint32_t(ta) + uint32_t(tb)), p.epi.out.outZp, p.epi.out.lo, p.epi.out.hi);
             }
+            if (TABLE) {
+                v = int32_t(__ldg(p.epi.table + 128 + v));
+            }
             if (ocValid && firstPixel + j < p.M) {
                 dst[int64_t(j) * p.ldOut] = int8_t(v);
             }
@@ -304,11 +307,11 @@ gemmI8Small(const __grid_constant__ CUtensorMap mapX, const __grid_constant__ CU
     }
 }
 
-template <int BNP, int SPLIT, bool IM2COL, bool RESIDUAL>
+template <int BNP, int SPLIT, bool IM2COL, bool RESIDUAL, bool TABLE = false>
 int launchSmall(const CUtensorMap &mapX, const CUtensorMap &mapW, const GemmI8Params &p, int tiles, cudaStream_t s) {
     constexpr size_t smem = size_t(smallStages(BNP)) * (kSmallChannels + BNP) * BK +
                             (SPLIT > 1 ? size_t(BNP) * kSmallChannels * 4 : 0) + sizeof(SmallBarriers) + 1024;
-    auto kernel = gemmI8Small<BNP, SPLIT, IM2COL, RESIDUAL>;
+    auto kernel = gemmI8Small<BNP, SPLIT, IM2COL, RESIDUAL, TABLE>;
     if (!allowDynamicSmem(reinterpret_cast<const void *>(kernel), smem)) {
         return MLEL_ERROR_DEVICE;
     }
@@ -337,6 +340,9 @@ int launchSmallMode(const CUtensorMap &mapX, const CUtensorMap &mapW, const Gemm
     if (im2col) {
         return p.epi.hasResidual ? launchSmall<BNP, SPLIT, true, true>(mapX, mapW, p, tiles, s)
                                  : launchSmall<BNP, SPLIT, true, false>(mapX, mapW, p, tiles, s);
+    }
+    if (p.epi.table != nullptr) {
+        return launchSmall<BNP, SPLIT, false, false, true>(mapX, mapW, p, tiles, s);
     }
     return p.epi.hasResidual ? launchSmall<BNP, SPLIT, false, true>(mapX, mapW, p, tiles, s)
                              : launchSmall<BNP, SPLIT, false, false>(mapX, mapW, p, tiles, s);

@@ -30,6 +30,8 @@ struct DevEpilogue {
     int32_t hasResidual;
     const int8_t *shortcut; // packed, same shape as the output
     DevRescale a, b, out;   // a: main path, b: shortcut, out: after the ADD
+    const int8_t *table;    // or null: byte v of the main stage becomes table[v + 128]; only the small and the paired
+                            // tensor-core kernel look it up, see launchMatmulTensorCore
 };
 
 // fused_generic.cu: one-thread-per-output fused kernels (always-correct path of the fused kinds)

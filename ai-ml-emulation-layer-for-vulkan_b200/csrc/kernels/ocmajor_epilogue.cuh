@@ -152,7 +152,7 @@ struct EpiConsts {
 // 16 pixels of one channel: accumulator slice -> bytes in the C/D tile (column `cd`, rows 128 bytes apart).
 // All shortcut bytes are read before the first result is written: the compiler must assume that a byte store
 // may alias any later load, and 16 load-compute-store chains in a row would run one after the other.
-template <bool RESIDUAL, int WORDS>
+template <bool RESIDUAL, bool TABLE, int WORDS>
 __device__ __forceinline__ void rescaleSliceImpl(const uint32_t (&acc)[16], const EpiConsts &k, uint32_t tab128,
                                                  uint32_t cd) {
     constexpr int CH = 8; // pixels per group: enough independent chains, few enough live registers
@@ -188,6 +188,12 @@ __device__ __forceinline__ void rescaleSliceImpl(const uint32_t (&acc)[16], cons
                 r[j] = int32_t(ldsU8(tab128 + sc[j] + uint32_t(r[j] * kResidualRowBytes)));
             }
         }
+        if (TABLE) {
+#pragma unroll
+            for (int j = 0; j < CH; ++j) {
+                r[j] = int32_t(ldsU8(tab128 + uint32_t(r[j])));
+            }
+        }
 #pragma unroll
         for (int j = 0; j < CH; ++j) {
             stsU8(cd + 128 * (g + j), r[j]);
@@ -196,15 +202,15 @@ __device__ __forceinline__ void rescaleSliceImpl(const uint32_t (&acc)[16], cons
 }
 
 // cd: shared address of this thread's column of the C/D tile at the slice's first pixel; tab128: shared address
-// of the residual table's row for the lowest main-stage value.
-template <bool RESIDUAL>
+// of the residual table's row for the lowest main-stage value (TABLE: of the byte table's entry for 0).
+template <bool RESIDUAL, bool TABLE>
 __device__ __forceinline__ void rescaleSlice(const uint32_t (&acc)[16], const EpiConsts &k, uint32_t tab128, uint32_t cd) {
     if (k.words == 2) {
-        rescaleSliceImpl<RESIDUAL, 2>(acc, k, tab128, cd);
+        rescaleSliceImpl<RESIDUAL, TABLE, 2>(acc, k, tab128, cd);
     } else if (k.words == 1) {
-        rescaleSliceImpl<RESIDUAL, 1>(acc, k, tab128, cd);
+        rescaleSliceImpl<RESIDUAL, TABLE, 1>(acc, k, tab128, cd);
     } else {
-        rescaleSliceImpl<RESIDUAL, 0>(acc, k, tab128, cd);
+        rescaleSliceImpl<RESIDUAL, TABLE, 0>(acc, k, tab128, cd);
     }
 }
 
@@ -226,7 +232,8 @@ __device__ __forceinline__ void mbarArriveCluster(uint32_t clusterAddr) {
 // The epilogue warps.  Warp w owns TMEM lanes 32 * (w & 3) .. +31 (output channels) and half of the tile's
 // pixels, which it walks in slices of 16 pixels; the tcgen05.ld of the next slice is in flight while the
 // current one is rescaled.  C_TILE: output channels per tile (128, or 256 for a pair of CTAs).
-template <int BNP, int EW, bool RESIDUAL, int C_TILE, bool STORE_WARP = false>
+// TABLE: resTab holds the 256 entries of a byte table that the results go through.
+template <int BNP, int EW, bool RESIDUAL, int C_TILE, bool STORE_WARP = false, bool TABLE = false>
 __device__ __forceinline__ void epilogueOcMajor(const CUtensorMap *tmapD, const GemmI8Params &p, OcBarriers *bars,
                                                 const uint8_t *resTab, uint8_t *cdTiles,
                                                 uint32_t tmemBase, int warp, int lane, int64_t numTiles, int pTiles,
@@ -249,8 +256,8 @@ __device__ __forceinline__ void epilogueOcMajor(const CUtensorMap *tmapD, const 
     EpiConsts k{};
     k.outZpMain = p.epi.main.outZp, k.loMain = p.epi.main.lo, k.hiMain = p.epi.main.hi;
     // row of the lowest main-stage value: the element loop counts rows from there
-    const uint32_t tab128 = smemAddr(resTab) + uint32_t((128 + p.epi.main.lo) * kResidualRowBytes);
-    bool tableReady = !RESIDUAL;
+    const uint32_t tab128 = smemAddr(resTab) + (TABLE ? 128u : uint32_t((128 + p.epi.main.lo) * kResidualRowBytes));
+    bool tableReady = !RESIDUAL && !TABLE;
     int curC0 = -1, curBatch = -1;
     const bool hasClasses = p.rowClass != nullptr;
     const int baseClass = p.baseClass;
@@ -378,7 +385,7 @@ __device__ __forceinline__ void epilogueOcMajor(const CUtensorMap *tmapD, const 
                     borderFix(accA, 16 * st);
                 }
                 if (warpLive) {
-                    rescaleSlice<RESIDUAL>(accA, k, tab128, cd + uint32_t((16 * st) * 128));
+                    rescaleSlice<RESIDUAL, TABLE>(accA, k, tab128, cd + uint32_t((16 * st) * 128));
                 }
             }
         } else {
@@ -391,7 +398,7 @@ __device__ __forceinline__ void epilogueOcMajor(const CUtensorMap *tmapD, const 
                 borderFix(accA, 16 * st);
             }
             if (warpLive) {
-                rescaleSlice<RESIDUAL>(accA, k, tab128, cd + uint32_t((16 * st) * 128));
+                rescaleSlice<RESIDUAL, TABLE>(accA, k, tab128, cd + uint32_t((16 * st) * 128));
             }
             tmemWait16(accB);
             if (st + 2 < kSteps) {
@@ -407,7 +414,7 @@ __device__ __forceinline__ void epilogueOcMajor(const CUtensorMap *tmapD, const 
                 borderFix(accB, 16 * (st + 1));
             }
             if (warpLive) {
-                rescaleSlice<RESIDUAL>(accB, k, tab128, cd + uint32_t((16 * (st + 1)) * 128));
+                rescaleSlice<RESIDUAL, TABLE>(accB, k, tab128, cd + uint32_t((16 * (st + 1)) * 128));
             }
         }
         }

@@ -99,6 +99,7 @@ DevEpilogue devEpilogue(const FusedEpilogue &e, const TView *T) {
         d.out = devRescale(e.out, T);
         d.shortcut = e.shortcutTensor >= 0 ? reinterpret_cast<const int8_t *>(T[e.shortcutTensor].ptr) : nullptr;
     }
+    d.table = e.tableTensor >= 0 ? reinterpret_cast<const int8_t *>(T[e.tableTensor].ptr) : nullptr;
     return d;
 }
 
@@ -236,7 +237,8 @@ int launchConvTensorCore(const OpDesc &op, const TView *T, cudaStream_t s, Launc
 }
 
 // MATMUL / fused MATMUL: second input constant and pre-transposed (tc == 1), or transposed here (tc == 3).
-int launchMatmulTensorCore(const OpDesc &op, const TView *T, cudaStream_t s) {
+// *tableDone: the kernel has looked up the epilogue's table, if there is one.
+int launchMatmulTensorCore(const OpDesc &op, const TView *T, cudaStream_t s, bool *tableDone) {
     const TView &a = T[op.in[0]], &out = T[op.out[0]];
     GemmI8Problem q{};
     GemmI8Params &p = q.params;
@@ -320,9 +322,30 @@ int launchMatmulTensorCore(const OpDesc &op, const TView *T, cudaStream_t s) {
     // ("pair_kernel" 2 asks for the paired kernel wherever it applies)
     const bool pairFirst = tensorCoreTuning().pairKernel.load(std::memory_order_relaxed) == 2;
     if ((pairFirst && tryPairKernel(q, false, s, &rc)) || trySmallKernel(q, s, &rc) || tryPairKernel(q, false, s, &rc)) {
+        *tableDone = true;
         return rc;
     }
     return gemmI8Launch(q, s);
+}
+
+int launchTable(const TView &in, const TView &out, const TView &table, cudaStream_t s) {
+    int rc = MLEL_SUCCESS;
+    return vecTable(in, out, table, s, &rc) ? rc : genericTable(in, out, table, s);
+}
+
+int launchMatmul(const OpDesc &op, const TView *T, cudaStream_t s) {
+    const TView &a = T[op.in[0]], &b = T[op.in[1]], &out = T[op.out[0]];
+    // Addresses are only known here: pointers that are not 16-byte aligned go to the generic kernels.
+    const bool tensorCore = op.tc != 0 && ((reinterpret_cast<uintptr_t>(a.ptr) | reinterpret_cast<uintptr_t>(out.ptr)) & 15u) == 0 &&
+                            (op.tc != 3 || (reinterpret_cast<uintptr_t>(b.ptr) & 15u) == 0);
+    bool tableDone = false;
+    const int rc = tensorCore                 ? launchMatmulTensorCore(op, T, s, &tableDone)
+                   : op.kind == OP_MATMUL ? genericMatmul(a, b, out, op.i[0], op.i[1], s)
+                                              : fusedMatmulGeneric(a, b, out, op.i[0], op.i[1], devEpilogue(op.epi, T), s);
+    if (rc != MLEL_SUCCESS || op.epi.tableTensor < 0 || tableDone) {
+        return rc;
+    }
+    return launchTable(out, out, T[op.epi.tableTensor], s); // in place, a thread reads what it writes
 }
 
 } // namespace
@@ -347,10 +370,6 @@ int launchOp(const OpDesc &op, const TView *T, cudaStream_t s, LaunchChain *chai
         if (aligned && (op.kind == OP_CONV2D || op.kind == OP_FUSED_CONV2D)) {
             return launchConvTensorCore(op, T, s, chain, &consumed);
         }
-        if (aligned && (op.kind == OP_MATMUL || op.kind == OP_FUSED_MATMUL) &&
-            (op.tc != 3 || (reinterpret_cast<uintptr_t>(in(1).ptr) & 15u) == 0)) {
-            return launchMatmulTensorCore(op, T, s);
-        }
     }
     switch (op.kind) {
     case OP_CONV2D:
@@ -361,7 +380,8 @@ int launchOp(const OpDesc &op, const TView *T, cudaStream_t s, LaunchChain *chai
         }
         return genericDepthwise(in(0), in(1), in(2), out, convAttr(op), s);
     case OP_MATMUL:
-        return genericMatmul(in(0), in(1), out, op.i[0], op.i[1], s);
+    case OP_FUSED_MATMUL:
+        return launchMatmul(op, T, s);
     case OP_RESCALE: {
         RescaleAttr a{op.i[0], op.i[1], op.i[2], op.i[3], op.i[4]};
         if (vecRescale(in(0), out, in(1), in(2), a, s, &rc)) {
@@ -380,10 +400,7 @@ int launchOp(const OpDesc &op, const TView *T, cudaStream_t s, LaunchChain *chai
         }
         return genericMaxPool(in(0), out, poolAttr(op), s);
     case OP_TABLE:
-        if (vecTable(in(0), out, in(1), s, &rc)) {
-            return rc;
-        }
-        return genericTable(in(0), out, in(1), s);
+        return launchTable(in(0), out, in(1), s);
     case OP_TRANSPOSE: {
         uint32_t perms[kMaxRank];
         for (int k = 0; k < kMaxRank; ++k) {
@@ -536,8 +553,6 @@ int launchOp(const OpDesc &op, const TView *T, cudaStream_t s, LaunchChain *chai
         }
         return fusedDepthwiseGeneric(in(0), in(1), in(2), out, convAttr(op), epi, s);
     }
-    case OP_FUSED_MATMUL:
-        return fusedMatmulGeneric(in(0), in(1), out, op.i[0], op.i[1], devEpilogue(op.epi, T), s);
     case OP_FUSED_ROWS:
         if (!op.rows) {
             setLastError("fused rows: no program");

@@ -187,6 +187,7 @@ struct FusedEpilogue {
     bool mainIsFirst{true}; // ADD(main, shortcut) or ADD(shortcut, main)
     int32_t shortcutTensor{-1};
     FusedRescale a, b, out;
+    int32_t tableTensor{-1}; // int8 TABLE (256 entries) behind the main stage
 };
 
 // A run of row-wise integer operators fused into one kernel (OP_FUSED_ROWS): every tensor of the run has the run's

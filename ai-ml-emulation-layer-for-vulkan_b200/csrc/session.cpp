@@ -328,6 +328,7 @@ int Session::resolve() {
             used.insert(f->shiftTensor);
         }
         used.insert(op.epi.shortcutTensor);
+        used.insert(op.epi.tableTensor);
         used.insert(std::begin(op.aux), std::end(op.aux));
         used.insert(op.scratch);
     }

@@ -1,0 +1,32 @@
+"""GPU parity of products whose RESCALE feeds an int8 TABLE: looked up in the small and the paired kernel's epilogue, applied
+in place behind the other kernels (run-time operand, NO_TENSOR_CORE), left alone where the rows are no whole 16 bytes.
+Bit-exact against the CPU oracle."""
+import numpy as np
+import pytest
+
+from mlel_b200.graph_builder import GraphBuilder
+from tests.test_gpu_vector_ops import check
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("batch,rows,k,n,constant,fused", [
+    (1, 5, 64, 144, True, True), (1, 200, 96, 256, True, True), (2, 300, 128, 400, True, True), (1, 1500, 768, 3072, True, True),
+    (1, 4000, 70, 272, True, True), (3, 257, 64, 512, False, True), (2, 65, 50, 160, False, True), (1, 64, 64, 128, True, False),
+    (1, 64, 64, 150, True, False),
+])
+@pytest.mark.parametrize("clamp", [False, True])
+def test_product_with_table(mlel, batch, rows, k, n, constant, fused, clamp):
+    from mlel_b200.runtime import GraphRunner
+    r = np.random.Generator(np.random.PCG64(rows + n))
+    a8, b8 = (r.integers(-128, 128, s, dtype=np.int8) for s in ((batch, rows, k), (batch, k, n)))
+    g = GraphBuilder()
+    a = g.input(np.int8, a8.shape)
+    b = g.constant(b8) if constant else g.input(np.int8, b8.shape)
+    lut = r.integers(-128, 128, (256,), dtype=np.int8)
+    for shift in (37, 31):
+        y = g.rescale(g.matmul(a, b, 3, 0), [1 << 30 | 12345], [shift], 0, 1, np.int8, double_round=True)
+        g.output(g.table(g.clamp(y, -100, 90) if clamp else y, lut))
+    names = GraphRunner(g).pipeline.exec_names()
+    assert all(x.endswith("+TABLE") for x in names) == fused, names
+    check(g, [a8] if constant else [a8, b8])
