@@ -1810,6 +1810,15 @@ void GraphPipeline::buildResidualTable(OpDesc &op) {
     op.aux[3] = addDerivedConstant(MLEL_U8, {int64_t(table.size())}, table.data());
 }
 
+// Sum of up to 65536 bytes (a function of its own: inside the loops around it the compiler did not vectorise it).
+static int32_t sumOfBytes(const int8_t *p, int64_t n) {
+    int32_t sum = 0;
+    for (int64_t i = 0; i < n; ++i) {
+        sum += p[i];
+    }
+    return sum;
+}
+
 void GraphPipeline::prepareTensorCore() {
     for (auto &op : exec_) {
         const bool conv = op.kind == OP_CONV2D || op.kind == OP_FUSED_CONV2D;
@@ -1893,12 +1902,7 @@ void GraphPipeline::prepareTensorCore() {
             std::vector<int64_t> wsum(size_t(KH * KW * OC), 0); // [ky][kx][oc]
             for (int64_t oc = 0; oc < OC; ++oc) {
                 for (int64_t t = 0; t < KH * KW; ++t) {
-                    int64_t acc = 0;
-                    const int8_t *row = wd + (oc * KH * KW + t) * IC;
-                    for (int64_t ic = 0; ic < IC; ++ic) {
-                        acc += row[ic];
-                    }
-                    wsum[size_t(t * OC + oc)] = acc;
+                    wsum[size_t(t * OC + oc)] = sumOfBytes(wd + (oc * KH * KW + t) * IC, IC);
                 }
             }
             const int64_t zx = op.i[8];
@@ -2048,15 +2052,27 @@ void GraphPipeline::prepareTensorCore() {
             std::vector<int8_t> bt(size_t(Nb * W * Cp), 0);
             std::vector<int32_t> corr(size_t(Nb * W));
             const int64_t za = op.i[0];
+            // 64 rows at a time: a strip's reads and writes stay in the cache (column by column over all rows it was a
+            // cache miss per byte, two thirds of the preparation of a transformer)
+            std::vector<int64_t> sums(size_t(W), 0);
             for (int64_t n = 0; n < Nb; ++n) {
-                for (int64_t w = 0; w < W; ++w) {
-                    int64_t sum = 0;
-                    for (int64_t c = 0; c < C; ++c) {
-                        const int8_t v = bdata[(n * C + c) * W + w];
-                        bt[size_t((n * W + w) * Cp + c)] = v;
-                        sum += v;
+                std::fill(sums.begin(), sums.end(), 0);
+                for (int64_t c0 = 0; c0 < C; c0 += 64) {
+                    const int64_t rows = std::min<int64_t>(64, C - c0);
+                    for (int64_t w = 0; w < W; ++w) {
+                        const int8_t *from = bdata + (n * C + c0) * W + w;
+                        int8_t *to = &bt[size_t((n * W + w) * Cp + c0)];
+                        int32_t sum = 0;
+                        for (int64_t c = 0; c < rows; ++c) {
+                            const int8_t v = from[c * W];
+                            to[c] = v;
+                            sum += v;
+                        }
+                        sums[size_t(w)] += sum;
                     }
-                    corr[size_t(n * W + w)] = int32_t(uint32_t(uint64_t(-za * sum)));
+                }
+                for (int64_t w = 0; w < W; ++w) {
+                    corr[size_t(n * W + w)] = int32_t(uint32_t(uint64_t(-za * sums[size_t(w)])));
                 }
             }
             op.aux[0] = addDerivedConstant(MLEL_I32, {Nb * W}, corr.data());
