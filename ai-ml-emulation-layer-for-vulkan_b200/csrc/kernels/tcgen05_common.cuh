@@ -398,21 +398,30 @@ template <class Encode> inline bool rememberedMap(CUtensorMap *map, const MapKey
         CUtensorMap map;
         bool valid = false;
     };
-    static thread_local std::vector<Entry> table(512);
+    constexpr size_t kWays = 4; // (with one, two maps of a program that shared a place were encoded anew on every pass)
+    static thread_local std::vector<Entry> table(128 * kWays);
+    static thread_local unsigned turn = 0;
     uint64_t h = 0xcbf29ce484222325ull;
     for (const uint64_t v : key.v) {
         h = (h ^ v) * 0x9e3779b97f4a7c15ull;
         h ^= h >> 29;
     }
-    Entry &e = table[h % table.size()];
-    if (e.valid && std::memcmp(&e.key, &key, sizeof(MapKey)) == 0) {
-        *map = e.map;
-        return true;
+    Entry *set = &table[h % (table.size() / kWays) * kWays];
+    Entry *slot = &set[turn % kWays];
+    for (size_t w = 0; w < kWays; ++w) {
+        if (set[w].valid && std::memcmp(&set[w].key, &key, sizeof(MapKey)) == 0) {
+            *map = set[w].map;
+            return true;
+        }
+        if (!set[w].valid) {
+            slot = &set[w];
+        }
     }
     if (!encode(map)) {
         return false;
     }
-    e.key = key, e.map = *map, e.valid = true;
+    ++turn;
+    slot->key = key, slot->map = *map, slot->valid = true;
     return true;
 }
 
