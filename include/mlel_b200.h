@@ -331,7 +331,7 @@ int mlel_selftest_wait_timeout(void *cuda_stream, int *recorded_code);
 
 /* Diagnostic (no counterpart in the reference): how often the library has enqueued tensor-core kernel
  * `kernel` since it was loaded -- 0 the pixel-major tcgen05 kernel, 1 the channel-major one, 2 the paired
- * (two-CTA) one, 3 the small-problem one; -1 for another index.  Tests use it to see which kernel took a case. */
+ * (two-CTA) one, 3 the small-problem one, 4 the window one; -1 for another index.  Tests use it to see which kernel took a case. */
 long long mlel_tensor_core_launches(int kernel);
 
 /* Number of kernels one dispatch launches. */
