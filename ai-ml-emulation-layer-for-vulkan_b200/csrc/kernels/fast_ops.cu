@@ -273,13 +273,13 @@ __global__ void __launch_bounds__(256) columnSumKernel(const int8_t *__restrict_
 }
 
 // ---- AVG_POOL2D, int8 NHWC (avgpool2d.comp:27-75) ---------------------------------------------------------
-// One output pixel and up to `width` channel units (a unit is four channels, or one where C % 4 != 0) belong to a cluster of
+// One output pixel and up to `width` channel units (a unit is 16 channels, or four or one where C asks for it) belong to a cluster of
 // `split` blocks.  The in-range part of a window is rows of contiguous bytes, one run when it spans whole image rows (a
 // global pool), so a thread keeps one channel unit and strides over the pixels of its block's share: consecutive threads
 // read consecutive bytes whatever the channel count.  Partial sums join in shared memory, first of the block, then of
 // the cluster's blocks in block 0 (distributed shared memory).
 // The classifier's pool has one output pixel per image: one block for each left the chip idle on small batches and large
-// windows (64 images of 112 x 112 x 64: 264 us with one block per pixel, 64 blocks, now 20.5; a channel count that is no
+// windows (64 images of 112 x 112 x 64: 264 us with one block per pixel, 64 blocks, now 16.6, with 16-byte units, 20.5 with 4-byte ones; a channel count that is no
 // multiple of 16 took the one-thread-per-output kernel: 3 x 57 x 57 x 36, 990 us, now 9).
 template <int CH>
 __global__ void __launch_bounds__(256) avgPoolI8Kernel(const int8_t *__restrict__ in, int8_t *__restrict__ out, int H, int W,
@@ -312,7 +312,14 @@ __global__ void __launch_bounds__(256) avgPoolI8Kernel(const int8_t *__restrict_
         const int line0 = joined ? 0 : int(int64_t(lines) * rank / split), line1 = joined ? 1 : int(int64_t(lines) * (rank + 1) / split);
         const int from = joined ? int(int64_t(length) * rank / split) : 0, to = joined ? int(int64_t(length) * (rank + 1) / split) : length;
         const auto take = [&](const int8_t *p) {
-            if (CH == 4) {
+            if (CH == 16) {
+                const int4 v = __ldg(reinterpret_cast<const int4 *>(p));
+                const int words[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+                for (int k = 0; k < CH; ++k) {
+                    acc[k] = __dp4a(words[k >> 2], 1 << (8 * (k & 3)), acc[k]);
+                }
+            } else if (CH == 4) {
                 const int word = __ldg(reinterpret_cast<const int *>(p));
 #pragma unroll
                 for (int k = 0; k < CH; ++k) {
@@ -714,14 +721,15 @@ bool avgPoolI8Eligible(const TView &in, const TView &out, const PoolAttr &a) {
 
 int avgPoolI8(const TView &in, const TView &out, const PoolAttr &a, cudaStream_t s) {
     const int C = int(in.dims[3]);
-    const int ch = poolUnit(in, out) == 1 ? 1 : 4, units = C / ch;
+    const int ch = poolUnit(in, out), units = C / ch; // 16, 4 or 1 channels
     const int64_t pixels = int64_t(out.dims[0]) * out.dims[1] * out.dims[2];
-    // More blocks while the SMs are not filled four times over: first of fewer channels, down to 32 units (full 32-byte
-    // sectors), so that a block has more pixels in flight; then a cluster per group while a block's share is no less than
-    // the 256 threads fetch in one go of eight words (below that the cluster's barriers cost more than the shorter walk
+    // More blocks while the SMs are not filled four times over: first of fewer channels, down to 128 bytes, so that a
+    // block has more pixels in flight; then a cluster per group while a block's share is no less than the 256 threads
+    // fetch in one go of eight units (below that the cluster's barriers cost more than the shorter walk
     // gives: 64 images of 7 x 7 x 2048 took 20.4 us as clusters of eight blocks of 256 units).
     int width = 256;
-    while (width > 32 && pixels * ((units + width - 1) / width) < 4 * kNumSMs) {
+    const int narrowest = ch == 16 ? 8 : 32;
+    while (width > narrowest && pixels * ((units + width - 1) / width) < 4 * kNumSMs) {
         width /= 2;
     }
     const int chunks = (units + width - 1) / width;
@@ -742,7 +750,7 @@ int avgPoolI8(const TView &in, const TView &out, const PoolAttr &a, cudaStream_t
     attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
     cfg.attrs = &attr;
     cfg.numAttrs = 1;
-    cudaLaunchKernelEx(&cfg, ch == 4 ? avgPoolI8Kernel<4> : avgPoolI8Kernel<1>, reinterpret_cast<const int8_t *>(in.ptr),
+    cudaLaunchKernelEx(&cfg, ch == 16 ? avgPoolI8Kernel<16> : (ch == 4 ? avgPoolI8Kernel<4> : avgPoolI8Kernel<1>), reinterpret_cast<const int8_t *>(in.ptr),
                        reinterpret_cast<int8_t *>(out.ptr), int(in.dims[1]), int(in.dims[2]), C, int(out.dims[1]),
                        int(out.dims[2]), chunks, width, split, a);
     return finish("AVG_POOL2D");
