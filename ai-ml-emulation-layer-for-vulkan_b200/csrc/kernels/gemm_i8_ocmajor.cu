@@ -49,7 +49,7 @@ constexpr int ocThreadsFor(int ew, int xMode) { return xMode == kXGather ? ocThr
 // X_MODE: how the pixel operand arrives: kXGather = gathered from the NHWC input described by p, kXTiled = tmapX
 // is a plain matrix, kXIm2col = tmapX is an im2col map of the NHWC input.
 // RESIDUAL: the fused residual tail is present (tmapC describes the shortcut tensor).
-template <int BNP, int NSTAGE, int EW, int X_MODE, bool RESIDUAL>
+template <int BNP, int NSTAGE, int EW, int X_MODE, bool RESIDUAL, bool ODD = false>
 __global__ void __launch_bounds__(ocThreadsFor(EW, X_MODE), 1)
 gemmI8OcMajor(const __grid_constant__ CUtensorMap tmapX, const __grid_constant__ CUtensorMap tmapW,
               const __grid_constant__ CUtensorMap tmapC, const __grid_constant__ CUtensorMap tmapD, const GemmI8Params p) {
@@ -260,7 +260,7 @@ gemmI8OcMajor(const __grid_constant__ CUtensorMap tmapX, const __grid_constant__
     } else if (warp >= kOcGatherWarp0) {
         if (X_TMA) {
             // ---------------- store warp ----------------
-            if (lane == 0) {
+            if (lane == 0 && !ODD) {
                 EpiWalk walk{};
                 walk.first = blockIdx.x, walk.stride = gridDim.x;
                 storeWarpOcMajor<BNP, EW, kOcTile>(&tmapD, p, bars, cdTiles, numTiles, pTiles, cTiles, walk);
@@ -301,7 +301,7 @@ gemmI8OcMajor(const __grid_constant__ CUtensorMap tmapX, const __grid_constant__
         // ---------------- epilogue ----------------
         EpiWalk walk{};
         walk.first = blockIdx.x, walk.stride = gridDim.x;
-        epilogueOcMajor<BNP, EW, RESIDUAL, kOcTile, X_TMA>(&tmapD, p, bars, resTab, cdTiles, tmemBase, warp, lane,
+        epilogueOcMajor<BNP, EW, RESIDUAL, kOcTile, X_TMA, false, ODD>(&tmapD, p, bars, resTab, cdTiles, tmemBase, warp, lane,
                                                            numTiles, pTiles, cTiles, walk);
     }
 
@@ -318,7 +318,7 @@ struct OcMaps {
     CUtensorMap x, w, c, d;
 };
 
-template <int BNP, int NSTAGE, int EW, int X_MODE, bool RESIDUAL>
+template <int BNP, int NSTAGE, int EW, int X_MODE, bool RESIDUAL, bool ODD = false>
 int launchOcMajor(const OcMaps &maps, const GemmI8Params &params, cudaStream_t s) {
     GemmI8Params p = params;
     p.divPlane = makeFastDiv(int64_t(p.OH) * p.OW), p.divOW = makeFastDiv(p.OW);
@@ -329,7 +329,7 @@ int launchOcMajor(const OcMaps &maps, const GemmI8Params &params, cudaStream_t s
                                  (RESIDUAL ? size_t(kResidualTableBytes) : 0) +
                                  kTapTabEntries * sizeof(int32_t) + sizeof(OcBarriers) + 1024;
     static_assert(smemBytes <= 232448, "shared memory per CTA");
-    auto kernel = gemmI8OcMajor<BNP, NSTAGE, EW, X_MODE, RESIDUAL>;
+    auto kernel = gemmI8OcMajor<BNP, NSTAGE, EW, X_MODE, RESIDUAL, ODD>;
     if (!allowDynamicSmem(reinterpret_cast<const void *>(kernel), smemBytes)) {
         return MLEL_ERROR_DEVICE;
     }
@@ -357,8 +357,15 @@ int launchOcMajorMode(const OcMaps &maps, const GemmI8Params &p, cudaStream_t s)
                              : launchOcMajor<BNP, NSTAGE, EW, X_MODE, false>(maps, p, s);
 }
 
+// Output rows that do not all start on 16-byte boundaries.
+bool oddRows(const GemmI8Params &p) { return p.ldOut % 16 != 0 || (reinterpret_cast<uintptr_t>(p.out8) & 15u) != 0; }
+
 template <int BNP, int NSTAGE, int EW>
 int launchOcMajorShape(const OcMaps &maps, const GemmI8Params &p, int xMode, cudaStream_t s) {
+    if (oddRows(p)) { // (never gathered, no residual tail: gemmI8OcMajorApplies)
+        return xMode == kXTiled ? launchOcMajor<BNP, NSTAGE, EW, kXTiled, false, true>(maps, p, s)
+                                : launchOcMajor<BNP, NSTAGE, EW, kXIm2col, false, true>(maps, p, s);
+    }
     if (xMode == kXTiled) {
         return launchOcMajorMode<BNP, NSTAGE, EW, kXTiled>(maps, p, s);
     }
@@ -375,8 +382,11 @@ bool gemmI8OcMajorApplies(const GemmI8Problem &q) {
     if (p.out8 == nullptr || !p.epi.hasMain || q.bMnMajor || p.batchedB || q.batches != 1 || p.N <= 64) {
         return false;
     }
-    // the output (and the shortcut) move as TMA tiles of 16-byte aligned rows
-    if (p.N % 16 != 0 || p.ldOut % 16 != 0 || (reinterpret_cast<uintptr_t>(p.out8) & 15u) != 0) {
+    // The shortcut, and the output where it can, move as TMA tiles of 16-byte aligned rows.  Rows at other addresses are
+    // stored by the epilogue warps of the TMA variants.
+    if (oddRows(p) && (p.epi.hasResidual || p.gatherTable != nullptr ||
+                       (q.aMatrix == nullptr && (p.IC % 16 != 0 || ((reinterpret_cast<uintptr_t>(p.in) |
+                                                                     reinterpret_cast<uintptr_t>(q.bMatrix)) & 15u) != 0)))) {
         return false;
     }
     // a gathered pixel operand goes through the segment gather
@@ -403,7 +413,6 @@ bool gemmI8OcMajorApplies(const GemmI8Problem &q) {
 // griddepcontrol.wait has returned, i.e. before B has ended.  (5) The counters are zeroed by a memset at the start of
 // the dispatch, which is ordered after the previous dispatch like any other operation of the stream.
 int gemmI8OcMajorLaunch(const GemmI8Problem &q, cudaStream_t s, LaunchChain *chain, const LaunchChain *consumed) {
-    g_tensorCoreLaunches[1].fetch_add(1, std::memory_order_relaxed);
     GemmI8Params p = q.params;
     p.batches = q.batches;
     p.progressOut = nullptr, p.progressIn = nullptr, p.channelFastest = 0;
@@ -459,9 +468,13 @@ int gemmI8OcMajorLaunch(const GemmI8Problem &q, cudaStream_t s, LaunchChain *cha
                                       uint64_t(q.bRowBytes) * uint64_t(p.N), BK, kOcTile)) {
         return MLEL_ERROR_DEVICE;
     }
+    if (oddRows(p) && xMode == kXGather) { // the driver refused the im2col map
+        return gemmI8Launch(q, s);
+    }
+    g_tensorCoreLaunches[1].fetch_add(1, std::memory_order_relaxed);
     // output and shortcut: [pixels][channels] bytes, unswizzled tiles of 128 channels x (128 or 256) pixels
     const uint64_t plane = uint64_t(p.ldOut) * uint64_t(p.M);
-    if (!makeMap(&maps.d, p.out8, uint64_t(p.N), uint64_t(p.M), 1, uint64_t(p.ldOut), plane, kOcTile, boxPixels, false)) {
+    if (!oddRows(p) && !makeMap(&maps.d, p.out8, uint64_t(p.N), uint64_t(p.M), 1, uint64_t(p.ldOut), plane, kOcTile, boxPixels, false)) {
         return MLEL_ERROR_DEVICE;
     }
     if (p.epi.hasResidual &&
@@ -481,7 +494,7 @@ int gemmI8OcMajorLaunch(const GemmI8Problem &q, cudaStream_t s, LaunchChain *cha
             p.progressInTarget = before.prevTarget;
         }
     }
-    if (handOver && chain->publishNext && (progressMode & 2)) {
+    if (handOver && chain->publishNext && (progressMode & 2) && !oddRows(p)) {
         const size_t pixelTiles = size_t((p.M + width - 1) / width);
         if (chain->used + pixelTiles <= chain->capacity) {
             p.progressOut = chain->words + chain->used;

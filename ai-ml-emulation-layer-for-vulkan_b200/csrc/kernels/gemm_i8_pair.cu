@@ -185,7 +185,7 @@ __device__ __forceinline__ uint32_t tmaStagePeekIm2colPair(uint64_t *fullOwn, ui
 // X_MODE: kXTiled = tmapX is a K-major matrix {K, M, batches}; kXIm2col = tmapX is an im2col map of the NHWC input
 //         and tmapW the {IC, taps, OC} weight map.
 // W_MN  : tmapW is {N, K, batches}, N contiguous (kXTiled only).
-template <int BNP, int NSTAGE, int EW, int X_MODE, bool W_MN, bool RESIDUAL, bool TABLE = false>
+template <int BNP, int NSTAGE, int EW, int X_MODE, bool W_MN, bool RESIDUAL, bool TABLE = false, bool ODD = false>
 __global__ void __launch_bounds__((EW + 4) * 32, 1)
 gemmI8Pair(const __grid_constant__ CUtensorMap tmapX, const __grid_constant__ CUtensorMap tmapW,
            const __grid_constant__ CUtensorMap tmapC, const __grid_constant__ CUtensorMap tmapD, const GemmI8Params p) {
@@ -412,7 +412,7 @@ gemmI8Pair(const __grid_constant__ CUtensorMap tmapX, const __grid_constant__ CU
         }
     } else if (warp == kStoreWarpP) {
         // ---------------- store warp (both CTAs) ----------------
-        if (lane == 0) {
+        if (lane == 0 && !ODD) {
             EpiWalk walk{};
             walk.first = pairIdx, walk.stride = numPairs;
             walk.cOffset = int(rank) * kOcTile;
@@ -425,7 +425,7 @@ gemmI8Pair(const __grid_constant__ CUtensorMap tmapX, const __grid_constant__ CU
         walk.cOffset = int(rank) * kOcTile;
         walk.accEmpty[0] = mapToCta(smemAddr(&bars->accEmpty[0]), 0u);
         walk.accEmpty[1] = mapToCta(smemAddr(&bars->accEmpty[1]), 0u);
-        epilogueOcMajor<BNP, EW, RESIDUAL, kPairChannels, true, TABLE>(&tmapD, p, bars, resTab, cdTiles, tmemBase,
+        epilogueOcMajor<BNP, EW, RESIDUAL, kPairChannels, true, TABLE, ODD>(&tmapD, p, bars, resTab, cdTiles, tmemBase,
                                                                 warp - kFirstEpiWarp, lane, numTiles, pTiles, cTiles, walk);
     }
 
@@ -443,7 +443,7 @@ struct PairMaps {
     CUtensorMap x, w, c, d;
 };
 
-template <int BNP, int NSTAGE, int EW, int X_MODE, bool W_MN, bool RESIDUAL, bool TABLE = false>
+template <int BNP, int NSTAGE, int EW, int X_MODE, bool W_MN, bool RESIDUAL, bool TABLE = false, bool ODD = false>
 int launchPair(const PairMaps &maps, const GemmI8Params &params, cudaStream_t s) {
     GemmI8Params p = params;
     p.divPlane = makeFastDiv(int64_t(p.OH) * p.OW), p.divOW = makeFastDiv(p.OW);
@@ -451,7 +451,7 @@ int launchPair(const PairMaps &maps, const GemmI8Params &params, cudaStream_t s)
     constexpr size_t smemBytes = size_t(NSTAGE) * (kOcTile * BK + (BNP / 2) * BK) + 2 * size_t(BNP) * 128 +
                                  (RESIDUAL ? size_t(kResidualTableBytes) : (TABLE ? 256 : 0)) + sizeof(OcBarriers) + 1024;
     static_assert(smemBytes <= 232448, "shared memory per CTA");
-    auto kernel = gemmI8Pair<BNP, NSTAGE, EW, X_MODE, W_MN, RESIDUAL, TABLE>;
+    auto kernel = gemmI8Pair<BNP, NSTAGE, EW, X_MODE, W_MN, RESIDUAL, TABLE, ODD>;
     if (!allowDynamicSmem(reinterpret_cast<const void *>(kernel), smemBytes)) {
         return MLEL_ERROR_DEVICE;
     }
@@ -482,6 +482,9 @@ int launchPair(const PairMaps &maps, const GemmI8Params &params, cudaStream_t s)
     return MLEL_SUCCESS;
 }
 
+// Output rows that do not all start on 16-byte boundaries (see ODD in epilogueOcMajor).
+bool pairOddRows(const GemmI8Params &p) { return p.ldOut % 16 != 0 || (reinterpret_cast<uintptr_t>(p.out8) & 15u) != 0; }
+
 template <int BNP, int NSTAGE, int NSTAGE_RES, int EW>
 int launchPairShape(const PairMaps &maps, const GemmI8Params &p, int xMode, bool wMn, cudaStream_t s) {
     if (p.epi.hasResidual) {
@@ -490,6 +493,9 @@ int launchPairShape(const PairMaps &maps, const GemmI8Params &p, int xMode, bool
     }
     if (xMode == kXIm2col) {
         return launchPair<BNP, NSTAGE, EW, kXIm2col, false, false>(maps, p, s);
+    }
+    if (pairOddRows(p)) { // (a matrix product with a K-contiguous second operand: gemmI8PairApplies)
+        return launchPair<BNP, NSTAGE, EW, kXTiled, false, false, false, true>(maps, p, s);
     }
     if (p.epi.table != nullptr && !wMn) {
         return launchPair<BNP, NSTAGE, EW, kXTiled, false, false, true>(maps, p, s);
@@ -505,7 +511,13 @@ bool gemmI8PairApplies(const GemmI8Problem &q) {
     if (p.out8 == nullptr || !p.epi.hasMain || p.N <= kOcTile || p.gatherTable != nullptr) {
         return false;
     }
-    if (p.N % 16 != 0 || p.ldOut % 16 != 0 || q.bRowBytes % 16 != 0 || (reinterpret_cast<uintptr_t>(p.out8) & 15u) != 0 ||
+    // Rows at odd addresses: where the tiles give half of the pairs work (4 x 300 x 200 x 301 with 16 tiles took 14.5 us here
+    // and 12.4 on the pixel-major kernel's smaller tiles; 40 x 300 x 511 x 511 37 and 48).
+    const int64_t tiles = int64_t((p.M + 191) / 192) * ((p.N + kPairChannels - 1) / kPairChannels) * q.batches;
+    if (pairOddRows(p) && (q.bMnMajor || q.aMatrix == nullptr || p.epi.hasResidual || p.epi.table != nullptr || 4 * tiles < smCount())) {
+        return false;
+    }
+    if (q.bRowBytes % 16 != 0 ||
         (reinterpret_cast<uintptr_t>(q.bMatrix) & 15u) != 0) {
         return false;
     }
@@ -586,7 +598,7 @@ int gemmI8PairLaunch(const GemmI8Problem &q, cudaStream_t s, bool *taken) {
         p.kbPerTap = (p.IC + 127) / 128;
     }
     const uint64_t plane = uint64_t(p.ldOut) * uint64_t(p.M);
-    if (!makeMap(&maps.d, p.out8, uint64_t(p.N), uint64_t(p.M), uint64_t(q.batches), uint64_t(p.ldOut), plane, kOcTile,
+    if (!pairOddRows(p) && !makeMap(&maps.d, p.out8, uint64_t(p.N), uint64_t(p.M), uint64_t(q.batches), uint64_t(p.ldOut), plane, kOcTile,
                  uint32_t(width), false)) {
         return MLEL_ERROR_DEVICE;
     }

@@ -130,11 +130,6 @@ __device__ __forceinline__ void tmaStore3d(const CUtensorMap *map, const void *s
 
 // Shared-memory accesses by 32-bit shared address (a pointer into dynamic shared memory that has been passed
 // through a few functions is otherwise accessed with generic 64-bit loads and stores).
-__device__ __forceinline__ uint32_t ldsU8(uint32_t addr) {
-    uint32_t v;
-    asm volatile("ld.shared.u8 %0, [%1];" : "=r"(v) : "r"(addr));
-    return v;
-}
 __device__ __forceinline__ void stsU8(uint32_t addr, int32_t v) {
     asm volatile("st.shared.u8 [%0], %1;" ::"r"(addr), "r"(v) : "memory");
 }
@@ -233,7 +228,11 @@ __device__ __forceinline__ void mbarArriveCluster(uint32_t clusterAddr) {
 // pixels, which it walks in slices of 16 pixels; the tcgen05.ld of the next slice is in flight while the
 // current one is rescaled.  C_TILE: output channels per tile (128, or 256 for a pair of CTAs).
 // TABLE: resTab holds the 256 entries of a byte table that the results go through.
-template <int BNP, int EW, bool RESIDUAL, int C_TILE, bool STORE_WARP = false, bool TABLE = false>
+// ODD: output rows start at any address (a TMA store wants 16-byte boundaries): the epilogue warps meet when a tile is
+// complete and store its rows themselves.  (The pixel-major kernel, which took such widths, needed twice to three times
+// as long: 8 x 56 x 56, 256 -> 255 channels 21.0 us, here 11.6, 128 -> 255 with a 3x3 window 26.0 and
+// 21.5; 16 x 1023^3 82 and 57.5.)
+template <int BNP, int EW, bool RESIDUAL, int C_TILE, bool STORE_WARP = false, bool TABLE = false, bool ODD = false>
 __device__ __forceinline__ void epilogueOcMajor(const CUtensorMap *tmapD, const GemmI8Params &p, OcBarriers *bars,
                                                 const uint8_t *resTab, uint8_t *cdTiles,
                                                 uint32_t tmemBase, int warp, int lane, int64_t numTiles, int pTiles,
@@ -258,6 +257,7 @@ __device__ __forceinline__ void epilogueOcMajor(const CUtensorMap *tmapD, const 
     // row of the lowest main-stage value: the element loop counts rows from there
     const uint32_t tab128 = smemAddr(resTab) + (TABLE ? 128u : uint32_t((128 + p.epi.main.lo) * kResidualRowBytes));
     bool tableReady = !RESIDUAL && !TABLE;
+    bool failed = false;
     int curC0 = -1, curBatch = -1;
     const bool hasClasses = p.rowClass != nullptr;
     const int baseClass = p.baseClass;
@@ -335,10 +335,12 @@ __device__ __forceinline__ void epilogueOcMajor(const CUtensorMap *tmapD, const 
         if (RESIDUAL && !mbarWait(&bars->cFull[buf], par, 6)) {
             break;
         }
-        if (STORE_WARP && !RESIDUAL && !mbarWait(&bars->cdEmpty[buf], par ^ 1u, 18)) {
+        if (STORE_WARP && !RESIDUAL && !ODD && !mbarWait(&bars->cdEmpty[buf], par ^ 1u, 18)) {
             break; // (the store that last read this C/D tile; passes at once for the first two tiles)
         }
-        if (!mbarWait(&bars->accFull[buf], par, 4)) {
+        if (ODD) { // after a wait that ran out the warp still meets the others
+            failed = failed || !mbarWait(&bars->accFull[buf], par, 4);
+        } else if (!mbarWait(&bars->accFull[buf], par, 4)) {
             break;
         }
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -417,6 +419,20 @@ __device__ __forceinline__ void epilogueOcMajor(const CUtensorMap *tmapD, const 
                 rescaleSlice<RESIDUAL, TABLE>(accB, k, tab128, cd + uint32_t((16 * (st + 1)) * 128));
             }
         }
+        }
+        if (ODD) {
+            if (p.progressIn != nullptr && tileCount == 0) {
+                gridDependencySync(); // (see below)
+            }
+            ocEpilogueSync<EW>(); // the tile is complete; its buffer's next writers come from the barrier of the tile after
+            const int rows = min(BNP, p.M - m0), length = min(kOcTile, p.N - c0);
+            int8_t *to = p.out8 + (int64_t(batch) * p.M + m0) * p.ldOut + c0;
+            const uint32_t from = smemAddr(cdTiles + buf * (BNP * 128));
+#pragma unroll 4
+            for (int r = warp; r < rows; r += EW) {
+                storeRowBytes(to + int64_t(r) * p.ldOut, from + uint32_t(r) * 128u, length, lane);
+            }
+            continue;
         }
         // make the tile visible to the TMA unit, then one thread stores it (pixels and channels past the
         // tensor's end are clipped by the tensor map)

@@ -274,6 +274,30 @@ __device__ __forceinline__ void gridDependencySync() {
     asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
+__device__ __forceinline__ uint32_t ldsU8(uint32_t addr) {
+    uint32_t v;
+    asm volatile("ld.shared.u8 %0, [%1];" : "=r"(v) : "r"(addr));
+    return v;
+}
+
+// `length` bytes (up to 128) from shared memory (address `from`, a word boundary) to any address: aligned words, lane l the
+// l-th, and the up to three bytes before and behind them from lanes of their own.  No loop and no branch: as a loop over
+// words with the ends byte by byte a row took a hundred instructions, as many as its arithmetic.
+__device__ __forceinline__ void storeRowBytes(int8_t *to, uint32_t from, int length, int lane) {
+    const int head = min(int((0u - uint32_t(reinterpret_cast<uintptr_t>(to))) & 3u), length);
+    const int words = (length - head) >> 2, tail = length - head - 4 * words;
+    const int edge = lane < 8 ? lane : length - tail + lane - 8; // lanes 0-2: bytes before the words, 8-10: behind them
+    if (lane < words) {
+        uint32_t here, next;
+        asm volatile("ld.shared.u32 %0, [%1];" : "=r"(here) : "r"(from + uint32_t(4 * lane)) : "memory");
+        asm volatile("ld.shared.u32 %0, [%1];" : "=r"(next) : "r"(from + uint32_t(4 * lane + 4)) : "memory");
+        reinterpret_cast<uint32_t *>(to + head)[lane] = __funnelshift_r(here, next, 8u * uint32_t(head));
+    }
+    if (lane < head || (lane >= 8 && lane < 8 + tail)) {
+        to[edge] = int8_t(ldsU8(from + uint32_t(edge)));
+    }
+}
+
 // Barrier among the epilogue warps only (named barrier 1).
 // n / f.d for n < 2^31 (see FastDiv)
 __device__ __forceinline__ uint32_t fastDiv(uint32_t n, const FastDiv &f) {

@@ -38,3 +38,17 @@ def test_rows_at_odd_addresses_with_residual_tail(mlel, channels):
     g.output(g.rescale(g.add(a, b), [int(r.integers(1 << 30, 1 << 31))], [40], 0, -20, np.int8, double_round=True))
     g.output(conv(g, r, x, channels, 3, 1, 1, 4, True))
     check(g, [r.integers(-128, 128, x.shape, dtype=np.int8)])
+
+
+@pytest.mark.parametrize("n,hw,ic,oc,k,stride", [
+    (2, 40, 64, 65, 1, 1), (8, 30, 256, 255, 1, 1), (4, 41, 128, 131, 3, 1), (3, 57, 48, 200 + 1, 3, 2), (1, 300, 16, 127, 1, 1),
+    (9, 56, 32, 385, 1, 1), (2, 33, 50, 90, 1, 1),
+])
+def test_wide_convolutions_with_rows_at_odd_addresses(mlel, n, hw, ic, oc, k, stride):
+    r = np.random.Generator(np.random.PCG64(hw + oc))
+    g = GraphBuilder()
+    x = g.input(np.int8, (n, hw, hw, ic))
+    y = conv(g, r, x, oc, k, stride, k // 2, -7, True)
+    g.output(conv(g, r, y, oc, 1, 1, 0, 4, False))
+    g.output(conv(g, r, x, oc, k, stride, k // 2, 5, False, 33))
+    check(g, [r.integers(-128, 128, x.shape, dtype=np.int8)])
