@@ -178,54 +178,41 @@ int launchConvTensorCore(const OpDesc &op, const TView *T, cudaStream_t s, Launc
         q.bMatrix = T[op.aux[3]].ptr;
         return gemmI8UnitsLaunch(q, u, s);
     }
+    const void *weights = w.ptr;
     if (op.tc == 2) {
-        // Channel count not a multiple of 16: gather, by a table of offsets, from a copy of the input with
-        // zero-padded channels and borders.
+        // Channel count not a multiple of 16: from a copy of the input with zero-padded channels.
         const TView &copy = T[op.scratch];
-        const int rc = padImageI8(p.in, reinterpret_cast<int8_t *>(copy.ptr), int(in.dims[0]), p.H, p.W, p.IC,
-                                  int(copy.dims[1]), int(copy.dims[2]), int(copy.dims[3]), p.padTop, p.padLeft, s);
+        const int ICp = int(copy.dims[3]);
+        const bool whole = op.aux[4] < 0; // else with borders, for the gather by a table of offsets
+        const int rc = padImageI8(p.in, reinterpret_cast<int8_t *>(copy.ptr), int(in.dims[0]), p.H, p.W, p.IC, int(copy.dims[1]),
+                                  int(copy.dims[2]), ICp, whole ? 0 : p.padTop, whole ? 0 : p.padLeft, s);
         if (rc != MLEL_SUCCESS) {
             return rc;
         }
         p.in = reinterpret_cast<const int8_t *>(copy.ptr);
-        p.H = int32_t(copy.dims[1]), p.W = int32_t(copy.dims[2]), p.IC = int32_t(copy.dims[3]);
-        p.padTop = p.padLeft = 0;
+        p.H = int32_t(copy.dims[1]), p.W = int32_t(copy.dims[2]), p.IC = ICp;
         p.K = int32_t(T[op.aux[3]].dims[1]);
-        if (p.KH == 1 && p.KW == 1 && p.strideY == 1 && p.strideX == 1 && p.H == p.OH && p.W == p.OW && p.IC % 16 == 0 &&
-            p.K == p.IC) {
-            // A 1x1 convolution over the copy (channels padded to a multiple of 16, weights padded alike) is a plain
-            // [pixels][channels] matrix product: TMA tiles instead of the table gather, and the channel-major kernel
-            // where it applies (e.g. the 24 -> 144 expansions of a MobileNetV2-shaped graph: 48 -> 20 us).
-            q.aMatrix = copy.ptr;
-            q.aRowBytes = uint64_t(p.IC);
-            q.aBatchBytes = uint64_t(p.IC) * uint64_t(p.M);
-            q.bMatrix = T[op.aux[3]].ptr;
+        weights = T[op.aux[3]].ptr;
+        if (!whole) {
+            p.padTop = p.padLeft = 0;
+            p.chunkBytes = op.auxi[2];
+            p.gatherTable = reinterpret_cast<const int32_t *>(T[op.aux[4]].ptr);
+            q.bMatrix = weights;
             q.bRowBytes = uint64_t(p.K);
             q.bBatchBytes = 0;
             q.bMnMajor = false;
-            int smallRc = MLEL_SUCCESS;
-            if (trySmallKernel(q, s, &smallRc)) {
-                return smallRc;
-            }
-            return gemmI8OcMajorApplies(q) ? gemmI8OcMajorLaunch(q, s) : gemmI8Launch(q, s);
+            return gemmI8Launch(q, s);
         }
-        p.chunkBytes = op.auxi[2];
-        p.gatherTable = reinterpret_cast<const int32_t *>(T[op.aux[4]].ptr);
-        q.bMatrix = T[op.aux[3]].ptr;
-        q.bRowBytes = uint64_t(p.K);
-        q.bBatchBytes = 0;
-        q.bMnMajor = false;
-        return gemmI8Launch(q, s);
     }
     // A 1x1, stride-1, unpadded convolution reads the input as a plain [pixels][IC] matrix.
     const bool plain = p.KH == 1 && p.KW == 1 && p.strideY == 1 && p.strideX == 1 && op.i[0] == 0 && op.i[1] == 0 &&
-                       op.i[2] == 0 && op.i[3] == 0 && (reinterpret_cast<uintptr_t>(in.ptr) & 15u) == 0;
+                       op.i[2] == 0 && op.i[3] == 0 && (reinterpret_cast<uintptr_t>(p.in) & 15u) == 0;
     if (plain) {
-        q.aMatrix = in.ptr;
+        q.aMatrix = p.in;
         q.aRowBytes = uint64_t(p.IC);
         q.aBatchBytes = uint64_t(p.IC) * uint64_t(p.M);
     }
-    q.bMatrix = w.ptr;
+    q.bMatrix = weights;
     q.bRowBytes = uint64_t(p.K);
     q.bBatchBytes = 0;
     q.bMnMajor = false;

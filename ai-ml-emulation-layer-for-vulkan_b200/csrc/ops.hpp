@@ -251,9 +251,10 @@ struct OpDesc {
     //   MATMUL kinds with a constant second input: aux[0] correction int32 [batches][W],
     //                 aux[3] the second input transposed to [batches][W][C]
     //   CONV2D kinds with tc == 2 (channel count not a multiple of 16): scratch = session tensor
-    //                 [N][Hp][Wp][ICp], a copy of the input with zero-padded channels and borders;
-    //                 aux[3] weights re-laid to the gather's K order [OC][kPad]; aux[4] int32 byte offset
-    //                 of every gathered piece from a pixel's window origin; auxi[2] = bytes per piece
+    //                 [N][Hp][Wp][ICp], a copy of the input with zero-padded channels; aux[3] weights [OC][kPad]
+    //                 padded alike.  With aux[4]: the copy has the borders, too, the weights are in the gather's K
+    //                 order, aux[4] int32 byte offset of every gathered piece from a pixel's window origin;
+    //                 auxi[2] = bytes per piece
     //   CONV2D kinds with tc == 4 (at most four channels): scratch = session tensor [N][Hu][Wu][16], units of four
     //                 pixels; aux[3] weights per unit [units][OC][16]
     int32_t tc{0};

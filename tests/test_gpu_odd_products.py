@@ -52,3 +52,18 @@ def test_wide_convolutions_with_rows_at_odd_addresses(mlel, n, hw, ic, oc, k, st
     g.output(conv(g, r, y, oc, 1, 1, 0, 4, False))
     g.output(conv(g, r, x, oc, k, stride, k // 2, 5, False, 33))
     check(g, [r.integers(-128, 128, x.shape, dtype=np.int8)])
+
+
+@pytest.mark.parametrize("n,hw,ic,oc,k,stride", [
+    (1, 17, 9, 51, 3, 1), (2, 23, 20, 48, 3, 1), (2, 30, 33, 32, 5, 2), (1, 14, 75, 125, 3, 2), (3, 28, 130, 64, 3, 1), (1, 40, 250, 200, 3, 1),
+    (1, 9, 24, 144, 1, 1), (2, 19, 17, 64, 1, 2),
+])
+def test_convolutions_over_padded_channels(mlel, n, hw, ic, oc, k, stride):
+    r = np.random.Generator(np.random.PCG64(hw + ic))
+    g = GraphBuilder()
+    x = g.input(np.int8, (n, hw, hw, ic))
+    g.output(conv(g, r, x, oc, k, stride, k // 2, -7, True))
+    g.output(conv(g, r, x, oc, k, stride, 0, 5, False, 33))
+    w, b = g.constant(r.integers(-128, 128, (oc, k, k, ic), dtype=np.int8)), g.constant(r.integers(-999, 999, (oc,), dtype=np.int32))
+    g.output(g.conv2d(x, w, b, [k // 2] * 4, [stride] * 2, [1, 1], 3, 0))
+    check(g, [r.integers(-128, 128, x.shape, dtype=np.int8)])
