@@ -1959,14 +1959,14 @@ void GraphPipeline::prepareTensorCore() {
             }
             // At most four channels, stride 1 or 2 (an RGB stem, tc == 4): the input is copied into 16-byte units of four
             // pixels, of which a window is a whole number, and runs on the window kernel.  Up to sixteen units (7x7 at
-            // stride 2) and whole 16-byte rows of output; other windows take the table gather below.
+            // stride 2); other windows take the table gather below.
             {
                 const int64_t perUnitX = sx == 1 ? 4 : 2, perUnitY = sx == 1 ? 1 : 2;
                 const int64_t unitsX = (KW + perUnitX - 1) / perUnitX, unitRows = (KH + perUnitY - 1) / perUnitY;
                 const int64_t units = (unitsX * unitRows + 1) / 2 * 2;
                 const int64_t remX = sx == 1 ? padLeft : padLeft & 1, remY = sx == 1 ? 0 : padTop & 1;
                 const int64_t Wu = sx == 1 ? W + padLeft : (W + remX + 1) / 2, Hu = sx == 1 ? H : (H + remY + 1) / 2;
-                if (IC <= 4 && sx == sy && sx <= 2 && dx == 1 && dy == 1 && padLeft >= 0 && padTop >= 0 && units <= 16 && OC % 16 == 0 &&
+                if (IC <= 4 && sx == sy && sx <= 2 && dx == 1 && dy == 1 && padLeft >= 0 && padTop >= 0 && units <= 16 &&
                     OC <= 4096 && op.kind == OP_FUSED_CONV2D && op.epi.hasMain && !op.epi.hasResidual &&
                     in.dims[0] * Hu * Wu < (int64_t(1) << 27)) {
                     std::vector<int8_t> wUnits(size_t(units * OC * 16), 0);
@@ -1992,7 +1992,7 @@ void GraphPipeline::prepareTensorCore() {
                 // that any window can touch.  The gather packs several taps into a K block, so up to 32 channels it stays
                 // where the window kernel does not apply (9 -> 51 channels 12.4 against 18.7 us; 20 -> 48 on the window
                 // kernel 8.5 against 10.7).
-                const bool window = sx == 1 && sy == 1 && OC % 16 == 0 && padLeft >= 0 && padTop >= 0 && fusedOut && !op.epi.hasResidual;
+                const bool window = sx == 1 && sy == 1 && padLeft >= 0 && padTop >= 0 && fusedOut && !op.epi.hasResidual;
                 const bool whole = ICp % 16 == 0 && (ICp > 32 || KH * KW == 1 || window);
                 const int64_t Hp = whole ? H : std::max<int64_t>(H + padTop, (OH - 1) * sy + (KH - 1) * dy + 1);
                 const int64_t xReach = rowRuns ? runBytes / ICp : (KW - 1) * dx + 1;

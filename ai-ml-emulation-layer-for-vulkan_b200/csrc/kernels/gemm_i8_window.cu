@@ -100,8 +100,14 @@ __device__ __forceinline__ void ummaLed(uint32_t leader, uint32_t tmemD, uint32_
                  : "memory");
 }
 
+// ODD: output rows start at any address.  The warps that share 32 rows of the accumulator put them together in shared memory
+// and store them as aligned words (storeRowBytes).  64 -> 63 channels, 8 x 56 x 56: 10.6 us on the pixel-major kernel, here
+// 8.8; 30 x 30, 64 -> 65: 9.7 and 6.1.
+template <int BN> constexpr int kOddPitch = BN + 4;                                        // bytes of a staged row
+template <int BN> constexpr int kOddBytes = 4 * 32 * kOddPitch<BN> * (BN == 32 ? 2 : 1) + 16; // quarters x rows x sets
+
 // BN: output channels of a tile (32, 64 or 128).  UNITS: the input is 16-byte units (see the head of the file).
-template <int BN, bool UNITS>
+template <int BN, bool UNITS, bool ODD>
 __global__ void __launch_bounds__(kThreadsTma, 1)
 gemmI8Window(const __grid_constant__ CUtensorMap mapX, const __grid_constant__ CUtensorMap mapW, const GemmI8Params p,
              const WindowTiling g) {
@@ -304,6 +310,10 @@ gemmI8Window(const __grid_constant__ CUtensorMap mapX, const __grid_constant__ C
         const bool rowInTile = yy < g.tileH && xx < g.tileW;
         const uint32_t tabAddr = smemAddr(colTab);
         uint32_t tileCount = 0;
+        bool failed = false;
+        // ODD: this quarter's (and set's) rows, after the barriers
+        const uint32_t staged = ((smemAddr(bars) + uint32_t(sizeof(WindowBarriers)) + 15u) & ~15u) + uint32_t((quarter + 4 * set) * 32 * kOddPitch<BN>);
+        const auto meet = [&] { asm volatile("bar.sync %0, %1;" ::"r"(2 + quarter + 4 * set), "r"(kGroups * 32) : "memory"); };
         for (int tile = firstTile; tile < g.pixelTiles; tile += tileStep, ++tileCount) {
             const uint32_t buf = tileCount & 1u;
             if (kSets == 2 && int(buf) != set) {
@@ -317,7 +327,9 @@ gemmI8Window(const __grid_constant__ CUtensorMap mapX, const __grid_constant__ C
                 cls = int(__ldg(p.rowClass + y)) * p.numColClasses + int(__ldg(p.colClass + x));
             }
             int8_t *dst = p.out8 + ((int64_t(n) * p.OH + y) * p.OW + x) * p.ldOut + c0;
-            if (!mbarWait(&bars->accFull[buf], (tileCount >> 1) & 1u, 95)) {
+            if (ODD) { // after a wait that ran out the warp still meets the others
+                failed = failed || !mbarWait(&bars->accFull[buf], (tileCount >> 1) & 1u, 95);
+            } else if (!mbarWait(&bars->accFull[buf], (tileCount >> 1) & 1u, 95)) {
                 break;
             }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -339,9 +351,18 @@ gemmI8Window(const __grid_constant__ CUtensorMap mapX, const __grid_constant__ C
                 }
                 if (cls != p.baseClass) {
                     // a pixel whose window crosses the border: swap the table's correction for its own class's
+                    if (ODD) {
+                        const int32_t *own = p.corr + int64_t(cls) * p.N + c0 + cl;
+#pragma unroll
+                        for (int j = 0; j < 16; ++j) {
+                            if (c0 + cl + j < p.N) {
+                                acc[j] += uint32_t(__ldg(own + j)) - uint32_t(colTab[cl + j].corr0);
+                            }
+                        }
+                    }
                     const int4 *own = reinterpret_cast<const int4 *>(p.corr + int64_t(cls) * p.N + c0 + cl);
 #pragma unroll
-                    for (int q = 0; q < 4; ++q) {
+                    for (int q = 0; q < (ODD ? 0 : 4); ++q) {
                         const int4 v = __ldg(own + q);
                         acc[4 * q] += uint32_t(v.x) - uint32_t(colTab[cl + 4 * q].corr0);
                         acc[4 * q + 1] += uint32_t(v.y) - uint32_t(colTab[cl + 4 * q + 1].corr0);
@@ -358,7 +379,27 @@ gemmI8Window(const __grid_constant__ CUtensorMap mapX, const __grid_constant__ C
                 } else {
                     rescale16General(acc, tab, zpMain, outZp, lo, hi, packed);
                 }
+                if (ODD) {
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) {
+                        asm volatile("st.shared.u32 [%0], %1;" ::"r"(staged + uint32_t(lane * kOddPitch<BN> + cl + 4 * q)), "r"(packed[q]) : "memory");
+                    }
+                    continue;
+                }
                 *reinterpret_cast<int4 *>(dst + cl) = make_int4(int(packed[0]), int(packed[1]), int(packed[2]), int(packed[3]));
+            }
+            if (ODD) {
+                meet();
+                const uint32_t live = __ballot_sync(0xffffffffu, valid);
+                const int length = min(BN, p.N - c0);
+#pragma unroll 2
+                for (int r = group; r < 32; r += kGroups) {
+                    int8_t *to = reinterpret_cast<int8_t *>(__shfl_sync(0xffffffffu, reinterpret_cast<unsigned long long>(dst), r));
+                    if ((live >> r) & 1u) {
+                        storeRowBytes(to, staged + uint32_t(r * kOddPitch<BN>), length, lane);
+                    }
+                }
+                meet(); // before the next tile's rows
             }
         }
     }
@@ -371,10 +412,10 @@ gemmI8Window(const __grid_constant__ CUtensorMap mapX, const __grid_constant__ C
 
 // ---- host side --------------------------------------------------------------------------------------------
 
-template <int BN, bool UNITS>
-int launchWindow(const CUtensorMap &mapX, const CUtensorMap &mapW, const GemmI8Params &p, const WindowTiling &g, size_t smem,
+template <int BN, bool UNITS, bool ODD>
+int launchWindowRows(const CUtensorMap &mapX, const CUtensorMap &mapW, const GemmI8Params &p, const WindowTiling &g, size_t smem,
                  cudaStream_t s) {
-    auto kernel = gemmI8Window<BN, UNITS>;
+    auto kernel = gemmI8Window<BN, UNITS, ODD>;
     if (!allowDynamicSmem(reinterpret_cast<const void *>(kernel), kWindowSmemLimit)) {
         return MLEL_ERROR_DEVICE;
     }
@@ -387,8 +428,19 @@ int launchWindow(const CUtensorMap &mapX, const CUtensorMap &mapW, const GemmI8P
     return MLEL_SUCCESS;
 }
 
-size_t windowSmem(const WindowTiling &g, int bn) {
-    return 1024 + size_t(g.weightBytes) + size_t(g.stages) * g.stageBytes + size_t(bn) * sizeof(ColConst) + sizeof(WindowBarriers);
+// Output rows that do not all start on 16-byte boundaries.
+bool windowOddRows(const GemmI8Params &p) { return p.ldOut % 16 != 0 || (reinterpret_cast<uintptr_t>(p.out8) & 15u) != 0; }
+
+template <int BN, bool UNITS>
+int launchWindow(const CUtensorMap &mapX, const CUtensorMap &mapW, const GemmI8Params &p, const WindowTiling &g, size_t smem,
+                 cudaStream_t s) {
+    return windowOddRows(p) ? launchWindowRows<BN, UNITS, true>(mapX, mapW, p, g, smem, s)
+                            : launchWindowRows<BN, UNITS, false>(mapX, mapW, p, g, smem, s);
+}
+
+size_t windowSmem(const WindowTiling &g, int bn, bool odd) {
+    return 1024 + size_t(g.weightBytes) + size_t(g.stages) * g.stageBytes + size_t(bn) * sizeof(ColConst) + sizeof(WindowBarriers) +
+           (odd ? size_t(bn == 32 ? kOddBytes<32> : (bn == 64 ? kOddBytes<64> : kOddBytes<128>)) : 0);
 }
 
 // What a tiling is chosen for: the reach of a window past its first pixel (unit) and the work of a tile.
@@ -419,7 +471,7 @@ bool windowTiling(const GemmI8Params &p, const WindowShape &w, int bn, WindowTil
         const int reach = w.reachY * g.boxW + w.reachX + (blocks ? 15 * g.boxW + 8 : 128) + (w.pixelBytes == 16 ? 1 : 0);
         g.stageBytes = (std::max(reach, g.boxW * g.boxH) * g.pixelBytes + 1023) / 1024 * 1024;
         g.stages = kWindowMaxStages;
-        while (g.stages > 1 && windowSmem(g, bn) > kWindowSmemLimit) {
+        while (g.stages > 1 && windowSmem(g, bn, windowOddRows(p)) > kWindowSmemLimit) {
             --g.stages;
         }
         if (g.stages < 2) {
@@ -511,10 +563,8 @@ bool gemmI8WindowApplies(const GemmI8Problem &q) {
     const GemmI8Params &p = q.params;
     const int mode = tensorCoreTuning().windowKernel.load(std::memory_order_relaxed);
     return mode != 0 && p.out8 != nullptr && p.epi.hasMain && !p.epi.hasResidual && q.aMatrix == nullptr && !q.bMnMajor && q.batches == 1 &&
-           p.gatherTable == nullptr && p.strideX == 1 && p.strideY == 1 && p.IC % 16 == 0 && p.IC <= 128 && p.N % 16 == 0 &&
-           p.ldOut % 16 == 0 && p.KH * p.KW > 1 && p.padLeft >= 0 && p.padTop >= 0 &&
-           ((reinterpret_cast<uintptr_t>(p.in) | reinterpret_cast<uintptr_t>(p.out8) | reinterpret_cast<uintptr_t>(q.bMatrix) |
-             reinterpret_cast<uintptr_t>(p.corr)) & 15u) == 0;
+           p.gatherTable == nullptr && p.strideX == 1 && p.strideY == 1 && p.IC % 16 == 0 && p.IC <= 128 && p.KH * p.KW > 1 && p.padLeft >= 0 && p.padTop >= 0 &&
+           ((reinterpret_cast<uintptr_t>(p.in) | reinterpret_cast<uintptr_t>(q.bMatrix) | reinterpret_cast<uintptr_t>(p.corr)) & 15u) == 0;
 }
 
 int gemmI8WindowLaunch(const GemmI8Problem &q, cudaStream_t s, bool *taken) {
@@ -539,7 +589,7 @@ int gemmI8WindowLaunch(const GemmI8Problem &q, cudaStream_t s, bool *taken) {
     }
     *taken = true;
     g_tensorCoreLaunches[4].fetch_add(1, std::memory_order_relaxed);
-    const size_t smem = windowSmem(g, bn);
+    const size_t smem = windowSmem(g, bn, windowOddRows(p));
     return bn == 32   ? launchWindow<32, false>(mapX, mapW, p, g, smem, s)
            : bn == 64 ? launchWindow<64, false>(mapX, mapW, p, g, smem, s)
                       : launchWindow<128, false>(mapX, mapW, p, g, smem, s);
@@ -568,7 +618,7 @@ int gemmI8UnitsLaunch(const GemmI8Problem &q, const UnitWindow &u, cudaStream_t 
         return MLEL_ERROR_DEVICE;
     }
     g_tensorCoreLaunches[4].fetch_add(1, std::memory_order_relaxed);
-    const size_t smem = windowSmem(g, bn);
+    const size_t smem = windowSmem(g, bn, windowOddRows(p));
     return bn == 32   ? launchWindow<32, true>(mapX, mapW, p, g, smem, s)
            : bn == 64 ? launchWindow<64, true>(mapX, mapW, p, g, smem, s)
                       : launchWindow<128, true>(mapX, mapW, p, g, smem, s);

@@ -1,6 +1,6 @@
 """GPU parity of the window kernel: both tile shapes, image sizes at and beside their edges, every pixel width (32, 64 and
 128 bytes, whole and padded), one to several channel tiles, windows of other sizes and dilations, border classes, shifts
-on both sides of 32.  Bit-exact against the CPU oracle; a counter tells that the kernel took the case."""
+on both sides of 32, widths that are no multiple of 16.  Bit-exact against the CPU oracle; a counter tells that the kernel took the case."""
 import ctypes
 
 import numpy as np
@@ -18,6 +18,8 @@ pytestmark = pytest.mark.gpu
     (1, 17, 9, 64, 64, 3, 1, 1, 37), (2, 40, 130, 32, 48, 3, 0, 1, 35), (1, 33, 257, 16, 16, 3, 1, 1, 34), (2, 23, 61, 48, 160, 3, 1, 1, 37),
     (1, 64, 70, 80, 96, 3, 1, 2, 37), (1, 30, 41, 32, 32, 5, 2, 1, 36), (2, 20, 120, 112, 16, 2, 0, 1, 30), (1, 50, 50, 16, 64, 7, 3, 1, 36),
     (5, 14, 14, 64, 256, 3, 1, 1, 29), (1, 3, 400, 32, 64, 3, 1, 1, 36), (1, 300, 2, 64, 16, 3, 1, 1, 36),
+    (2, 56, 56, 64, 63, 3, 1, 1, 37), (1, 45, 131, 96, 21, 3, 1, 1, 37), (3, 28, 28, 128, 129, 3, 1, 1, 38), (1, 33, 70, 32, 5, 3, 1, 1, 31),
+    (2, 23, 61, 48, 150, 3, 0, 1, 37),
 ])
 def test_windows(mlel, n, h, w, ic, oc, k, pad, dil, shift):
     from mlel_b200.runtime import GraphRunner
@@ -47,6 +49,7 @@ def test_windows(mlel, n, h, w, ic, oc, k, pad, dil, shift):
     (2, 56, 56, 3, 64, 7, 2, 3, 36), (1, 45, 131, 3, 32, 3, 1, 1, 33), (3, 33, 47, 3, 32, 3, 2, 1, 33), (1, 16, 8, 4, 16, 3, 1, 0, 33),
     (1, 20, 120, 1, 48, 5, 1, 2, 31), (2, 21, 257, 2, 16, 3, 2, 0, 32), (1, 40, 40, 3, 160, 7, 1, 3, 36), (1, 9, 300, 3, 64, 5, 2, 2, 29),
     (1, 5, 5, 4, 32, 2, 2, 0, 31), (2, 7, 7, 3, 16, 1, 2, 0, 30), (1, 70, 3, 3, 64, 3, 2, 2, 33),
+    (2, 40, 50, 3, 37, 3, 1, 1, 33), (1, 56, 57, 3, 65, 7, 2, 3, 36), (3, 20, 21, 2, 1, 3, 2, 1, 31),
 ])
 def test_windows_of_few_channels(mlel, n, h, w, ic, oc, k, stride, pad, shift):
     from mlel_b200.runtime import GraphRunner
