@@ -265,21 +265,21 @@ gemmI8Window(const __grid_constant__ CUtensorMap mapX, const __grid_constant__ C
         if (UNITS) {
             tiles(std::integral_constant<int, 1>{}, std::false_type{});
         } else {
-        using Three = std::true_type;
-        using Any = std::false_type;
-        switch ((p.IC + UMMA_K - 1) / UMMA_K) {
-        case 1:
-            three ? tiles(std::integral_constant<int, 1>{}, Three{}) : tiles(std::integral_constant<int, 1>{}, Any{});
-            break;
-        case 2:
-            three ? tiles(std::integral_constant<int, 2>{}, Three{}) : tiles(std::integral_constant<int, 2>{}, Any{});
-            break;
-        case 3:
-            three ? tiles(std::integral_constant<int, 3>{}, Three{}) : tiles(std::integral_constant<int, 3>{}, Any{});
-            break;
-        default:
-            three ? tiles(std::integral_constant<int, 4>{}, Three{}) : tiles(std::integral_constant<int, 4>{}, Any{});
-        }
+            using Three = std::true_type;
+            using Any = std::false_type;
+            switch ((p.IC + UMMA_K - 1) / UMMA_K) {
+            case 1:
+                three ? tiles(std::integral_constant<int, 1>{}, Three{}) : tiles(std::integral_constant<int, 1>{}, Any{});
+                break;
+            case 2:
+                three ? tiles(std::integral_constant<int, 2>{}, Three{}) : tiles(std::integral_constant<int, 2>{}, Any{});
+                break;
+            case 3:
+                three ? tiles(std::integral_constant<int, 3>{}, Three{}) : tiles(std::integral_constant<int, 3>{}, Any{});
+                break;
+            default:
+                three ? tiles(std::integral_constant<int, 4>{}, Three{}) : tiles(std::integral_constant<int, 4>{}, Any{});
+            }
         }
     } else {
         // ---- epilogue: the table of this CTA's channels, then a tile row (pixel) per lane, 16 columns per step
