@@ -283,7 +283,9 @@ __device__ __forceinline__ bool wordsScaleApplies(int32_t mult, int32_t shift, b
     return shift >= 32 && shift <= 50 && (!doubleRound || mult >= 0);
 }
 __device__ __forceinline__ bool wordsScaleSignFree(bool doubleRound, int32_t outZp, int32_t lo) { return !doubleRound || lo >= outZp; }
-// x0 = offset - input zero point, whole = what is added to the result (the output zero point)
+// x0 = offset - input zero point, whole = what is added to the result (the output zero point).  The product takes 62 bits
+// and the rounding term 49, so |whole| * 2^50 has to stay below 2^62: |whole| at most 2^11, which the zero points and bounds
+// of int8 results are; wider ones are added afterwards.
 template <bool SIGNED>
 __device__ __forceinline__ WordsScale makeWordsScale(int32_t mult, int32_t shift, bool doubleRound, int32_t x0, int32_t whole) {
     const int64_t bump = doubleRound ? int64_t(1) << 30 : 0;

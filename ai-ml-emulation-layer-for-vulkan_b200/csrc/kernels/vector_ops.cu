@@ -142,6 +142,11 @@ template <typename T, typename LOAD, typename STORE> __device__ __forceinline__ 
 // groups side by side a load touched 32 lines for 16 bytes each.)  What the blocks leave goes four elements or one at a
 // time.  FORM: 0 fastRescale, 1 and 2 WordsScale with and without the sign (per-tensor scales; picked by each thread, the
 // scale is in device memory).  192 x 384 x 384 int32 -> int8: 32.8 us, now 28.6.
+//
+// Only int8 results have the zero point in WordsScale's addend: 2^7 times 2^50 leaves room for the product (2^62).  An
+// int16 zero point would not from a shift of 48 on, an int32 one of 100 000 from 46 on; there it is added to the result.
+template <typename OUT> constexpr bool foldsZeroPoint = sizeof(OUT) == 1;
+
 template <int FORM, typename OUT>
 __device__ __forceinline__ void rescaleFour(const int32_t (&v)[4], int32_t (&r)[4], FastRescale f, const WordsScale &words,
                                             const int32_t *mult, const int8_t *shift, int perChannel, int c0, int C, int32_t inZp,
@@ -149,7 +154,10 @@ __device__ __forceinline__ void rescaleFour(const int32_t (&v)[4], int32_t (&r)[
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
         if (FORM != 0) {
-            const int32_t q = FORM == 1 ? wordsScale<true>(words, v[k]) + outZp : wordsScale<false>(words, v[k]);
+            int32_t q = wordsScale<FORM == 1>(words, v[k]);
+            if (FORM == 1 || !foldsZeroPoint<OUT>) {
+                q = int32_t(uint32_t(q) + uint32_t(outZp)); // 32-bit wrap, as fastRescale
+            }
             r[k] = min(max(q, lowestOf<OUT>()), highestOf<OUT>());
             continue;
         }
@@ -198,7 +206,7 @@ __global__ void rescaleVecKernel(const IN *__restrict__ in, OUT *__restrict__ ou
             words = makeWordsScale<true>(f.mult, s, true, int32_t(uint32_t(0) - uint32_t(inZp)), 0);
             rescaleBlocks<1, IN, OUT>(in, out, blocks, f, words, mult, shift, 0, C, inZp, outZp, doubleRound);
         } else {
-            words = makeWordsScale<false>(f.mult, s, false, int32_t(uint32_t(0) - uint32_t(inZp)), outZp);
+            words = makeWordsScale<false>(f.mult, s, false, int32_t(uint32_t(0) - uint32_t(inZp)), foldsZeroPoint<OUT> ? outZp : 0);
             rescaleBlocks<2, IN, OUT>(in, out, blocks, f, words, mult, shift, 0, C, inZp, outZp, doubleRound);
         }
     } else {
