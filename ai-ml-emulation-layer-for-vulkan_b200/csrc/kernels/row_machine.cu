@@ -313,6 +313,13 @@ int rowMachine(const RowProgram &program, const TView *T, cudaStream_t s) {
         setLastError("fused rows: program out of range");
         return MLEL_ERROR_UNKNOWN;
     }
+    // Both kernels load and store words: application tensors at other addresses are refused.
+    for (const RowInst &in : program.insts) {
+        if ((in.op == ROW_LOAD || in.op == ROW_STORE) && (reinterpret_cast<uintptr_t>(T[in.tensor].ptr) & 15u) != 0) {
+            setLastError("fused rows: a tensor is not 16-byte aligned");
+            return MLEL_ERROR_UNKNOWN;
+        }
+    }
     if (rowNormMatch(program)) {
         return rowNorm(program, T, s);
     }
@@ -335,10 +342,6 @@ int rowMachine(const RowProgram &program, const TView *T, cudaStream_t s) {
         d.ptr = in.tensor >= 0 ? T[in.tensor].ptr : nullptr;
         for (int k = 0; k < 7; ++k) {
             d.p[k] = in.p[k];
-        }
-        if ((in.op == ROW_LOAD || in.op == ROW_STORE) && (reinterpret_cast<uintptr_t>(d.ptr) & 15u) != 0) {
-            setLastError("fused rows: a tensor is not 16-byte aligned");
-            return MLEL_ERROR_UNKNOWN;
         }
     }
     const size_t smemBytes = size_t(prog.warps) * (size_t(prog.slots) * prog.len + kMaxRowValues) * sizeof(int32_t);

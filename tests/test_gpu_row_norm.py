@@ -33,3 +33,28 @@ def test_residual_layer_norm(mlel, rows, length, mult, shift, out_shift, in_zp, 
     rsqrt = np.clip(np.round(32767.0 * 16.0 / np.sqrt(x + 32768.0 + 256.0)), 0, 32767).astype(np.int16)
     g.output(g.rescale(g.mul(cen, g.table(var16, rsqrt), 12), [mult], [out_shift], 0, -3, np.int8, double_round=double_round))
     check_fused(mlel, g, [full_range(r, np.int8, a.shape), full_range(r, np.int8, b.shape)], [NORM])
+
+
+@pytest.mark.parametrize("tensor", ["first", "second", "result"])
+@pytest.mark.parametrize("offset", [4, 8])
+def test_tensors_off_16_byte_boundaries_are_refused(mlel, tensor, offset):
+    """As by the row machine: both kernels load and store words.  Nothing is launched."""
+    import torch
+    from mlel_b200.runtime import GraphRunner
+    from tests.test_gpu_vector_ops import _norm_chain
+    shape = (1, 3, 128)
+    g = GraphBuilder()
+    a, b = g.input(np.int8, shape), g.input(np.int8, shape)
+    t = g.add(g.rescale(a, [1 << 30], [24], 0, 0, np.int32), g.rescale(b, [1 << 30], [24], 0, 0, np.int32))
+    g.output(_norm_chain(g, rng(1), t, shape[-1])[0])
+    runner = GraphRunner(g)
+    assert runner.pipeline.exec_names() == [NORM]
+    set_, binding = {"first": runner._in_keys[0], "second": runner._in_keys[1], "result": runner._out_keys[0]}[tensor][:2]
+    buffer = torch.zeros(3 * 128 + 16, dtype=torch.uint8, device="cuda")
+    runner.session.set_external(set_, binding, buffer.data_ptr() + offset)
+    for use_cuda_graph in (False, True):
+        with pytest.raises(mlel.MlelError, match="not 16-byte aligned"):
+            runner.dispatch(use_cuda_graph=use_cuda_graph)
+    runner.session.set_external(set_, binding, buffer.data_ptr())  # a boundary is accepted again
+    runner.dispatch()
+    torch.cuda.synchronize()
