@@ -1925,9 +1925,9 @@ void GraphPipeline::prepareTensorCore() {
                 }
             }
             {
-                // With corrections this small, accumulator + correction - zero point cannot leave int32 (the raw sum
-                // of at most 65536 products is at most 2^30 in size): the epilogue may then fold the three terms into
-                // one 32-bit addition without changing the reference's 64-bit arithmetic.
+                // With corrections this small, accumulator + correction - zero point of at most 256 cannot leave int32 (the
+                // raw sum of at most 65536 products is at most 2^30 in size): the epilogue may then fold the three terms
+                // into one 32-bit addition without changing the reference's 64-bit arithmetic.
                 bool small = true;
                 for (const int32_t c : corr) {
                     small = small && c >= -((1 << 30) - 256) && c <= (1 << 30) - 256;

@@ -338,7 +338,8 @@ __global__ void __launch_bounds__(128, 4) depthwise3x3RowsKernel(const int8_t *_
             if (OUT8) {
                 const int ci = epi.main.perChannel ? c0 + k : 0;
                 // |sum of nine products| <= 9 * 2^14: with this bound sum + add - zero point stays inside int32
-                words = words && abs(int64_t(add[k])) < (int64_t(1) << 30) &&
+                words = words && abs(int64_t(add[k]) - int64_t(epi.main.inZp)) < (int64_t(1) << 30) && // (a zero point of any int32)
+                        abs(int64_t(add[k])) < (int64_t(1) << 30) &&
                         wordsScaleApplies(__ldg(epi.main.mult + ci), int32_t(__ldg(epi.main.shift + ci)), epi.main.doubleRound != 0);
             }
         }

@@ -63,7 +63,8 @@ struct GemmI8Params {
                              // one; kLateCorrections: only the corrections, and that launch waits for all older ones
                              // before it lets this one start
     int32_t baseClass;       // the most common class: its correction row is staged in shared memory
-    int32_t corrSmall;       // 1: every |corr| <= 2^30 - 256: accumulator + correction - zero point stays inside int32
+    int32_t corrSmall;       // 1: every |corr| <= 2^30 - 256 and the main stage's input zero point is at most 256 in size:
+                             // accumulator + correction - zero point stays inside int32
     // outputs: exactly one of out32 / out8 is set
     int32_t *out32;
     int8_t *out8;

@@ -103,6 +103,12 @@ DevEpilogue devEpilogue(const FusedEpilogue &e, const TView *T) {
     return d;
 }
 
+// GemmI8Params::corrSmall: the corrections have been bounded by 2^30 - 256, the main stage's input zero point is here.  (An
+// int32 zero point may have any value; the general form takes it in 64 bits.)
+int32_t corrSmall(bool corrections, const DevEpilogue &epi) {
+    return corrections && epi.main.inZp >= -256 && epi.main.inZp <= 256 ? 1 : 0;
+}
+
 int64_t numelOf(const TView &t) {
     int64_t n = 1;
     for (int i = 0; i < t.rank; ++i) {
@@ -146,7 +152,6 @@ int launchConvTensorCore(const OpDesc &op, const TView *T, cudaStream_t s, Launc
     p.numColClasses = op.auxi[0];
     p.numClasses = op.auxi[1];
     p.baseClass = op.auxi[3];
-    p.corrSmall = op.auxi[4];
     if (p.numClasses <= 1) {
         p.rowClass = p.colClass = nullptr; // no window crosses the border: one correction row serves every pixel
         p.baseClass = 0;
@@ -154,6 +159,7 @@ int launchConvTensorCore(const OpDesc &op, const TView *T, cudaStream_t s, Launc
     if (op.kind == OP_FUSED_CONV2D) {
         p.out8 = reinterpret_cast<int8_t *>(out.ptr);
         p.epi = devEpilogue(op.epi, T);
+        p.corrSmall = corrSmall(op.auxi[4] != 0, p.epi);
         if (op.epi.hasResidual && op.tc == 1 && op.aux[3] >= 0) {
             p.residualTable = reinterpret_cast<const uint8_t *>(T[op.aux[3]].ptr);
         }
@@ -235,15 +241,13 @@ int launchMatmulTensorCore(const OpDesc &op, const TView *T, cudaStream_t s, boo
     p.numClasses = 1;
     p.numColClasses = 1;
     p.batchedCorr = 1;
-    // |correction| = |zero point of A| * |column sum of B| <= 128 * K * |zp|: small enough for the short RESCALE form
-    // whenever that bound is (see GemmI8Params::corrSmall)
-    {
-        const int64_t corrBound = int64_t(op.i[0] < 0 ? -op.i[0] : op.i[0]) * p.K * 128;
-        p.corrSmall = corrBound <= (int64_t(1) << 30) - 256 ? 1 : 0;
-    }
     if (op.kind == OP_FUSED_MATMUL) {
         p.out8 = reinterpret_cast<int8_t *>(out.ptr);
         p.epi = devEpilogue(op.epi, T);
+        // |correction| = |zero point of A| * |column sum of B| <= 128 * K * |zp|: small enough for the short RESCALE form
+        // whenever that bound is
+        const int64_t corrBound = int64_t(op.i[0] < 0 ? -op.i[0] : op.i[0]) * p.K * 128;
+        p.corrSmall = corrSmall(corrBound <= (int64_t(1) << 30) - 256, p.epi);
     } else {
         p.out32 = reinterpret_cast<int32_t *>(out.ptr);
     }
