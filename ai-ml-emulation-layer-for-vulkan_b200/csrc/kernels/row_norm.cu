@@ -154,7 +154,11 @@ bool makeNormScale(const int32_t (&q)[7], int64_t xMax, bool signedAllowed, Norm
         m >>= 1, bump >>= 1, round >>= 1; // at k + 1 == shift the rounding term is below one unit and falls away
         ++k;
     }
-    const int64_t most = (xMax + std::abs(int64_t(q[2]))) * m + round + 2 * bump + std::abs(int64_t(q[2])) * m;
+    const int64_t reach = xMax + 2 * std::abs(int64_t(q[2]));
+    if (reach >= (int64_t(1) << 31)) {
+        return false; // (the product below would leave 64 bits)
+    }
+    const int64_t most = reach * m + round + 2 * bump;
     if (shift - k > 31 || most >= (int64_t(1) << 31)) {
         return false;
     }

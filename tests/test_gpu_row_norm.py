@@ -58,3 +58,21 @@ def test_tensors_off_16_byte_boundaries_are_refused(mlel, tensor, offset):
     runner.session.set_external(set_, binding, buffer.data_ptr())  # a boundary is accepted again
     runner.dispatch()
     torch.cuda.synchronize()
+
+
+@pytest.mark.parametrize("in_zp", [-(1 << 31), (1 << 31) - 1, -(1 << 30), 1 << 24, 256])
+@pytest.mark.parametrize("mult,shift", [((1 << 31) - 1, 31), (1 << 30, 45)])
+def test_result_scale_with_any_zero_point(mlel, in_zp, mult, shift):
+    """The last RESCALE reads int32: bounds of the 32-bit form with zero points whose product leaves 64 bits."""
+    from tests.test_gpu_vector_ops import _lut16
+    r = rng(shift)
+    shape = (1, 9, 132)
+    g = GraphBuilder()
+    a, b = g.input(np.int8, shape), g.input(np.int8, shape)
+    t = g.add(g.rescale(a, [1 << 30], [24], 0, 0, np.int32), g.rescale(b, [1 << 30], [24], 0, 0, np.int32))
+    inv = g.inline(np.asarray([(1 << 20) // shape[-1]], np.int32).reshape(1, 1, 1))
+    cen = g.sub(t, g.mul(g.reduce("REDUCE_SUM", t, 2), inv, 20))
+    var = g.mul(g.reduce("REDUCE_SUM", g.mul(cen, cen, 8), 2), inv, 20)
+    factor = g.table(g.rescale(var, [1 << 30], [34], 0, -32768, np.int16), _lut16(r))
+    g.output(g.rescale(g.mul(cen, factor, 12), [mult], [shift], in_zp, 3, np.int8))
+    check_fused(mlel, g, [full_range(r, np.int8, shape), full_range(r, np.int8, shape)], [NORM])
