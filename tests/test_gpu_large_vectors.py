@@ -1,5 +1,6 @@
 """GPU parity of the forms that the vectorised kernels take for large tensors only (vector_ops.cu): RESCALE by blocks of 512
-elements a warp (from 606 208 elements) with its one-multiply-add forms.  Bit-exact against the CPU oracle."""
+elements a warp (from 606 208 elements) with its one-multiply-add forms, TABLE with a copy of the table per lane (from 2^23
+elements), four groups in flight a thread (from 7.3 M int32 or 29 M int8 elements).  Bit-exact against the CPU oracle."""
 import numpy as np
 import pytest
 
@@ -59,3 +60,51 @@ def test_rescale_by_blocks_per_channel(mlel, channels):
         for double_round in (False, True):
             g.output(g.rescale(x, mult, shift, 0, out_zp, out_dtype, double_round=double_round, per_channel=True))
     check(g, [full_range(r, np.int32, shape)])
+
+
+GROUPS = 4 * 148 * 16 * 256 + 1000  # groups of which every thread takes four at a time, some a fifth by itself
+
+
+def test_int8_beyond_four_groups_a_thread(mlel):
+    """CLAMP and TABLE: the unrolled part, the rest and the last elements."""
+    r = rng(1)
+    shape = (16 * GROUPS + 13,)
+    g = GraphBuilder()
+    x = g.input(np.int8, shape)
+    g.output(g.clamp(x, -100, 93))
+    g.output(g.table(x, full_range(r, np.int8, (256,))))
+    check(g, [full_range(r, np.int8, shape)])
+
+
+@pytest.mark.parametrize("elements", [(1 << 23) - 1, 1 << 23, (1 << 23) + 15, 16 * 4 * 148 * 2 * 1024 + 1])
+def test_table_by_lanes(mlel, elements):
+    """TABLE's copy per lane begins at 2^23 elements; its threads take four groups at a time from 14.5 M on."""
+    r = rng(elements & 7)
+    g = GraphBuilder()
+    x = g.input(np.int8, (elements,))
+    g.output(g.table(x, full_range(r, np.int8, (256,))))
+    check(g, [full_range(r, np.int8, (elements,))])
+
+
+def test_int16_table_beyond_four_groups_a_thread(mlel):
+    r = rng(2)
+    shape = (4 * GROUPS + 3,)
+    g = GraphBuilder()
+    x = g.input(np.int16, shape)
+    g.output(g.table(x, full_range(r, np.int16, (513,))))
+    check(g, [full_range(r, np.int16, shape)])
+
+
+@pytest.mark.parametrize("length", [196, 197])
+def test_int32_beyond_four_groups_a_thread(mlel, length):
+    """ADD, SUB and MUL with an operand of the same shape, one value per row (of whole groups or not) and one value."""
+    r = rng(length)
+    shape = (4 * GROUPS // length + 1, length)
+    same, row, one = (full_range(r, np.int32, s) for s in (shape, (shape[0], 1), (1, 1)))
+    g = GraphBuilder()
+    x, y, rw, v = g.input(np.int32, shape), g.input(np.int32, shape), g.input(np.int32, row.shape), g.input(np.int32, (1, 1))
+    g.output(g.add(x, y))
+    g.output(g.sub(x, rw))
+    g.output(g.mul(x, rw, 17))
+    g.output(g.mul(x, v, 31))
+    check(g, [full_range(r, np.int32, shape), same, row, one])
