@@ -229,9 +229,10 @@ int launchConvTensorCore(const OpDesc &op, const TView *T, cudaStream_t s, Launc
     return gemmI8OcMajorApplies(q) ? gemmI8OcMajorLaunch(q, s, chain, consumed) : gemmI8Launch(q, s);
 }
 
-// MATMUL / fused MATMUL: second input constant and pre-transposed (tc == 1), or transposed here (tc == 3).
-// *tableDone: the kernel has looked up the epilogue's table, if there is one.
-int launchMatmulTensorCore(const OpDesc &op, const TView *T, cudaStream_t s, bool *tableDone) {
+// MATMUL / fused MATMUL on the tensor cores: everything but what has to be copied or transposed first.  A product of two
+// activations (tc == 3) is described as the paired kernel reads it: the second operand where it lies ([C][W], the output
+// column contiguous: an MN-major tensor-core operand).
+GemmI8Problem matmulProblem(const OpDesc &op, const TView *T) {
     const TView &a = T[op.in[0]], &out = T[op.out[0]];
     GemmI8Problem q{};
     GemmI8Params &p = q.params;
@@ -253,35 +254,60 @@ int launchMatmulTensorCore(const OpDesc &op, const TView *T, cudaStream_t s, boo
     }
     q.batches = int32_t(a.dims[0]);
     const int Cp = (p.K + 15) / 16 * 16; // row pitch of what is read with K contiguous
-    q.aMatrix = a.ptr;
+    q.aMatrix = Cp == p.K ? a.ptr : T[op.scratch].ptr; // (a copy with rows of Cp bytes)
     q.aRowBytes = uint64_t(Cp);
     q.aBatchBytes = uint64_t(Cp) * uint64_t(p.M);
-    if (Cp != p.K) {
-        int8_t *copy = reinterpret_cast<int8_t *>(T[op.scratch].ptr);
-        const int rows = int(a.dims[0]) * p.M;
-        const int rc = padImageI8(reinterpret_cast<const int8_t *>(a.ptr), copy, 1, 1, rows, p.K, 1, rows, Cp, 0, 0, s);
-        if (rc != MLEL_SUCCESS) {
-            return rc;
-        }
-        q.aMatrix = copy;
-    }
-    const void *bt = nullptr;
     if (op.tc == 3) {
         const TView &b = T[op.in[1]];
         p.N = int32_t(b.dims[2]);
-        p.ldOut = p.N;
-        int8_t *scratch = reinterpret_cast<int8_t *>(T[op.scratch].ptr) + op.auxi[0];
-        int32_t *corr = reinterpret_cast<int32_t *>(reinterpret_cast<int8_t *>(T[op.scratch].ptr) + op.auxi[2]);
-        p.corr = corr;
+        p.corr = reinterpret_cast<int32_t *>(T[op.scratch].ptr + op.auxi[2]);
         p.lateOperand = kLateCorrections;
-        // The paired kernel reads the run-time operand where it lies ([C][W], the output column contiguous: an
-        // MN-major tensor-core operand) and only needs the column sums; the single-CTA kernel takes a transposed
-        // copy, made together with the sums.
         q.bMatrix = b.ptr;
         q.bRowBytes = uint64_t(p.N);
         q.bBatchBytes = uint64_t(p.K) * uint64_t(p.N);
         q.bMnMajor = true;
-        if (tensorCoreTuning().pairKernel.load(std::memory_order_relaxed) != 0 && gemmI8PairApplies(q)) {
+    } else {
+        p.N = int32_t(T[op.aux[3]].dims[1]);
+        p.corr = reinterpret_cast<const int32_t *>(T[op.aux[0]].ptr);
+        q.bMatrix = T[op.aux[3]].ptr;
+        q.bRowBytes = uint64_t(Cp);
+        q.bBatchBytes = uint64_t(Cp) * uint64_t(p.N);
+    }
+    p.ldOut = p.N;
+    return q;
+}
+
+// Whether the paired kernel takes a product of two activations where its second operand lies.
+bool pairTakesActivations(const GemmI8Problem &q) {
+    return tensorCoreTuning().pairKernel.load(std::memory_order_relaxed) != 0 && gemmI8PairApplies(q);
+}
+
+// Addresses are only known at dispatch: pointers that are not 16-byte aligned go to the generic kernels.
+bool matmulOnTensorCores(const OpDesc &op, const TView *T) {
+    const auto bits = [&](int32_t t) { return reinterpret_cast<uintptr_t>(T[t].ptr) & 15u; };
+    return op.tc != 0 && (bits(op.in[0]) | bits(op.out[0])) == 0 && (op.tc != 3 || bits(op.in[1]) == 0);
+}
+
+// Second input constant and pre-transposed (tc == 1), or a run-time tensor (tc == 3): the paired kernel only needs its
+// column sums, the single-CTA kernels take a transposed copy, made together with the sums.
+// *tableDone: the kernel has looked up the epilogue's table, if there is one.
+int launchMatmulTensorCore(const OpDesc &op, const TView *T, cudaStream_t s, bool *tableDone) {
+    const TView &a = T[op.in[0]];
+    GemmI8Problem q = matmulProblem(op, T);
+    GemmI8Params &p = q.params;
+    const int Cp = int(q.aRowBytes);
+    if (Cp != p.K) {
+        const int rows = int(a.dims[0]) * p.M;
+        const int rc = padImageI8(reinterpret_cast<const int8_t *>(a.ptr), reinterpret_cast<int8_t *>(T[op.scratch].ptr), 1, 1, rows,
+                                  p.K, 1, rows, Cp, 0, 0, s);
+        if (rc != MLEL_SUCCESS) {
+            return rc;
+        }
+    }
+    if (op.tc == 3) {
+        const TView &b = T[op.in[1]];
+        int32_t *corr = reinterpret_cast<int32_t *>(T[op.scratch].ptr + op.auxi[2]);
+        if (pairTakesActivations(q)) {
             int rc = columnSumsForMatmul(reinterpret_cast<const int8_t *>(b.ptr), corr, int(b.dims[0]), p.K, p.N, op.i[0], s);
             if (rc != MLEL_SUCCESS) {
                 return rc;
@@ -292,23 +318,17 @@ int launchMatmulTensorCore(const OpDesc &op, const TView *T, cudaStream_t s, boo
                 return rc;
             }
         }
-        p.lateOperand = kLateOperand;
-        const int rc = transposeForMatmul(reinterpret_cast<const int8_t *>(b.ptr), scratch, corr, int(b.dims[0]), p.K, p.N,
-                                          op.i[0], s);
+        int8_t *transposed = reinterpret_cast<int8_t *>(T[op.scratch].ptr) + op.auxi[0];
+        const int rc = transposeForMatmul(reinterpret_cast<const int8_t *>(b.ptr), transposed, corr, int(b.dims[0]), p.K, p.N, op.i[0], s);
         if (rc != MLEL_SUCCESS) {
             return rc;
         }
-        bt = scratch;
-    } else {
-        p.N = int32_t(T[op.aux[3]].dims[1]);
-        p.ldOut = p.N;
-        bt = T[op.aux[3]].ptr;
-        p.corr = reinterpret_cast<const int32_t *>(T[op.aux[0]].ptr);
+        p.lateOperand = kLateOperand;
+        q.bMatrix = transposed;
+        q.bRowBytes = uint64_t(Cp);
+        q.bBatchBytes = uint64_t(Cp) * uint64_t(p.N);
+        q.bMnMajor = false;
     }
-    q.bMatrix = bt;
-    q.bRowBytes = uint64_t(Cp);
-    q.bBatchBytes = uint64_t(Cp) * uint64_t(p.N);
-    q.bMnMajor = false;
     int rc = MLEL_SUCCESS;
     // ("pair_kernel" 2 asks for the paired kernel wherever it applies)
     const bool pairFirst = tensorCoreTuning().pairKernel.load(std::memory_order_relaxed) == 2;
@@ -326,11 +346,8 @@ int launchTable(const TView &in, const TView &out, const TView &table, cudaStrea
 
 int launchMatmul(const OpDesc &op, const TView *T, cudaStream_t s) {
     const TView &a = T[op.in[0]], &b = T[op.in[1]], &out = T[op.out[0]];
-    // Addresses are only known here: pointers that are not 16-byte aligned go to the generic kernels.
-    const bool tensorCore = op.tc != 0 && ((reinterpret_cast<uintptr_t>(a.ptr) | reinterpret_cast<uintptr_t>(out.ptr)) & 15u) == 0 &&
-                            (op.tc != 3 || (reinterpret_cast<uintptr_t>(b.ptr) & 15u) == 0);
     bool tableDone = false;
-    const int rc = tensorCore                 ? launchMatmulTensorCore(op, T, s, &tableDone)
+    const int rc = matmulOnTensorCores(op, T) ? launchMatmulTensorCore(op, T, s, &tableDone)
                    : op.kind == OP_MATMUL ? genericMatmul(a, b, out, op.i[0], op.i[1], s)
                                               : fusedMatmulGeneric(a, b, out, op.i[0], op.i[1], devEpilogue(op.epi, T), s);
     if (rc != MLEL_SUCCESS || op.epi.tableTensor < 0 || tableDone) {
@@ -343,6 +360,11 @@ int launchMatmul(const OpDesc &op, const TView *T, cudaStream_t s) {
 
 void setLastError(const std::string &msg) { g_lastError = msg; }
 const std::string &lastError() { return g_lastError; }
+
+bool overlappingProduct(const OpDesc &op, const TView *T) {
+    return op.kind == OP_FUSED_MATMUL && op.tc == 3 && op.epi.tableTensor < 0 && T[op.in[0]].dims[2] % 16 == 0 &&
+           matmulOnTensorCores(op, T) && pairTakesActivations(matmulProblem(op, T));
+}
 
 int launchOp(const OpDesc &op, const TView *T, cudaStream_t s, LaunchChain *chain) {
     const auto in = [&](size_t k) -> const TView & { return T[op.in[k]]; };

@@ -470,15 +470,14 @@ int Session::dispatchGraph(cudaStream_t stream) {
     // convolution, the host having 5.3 and 1.8 us to do.
     // So are the two of a product of two activations on the paired kernel, which overlap (as a graph 10.3, enqueued 8.1 us
     // for 4 x 512^3; 38.1 and 32.9 for 16 x 1024^3 out of memory), from 2^24 products on: below that the device would wait
-    // for the host.  Copies and transposes in front of a contraction do not
-    // overlap with it, and three launches cost the host more than a replay.
+    // for the host.  Copies and transposes in front of a contraction do not overlap with it, and three launches (a TABLE
+    // behind the product is the third) cost the host more than a replay.
     const auto &exec = pipeline_->getExecList();
     if (exec.size() == 1) {
         const OpDesc &op = exec[0];
-        const auto inner = [&](size_t k) { return pipeline_->tensor(op.in[k]).dims.back(); };
-        const bool paired = op.kind == OP_FUSED_MATMUL && op.tc == 3 && inner(0) % 16 == 0 && inner(1) % 16 == 0 && inner(1) > 128 &&
-                            pipeline_->tensor(op.in[0]).numel() * inner(1) >= int64_t(1) << 24;
-        if (op.scratch < 0 || paired) {
+        if (op.scratch < 0 ||
+            (overlappingProduct(op, views_.data()) &&
+             pipeline_->tensor(op.in[0]).numel() * pipeline_->tensor(op.in[1]).dims.back() >= int64_t(1) << 24)) {
             return dispatch(stream);
         }
     }

@@ -30,3 +30,33 @@ def test_product_with_table(mlel, batch, rows, k, n, constant, fused, clamp):
     names = GraphRunner(g).pipeline.exec_names()
     assert all(x.endswith("+TABLE") for x in names) == fused, names
     check(g, [a8] if constant else [a8, b8])
+
+
+@pytest.mark.parametrize("table", [False, True])
+@pytest.mark.parametrize("k,n", [(256, 256), (256, 144), (250, 256), (256, 128)])
+def test_product_of_activations_dispatched_by_either_way(mlel, table, k, n):
+    """Enqueued (column sums and the paired kernel) or replayed (anything else), by the kernel that takes it: with the paired
+    kernel and without, with a TABLE as third launch, with addresses that go to the generic kernel."""
+    import torch
+    from mlel_b200.runtime import GraphRunner
+    from tests.graph_eval import evaluate
+    r = np.random.Generator(np.random.PCG64(k + n))
+    a8, b8 = (r.integers(-128, 128, s, dtype=np.int8) for s in ((2, 300, k), (2, k, n)))
+    g = GraphBuilder()
+    a, b = g.input(np.int8, a8.shape), g.input(np.int8, b8.shape)
+    y = g.rescale(g.matmul(a, b, 3, 0), [1 << 30 | 12345], [37], 0, 1, np.int8, double_round=True)
+    g.output(g.table(y, r.integers(-128, 128, (256,), dtype=np.int8)) if table else y)
+    want = evaluate(g, [a8, b8])[0]
+    lib = mlel.lib()
+    runner = GraphRunner(g)
+    buffer = torch.zeros(b8.size + 16, dtype=torch.uint8, device="cuda")
+    try:
+        for pair in (1, 0, 1):
+            assert lib.mlel_set_tuning(b"pair_kernel", pair) == 0
+            for use_cuda_graph in (True, False):
+                assert np.array_equal(runner.run([a8, b8], use_cuda_graph=use_cuda_graph)[0], want)
+    finally:
+        assert lib.mlel_set_tuning(b"pair_kernel", 1) == 0
+    buffer[1:1 + b8.size] = torch.from_numpy(b8.reshape(-1).view(np.uint8)).cuda()
+    runner.session.set_external(*runner._in_keys[1][:2], buffer.data_ptr() + 1)
+    assert np.array_equal(runner.run([a8, b8], use_cuda_graph=True)[0], want)
