@@ -412,26 +412,35 @@ __device__ __forceinline__ void gatherBlock(const GatherRow (&rows)[ROWS], const
 // ---- host side ----
 // Encoded tensor maps by their description.  A map is a function of its arguments alone (the address among them), and the
 // driver takes about half a microsecond to encode one: three of them were a third of what enqueueing a convolution costs
-// the host.  A session that enqueues the same launches again finds them here; one table of fixed size per host thread.
+// the host.  A session that enqueues the same launches again finds them here; one table of 512 maps (160 KB) per host
+// thread, made at its first map.
 struct MapKey {
-    uint64_t v[16] = {};
+    uint64_t v[16] = {}; // v[0] names the kind of map
 };
-template <class Encode> inline bool rememberedMap(CUtensorMap *map, const MapKey &key, Encode &&encode) {
+struct RememberedMaps {
     struct Entry {
         MapKey key;
         CUtensorMap map;
         bool valid = false;
     };
-    constexpr size_t kWays = 4; // (with one, two maps of a program that shared a place were encoded anew on every pass)
-    static thread_local std::vector<Entry> table(128 * kWays);
-    static thread_local unsigned turn = 0;
+    static constexpr size_t kWays = 4; // (with one, two maps of a program that shared a place were encoded anew on every pass)
+    std::vector<Entry> table = std::vector<Entry>(128 * kWays);
+    unsigned turn = 0;
+};
+inline RememberedMaps &rememberedMaps() {
+    static thread_local RememberedMaps maps;
+    return maps;
+}
+template <class Encode> inline bool rememberedMap(CUtensorMap *map, const MapKey &key, Encode &&encode) {
+    RememberedMaps &known = rememberedMaps();
+    constexpr size_t kWays = RememberedMaps::kWays;
     uint64_t h = 0xcbf29ce484222325ull;
     for (const uint64_t v : key.v) {
         h = (h ^ v) * 0x9e3779b97f4a7c15ull;
         h ^= h >> 29;
     }
-    Entry *set = &table[h % (table.size() / kWays) * kWays];
-    Entry *slot = &set[turn % kWays];
+    RememberedMaps::Entry *set = &known.table[h % (known.table.size() / kWays) * kWays];
+    RememberedMaps::Entry *slot = &set[known.turn % kWays];
     for (size_t w = 0; w < kWays; ++w) {
         if (set[w].valid && std::memcmp(&set[w].key, &key, sizeof(MapKey)) == 0) {
             *map = set[w].map;
@@ -444,7 +453,7 @@ template <class Encode> inline bool rememberedMap(CUtensorMap *map, const MapKey
     if (!encode(map)) {
         return false;
     }
-    ++turn;
+    ++known.turn;
     slot->key = key, slot->map = *map, slot->valid = true;
     return true;
 }
