@@ -104,7 +104,8 @@ __device__ __forceinline__ void storeRun(int8_t *to, const uint32_t *words, int 
     }
 }
 
-// ROWS16: every row of the output starts on a 16-byte boundary, a thread stores its own row's 16 columns at once.
+// ROWS16: every row of the output and of the shortcut starts on a 16-byte boundary, a thread stores (and reads) its own
+// row's 16 columns at once.
 template <int BN, int NSTAGE, bool RESIDUAL, bool ROWS16, bool GATHER>
 __device__ __forceinline__ void epilogueInt8(const GemmI8Params &p, PipeBarriers *bars, ColConst *colTab,
                                              uint32_t tmemBase, int warp, int lane, int64_t numTiles, int mTiles,
@@ -858,7 +859,9 @@ int gemmI8Launch(const GemmI8Problem &q, cudaStream_t s) {
         return aMode == kATiled ? launchVariant<128, 6, kATiled, true>(mapA, mapB, p, s)
                                 : launchVariant<128, 6, kAGather, true>(mapA, mapB, p, s);
     }
-    const bool rows16 = p.out8 == nullptr || (p.ldOut % 16 == 0 && (reinterpret_cast<uintptr_t>(p.out8) & 15u) == 0);
+    // (the shortcut of a residual tail has the output's rows at an address of its own)
+    const uintptr_t rowBits = reinterpret_cast<uintptr_t>(p.out8) | (p.epi.hasResidual ? reinterpret_cast<uintptr_t>(p.epi.shortcut) : 0);
+    const bool rows16 = p.out8 == nullptr || (p.ldOut % 16 == 0 && (rowBits & 15u) == 0);
     if (!rows16) {
         if (bn == 64) {
             return aMode == kATiled    ? launchVariant<64, 8, kATiled, false, false, false>(mapA, mapB, p, s)
