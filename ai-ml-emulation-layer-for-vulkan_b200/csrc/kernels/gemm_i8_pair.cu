@@ -511,10 +511,14 @@ bool gemmI8PairApplies(const GemmI8Problem &q) {
     if (p.out8 == nullptr || !p.epi.hasMain || p.N <= kOcTile || p.gatherTable != nullptr) {
         return false;
     }
-    // Rows at odd addresses: where the tiles give half of the pairs work (4 x 300 x 200 x 301 with 16 tiles took 14.5 us here
-    // and 12.4 on the pixel-major kernel's smaller tiles; 40 x 300 x 511 x 511 37 and 48).
-    const int64_t tiles = int64_t((p.M + 191) / 192) * ((p.N + kPairChannels - 1) / kPairChannels) * q.batches;
-    if (pairOddRows(p) && (q.bMnMajor || q.aMatrix == nullptr || p.epi.hasResidual || p.epi.table != nullptr || 4 * tiles < smCount())) {
+    // Rows at odd addresses, whose stores cost this kernel's epilogue more: where the pixel-major kernel's tiles of 128 x 128
+    // would not all run at once.  Of 74 products (48 to 3000 deep) 24 are one round there: 22 took 6 to 24 % longer here (16 x
+    // 384 x 64 x 383 8.0 us and 6.4, 1 x 4000 x 1024 x 511 9.2 and 8.0), two over 2500 deep 2 % shorter.  Of the other 50 42
+    // took 2 to 29 % shorter (32 x 384 x 64 x 255 8.0 and 10.7, 8 x 1857 x 1286 x 2505 74.6 and 97.8) and 8, whose last
+    // round there is full, 1 to 19 % longer (48 x 384 x 1024 x 383 22.0 and 18.5).
+    const int64_t pixelMajorTiles = int64_t((p.M + 127) / 128) * ((p.N + 127) / 128) * q.batches;
+    if (pairOddRows(p) &&
+        (q.bMnMajor || q.aMatrix == nullptr || p.epi.hasResidual || p.epi.table != nullptr || pixelMajorTiles <= smCount())) {
         return false;
     }
     if (q.bRowBytes % 16 != 0 ||

@@ -5,7 +5,7 @@ import pytest
 
 from mlel_b200.graph_builder import GraphBuilder
 from tests.test_gpu_small import conv
-from tests.test_gpu_vector_ops import check
+from tests.test_gpu_vector_ops import check, check_fused
 
 pytestmark = pytest.mark.gpu
 
@@ -67,3 +67,25 @@ def test_convolutions_over_padded_channels(mlel, n, hw, ic, oc, k, stride):
     w, b = g.constant(r.integers(-128, 128, (oc, k, k, ic), dtype=np.int8)), g.constant(r.integers(-999, 999, (oc,), dtype=np.int32))
     g.output(g.conv2d(x, w, b, [k // 2] * 4, [stride] * 2, [1, 1], 3, 0))
     check(g, [r.integers(-128, 128, x.shape, dtype=np.int8)])
+
+
+@pytest.mark.parametrize("batch,rows,k,n,paired", [
+    (37, 130, 70, 151, False), (38, 130, 70, 151, True), (1, 19 * 128, 33, 8 * 128 - 1, True), (3, 5000, 64, 255, True), (40, 200, 300, 385, True),
+])
+@pytest.mark.parametrize("constant", [False, True])
+def test_products_with_rows_at_odd_addresses_where_the_paired_kernel_begins(mlel, batch, rows, k, n, paired, constant):
+    """More 128 x 128 tiles than SMs (148); widths of all three tile sizes, one to four channel tiles."""
+    import ctypes
+    lib = mlel.lib()
+    lib.mlel_tensor_core_launches.restype = ctypes.c_longlong
+    r = np.random.Generator(np.random.PCG64(rows * k + n))
+    a8, b8 = (r.integers(-128, 128, s, dtype=np.int8) for s in ((batch, rows, k), (batch, k, n)))
+    g = GraphBuilder()
+    a = g.input(np.int8, a8.shape)
+    b = g.constant(b8) if constant else g.input(np.int8, b8.shape)
+    for shift in (34, 40):
+        y = g.rescale(g.matmul(a, b, 3, 0), [1 << 30 | 12345], [shift], 0, 1, np.int8, double_round=True)
+        g.output(y)
+    before = lib.mlel_tensor_core_launches(2)
+    check_fused(mlel, g, [a8] if constant else [a8, b8], ["MATMUL+RESCALE"])
+    assert (lib.mlel_tensor_core_launches(2) > before) == paired
