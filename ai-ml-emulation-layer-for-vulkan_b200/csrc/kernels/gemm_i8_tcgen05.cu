@@ -75,7 +75,7 @@ struct TileCoord {
 // Int8 rows at odd addresses: the 32 rows of a quarter of the tile are put together in shared memory by the four warps that
 // compute them, and leave as runs of aligned words -- a run per row, or one run for all of them where a row is one tile
 // wide.  Stored byte by byte a step was 16 store instructions, each to 32 lines (1 x 270 x 480 pixels of 21 channels: 18.5
-// us; 16 products of 1024 x 1024 x 1023: see launchMatmulTensorCore).
+// us, now 13.2).
 template <int BN> constexpr int kRowPitchWords = BN / 4 + 1; // no bank conflicts
 template <int BN> constexpr int kStageBytesRows8 = 4 * 32 * kRowPitchWords<BN> * 4;
 
@@ -301,8 +301,9 @@ __device__ __forceinline__ void epilogueInt8(const GemmI8Params &p, PipeBarriers
             int8_t *to = p.out8 + (int64_t(batch) * p.M + firstRow) * p.ldOut + n0;
             const uint32_t from = smemAddr(rows);
             if (nTiles == 1 && GATHER) {
-                // (with 80 registers a thread this form is the quicker one: 16.6 against 18.5 us for a 3x3 window over 65
-                // channels, 8 x 56 x 56 x 63; the other one 13.2 against 14.0 for 270 x 480 x 21)
+                // (with the gather warps' 80 registers a thread this form is the quicker one: 3x3 at stride 2, 8 x 112 x 112,
+                // 9 -> 63 channels 11.8 us against 12.5, 20 -> 45 11.6 and 12.3, 56 x 56, 9 -> 21 7.0 and 7.2; the other one
+                // where TMA fetches: 1x1, 270 x 480, 32 -> 21 13.2 against 14.0)
                 storeRun(to, rows, rowsHere * p.N, half * 32 + lane, 128);
             } else if (nTiles == 1) { // one run of bytes, 128 at a time
                 const int length = rowsHere * p.N;
