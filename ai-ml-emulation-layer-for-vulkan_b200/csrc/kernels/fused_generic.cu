@@ -330,16 +330,16 @@ __global__ void __launch_bounds__(128, 4) depthwise3x3RowsKernel(const int8_t *_
             convolve(std::false_type{});
         }
         int32_t add[4];
-        bool words = OUT8; // the four channels' RESCALEs are one multiply-add each (WordsScale)
+        // The four channels' RESCALEs are one multiply-add each (WordsScale).  (An int32 zero point may have any value.)
+        bool words = OUT8 && (uint32_t(epi.main.inZp) + 256u) <= 512u;
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
             const int32_t b = __ldg(bias + (biasCount == 1 ? 0 : c0 + k));
             add[k] = int32_t(uint32_t(b) - uint32_t(a.inZp) * uint32_t(wsum[k]));
             if (OUT8) {
                 const int ci = epi.main.perChannel ? c0 + k : 0;
-                // |sum of nine products| <= 9 * 2^14: with this bound sum + add - zero point stays inside int32
-                words = words && abs(int64_t(add[k]) - int64_t(epi.main.inZp)) < (int64_t(1) << 30) && // (a zero point of any int32)
-                        abs(int64_t(add[k])) < (int64_t(1) << 30) &&
+                // |sum of nine products| <= 9 * 2^14: with these bounds sum + add - zero point stays inside int32
+                words = words && abs(int64_t(add[k])) < (int64_t(1) << 30) &&
                         wordsScaleApplies(__ldg(epi.main.mult + ci), int32_t(__ldg(epi.main.shift + ci)), epi.main.doubleRound != 0);
             }
         }
