@@ -1285,7 +1285,7 @@ void GraphPipeline::fuseAttention(std::vector<int> &group, const std::vector<Use
         plan->denomOutZp = den.outZp;
         plan->mulShift = int32_t(mulShift), plan->mulRound = int64_t(1) << (mulShift - 1);
         plan->context = makeFastRescale(ctx.mult, ctx.shift, ctx.inZp, ctx.doubleRound);
-        plan->contextOutZp = ctx.outZp, plan->contextLo = -128, plan->contextHi = 127;
+        plan->contextOutZp = ctx.outZp;
 
         // ---- operands
         const int32_t vT = ops_[size_t(pv)].in[1];

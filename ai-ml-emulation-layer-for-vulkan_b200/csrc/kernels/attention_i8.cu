@@ -116,17 +116,10 @@ __device__ __forceinline__ void tmemStore32(uint32_t taddr, const uint32_t (&r)[
 
 // 4-D tensor map {head dimension, token, head, sequence} over an int8 operand with a box of 32 tokens by one 128-byte
 // SWIZZLE_128B row: bytes past the head dimension and tokens past the last arrive as zeros.
-__device__ __forceinline__ void tmaLoad4d(const CUtensorMap *map, void *dst, uint64_t *bar, int c1, int c2, int c3) {
-    asm volatile(
-        "cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6}], [%2];" ::"r"(
-            smemAddr(dst)),
-        "l"(reinterpret_cast<uint64_t>(map)), "r"(smemAddr(bar)), "r"(0), "r"(c1), "r"(c2), "r"(c3)
-        : "memory");
-}
 __device__ __forceinline__ void loadTokens(const CUtensorMap *map, uint8_t *dst, uint64_t *bar, int first, int count, int head,
                                            int sequence) {
     for (int r = 0; r < count; r += kTokenBox) {
-        tmaLoad4d(map, dst + r * kRowBytes, bar, first + r, head, sequence);
+        tmaLoad4d(map, dst + r * kRowBytes, bar, 0, first + r, head, sequence);
     }
 }
 
@@ -189,7 +182,7 @@ attentionI8Kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constan
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmemBase = shared->tmemBase;
-    gridDependencySync(); // from here on activations are read and written
+    dependencySync(); // from here on activations are read and written
 
     struct Tile {
         uint32_t n, h;
@@ -302,7 +295,7 @@ attentionI8Kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constan
                 uint32_t w = 0;
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
-                    w |= uint32_t(uint8_t(fastRescale(a.context, int32_t(s[4 * q + j]), a.contextOutZp, a.contextLo, a.contextHi)))
+                    w |= uint32_t(uint8_t(fastRescale(a.context, int32_t(s[4 * q + j]), a.contextOutZp, -128, 127)))
                          << (8 * j);
                 }
                 packed[q] = w;
@@ -505,7 +498,7 @@ int launchAttention(const CUtensorMap (&maps)[3], AttentionParams p, cudaStream_
     const int blocksPerSm = WARPS == 8 ? 2 : 1;
     p.contextColumn = p.keysPad + p.d <= 512 / blocksPerSm ? p.keysPad : 0;
     const int grid = int(std::min<int64_t>(p.tiles, int64_t(smCount()) * blocksPerSm));
-    if (launchDependent(kernel, grid, WARPS * 32 + 32, smem, s, maps[0], maps[1], maps[2], p) != cudaSuccess) {
+    if (launchOverlapped(kernel, grid, WARPS * 32 + 32, smem, s, maps[0], maps[1], maps[2], p) != cudaSuccess) {
         setLastError(std::string("attention: ") + cudaGetErrorString(cudaGetLastError()));
         return MLEL_ERROR_DEVICE;
     }

@@ -25,7 +25,7 @@ struct AttentionPlan {
     bool narrow;       // both RESCALEs divided by a power of two of their multipliers: (x * mult + addend) >> shift in 32 bits
     bool unsignedProb;                      // zero point -128: probabilities are stored as unsigned bytes
     FastRescale context;
-    int32_t contextOutZp, contextLo, contextHi;
+    int32_t contextOutZp;
 };
 
 // Limits of the kernel: a row of scores fits tensor memory (512 columns) and, with the operands, shared memory; below

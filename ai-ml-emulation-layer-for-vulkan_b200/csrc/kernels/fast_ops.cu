@@ -65,14 +65,13 @@ template <bool BORDER>
 __global__ void __launch_bounds__(256) padPixels16Kernel(const int8_t *__restrict__ in, int4 *__restrict__ out, uint32_t units, int H,
                                                          int W, int C, FastDiv perPixel, FastDiv divWp, FastDiv divHp, int padTop,
                                                          int padLeft) {
-    const auto div = [](uint32_t v, const FastDiv &f) { return f.mul == 0u ? v : __umulhi(v, f.mul) >> f.shift; };
     for (uint32_t e = blockIdx.x * blockDim.x + threadIdx.x; e < units; e += gridDim.x * blockDim.x) {
-        const uint32_t pix = div(e, perPixel);
+        const uint32_t pix = fastDiv(e, perPixel);
         const int c0 = int(e - pix * perPixel.d) * 16;
         int64_t from = pix;
         bool live = c0 < C;
         if (BORDER) {
-            const uint32_t line = div(pix, divWp), n = div(line, divHp);
+            const uint32_t line = fastDiv(pix, divWp), n = fastDiv(line, divHp);
             const int x = int(pix - line * divWp.d) - padLeft, y = int(line - n * divHp.d) - padTop;
             live = live && unsigned(x) < unsigned(W) && unsigned(y) < unsigned(H);
             from = (int64_t(n) * H + y) * W + x;
@@ -89,11 +88,10 @@ template <int STRIDE>
 __global__ void __launch_bounds__(256) gatherUnitsKernel(const int8_t *__restrict__ in, int4 *__restrict__ out, uint32_t units, int H,
                                                          int W, int C, FastDiv divWu, FastDiv divHu, int padTop, int padLeft) {
     dependencySync();
-    const auto div = [](uint32_t v, const FastDiv &f) { return f.mul == 0u ? v : __umulhi(v, f.mul) >> f.shift; };
     const uint32_t mask = C == 4 ? 0xffffffffu : (1u << (8 * C)) - 1u;
     const uint32_t *words = reinterpret_cast<const uint32_t *>(in);
     for (uint32_t e = blockIdx.x * blockDim.x + threadIdx.x; e < units; e += gridDim.x * blockDim.x) {
-        const uint32_t line = div(e, divWu), n = div(line, divHu);
+        const uint32_t line = fastDiv(e, divWu), n = fastDiv(line, divHu);
         const int x0 = int(e - line * divWu.d) * STRIDE - padLeft, y0 = int(line - n * divHu.d) * STRIDE - padTop;
         uint32_t px[4];
 #pragma unroll
@@ -475,8 +473,7 @@ __global__ void __launch_bounds__(256) maxPoolNarrowKernel(const int8_t *__restr
     const uint32_t step = gridDim.x * blockDim.x;
     for (uint64_t e64 = blockIdx.x * blockDim.x + threadIdx.x; e64 < total; e64 += step) {
         const uint32_t e = uint32_t(e64);
-        const auto div = [](uint32_t v, const FastDiv &f) { return f.mul == 0u ? v : __umulhi(v, f.mul) >> f.shift; };
-        const uint32_t pix = div(e, groups), line = div(pix, divOW), n = div(line, divOH);
+        const uint32_t pix = fastDiv(e, groups), line = fastDiv(pix, divOW), n = fastDiv(line, divOH);
         const int c0 = int(e - pix * groups.d) * CH;
         const int ox = int(pix - line * divOW.d), oy = int(line - n * divOH.d);
         const int iy0 = oy * max(a.stride[0], 1) - a.pad[0], ix0 = ox * max(a.stride[1], 1) - a.pad[2];

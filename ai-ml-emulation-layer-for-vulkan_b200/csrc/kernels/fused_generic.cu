@@ -11,6 +11,7 @@
 #include "device_common.cuh"
 #include "gemm_i8_tcgen05.hpp"
 #include "kernels.hpp"
+#include "launch_overlapped.cuh"
 
 namespace mlel {
 
@@ -244,8 +245,7 @@ __global__ void __launch_bounds__(128, 4) depthwise3x3RowsKernel(const int8_t *_
     const uint32_t zword = uint32_t(uint8_t(a.inZp)) * 0x01010101u;
     GRID_STRIDE(e, total) {
         // (four 64-bit divisions here were a tenth of the kernel's instructions)
-        const auto div = [](uint32_t v, const FastDiv &f) { return f.mul == 0u ? v : __umulhi(v, f.mul) >> f.shift; };
-        const uint32_t tx = div(uint32_t(e), divC), ty = div(tx, divX), tn = div(ty, divY);
+        const uint32_t tx = fastDiv(uint32_t(e), divC), ty = fastDiv(tx, divX), tn = fastDiv(ty, divY);
         const int c0 = int(uint32_t(e) - tx * divC.d) * 4, ox0 = int(tx - ty * divX.d) * PX, oy0 = int(ty - tn * divY.d) * R;
         const int n = int(tn);
         // the three weights of a window row of one channel at byte offsets 0 and 1, and their sum
@@ -522,22 +522,6 @@ bool depthwise3x3Eligible(const TView &in, const TView &w, const TView &bias, co
     return (ptrs & 3u) == 0 && (reinterpret_cast<uintptr_t>(out.ptr) & (fused ? 3u : 15u)) == 0;
 }
 
-// Launch with programmatic stream serialization (the kernel must execute griddepcontrol.wait before it touches
-// memory): its blocks may be scheduled while the previous kernel of the stream drains.
-template <class... Params, class... Args>
-static void launchOverlapping(void (*kernel)(Params...), int grid, int threads, cudaStream_t stream, Args &&...args) {
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(unsigned(grid));
-    cfg.blockDim = dim3(unsigned(threads));
-    cfg.stream = stream;
-    cudaLaunchAttribute attr{};
-    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr.val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = &attr;
-    cfg.numAttrs = tensorCoreTuning().dependentLaunch.load(std::memory_order_relaxed) != 0 ? 1 : 0;
-    cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
-}
-
 int depthwise3x3(const TView &in, const TView &w, const TView &bias, const TView &out, const ConvAttr &a,
                  const DevEpilogue *epi, cudaStream_t s) {
     constexpr int PX = 4;
@@ -557,7 +541,7 @@ int depthwise3x3(const TView &in, const TView &w, const TView &bias, const TView
         const int64_t total = int64_t(N) * ((OH + R - 1) / R) * ((OW + PX - 1) / PX) * (C / 4);
         const int grid = gridFor(total, 128, 16);
 #define MLEL_LAUNCH_ROWS(RR, SS, O8) \
-    launchOverlapping(depthwise3x3RowsKernel<RR, SS, O8>, grid, 128, s, pi, pw, pb, nb, out.ptr, N, H, W, C, OH, OW, makeFastDiv(C / 4), \
+    launchOverlapped(depthwise3x3RowsKernel<RR, SS, O8>, grid, 128, 0, s, pi, pw, pb, nb, out.ptr, N, H, W, C, OH, OW, makeFastDiv(C / 4), \
                       makeFastDiv((OW + PX - 1) / PX), makeFastDiv((OH + R - 1) / R), a, e)
         if (epi != nullptr) {
             if (a.stride[1] == 1) {

@@ -123,7 +123,7 @@ gemmI8OcMajor(const __grid_constant__ CUtensorMap tmapX, const __grid_constant__
     // grid before its first store; nobody else touches activations.
     const bool byTiles = X_TMA && p.progressIn != nullptr;
     if (!byTiles) {
-        gridDependencySync();
+        dependencySync();
     } else {
         asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     }
@@ -339,7 +339,7 @@ int launchOcMajor(const OcMaps &maps, const GemmI8Params &params, cudaStream_t s
         return MLEL_ERROR_UNKNOWN;
     }
     const int grid = int(tiles < smCount() ? tiles : smCount());
-    const cudaError_t err = launchDependent(kernel, grid, ocThreadsFor(EW, X_MODE), smemBytes, s, maps.x, maps.w,
+    const cudaError_t err = launchOverlapped(kernel, grid, ocThreadsFor(EW, X_MODE), smemBytes, s, maps.x, maps.w,
                                             maps.c, maps.d, p);
     if (err != cudaSuccess) {
         setLastError(std::string("tcgen05 channel-major convolution launch: ") + cudaGetErrorString(err));

@@ -556,7 +556,7 @@ gemmI8Tcgen05(const __grid_constant__ CUtensorMap tmapA, const __grid_constant__
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmemBase = bars->tmemBase;
-    gridDependencySync(); // from here on activations are read and written
+    dependencySync(); // from here on activations are read and written
 
     if (warp == kTmaWarp) {
         // ---------------- TMA producer ----------------
@@ -797,7 +797,7 @@ int launchVariant(const CUtensorMap &mapA, const CUtensorMap &mapB, const GemmI8
         return MLEL_ERROR_UNKNOWN;
     }
     const int grid = int(tiles < smCount() ? tiles : smCount()); // persistent: one CTA per SM
-    const cudaError_t err = launchDependent(kernel, grid, A_MODE != kAGather ? kThreadsTma : kThreadsGather, smemBytes, s, mapA, mapB, p);
+    const cudaError_t err = launchOverlapped(kernel, grid, A_MODE != kAGather ? kThreadsTma : kThreadsGather, smemBytes, s, mapA, mapB, p);
     if (err != cudaSuccess) {
         setLastError(std::string("tcgen05 int8 GEMM launch: ") + cudaGetErrorString(err));
         return MLEL_ERROR_DEVICE;

@@ -31,6 +31,10 @@ inline FastDiv makeFastDiv(int64_t divisor) {
     }
     return f;
 }
+// n / f.d for n < 2^31
+__device__ __forceinline__ uint32_t fastDiv(uint32_t n, const FastDiv &f) {
+    return f.mul == 0u ? n : __umulhi(n, f.mul) >> f.shift;
+}
 
 enum : int32_t { kLateOperand = 1, kLateCorrections = 2 };
 

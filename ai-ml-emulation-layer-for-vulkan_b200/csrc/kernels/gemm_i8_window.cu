@@ -68,13 +68,6 @@ struct __align__(8) WindowBarriers {
     uint32_t tmemBase, forms;
 };
 
-__device__ __forceinline__ void tmaLoad4d(const CUtensorMap *map, void *dst, uint64_t *bar, int c0, int c1, int c2, int c3) {
-    asm volatile(
-        "cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6}], [%2];"
-        ::"r"(smemAddr(dst)), "l"(reinterpret_cast<uint64_t>(map)), "r"(smemAddr(bar)), "r"(c0), "r"(c1), "r"(c2), "r"(c3)
-        : "memory");
-}
-
 // Descriptor of a K-major operand whose rows are `rowBytes` long in the swizzle of that width.
 __device__ __forceinline__ uint64_t rowDesc(uint32_t addr, uint32_t rowBytes, uint32_t groupBytes) {
     const uint64_t layout = rowBytes == 128 ? 2 : (rowBytes == 64 ? 4 : 6);
@@ -160,7 +153,7 @@ gemmI8Window(const __grid_constant__ CUtensorMap mapX, const __grid_constant__ C
                     tmaLoad3d(&mapW, weights + t * tapBytes, &bars->weights, 0, t, c0);
                 }
             }
-            gridDependencySync();
+            dependencySync();
             int s = 0;
             uint32_t phase = 0;
             for (int tile = firstTile; tile < g.pixelTiles; tile += tileStep) {
@@ -187,7 +180,7 @@ gemmI8Window(const __grid_constant__ CUtensorMap mapX, const __grid_constant__ C
         // registers.  (With the loop inside `if (lane == 0)` every MMA cost the thread some 200 cycles of moves and waits behind
         // the epilogue warps of its scheduler, 4000 of a 64-channel tile's 4600.)  A wait that runs out only ends the waiting:
         // the later MMAs read old bytes, the recorded error tells.
-        gridDependencySync();
+        dependencySync();
         constexpr uint32_t idesc = instrDesc(BN, false);
         const uint32_t groupBytes = uint32_t((g.blocks ? g.boxW : 8) * g.pixelBytes), leader = lane == 0 ? 1u : 0u;
         const uint64_t descX = rowDesc(smemAddr(stages), uint32_t(g.pixelBytes), groupBytes);
@@ -302,7 +295,7 @@ gemmI8Window(const __grid_constant__ CUtensorMap mapX, const __grid_constant__ C
             colTab[threadIdx.x] = makeColConst(f, corr0, p.epi.main, form);
         }
         epilogueSync();
-        gridDependencySync();
+        dependencySync();
 
         const int quarter = warp & 3, part = warp >> 2, set = part / kGroups, group = part - set * kGroups;
         const int row = quarter * 32 + lane;
@@ -420,7 +413,7 @@ int launchWindowRows(const CUtensorMap &mapX, const CUtensorMap &mapW, const Gem
         return MLEL_ERROR_DEVICE;
     }
     const int perChannelTile = std::max(1, std::min(smCount() / g.channelTiles, g.pixelTiles));
-    const cudaError_t err = launchDependent(kernel, perChannelTile * g.channelTiles, kThreadsTma, smem, s, mapX, mapW, p, g);
+    const cudaError_t err = launchOverlapped(kernel, perChannelTile * g.channelTiles, kThreadsTma, smem, s, mapX, mapW, p, g);
     if (err != cudaSuccess) {
         setLastError(std::string("int8 window launch: ") + cudaGetErrorString(err));
         return MLEL_ERROR_DEVICE;

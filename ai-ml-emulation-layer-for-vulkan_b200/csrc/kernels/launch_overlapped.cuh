@@ -1,10 +1,14 @@
-// Programmatic dependent launch for the kernels between the tensor-core launches.
+// Programmatic dependent launch.  A kernel launched this way may start while the kernel before it in the stream is still
+// running (on SMs that kernel has already left): everything up to dependencySync() - barrier and TMEM set-up, tables built
+// from graph constants - overlaps the predecessor's tail.  The wait returns when the predecessor has completed and its
+// writes are visible; nothing before it may touch memory that another kernel of the stream writes or reads for writing
+// later.  The trigger lets the successor start as early as it finds room.  Both are no-ops in a kernel launched the
+// ordinary way.
 //
-// A kernel launched this way is set up and its blocks are scheduled while the kernel before it in the stream drains; it
-// calls dependencySync() before it touches memory that another kernel writes or will write.  Worth it between two
-// tensor-core launches (the layer norms and the GELU of a BERT-shaped encoder: 2.495 -> 2.451 ms per dispatch of 168
-// nodes); not in a chain of short element-wise kernels, where a replayed graph's ordinary edges are as quick (the twelve
-// operators of a graph of small ones: 31 us with ordinary launches, 34 with these).
+// Beside the tensor-core kernels it is worth it between two of their launches (the layer norms and the GELU of a
+// BERT-shaped encoder: 2.495 -> 2.451 ms per dispatch of 12 layers); not in a chain of short element-wise kernels, where a
+// replayed graph's ordinary edges are as quick (the twelve operators of a graph of small ones: 31 us with ordinary
+// launches, 34 with these).
 #pragma once
 
 #include <cuda_runtime.h>
@@ -15,16 +19,14 @@
 
 namespace mlel {
 
-// Lets the next kernel of the stream be scheduled, then waits for the one before to complete with its writes visible.
-// Both are no-ops in a kernel launched the ordinary way.
 __device__ __forceinline__ void dependencySync() {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
 template <class... Params, class... Args>
-inline void launchOverlapped(void (*kernel)(Params...), dim3 grid, unsigned threads, size_t smemBytes, cudaStream_t stream,
-                             Args &&...args) {
+inline cudaError_t launchOverlapped(void (*kernel)(Params...), dim3 grid, unsigned threads, size_t smemBytes, cudaStream_t stream,
+                                    Args &&...args) {
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = grid;
     cfg.blockDim = dim3(threads);
@@ -35,7 +37,7 @@ inline void launchOverlapped(void (*kernel)(Params...), dim3 grid, unsigned thre
     attr.val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = &attr;
     cfg.numAttrs = tensorCoreTuning().dependentLaunch.load(std::memory_order_relaxed) != 0 ? 1 : 0;
-    cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
+    return cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
 }
 
 } // namespace mlel

@@ -32,8 +32,6 @@ int finish(const char *what) {
     return MLEL_SUCCESS;
 }
 
-__device__ __forceinline__ uint32_t divBy(uint32_t n, const FastDiv &f) { return f.mul == 0u ? n : __umulhi(n, f.mul) >> f.shift; }
-
 // One strided copy: `axes` outer axes (the last varies fastest) over runs of contiguous bytes.
 struct RunMove {
     const uint8_t *src;
@@ -60,11 +58,11 @@ template <typename UNIT> __global__ void __launch_bounds__(256) runMoveKernel(co
             const uint64_t e = first + uint64_t(u) * step;
             dst[u] = -1;
             if (e < m.units) {
-                uint32_t row = divBy(uint32_t(e), m.unitsPerRun);
+                uint32_t row = fastDiv(uint32_t(e), m.unitsPerRun);
                 const int64_t r = int64_t(uint32_t(e) - row * m.unitsPerRun.d) * int64_t(sizeof(UNIT));
                 int64_t so = r, to = r;
                 for (int k = m.axes - 1; k >= 0; --k) {
-                    const uint32_t q = k > 0 ? divBy(row, m.dims[k]) : 0u;
+                    const uint32_t q = k > 0 ? fastDiv(row, m.dims[k]) : 0u;
                     const int64_t i = row - q * m.dims[k].d;
                     so += i * m.srcStride[k];
                     to += i * m.dstStride[k];
@@ -217,13 +215,13 @@ __global__ void __launch_bounds__(256) tileTransposeKernel(const uint8_t *__rest
     __shared__ __align__(16) uint8_t tile[64 * kPitch];
     const int x = threadIdx.x & 63, y0 = threadIdx.x >> 6;
     for (uint32_t t = blockIdx.x; t < tiles; t += gridDim.x) {
-        uint32_t matrix = divBy(t, p.tilesPerMatrix);
+        uint32_t matrix = fastDiv(t, p.tilesPerMatrix);
         const uint32_t inMatrix = t - matrix * p.tilesPerMatrix.d;
-        const uint32_t tr = divBy(inMatrix, p.tilesC);
+        const uint32_t tr = fastDiv(inMatrix, p.tilesC);
         const int r0 = int(tr) * 64, c0 = int(inMatrix - tr * p.tilesC.d) * 64;
         int64_t so = 0, to = 0;
         for (int k = p.axes - 1; k >= 0; --k) {
-            const uint32_t q = divBy(matrix, p.dims[k]);
+            const uint32_t q = fastDiv(matrix, p.dims[k]);
             const int64_t i = matrix - q * p.dims[k].d;
             so += i * p.srcStride[k];
             to += i * p.dstStride[k];
@@ -278,9 +276,9 @@ __global__ void __launch_bounds__(256)
                         FastDiv divOH, uint32_t H, uint32_t W, ResizeAttr a) {
     const uint32_t step = gridDim.x * blockDim.x;
     for (uint32_t e = blockIdx.x * blockDim.x + threadIdx.x; e < units; e += step) {
-        const uint32_t pixel = divBy(e, perPixel), u = e - pixel * perPixel.d;
-        const uint32_t line = divBy(pixel, divOW), ox = pixel - line * divOW.d;
-        const uint32_t n = divBy(line, divOH), oy = line - n * divOH.d;
+        const uint32_t pixel = fastDiv(e, perPixel), u = e - pixel * perPixel.d;
+        const uint32_t line = fastDiv(pixel, divOW), ox = pixel - line * divOW.d;
+        const uint32_t n = fastDiv(line, divOH), oy = line - n * divOH.d;
         const uint32_t y = nearestSource(oy, a.scale[0], a.scale[1], a.offset[0], H);
         const uint32_t x = nearestSource(ox, a.scale[2], a.scale[3], a.offset[1], W);
         UNIT v{}; // a position outside the image reads zero

@@ -422,7 +422,7 @@ __device__ __forceinline__ void epilogueOcMajor(const CUtensorMap *tmapD, const 
         }
         if (ODD) {
             if (p.progressIn != nullptr && tileCount == 0) {
-                gridDependencySync(); // (see below)
+                dependencySync(); // (see below)
             }
             ocEpilogueSync<EW>(); // the tile is complete; its buffer's next writers come from the barrier of the tile after
             const int rows = min(BNP, p.M - m0), length = min(kOcTile, p.N - c0);
@@ -464,7 +464,7 @@ __device__ __forceinline__ void epilogueOcMajor(const CUtensorMap *tmapD, const 
                 // This launch started on the finished tiles of the launch before it.  Its output may lie where that
                 // launch's input lay (the session plans memory by life times), so nothing is written before that
                 // launch has ended.
-                gridDependencySync();
+                dependencySync();
             }
             tmaStore3d(tmapD, cdTiles + buf * (BNP * 128), c0, m0, batch);
             asm volatile("cp.async.bulk.commit_group;" ::: "memory");
@@ -499,7 +499,7 @@ __device__ __forceinline__ void storeWarpOcMajor(const CUtensorMap *tmapD, const
             // This launch started on the finished tiles of the launch before it.  Its output may lie where that
             // launch's input lay (the session plans memory by life times), so nothing is written before that
             // launch has ended.
-            gridDependencySync();
+            dependencySync();
         }
         tmaStore3d(tmapD, cdTiles + buf * (BNP * 128), int(ti.chan) * C_TILE + walk.cOffset, int(ti.pix) * BNP, int(ti.batch));
         asm volatile("cp.async.bulk.commit_group;" ::: "memory");

@@ -17,6 +17,7 @@
 
 #include "device_common.cuh"
 #include "gemm_i8_tcgen05.hpp"
+#include "launch_overlapped.cuh"
 
 namespace mlel {
 
@@ -263,15 +264,12 @@ __device__ __forceinline__ void tmemWait16(uint32_t (&r)[16]) {
                  : "memory");
 }
 
-// Programmatic dependent launch.  A kernel launched with launchDependent() may start while the kernel before
-// it in the stream is still running (on SMs that kernel has already left): everything up to this call - barrier
-// and TMEM set-up, tables built from graph constants - overlaps the predecessor's tail.  The wait returns when
-// the predecessor has completed and its writes are visible; nothing before it may touch memory that another
-// kernel of the stream writes or reads for writing later.  The trigger lets the successor start as early as
-// it finds room.  Both are no-ops in a kernel launched the ordinary way.
-__device__ __forceinline__ void gridDependencySync() {
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    asm volatile("griddepcontrol.wait;" ::: "memory");
+// A box of a 4-D tensor map, at the coordinates c0 (fastest) to c3.
+__device__ __forceinline__ void tmaLoad4d(const CUtensorMap *map, void *dst, uint64_t *bar, int c0, int c1, int c2, int c3) {
+    asm volatile(
+        "cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6}], [%2];"
+        ::"r"(smemAddr(dst)), "l"(reinterpret_cast<uint64_t>(map)), "r"(smemAddr(bar)), "r"(c0), "r"(c1), "r"(c2), "r"(c3)
+        : "memory");
 }
 
 __device__ __forceinline__ uint32_t ldsU8(uint32_t addr) {
@@ -299,11 +297,6 @@ __device__ __forceinline__ void storeRowBytes(int8_t *to, uint32_t from, int len
 }
 
 // Barrier among the epilogue warps only (named barrier 1).
-// n / f.d for n < 2^31 (see FastDiv)
-__device__ __forceinline__ uint32_t fastDiv(uint32_t n, const FastDiv &f) {
-    return f.mul == 0u ? n : __umulhi(n, f.mul) >> f.shift;
-}
-
 __device__ __forceinline__ void epilogueSync() {
     asm volatile("bar.sync 1, %0;" ::"r"(kEpilogueWarps * 32) : "memory");
 }
@@ -573,24 +566,6 @@ inline bool makeIm2colMap(CUtensorMap *map, const void *base, int N, int H, int 
                   elemStrides, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
     });
-}
-
-// Launches `kernel` so that it may overlap the end of its predecessor in the stream (see gridDependencySync).
-template <class... Params, class... Args>
-inline cudaError_t launchDependent(void (*kernel)(Params...), int grid, int threads, size_t smemBytes, cudaStream_t stream,
-                                   Args &&...args) {
-    const bool disabled = tensorCoreTuning().dependentLaunch.load(std::memory_order_relaxed) == 0;
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(unsigned(grid));
-    cfg.blockDim = dim3(unsigned(threads));
-    cfg.dynamicSmemBytes = smemBytes;
-    cfg.stream = stream;
-    cudaLaunchAttribute attr{};
-    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr.val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = &attr;
-    cfg.numAttrs = disabled ? 0 : 1;
-    return cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
 }
 
 // Number of SMs of the device that is current (cached per device).

@@ -72,8 +72,6 @@ bool rowBroadcast(const TView &b, const TView &out) {
 
 bool aligned16(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
-__device__ __forceinline__ uint32_t divBy(uint32_t n, const FastDiv &f) { return f.mul == 0u ? n : __umulhi(n, f.mul) >> f.shift; }
-
 bool signedInt(int32_t dtype) { return dtype == MLEL_I8 || dtype == MLEL_I16 || dtype == MLEL_I32; }
 
 // Four consecutive elements of a signed integer type, widened to int32.
@@ -376,8 +374,8 @@ __global__ void binaryI32Kernel(const int32_t *__restrict__ a, const int32_t *__
                 v.y = *reinterpret_cast<const int4 *>(b + 4 * g);
             } else if (B_MODE == 3) {
                 const uint32_t e = uint32_t(4 * g);
-                v.y = make_int4(__ldg(b + divBy(e, divRow)), __ldg(b + divBy(e + 1, divRow)), __ldg(b + divBy(e + 2, divRow)),
-                                __ldg(b + divBy(e + 3, divRow)));
+                v.y = make_int4(__ldg(b + fastDiv(e, divRow)), __ldg(b + fastDiv(e + 1, divRow)), __ldg(b + fastDiv(e + 2, divRow)),
+                                __ldg(b + fastDiv(e + 3, divRow)));
             } else {
                 const int32_t y = __ldg(b + (B_MODE == 1 ? (4 * g) / rowLen : 0));
                 v.y = make_int4(y, y, y, y);
@@ -627,13 +625,13 @@ struct RowPermute {
 
 __global__ void transposeRowsKernel(const uint8_t *__restrict__ in, uint8_t *__restrict__ out, int64_t chunks, RowPermute p) {
     GRID_STRIDE(e, chunks) { // the launcher refuses 2^31 chunks and more
-        uint32_t row = divBy(uint32_t(e), p.chunksPerRow);
+        uint32_t row = fastDiv(uint32_t(e), p.chunksPerRow);
         const uint32_t chunk = uint32_t(e) - row * p.chunksPerRow.d;
         int64_t src = 0;
 #pragma unroll
         for (int i = kMaxRank - 1; i >= 0; --i) {
             if (i < p.rank) {
-                const uint32_t q = divBy(row, p.outDims[i]);
+                const uint32_t q = fastDiv(row, p.outDims[i]);
                 src += int64_t(row - q * p.outDims[i].d) * p.inStride[i];
                 row = q;
             }
@@ -663,9 +661,9 @@ __global__ void __launch_bounds__(256) transposeLast2BytesKernel(const uint8_t *
     const int lane = threadIdx.x & 31;
     for (int64_t wid = (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5; wid < warps;
          wid += (int64_t(gridDim.x) * blockDim.x) >> 5) {
-        uint32_t batch = divBy(uint32_t(wid), p.perBatch);
+        uint32_t batch = fastDiv(uint32_t(wid), p.perBatch);
         const uint32_t inMat = uint32_t(wid) - batch * p.perBatch.d;
-        const uint32_t rowGroup = divBy(inMat, p.colGroups);
+        const uint32_t rowGroup = fastDiv(inMat, p.colGroups);
         const int c0 = int(inMat - rowGroup * p.colGroups.d) * 32 + (lane & 1) * 16;
         const int r = (int(rowGroup) * 16 + (lane >> 1)) * 8;
         uint8_t *dst = out + int64_t(batch) * R * Ccols;
@@ -673,7 +671,7 @@ __global__ void __launch_bounds__(256) transposeLast2BytesKernel(const uint8_t *
 #pragma unroll
         for (int i = kMaxRank - 1; i >= 0; --i) {
             if (i < p.rank) {
-                const uint32_t q = divBy(batch, p.outDims[i]);
+                const uint32_t q = fastDiv(batch, p.outDims[i]);
                 src += int64_t(batch - q * p.outDims[i].d) * p.inStride[i];
                 batch = q;
             }
