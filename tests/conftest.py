@@ -12,7 +12,7 @@ from __graft_entry__ import load_package  # noqa: E402
 load_package()  # registers the package as module "mlel_b200" so that tests can import its submodules
 
 # checkout of the reference project: present only where the fixtures were authored, never needed on a GPU box
-REFERENCE_ROOT = os.environ.get("MLEL_REFERENCE_ROOT", "/root/reference")
+REFERENCE_ROOT = os.environ.get("MLEL_REFERENCE_ROOT")
 
 
 def pytest_configure(config):
@@ -29,7 +29,7 @@ def mlel():
 
 @pytest.fixture(scope="session")
 def reference_root():
-    if not os.path.isdir(os.path.join(REFERENCE_ROOT, "tests")):  # absent, or an empty mount point
+    if not REFERENCE_ROOT or not os.path.isdir(os.path.join(REFERENCE_ROOT, "tests")):  # absent, or an empty mount point
         pytest.skip("reference checkout not present")
     return REFERENCE_ROOT
 

@@ -105,4 +105,4 @@ def main(ref_root: str) -> None:
 
 
 if __name__ == "__main__":
-    main(sys.argv[1] if len(sys.argv) > 1 else os.environ.get("MLEL_REFERENCE_ROOT", "/root/reference"))
+    main(sys.argv[1] if len(sys.argv) > 1 else os.environ["MLEL_REFERENCE_ROOT"])
