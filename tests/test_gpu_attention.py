@@ -68,3 +68,43 @@ def test_attention_outside_the_kernel_stays_with_the_operators(mlel, n, heads, s
     runner = GraphRunner(g)
     assert ATTENTION not in runner.pipeline.exec_names()
     np.testing.assert_array_equal(runner.run(data)[0], evaluate(g, data)[0])
+
+
+def softmax_variant(form, n, heads, s, d, seed):
+    """An attention that is not the fused node's: a mask added to the scores, the factors of MUL the other way round, a
+    second reader of the probabilities."""
+    rng = np.random.Generator(np.random.PCG64(seed))
+    x = (np.arange(513, dtype=np.float64) - 256.0) * 128.0
+    exp_lut = np.round(32767.0 * np.exp(np.minimum(x, 0.0) / 4096.0)).astype(np.int16)
+    recip_lut = np.clip(np.round(32767.0 * 256.0 / (x + 32768.0 + 256.0)), 0, 32767).astype(np.int16)
+    g = GraphBuilder("attention_variant")
+    q, k, v = g.input(np.int8, (n * heads, s, d)), g.input(np.int8, (n * heads, d, s)), g.input(np.int8, (n * heads, s, d))
+    data = [rng.integers(-128, 128, t.shape, dtype=np.int8) for t in (q, k, v)]
+    q, k, v = (g.clamp(t, -128, 127) for t in (q, k, v))
+    scores = g.matmul(q, k, 0, 0)
+    if form == "mask":
+        mask = g.input(np.int32, (n * heads, 1, s))
+        data.append(np.where(rng.random((n * heads, 1, s)) < 0.3, -(1 << 22), 0).astype(np.int32))
+        scores = g.add(scores, mask)
+    diff = g.sub(scores, g.reduce("REDUCE_MAX", scores, 2))
+    e = g.table(g.rescale(diff, [1 << 30], [30 + max(2, int(math.log2(d)) - 2)], 0, 0, np.int16), exp_lut)
+    log_keys = max(1, math.ceil(math.log2(s)))
+    r = g.table(g.rescale(g.reduce("REDUCE_SUM", e, 2), [1 << 30], [37 + log_keys], 0, -32768, np.int16), recip_lut)
+    p = g.rescale(g.mul(r, e, 22) if form == "swapped" else g.mul(e, r, 22), [1 << 30], [37 + log_keys], 0, -128, np.int8)
+    if form == "read twice":
+        g.output(g.clamp(p, -100, 100))
+    g.output(g.rescale(g.matmul(p, v, -128, 0), [(1 << 30) + 3], [38], 0, 3, np.int8, double_round=True))
+    return g, data
+
+
+@pytest.mark.parametrize("form", ["mask", "swapped", "read twice"])
+@pytest.mark.parametrize("n,heads,s,d", [(2, 3, 64, 32), (1, 2, 197, 64)])
+def test_attention_of_another_form_stays_with_the_operators(mlel, form, n, heads, s, d):
+    from mlel_b200.runtime import GraphRunner
+    g, data = softmax_variant(form, n, heads, s, d, s)
+    runner = GraphRunner(g)
+    assert ATTENTION not in runner.pipeline.exec_names()
+    want = evaluate(g, data)
+    for use_cuda_graph in (False, True):
+        for a, b in zip(runner.run(data, use_cuda_graph=use_cuda_graph), want):
+            np.testing.assert_array_equal(a, b)

@@ -76,3 +76,27 @@ def test_result_scale_with_any_zero_point(mlel, in_zp, mult, shift):
     factor = g.table(g.rescale(var, [1 << 30], [34], 0, -32768, np.int16), _lut16(r))
     g.output(g.rescale(g.mul(cen, factor, 12), [mult], [shift], in_zp, 3, np.int8))
     check_fused(mlel, g, [full_range(r, np.int8, shape), full_range(r, np.int8, shape)], [NORM])
+
+
+@pytest.mark.parametrize("length", [64, 132])
+def test_layer_norm_with_gain_and_bias(mlel, length):
+    """Per-channel gain and bias behind the normalisation: not the register kernel's program, the operators' results."""
+    from mlel_b200.runtime import GraphRunner
+    from tests.graph_eval import evaluate
+    from tests.test_gpu_vector_ops import _lut16
+    r = rng(length)
+    shape = (1, 19, length)
+    g = GraphBuilder()
+    a, b = g.input(np.int8, shape), g.input(np.int8, shape)
+    t = g.add(g.rescale(a, [1 << 30], [24], 0, 0, np.int32), g.rescale(b, [1 << 30], [24], 0, 0, np.int32))
+    inv = g.inline(np.asarray([(1 << 20) // length], np.int32).reshape(1, 1, 1))
+    cen = g.sub(t, g.mul(g.reduce("REDUCE_SUM", t, 2), inv, 20))
+    var = g.mul(g.reduce("REDUCE_SUM", g.mul(cen, cen, 8), 2), inv, 20)
+    y = g.mul(cen, g.table(g.rescale(var, [1 << 30], [34], 0, -32768, np.int16), _lut16(r)), 12)
+    gain, bias = (g.constant(r.integers(lo, hi, (1, 1, length)).astype(np.int32)) for lo, hi in ((200, 300), (-99, 99)))
+    g.output(g.rescale(g.add(g.mul(y, gain, 8), bias), [1 << 30], [45], 0, 3, np.int8, double_round=True))
+    data = [full_range(r, np.int8, shape), full_range(r, np.int8, shape)]
+    runner = GraphRunner(g)
+    assert NORM not in runner.pipeline.exec_names()
+    for use_cuda_graph in (False, True):
+        np.testing.assert_array_equal(runner.run(data, use_cuda_graph=use_cuda_graph)[0], evaluate(g, data)[0])
