@@ -1752,7 +1752,7 @@ int32_t GraphPipeline::addScratchTensor(int32_t dtype, const std::vector<int64_t
 // needs beyond the graph's own tensors.  Everything here is derived once from constant data.
 //
 // CONV2D (plain or fused): int8 NHWC input, packed; constant int8 OHWI weights with zero point 0;
-// constant int32 bias; IC and OC multiples of 16; K = KH*KW*IC <= 65536 so that the raw int32 sum of
+// constant int32 bias; K = KH*KW*IC (channels padded) <= 65536 so that the raw int32 sum of
 // products cannot overflow.  The correction table holds, per border class of an output pixel,
 //     corr[class][oc] = bias[oc] - inputZeroPoint * sum over the taps that are in range of w[oc, tap, :]
 // which turns the tensor core's sum(x * w) over zero-filled taps into the reference's
@@ -2048,8 +2048,6 @@ void GraphPipeline::prepareTensorCore() {
                 // correction; all land in one scratch tensor: the copy of the first input (if any), [Nb][W][Cp] bytes,
                 // then [Nb][W] int32.
                 const int64_t btBytes = (Nb * W * Cp + 255) / 256 * 256;
-                // (Copy, transpose and product are three launches, about 8 us for the smallest sizes; one thread per
-                // output is quicker while its chain of C products and the total are short.)
                 if (aBytes + btBytes + Nb * W * 4 >= (int64_t(1) << 31)) {
                     continue;
                 }

@@ -1,11 +1,12 @@
 // Vectorised kernels for the element-wise, table, reduction and data-movement operators on packed
 // tensors.  Each has a generic counterpart in generic_ops.cu that defines the result for every rank, stride
 // and type; these take the common case - contiguous tensors, signed integer types, operands of the same
-// shape or broadcast along the last axis - and only change how the bytes move: four elements per thread
-// with 4-, 8- or 16-byte accesses, no index unravelling, a warp per row for reductions.  The arithmetic is
-// the same functions (device_common.cuh), so the results are the same bits.  Element counts that are no multiple of a
-// thread's group leave one to fifteen elements, which a thread each takes (REDUCE_SUM over 2364 rows of 197 in the
-// one-thread-per-row generic kernel: 132 us, here 6.1; SUB by rows of 197: 16.4 -> 6.1 us).
+// shape or broadcast along the last axis - and move 16 bytes a thread and access where they can, several accesses in
+// flight, without index unravelling; reductions have a warp per row.  Where the arithmetic is not the generic kernels'
+// own function (RESCALE as one multiply-add, CLAMP on 16-bit lanes, TABLE from words that hold two entries) it gives the
+// same bits.  Element counts that are no multiple of a thread's group leave one to fifteen elements, which a thread each
+// takes (REDUCE_SUM over 2364 rows of 197 in the one-thread-per-row generic kernel: 132 us, here 6.1; SUB by rows of 197:
+// 16.4 -> 6.1 us).
 //
 // Every entry point returns false when it does not apply; the caller then runs the generic kernel.
 #include <algorithm>

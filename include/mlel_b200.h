@@ -250,7 +250,8 @@ int mlel_session_set_external(mlel_session *s, uint32_t set, uint32_t binding, u
 /* vkCmdDispatchDataGraphARM + queue submission: enqueues every kernel of the graph on `stream`. */
 int mlel_session_dispatch(mlel_session *s, void *cuda_stream);
 /* Same, replayed from a CUDA graph captured on first use.  One graph is kept per set of bound addresses (up to
- * 64 sets), so a host that alternates between a few input and output buffers replays a graph for each. */
+ * 64 sets), so a host that alternates between a few input and output buffers replays a graph for each.  The first dispatch
+ * of a pipeline (of either kind) uploads its constants, and the first with a set of addresses captures its graph. */
 int mlel_session_dispatch_graph(mlel_session *s, void *cuda_stream);
 /* Dispatch with a CUDA event pair around every launched kernel, the counterpart of the reference's
  * per-operator timestamp profiling (VMEL_GRAPH_PROFILING, graph/graph_profiler.cpp:157-191).
@@ -334,7 +335,8 @@ int mlel_selftest_wait_timeout(void *cuda_stream, int *recorded_code);
  * (two-CTA) one, 3 the small-problem one, 4 the window one; -1 for another index.  Tests use it to see which kernel took a case. */
 long long mlel_tensor_core_launches(int kernel);
 
-/* Number of kernels one dispatch launches. */
+/* Number of entries of the list that one dispatch runs (mlel_pipeline_exec_name).  A RESHAPE whose tensors share storage is
+ * an entry and launches nothing; an operator whose operand is copied or transposed first launches two or three kernels. */
 int mlel_session_launch_count(const mlel_session *s);
 /* Host-buffer convenience used for end-to-end timing: copies `n_in` host inputs to their bound
  * device tensors, dispatches, copies `n_out` outputs back, and synchronises the stream. */
