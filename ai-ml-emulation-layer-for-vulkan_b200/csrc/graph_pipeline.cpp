@@ -1054,7 +1054,10 @@ void GraphPipeline::fuseRowRuns(std::vector<int> &group, const std::vector<UseIn
 
 // MATMUL(Q, K^T) -> row-wise softmax -> MATMUL(P, V) -> RESCALE -> OP_FUSED_ATTENTION (kernels/attention_i8.cu), with the
 // transposes that split Q, K and V into heads and merge the context again taken in as strides where nothing else reads
-// them.  Conditions beyond the pattern itself:
+// them.  The pattern is a sequence, not a meaning: scores with two readers, REDUCE_MAX along the last axis and SUB(scores,
+// maximum); RESCALE to int16, TABLE; exponentials with two readers, REDUCE_SUM along the last axis and MUL(exponentials,
+// reciprocal) in this order; RESCALE to int16 and TABLE for the reciprocal; RESCALE to int8.  A graph that states it another
+// way (a mask ADD on the scores, MUL's operands swapped) keeps its operators.  Conditions beyond the pattern itself:
 //   * a row of scores fits the kernel (at most kAttentionMaxKeys keys), head dimension a multiple of 32 up to 128: 32 is
 //     the tensor core's K step, below it the score product would be mostly padding;
 //   * zero points 0 on Q, K and V, and 0 or -128 on the probabilities (signed or unsigned operand bytes);

@@ -2,9 +2,10 @@
 //   t = RESCALE(a) + RESCALE(b);  c = t - MUL(SUM(t), k1, s1);  d = TABLE(RESCALE(MUL(SUM(MUL(c, c, s2)), k2, s3)))
 //   out = RESCALE(MUL(c, d, s4))
 // on int8 rows (reduce.comp, elementwise_binary.comp, mul.comp, rescale.comp, table.comp).  rowMachine() hands a program
-// over when rowNormMatch() recognises it; anything else runs in the row machine, which keeps every value of a row in
-// shared memory and pays its interpreter and a shared-memory round trip per operator: 63 us for 12 288 rows of 768,
-// where the bytes (28 MB, mostly in L2) take about 5.
+// over when rowNormMatch() recognises it: these instructions in this order, operands of ADD and MUL either way round.
+// Anything else (a gain or bias per channel) runs in the row machine or as kernels of its own.  The row machine keeps every
+// value of a row in shared memory and pays its interpreter and a shared-memory round trip per operator: 63 us for 12 288
+// rows of 768, where the bytes (28 MB, mostly in L2) take about 5.
 //
 // A warp owns a row and keeps it in registers, four neighbouring elements per lane and 128-element group.  What is left
 // is bound by the integer instructions of the arithmetic.  NARROW: RESCALEs whose multiplier is a small number times a
