@@ -480,6 +480,11 @@ int Session::dispatchGraph(cudaStream_t stream) {
              pipeline_->tensor(op.in[0]).numel() * pipeline_->tensor(op.in[1]).dims.back() >= int64_t(1) << 24)) {
             return dispatch(stream);
         }
+        // (a stream that is being captured takes kernels, not the launch of a graph)
+        cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+        if (cudaStreamIsCapturing(stream, &status) == cudaSuccess && status == cudaStreamCaptureStatusActive) {
+            return dispatch(stream);
+        }
     }
     // A captured graph holds the addresses that were bound when it was taken: one graph per set of bindings.
     constexpr size_t kMaxCapturedGraphs = 64;

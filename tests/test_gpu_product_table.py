@@ -60,3 +60,30 @@ def test_product_of_activations_dispatched_by_either_way(mlel, table, k, n):
     buffer[1:1 + b8.size] = torch.from_numpy(b8.reshape(-1).view(np.uint8)).cuda()
     runner.session.set_external(*runner._in_keys[1][:2], buffer.data_ptr() + 1)
     assert np.array_equal(runner.run([a8, b8], use_cuda_graph=True)[0], want)
+
+
+@pytest.mark.parametrize("table", [False, True])
+@pytest.mark.parametrize("dispatched_before", [False, True])
+def test_product_of_activations_inside_a_capture(mlel, table, dispatched_before):
+    """A host that captures its stream gets the kernels, whichever way the session dispatches otherwise."""
+    import torch
+    from mlel_b200.runtime import GraphRunner
+    from tests.graph_eval import evaluate
+    r = np.random.Generator(np.random.PCG64(5))
+    a8, b8 = (r.integers(-128, 128, s, dtype=np.int8) for s in ((2, 300, 256), (2, 256, 256)))
+    g = GraphBuilder()
+    a, b = g.input(np.int8, a8.shape), g.input(np.int8, b8.shape)
+    y = g.rescale(g.matmul(a, b, 3, 0), [1 << 30 | 12345], [37], 0, 1, np.int8, double_round=True)
+    g.output(g.table(y, r.integers(-128, 128, (256,), dtype=np.int8)) if table else y)
+    runner = GraphRunner(g)
+    runner.run([a8, b8])  # uploads the constants
+    if dispatched_before:
+        runner.dispatch(use_cuda_graph=True)
+    torch.cuda.synchronize()
+    runner.outputs[0].zero_()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        runner.dispatch(use_cuda_graph=True)
+    assert not np.array_equal(runner.get_outputs()[0], evaluate(g, [a8, b8])[0])  # captured, not run
+    graph.replay()
+    assert np.array_equal(runner.get_outputs()[0], evaluate(g, [a8, b8])[0])
