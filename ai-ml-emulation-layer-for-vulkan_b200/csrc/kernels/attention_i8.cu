@@ -194,25 +194,32 @@ attentionI8Kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constan
     };
 
     if (warp == WARPS) {
-        if (lane == 0) {
-            // ---------------- loads and MMAs ----------------
+        {
+            // ---------------- loads (by one lane) and MMAs (by the whole warp, see ummaBlockPeek) ----------------
             const auto loadQK = [&](const Tile &t) {
-                mbarArriveExpectTx(&shared->loadedQK, uint32_t((BM + p.keysPad) * kRowBytes));
-                loadTokens(&mapQ, tileQ, &shared->loadedQK, t.q0, BM, int(t.h), int(t.n));
-                loadTokens(&mapK, tileK, &shared->loadedQK, 0, p.keysPad, int(t.h), int(t.n));
+                if (lane == 0) {
+                    mbarArriveExpectTx(&shared->loadedQK, uint32_t((BM + p.keysPad) * kRowBytes));
+                    loadTokens(&mapQ, tileQ, &shared->loadedQK, t.q0, BM, int(t.h), int(t.n));
+                    loadTokens(&mapK, tileK, &shared->loadedQK, 0, p.keysPad, int(t.h), int(t.n));
+                }
+                __syncwarp();
             };
             const auto loadV = [&](const Tile &t) {
-                mbarArriveExpectTx(&shared->loadedV, uint32_t(p.keysPad * kRowBytes));
-                loadTokens(&mapV, tileV, &shared->loadedV, 0, p.keysPad, int(t.h), int(t.n));
+                if (lane == 0) {
+                    mbarArriveExpectTx(&shared->loadedV, uint32_t(p.keysPad * kRowBytes));
+                    loadTokens(&mapV, tileV, &shared->loadedV, 0, p.keysPad, int(t.h), int(t.n));
+                }
+                __syncwarp();
             };
-            const uint64_t descQ = smemDesc(smemAddr(tileQ), 16, 1024), descK = smemDesc(smemAddr(tileK), 16, 1024);
-            const uint64_t descP = smemDesc(smemAddr(tileP), 16, 1024), descV = smemDesc(smemAddr(tileV), BK * 128, 1024);
+            const auto wait = [&](uint64_t *bar, uint32_t parity, int code) { return __all_sync(0xffffffffu, mbarWait(bar, parity, code)) != 0; };
+            const DescWords descQ = descWords(smemDesc(smemAddr(tileQ), 16, 1024)), descK = descWords(smemDesc(smemAddr(tileK), 16, 1024));
+            const DescWords descP = descWords(smemDesc(smemAddr(tileP), 16, 1024)), descV = descWords(smemDesc(smemAddr(tileV), BK * 128, 1024));
             const auto scoreProduct = [&] {
                 for (int n0 = 0; n0 < p.keysPad; n0 += 256) {
                     const int n = min(256, p.keysPad - n0);
                     for (int ks = 0; ks * UMMA_K < p.d; ++ks) {
-                        umma(tmemBase + uint32_t(n0), descQ + uint64_t(2 * ks),
-                             descK + uint64_t(n0 * (kRowBytes >> 4) + 2 * ks), instrDesc(n, false), ks > 0 ? 1u : 0u);
+                        umma(tmemBase + uint32_t(n0), {descQ.low + uint32_t(2 * ks), descQ.high},
+                             {descK.low + uint32_t(n0 * (kRowBytes >> 4) + 2 * ks), descK.high}, instrDesc(n, false), ks > 0 ? 1u : 0u);
                     }
                 }
                 ummaCommit(&shared->scoresDone);
@@ -221,8 +228,8 @@ attentionI8Kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constan
                 // A format 0: unsigned 8-bit
                 const uint32_t idesc = instrDesc(p.d, true) & (UNSIGNED_P ? ~(7u << 7) : ~0u);
                 for (int ks = 0; ks * UMMA_K < p.keysPad; ++ks) {
-                    umma(tmemBase + uint32_t(p.contextColumn), descP + uint64_t((ks >> 2) * ((BM * BK) >> 4) + 2 * (ks & 3)),
-                         descV + uint64_t(ks * ((UMMA_K * kRowBytes) >> 4)), idesc, ks > 0 ? 1u : 0u);
+                    umma(tmemBase + uint32_t(p.contextColumn), {descP.low + uint32_t((ks >> 2) * ((BM * BK) >> 4) + 2 * (ks & 3)), descP.high},
+                         {descV.low + uint32_t(ks * ((UMMA_K * kRowBytes) >> 4)), descV.high}, idesc, ks > 0 ? 1u : 0u);
                 }
                 ummaCommit(&shared->contextDone);
             };
@@ -231,7 +238,7 @@ attentionI8Kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constan
             if (t < p.tiles) {
                 loadQK(tileOf(t));
                 loadV(tileOf(t));
-                ok = mbarWait(&shared->loadedQK, 0, 71);
+                ok = wait(&shared->loadedQK, 0, 71);
                 if (ok) {
                     scoreProduct();
                 }
@@ -240,12 +247,12 @@ attentionI8Kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constan
                 const uint32_t parity = i & 1u;
                 const uint32_t next = t + gridDim.x;
                 const bool more = next < p.tiles;
-                ok = mbarWait(&shared->scoresDone, parity, 72); // Q and K have been read
+                ok = wait(&shared->scoresDone, parity, 72); // Q and K have been read
                 if (ok && more) {
                     loadQK(tileOf(next));
                 }
-                ok = ok && mbarWait(&shared->probsReady, parity, 73) && mbarWait(&shared->loadedV, parity, 74) &&
-                     (!more || mbarWait(&shared->loadedQK, parity ^ 1u, 71));
+                ok = ok && wait(&shared->probsReady, parity, 73) && wait(&shared->loadedV, parity, 74) &&
+                     (!more || wait(&shared->loadedQK, parity ^ 1u, 71));
                 if (!ok) {
                     break;
                 }
@@ -254,19 +261,19 @@ attentionI8Kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constan
                     scoreProduct();
                 }
                 if (sideBySide && i > 0) { // the previous tile's context has been stored
-                    ok = mbarWait(&shared->contextRead, parity ^ 1u, 76);
+                    ok = wait(&shared->contextRead, parity ^ 1u, 76);
                     if (!ok) {
                         break;
                     }
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 }
                 contextProduct();
-                ok = mbarWait(&shared->contextDone, parity, 75); // V and the probabilities have been read
+                ok = wait(&shared->contextDone, parity, 75); // V and the probabilities have been read
                 if (ok && more) {
                     loadV(tileOf(next));
                 }
                 if (!sideBySide && more) {
-                    ok = ok && mbarWait(&shared->contextRead, parity, 76);
+                    ok = ok && wait(&shared->contextRead, parity, 76);
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                     if (ok) {
                         scoreProduct();

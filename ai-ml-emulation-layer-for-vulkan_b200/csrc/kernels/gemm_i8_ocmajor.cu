@@ -218,7 +218,6 @@ gemmI8OcMajor(const __grid_constant__ CUtensorMap tmapX, const __grid_constant__
         // ---------------- MMA issuer (the whole warp: see ummaBlockPeek) ----------------
         constexpr uint32_t idesc = instrDesc(BNP, false);
         static_assert(BK / UMMA_K == 4, "ummaBlockPeek issues the four MMAs of a K block");
-        const uint32_t leader = lane == 0 ? 1u : 0u;
         const DescWords descW0 = descWords(smemDesc(smemAddr(tilesW), 16, 1024)), descX0 = descWords(smemDesc(smemAddr(tilesX), 16, 1024));
         uint32_t tileCount = 0;
         uint32_t ready = 0; // 1: the stage of the coming K block is known to be full (see ummaBlockPeek)
@@ -241,7 +240,7 @@ gemmI8OcMajor(const __grid_constant__ CUtensorMap tmapX, const __grid_constant__
                 // the ring runs on across tiles: the next K block's stage follows this one whatever tile it is in
                 const int sNext = s + 1 == NSTAGE ? 0 : s + 1;
                 const uint32_t phaseNext = sNext == 0 ? phase ^ 1u : phase;
-                ready = ummaBlockPeek(leader, tmemD, {descW0.low + uint32_t(s) * uint32_t(kTileW >> 4), descW0.high}, 2,
+                ready = ummaBlockPeek(tmemD, {descW0.low + uint32_t(s) * uint32_t(kTileW >> 4), descW0.high}, 2,
                                       {descX0.low + uint32_t(s) * uint32_t(kTileX >> 4), descX0.high}, 2, idesc, kb != 0 ? 1u : 0u,
                                       ummaCountFor(kLeft), &bars->empty[s], &bars->full[sNext], phaseNext);
                 // bytes of K in the next block: the rest of the tap's channels (im2col) or of the whole K axis
@@ -252,10 +251,7 @@ gemmI8OcMajor(const __grid_constant__ CUtensorMap tmapX, const __grid_constant__
                 s = sNext;
                 phase = phaseNext;
             }
-            if (lane == 0) {
-                ummaCommit(&bars->accFull[buf]);
-            }
-            __syncwarp();
+            ummaCommit(&bars->accFull[buf]);
         }
     } else if (warp >= kOcGatherWarp0) {
         if (X_TMA) {

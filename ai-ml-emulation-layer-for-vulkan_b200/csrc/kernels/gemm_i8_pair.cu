@@ -101,37 +101,41 @@ __device__ __forceinline__ void ummaPair(uint32_t tmemD, uint64_t descA, uint64_
 }
 
 // Makes the barrier at `barAddr` (shared::cluster address, this CTA's or the peer's) complete one arrival when
-// all MMAs issued so far by this thread have finished.
+// all MMAs issued so far by this warp have finished.
 __device__ __forceinline__ void ummaCommitPair(uint32_t barAddr) {
-    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(barAddr) : "memory");
+    asm volatile("{\n\t.reg .pred l;\n\telect.sync _|l, 0xffffffff;\n\t"
+                 "@l tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(barAddr) : "memory");
 }
 
 // One K block of the pair: the four MMAs, the two commits that hand the stage back to both CTAs and, issued ahead
 // of them, a non-blocking test of the barrier the next K block waits for (see ummaBlockPeek).
-__device__ __forceinline__ uint32_t ummaBlockPeekPair(uint32_t tmemD, uint64_t descA, uint64_t stepA, uint64_t descB,
-                                                      uint64_t stepB, uint32_t idesc, uint32_t accumulateFirst, int count,
-                                                      uint32_t commitOwn, uint32_t commitPeer, uint64_t *peekBar,
-                                                      uint32_t peekParity) {
+__device__ __forceinline__ uint32_t ummaBlockPeekPair(uint32_t tmemD, DescWords a, uint32_t stepA, DescWords b, uint32_t stepB,
+                                                      uint32_t idesc, uint32_t accumulateFirst, int count, uint32_t commitOwn,
+                                                      uint32_t commitPeer, uint64_t *peekBar, uint32_t peekParity) {
     uint32_t ready;
-    asm volatile("{\n\t.reg .pred q, a0, a1, g1, g2, g3;\n\t"
+    asm volatile("{\n\t.reg .pred q, l, a0, a1, g1, g2, g3;\n\t"
+                 ".reg .b32 la, lb;\n\t.reg .b64 da, db;\n\t"
                  "mbarrier.test_wait.parity.shared::cta.b64 q, [%1], %2;\n\t"
+                 "elect.sync _|l, 0xffffffff;\n\t"
                  "setp.ne.b32 a0, %9, 0;\n\t"
-                 "setp.ne.b32 a1, %10, 0;\n\t"
-                 "setp.gt.s32 g1, %18, 1;\n\t"
-                 "setp.gt.s32 g2, %18, 2;\n\t"
-                 "setp.gt.s32 g3, %18, 3;\n\t"
-                 "tcgen05.mma.cta_group::2.kind::i8 [%3], %4, %5, %8, {%11, %11, %11, %11, %11, %11, %11, %11}, a0;\n\t"
-                 "@g1 tcgen05.mma.cta_group::2.kind::i8 [%3], %6, %7, %8, {%11, %11, %11, %11, %11, %11, %11, %11}, a1;\n\t"
-                 "@g2 tcgen05.mma.cta_group::2.kind::i8 [%3], %12, %13, %8, {%11, %11, %11, %11, %11, %11, %11, %11}, a1;\n\t"
-                 "@g3 tcgen05.mma.cta_group::2.kind::i8 [%3], %14, %15, %8, {%11, %11, %11, %11, %11, %11, %11, %11}, a1;\n\t"
-                 "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%16];\n\t"
-                 "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%17];\n\t"
+                 "setp.eq.b32 a1, %10, 0;\n\t"
+                 "setp.gt.and.s32 g1, %11, 1, l;\n\t"
+                 "setp.gt.and.s32 g2, %11, 2, l;\n\t"
+                 "setp.gt.and.s32 g3, %11, 3, l;\n\t"
+                 "mov.b64 da, {%4, %5};\n\tmov.b64 db, {%6, %7};\n\t"
+                 "@l tcgen05.mma.cta_group::2.kind::i8 [%3], da, db, %8, {%10, %10, %10, %10, %10, %10, %10, %10}, a0;\n\t"
+                 "add.u32 la, %4, %14;\n\tadd.u32 lb, %6, %15;\n\tmov.b64 da, {la, %5};\n\tmov.b64 db, {lb, %7};\n\t"
+                 "@g1 tcgen05.mma.cta_group::2.kind::i8 [%3], da, db, %8, {%10, %10, %10, %10, %10, %10, %10, %10}, a1;\n\t"
+                 "add.u32 la, la, %14;\n\tadd.u32 lb, lb, %15;\n\tmov.b64 da, {la, %5};\n\tmov.b64 db, {lb, %7};\n\t"
+                 "@g2 tcgen05.mma.cta_group::2.kind::i8 [%3], da, db, %8, {%10, %10, %10, %10, %10, %10, %10, %10}, a1;\n\t"
+                 "add.u32 la, la, %14;\n\tadd.u32 lb, lb, %15;\n\tmov.b64 da, {la, %5};\n\tmov.b64 db, {lb, %7};\n\t"
+                 "@g3 tcgen05.mma.cta_group::2.kind::i8 [%3], da, db, %8, {%10, %10, %10, %10, %10, %10, %10, %10}, a1;\n\t"
+                 "@l tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%12];\n\t"
+                 "@l tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%13];\n\t"
                  "selp.u32 %0, 1, 0, q;\n\t}"
                  : "=r"(ready)
-                 : "r"(smemAddr(peekBar)), "r"(peekParity), "r"(tmemD), "l"(descA), "l"(descB), "l"(descA + stepA),
-                   "l"(descB + stepB), "r"(idesc), "r"(accumulateFirst), "r"(1u), "r"(0u), "l"(descA + 2 * stepA),
-                   "l"(descB + 2 * stepB), "l"(descA + 3 * stepA), "l"(descB + 3 * stepB), "r"(commitOwn), "r"(commitPeer),
-                   "r"(count)
+                 : "r"(smemAddr(peekBar)), "r"(peekParity), "r"(tmemD), "r"(a.low), "r"(a.high), "r"(b.low), "r"(b.high), "r"(idesc),
+                   "r"(accumulateFirst), "r"(0u), "r"(count), "r"(commitOwn), "r"(commitPeer), "r"(stepA), "r"(stepB)
                  : "memory");
     return ready;
 }
@@ -353,61 +357,47 @@ gemmI8Pair(const __grid_constant__ CUtensorMap tmapX, const __grid_constant__ CU
         }
     } else if (warp == kMmaWarpP) {
         // ---------------- MMA issuer (leader only) ----------------
-        if (lane == 0 && rank == 0) {
+        if (rank == 0) { // (the whole warp: see ummaBlockPeek)
             constexpr uint32_t idesc = instrDescPair(BNP, W_MN);
-            // Everything the loop needs per K block is kept in registers and stepped, not recomputed: the stage's two
-            // operand descriptors (the address field counts 16-byte units and never leaves its 14 bits), its barrier
-            // addresses in both CTAs, its phase.  This one thread's instruction stream paces the pair: with the
-            // barrier tested after the MMAs and commits about 630 cycles per K block were measured, with or without
+            // With the barrier tested after the MMAs and commits about 630 cycles per K block were measured, with or without
             // the copies, against 512 that the MMAs take; hence the test ahead of them (ummaBlockPeekPair).
-            const uint64_t descW0 =
-                W_MN ? smemDesc(smemAddr(tilesW), BK * 128, 1024) : smemDesc(smemAddr(tilesW), 16, 1024);
-            const uint64_t descX0 = smemDesc(smemAddr(tilesX), 16, 1024);
-            constexpr uint64_t kStepW = uint64_t(W_MN ? UMMA_K * 128 : UMMA_K) >> 4, kStepX = uint64_t(UMMA_K) >> 4;
+            const DescWords descW0 =
+                descWords(W_MN ? smemDesc(smemAddr(tilesW), BK * 128, 1024) : smemDesc(smemAddr(tilesW), 16, 1024));
+            const DescWords descX0 = descWords(smemDesc(smemAddr(tilesX), 16, 1024));
+            constexpr uint32_t kStepW = uint32_t(W_MN ? UMMA_K * 128 : UMMA_K) >> 4, kStepX = uint32_t(UMMA_K) >> 4;
             const uint32_t emptyOwn0 = smemAddr(&bars->empty[0]), emptyPeer0 = mapToCta(emptyOwn0, 1u);
             const uint32_t accFullOwn = smemAddr(&bars->accFull[0]), accFullPeer = mapToCta(accFullOwn, 1u);
-            uint64_t dw = descW0, dx = descX0;
             uint32_t s = 0, phase = 0, tileCount = 0;
             uint32_t ready = 0; // 1: the stage of the coming K block is known to be full (see ummaBlockPeek)
-            bool ok = true;
-            for (int64_t t = pairIdx; t < numTiles && ok; t += numPairs, ++tileCount) {
+            bool failed = false; // a wait ran out: no more waits, the later MMAs read old bytes, the recorded error tells
+            for (int64_t t = pairIdx; t < numTiles; t += numPairs, ++tileCount) {
                 const uint32_t buf = tileCount & 1u;
-                ok = mbarWait(&bars->accEmpty[buf], ((tileCount >> 1) & 1u) ^ 1u, 25);
-                if (!ok) {
-                    break;
-                }
+                failed = failed || !mbarWait(&bars->accEmpty[buf], ((tileCount >> 1) & 1u) ^ 1u, 25);
+                __syncwarp();
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const uint32_t tmemD = tmemBase + buf * uint32_t(BNP);
                 int kLeft = X_MODE == kXIm2col ? p.IC : p.K; // bytes of K in the coming block's tap or K axis
                 for (int kb = 0; kb < numKb; ++kb) {
                     if (ready == 0) {
-                        ok = mbarWait(&bars->full[s], phase, 22);
-                        if (!ok) {
-                            break;
-                        }
+                        failed = failed || !mbarWait(&bars->full[s], phase, 22);
                     }
+                    __syncwarp();
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                     const uint32_t sNext = s + 1 == uint32_t(NSTAGE) ? 0u : s + 1;
                     const uint32_t phaseNext = sNext == 0 ? phase ^ 1u : phase;
                     // the stage is free in both CTAs once these MMAs have read it
-                    ready = ummaBlockPeekPair(tmemD, dw, kStepW, dx, kStepX, idesc, kb != 0 ? 1u : 0u, ummaCountFor(kLeft),
-                                              emptyOwn0 + s * 8u, emptyPeer0 + s * 8u, &bars->full[sNext], phaseNext);
+                    ready = ummaBlockPeekPair(tmemD, {descW0.low + s * uint32_t(kTileW >> 4), descW0.high}, kStepW,
+                                              {descX0.low + s * uint32_t(kTileX >> 4), descX0.high}, kStepX, idesc, kb != 0 ? 1u : 0u,
+                                              ummaCountFor(kLeft), emptyOwn0 + s * 8u, emptyPeer0 + s * 8u, &bars->full[sNext], phaseNext);
                     kLeft -= BK;
                     if (kLeft <= 0) {
                         kLeft = X_MODE == kXIm2col ? p.IC : 0;
                     }
-                    if (sNext == 0) {
-                        dw = descW0, dx = descX0;
-                    } else {
-                        dw += uint64_t(kTileW >> 4), dx += uint64_t(kTileX >> 4);
-                    }
                     s = sNext;
                     phase = phaseNext;
                 }
-                if (ok) {
-                    ummaCommitPair(accFullOwn + buf * 8u);
-                    ummaCommitPair(accFullPeer + buf * 8u);
-                }
+                ummaCommitPair(accFullOwn + buf * 8u);
+                ummaCommitPair(accFullPeer + buf * 8u);
             }
         }
     } else if (warp == kStoreWarpP) {

@@ -124,75 +124,95 @@ gemmI8Small(const __grid_constant__ CUtensorMap mapX, const __grid_constant__ CU
 
     if (warp == kSmallTmaWarp) {
         if (lane == 0) {
-            const auto loadW = [&](int i) {
-                const int kb = kb0 + i, s = i % kStages;
-                mbarArriveExpectTx(&bars->full[s], uint32_t(kTileW + kTileX));
+            // (running positions on the K axis: the divisions that they take are done once)
+            const int tap0 = IM2COL ? kb0 / p.kbPerTap : 0, cb0 = IM2COL ? (kb0 - tap0 * p.kbPerTap) * BK : kb0 * BK;
+            int tapW = tap0, cbW = cb0, stageW = 0;
+            const auto loadW = [&] {
+                uint64_t *full = &bars->full[stageW];
+                mbarArriveExpectTx(full, uint32_t(kTileW + kTileX));
                 if (IM2COL) {
-                    const int tap = kb / p.kbPerTap, cb = (kb - tap * p.kbPerTap) * BK;
-                    tmaLoad3d(&mapW, tilesW + s * kTileW, &bars->full[s], cb, tap, c0);
+                    tmaLoad3d(&mapW, tilesW + stageW * kTileW, full, cbW, tapW, c0);
                 } else {
-                    tmaLoad3d(&mapW, tilesW + s * kTileW, &bars->full[s], kb * BK, c0, 0);
+                    tmaLoad3d(&mapW, tilesW + stageW * kTileW, full, cbW, c0, 0);
                 }
+                cbW += BK;
+                if (IM2COL && cbW >= p.IC) {
+                    cbW = 0;
+                    ++tapW;
+                }
+                stageW = stageW + 1 == kStages ? 0 : stageW + 1;
             };
             int w0 = 0, h0 = 0, n0 = 0; // first tap of the tile's first window
+            int cbX = cb0, stageX = 0, ky = IM2COL ? tap0 / p.KW : 0, kx = tap0 - ky * p.KW;
             if (IM2COL) {
                 n0 = int(fastDiv(uint32_t(m0), p.divPlane));
                 const int rem = m0 - n0 * p.OH * p.OW, oy = int(fastDiv(uint32_t(rem), p.divOW));
                 h0 = oy * p.strideY - p.padTop, w0 = (rem - oy * p.OW) * p.strideX - p.padLeft;
             }
-            const auto loadX = [&](int i) {
-                const int kb = kb0 + i, s = i % kStages;
+            const auto loadX = [&] {
+                uint64_t *full = &bars->full[stageX];
                 if (IM2COL) {
-                    const int tap = kb / p.kbPerTap, cb = (kb - tap * p.kbPerTap) * BK, ky = tap / p.KW, kx = tap - ky * p.KW;
-                    tmaLoadIm2col4d(&mapX, tilesX + s * kTileX, &bars->full[s], cb, w0, h0, n0, uint16_t(kx * p.dilX),
+                    tmaLoadIm2col4d(&mapX, tilesX + stageX * kTileX, full, cbX, w0, h0, n0, uint16_t(kx * p.dilX),
                                     uint16_t(ky * p.dilY));
                 } else {
-                    tmaLoad3d(&mapX, tilesX + s * kTileX, &bars->full[s], kb * BK, m0, 0);
+                    tmaLoad3d(&mapX, tilesX + stageX * kTileX, full, cbX, m0, 0);
                 }
+                cbX += BK;
+                if (IM2COL && cbX >= p.IC) {
+                    cbX = 0;
+                    if (++kx == p.KW) {
+                        kx = 0;
+                        ++ky;
+                    }
+                }
+                stageX = stageX + 1 == kStages ? 0 : stageX + 1;
             };
             const int ahead = min(kbCount, kStages);
             if (p.lateOperand != 0) {
                 asm volatile("griddepcontrol.wait;" ::: "memory");
             }
             for (int i = 0; i < ahead; ++i) {
-                loadW(i);
+                loadW();
             }
             asm volatile("griddepcontrol.wait;" ::: "memory"); // the pixels are the launch before's results
             for (int i = 0; i < ahead; ++i) {
-                loadX(i);
+                loadX();
             }
             for (int i = ahead; i < kbCount; ++i) {
                 if (!mbarWait(&bars->empty[i % kStages], uint32_t(i / kStages - 1) & 1u, 81)) {
                     break;
                 }
-                loadW(i);
-                loadX(i);
+                loadW();
+                loadX();
             }
         }
         __syncwarp();
     } else if (warp == kSmallMmaWarp) {
-        if (lane == 0) {
-            const uint64_t descW = smemDesc(smemAddr(tilesW), 16, 1024), descX = smemDesc(smemAddr(tilesX), 16, 1024);
-            bool ok = true;
-            for (int i = 0; i < kbCount; ++i) {
-                const int kb = kb0 + i, s = i % kStages;
-                ok = mbarWait(&bars->full[s], uint32_t(i / kStages) & 1u, 82);
-                if (!ok) {
-                    break;
-                }
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const int valid = IM2COL ? p.IC - (kb % p.kbPerTap) * BK : p.K - kb * BK;
-                const int count = ummaCountFor(valid);
-                for (int u = 0; u < count; ++u) {
-                    umma(tmemBase, descW + uint64_t(s * (kTileW >> 4) + 2 * u), descX + uint64_t(s * (kTileX >> 4) + 2 * u),
-                         instrDesc(BNP, false), i > 0 || u > 0 ? 1u : 0u);
-                }
-                ummaCommit(&bars->empty[s]);
+        // The whole warp (see ummaBlockPeek).  From one divergent lane a K block took 0.3-0.4 us between its operands' arrival and
+        // the next one's MMAs: 1.1 us of a layer's 4 with three K blocks, 2.3 with six.  (All K blocks on one barrier, one wait and
+        // one train of MMAs: slower, one image 228 us against 219 -- the first block's MMAs run while the others arrive.)  A wait
+        // that runs out only ends the waiting, the recorded error tells.
+        const DescWords descW = descWords(smemDesc(smemAddr(tilesW), 16, 1024)), descX = descWords(smemDesc(smemAddr(tilesX), 16, 1024));
+        int left = IM2COL ? p.IC - kb0 % p.kbPerTap * BK : p.K - kb0 * BK; // bytes of K from here to the end of the tap or row
+        bool failed = false;
+        uint32_t ready = 0, phase = 0;
+        int s = 0;
+        for (int i = 0; i < kbCount; ++i) {
+            if (ready == 0) {
+                failed = failed || !mbarWait(&bars->full[s], phase, 82);
             }
-            if (ok) {
-                ummaCommit(&bars->accFull);
-            }
+            __syncwarp();
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const int sNext = s + 1 == kStages ? 0 : s + 1;
+            const uint32_t phaseNext = sNext == 0 ? phase ^ 1u : phase;
+            ready = ummaBlockPeek(tmemBase, {descW.low + uint32_t(s * (kTileW >> 4)), descW.high}, 2,
+                                  {descX.low + uint32_t(s * (kTileX >> 4)), descX.high}, 2, instrDesc(BNP, false), i > 0 ? 1u : 0u,
+                                  ummaCountFor(left), &bars->empty[s], &bars->full[sNext], phaseNext);
+            left = IM2COL && left <= BK ? p.IC : left - BK;
+            s = sNext;
+            phase = phaseNext;
         }
+        ummaCommit(&bars->accFull);
         __syncwarp();
     } else {
         const int ci = p.epi.main.perChannel && ocValid ? oc : 0;

@@ -626,7 +626,6 @@ gemmI8Tcgen05(const __grid_constant__ CUtensorMap tmapA, const __grid_constant__
         // ---------------- MMA issuer (the whole warp: see ummaBlockPeek) ----------------
         constexpr uint32_t idesc = instrDesc(BN, B_MN);
         static_assert(BK / UMMA_K == 4, "ummaBlockPeek issues the four MMAs of a K block");
-        const uint32_t leader = lane == 0 ? 1u : 0u;
         // K-major: step 32 bytes inside the 128-byte swizzle row; MN-major: step 32 K-rows of 128 bytes
         const DescWords descA0 = descWords(smemDesc(smemAddr(tilesA), 16, 1024));
         const DescWords descB0 = descWords(B_MN ? smemDesc(smemAddr(tilesB), BK * 128, 1024) : smemDesc(smemAddr(tilesB), 16, 1024));
@@ -653,7 +652,7 @@ gemmI8Tcgen05(const __grid_constant__ CUtensorMap tmapA, const __grid_constant__
                 // the ring runs on across tiles: the next K block's stage follows this one whatever tile it is in
                 const int sNext = s + 1 == NSTAGE ? 0 : s + 1;
                 const uint32_t phaseNext = sNext == 0 ? phase ^ 1u : phase;
-                ready = ummaBlockPeek(leader, tmemD, {descA0.low + uint32_t(s) * uint32_t(kTileA >> 4), descA0.high}, 2,
+                ready = ummaBlockPeek(tmemD, {descA0.low + uint32_t(s) * uint32_t(kTileA >> 4), descA0.high}, 2,
                                       {descB0.low + uint32_t(s) * uint32_t(kTileB >> 4), descB0.high}, kStepB, idesc,
                                       kb != 0 ? 1u : 0u, ummaCountFor(kLeft), &bars->empty[s], &bars->full[sNext], phaseNext);
                 kLeft -= BK;
@@ -663,10 +662,7 @@ gemmI8Tcgen05(const __grid_constant__ CUtensorMap tmapA, const __grid_constant__
                 s = sNext;
                 phase = phaseNext;
             }
-            if (lane == 0) {
-                ummaCommit(&bars->accFull[buf]);
-            }
-            __syncwarp();
+            ummaCommit(&bars->accFull[buf]);
         }
     } else if (warp >= kGatherWarp0) {
         // ---------------- A gather (implicit GEMM): one tile row per thread ----------------

@@ -79,20 +79,6 @@ __device__ __forceinline__ uint64_t smemDescPlain(uint32_t addr, uint32_t leadin
     return smemDesc(addr, leadingBytes, groupBytes) & ~(uint64_t(7) << 61);
 }
 
-// One MMA by the leading lane of a warp that executes this as a whole (see the MMA warp).  The descriptors come as low words
-// (address; no sum of these carries) and constant high words.
-__device__ __forceinline__ void ummaLed(uint32_t leader, uint32_t tmemD, uint32_t lowA, uint32_t highA, uint32_t lowB, uint32_t highB,
-                                        uint32_t idesc, uint32_t accumulate) {
-    asm volatile("{\n\t.reg .pred p, l;\n\t.reg .b64 a, b;\n\t"
-                 "setp.ne.b32 l, %8, 0;\n\t"
-                 "setp.ne.b32 p, %6, 0;\n\t"
-                 "mov.b64 a, {%1, %2};\n\t"
-                 "mov.b64 b, {%3, %4};\n\t"
-                 "@l tcgen05.mma.cta_group::1.kind::i8 [%0], a, b, %5, {%7, %7, %7, %7}, p;\n\t}"
-                 ::"r"(tmemD), "r"(lowA), "r"(highA), "r"(lowB), "r"(highB), "r"(idesc), "r"(accumulate), "r"(0u), "r"(leader)
-                 : "memory");
-}
-
 // ODD: output rows start at any address.  The warps that share 32 rows of the accumulator put them together in shared memory
 // and store them as aligned words (storeRowBytes).  64 -> 63 channels, 8 x 56 x 56: 10.6 us on the pixel-major kernel, here
 // 8.8; 30 x 30, 64 -> 65: 9.7 and 6.1.
@@ -182,7 +168,7 @@ gemmI8Window(const __grid_constant__ CUtensorMap mapX, const __grid_constant__ C
         // the later MMAs read old bytes, the recorded error tells.
         dependencySync();
         constexpr uint32_t idesc = instrDesc(BN, false);
-        const uint32_t groupBytes = uint32_t((g.blocks ? g.boxW : 8) * g.pixelBytes), leader = lane == 0 ? 1u : 0u;
+        const uint32_t groupBytes = uint32_t((g.blocks ? g.boxW : 8) * g.pixelBytes);
         const uint64_t descX = rowDesc(smemAddr(stages), uint32_t(g.pixelBytes), groupBytes);
         const uint64_t descW = rowDesc(smemAddr(weights), uint32_t(g.pixelBytes), uint32_t(8 * g.pixelBytes));
         const uint32_t lowX = uint32_t(descX), highX = uint32_t(descX >> 32), lowW = uint32_t(descW), highW = uint32_t(descW >> 32);
@@ -214,17 +200,14 @@ gemmI8Window(const __grid_constant__ CUtensorMap mapX, const __grid_constant__ C
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const uint32_t tmemD = tmemBase + buf * uint32_t(BN);
                 const auto tap = [&](uint32_t x, uint32_t w, bool first) {
-#pragma unroll
-                    for (int u = 0; u < kSlices; ++u) {
-                        ummaLed(leader, tmemD, x + uint32_t(2 * u), highX, w + uint32_t(2 * u), highW, idesc, first && u == 0 ? 0u : 1u);
-                    }
+                    ummaBlock(tmemD, {x, highX}, 2, {w, highW}, 2, idesc, first ? 0u : 1u, kSlices);
                 };
                 if (UNITS) {
                     const uint32_t stage = smemAddr(stages + s * g.stageBytes) >> 4, w = (smemAddr(weights) >> 4) + (uint32_t(BN) << 16);
 #pragma unroll
                     for (int m = 0; m < kMaxUnitPairs; ++m) {
                         if (m < g.unitPairs) {
-                            ummaLed(leader, tmemD, stage + pairX[m], pairHigh, w + uint32_t(2 * m * BN), weightHigh, idesc, m == 0 ? 0u : 1u);
+                            umma(tmemD, {stage + pairX[m], pairHigh}, {w + uint32_t(2 * m * BN), weightHigh}, idesc, m == 0 ? 0u : 1u);
                         }
                     }
                 } else if (kThree) {
@@ -241,11 +224,8 @@ gemmI8Window(const __grid_constant__ CUtensorMap mapX, const __grid_constant__ C
                         }
                     }
                 }
-                if (lane == 0) {
-                    ummaCommit(&bars->empty[s]);
-                    ummaCommit(&bars->accFull[buf]);
-                }
-                __syncwarp();
+                ummaCommit(&bars->empty[s]);
+                ummaCommit(&bars->accFull[buf]);
                 stageX += stageStep;
                 if (++s == stageCount) {
                     s = 0;

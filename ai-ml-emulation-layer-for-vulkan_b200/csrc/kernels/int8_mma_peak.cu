@@ -38,7 +38,7 @@ __global__ void __launch_bounds__(128, 1) int8MmaPeakKernel(int batches) {
     uint8_t *tileA = smem;
     uint8_t *tileB = smem + kPeakTileA;
     PeakBarriers *bars = reinterpret_cast<PeakBarriers *>(tileB + kPeakTileB);
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = threadIdx.x >> 5;
 
     // operand bytes: any values do (the rate does not depend on them); not all zero, so that the multipliers toggle
     for (int i = threadIdx.x; i < (kPeakTileA + kPeakTileB) / 4; i += blockDim.x) {
@@ -62,7 +62,7 @@ __global__ void __launch_bounds__(128, 1) int8MmaPeakKernel(int batches) {
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmemBase = bars->tmemBase;
 
-    if (warp == 0 && lane == 0) {
+    if (warp == 0) { // (as a whole, see umma)
         constexpr uint32_t idesc = instrDesc(kPeakN, false);
         const uint32_t aAddr = smemAddr(tileA), bAddr = smemAddr(tileB);
         bool ok = true;
@@ -74,13 +74,14 @@ __global__ void __launch_bounds__(128, 1) int8MmaPeakKernel(int batches) {
                 if (!ok) {
                     break;
                 }
+                __syncwarp();
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             }
             const uint32_t tmemD = tmemBase + buf * uint32_t(kPeakN);
 #pragma unroll 4
             for (int i = 0; i < kPeakBatch; ++i) {
                 const int k = i & 3;
-                umma(tmemD, smemDesc(aAddr + k * UMMA_K, 16, 1024), smemDesc(bAddr + k * UMMA_K, 16, 1024), idesc,
+                umma(tmemD, descWords(smemDesc(aAddr + k * UMMA_K, 16, 1024)), descWords(smemDesc(bAddr + k * UMMA_K, 16, 1024)), idesc,
                      i != 0 ? 1u : 0u);
             }
             ummaCommit(&bars->done[buf]);

@@ -187,22 +187,33 @@ __host__ __device__ constexpr uint32_t instrDesc(int n, bool bMnMajor) {
            (uint32_t(BM >> 4) << 24);
 }
 
-__device__ __forceinline__ void umma(uint32_t tmemD, uint64_t descA, uint64_t descB, uint32_t idesc, uint32_t accumulate) {
-    asm volatile("{\n\t.reg .pred p;\n\t"
-                 "setp.ne.b32 p, %4, 0;\n\t"
-                 "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, {%5, %5, %5, %5}, p;\n\t}"
-                 ::"r"(tmemD), "l"(descA), "l"(descB), "r"(idesc), "r"(accumulate), "r"(0u)
-                 : "memory");
-}
-__device__ __forceinline__ void ummaCommit(uint64_t *bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smemAddr(bar))
-                 : "memory");
-}
-// The warp that issues MMAs runs its loops as a whole, one lane (`leader`) issues: with nothing divergent around them the
+// The warp that issues MMAs runs its loops as a whole and one elected lane issues: with nothing divergent around them the
 // operands of tcgen05.mma stay in uniform registers.  From inside `if (lane == 0)` every MMA took the thread a dozen moves
 // and waits behind the epilogue warps that share its scheduler (3x3 windows over 64 channels: some 200 cycles per MMA that
-// the pipe does in 50).  Descriptors are given as low words (address; no sum of these carries) and constant high words.
-//
+// the pipe does in 50).  The lane is elected by elect.sync in the statement itself: for a predicate like `lane == 0` the
+// compiler has to allow for several lanes, and an MMA took 62 cycles to issue whatever its width, elected 21 (one warp alone;
+// the pipe takes 40 at N = 32, 50 at 64, 67 at 128, 134 at 256).  A K block with its commit and test 418 -> 313 cycles at
+// N <= 64, 416 -> 384 (the pipe) at 192.  The calls below want the whole warp, converged.
+__device__ __forceinline__ void ummaCommit(uint64_t *bar) {
+    asm volatile("{\n\t.reg .pred l;\n\telect.sync _|l, 0xffffffff;\n\t"
+                 "@l tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(smemAddr(bar))
+                 : "memory");
+}
+// One MMA.  Descriptors are given as low words (address; no sum of these carries) and constant high words.
+struct DescWords {
+    uint32_t low, high;
+};
+__device__ __forceinline__ DescWords descWords(uint64_t d) { return {uint32_t(d), uint32_t(d >> 32)}; }
+__device__ __forceinline__ void umma(uint32_t tmemD, DescWords a, DescWords b, uint32_t idesc, uint32_t accumulate) {
+    asm volatile("{\n\t.reg .pred p, l;\n\t.reg .b64 a, b;\n\t"
+                 "elect.sync _|l, 0xffffffff;\n\t"
+                 "setp.ne.b32 p, %6, 0;\n\t"
+                 "mov.b64 a, {%1, %2};\n\t"
+                 "mov.b64 b, {%3, %4};\n\t"
+                 "@l tcgen05.mma.cta_group::1.kind::i8 [%0], a, b, %5, {%7, %7, %7, %7}, p;\n\t}"
+                 ::"r"(tmemD), "r"(a.low), "r"(a.high), "r"(b.low), "r"(b.high), "r"(idesc), "r"(accumulate), "r"(0u)
+                 : "memory");
+}
 // One 128-byte K block: up to four MMAs of 32 bytes of K each (`count` of them: the tail of a K block that only
 // holds zero fill is skipped; descriptors advance by stepA / stepB units of 16 bytes, 2 for a K-major SWIZZLE_128B
 // tile), the commit that hands the stage back, and -- issued AHEAD of them -- a non-blocking test of the barrier the
@@ -210,20 +221,16 @@ __device__ __forceinline__ void ummaCommit(uint64_t *bar) {
 // cycles to answer even when the phase has long completed (it queues behind them), and the warp that needs the
 // answer stalls for it.  Returns 1 when the next barrier's phase `peekParity` is complete; 0 means "not yet known":
 // wait for it in the ordinary way.
-struct DescWords {
-    uint32_t low, high;
-};
-__device__ __forceinline__ DescWords descWords(uint64_t d) { return {uint32_t(d), uint32_t(d >> 32)}; }
-__device__ __forceinline__ uint32_t ummaBlockPeek(uint32_t leader, uint32_t tmemD, DescWords a, uint32_t stepA, DescWords b,
+__device__ __forceinline__ uint32_t ummaBlockPeek(uint32_t tmemD, DescWords a, uint32_t stepA, DescWords b,
                                                   uint32_t stepB, uint32_t idesc, uint32_t accumulateFirst, int count,
                                                   uint64_t *commitBar, uint64_t *peekBar, uint32_t peekParity) {
     uint32_t ready;
     asm volatile("{\n\t.reg .pred q, l, a0, a1, g1, g2, g3;\n\t"
                  ".reg .b32 la, lb;\n\t.reg .b64 da, db;\n\t"
                  "mbarrier.test_wait.parity.shared::cta.b64 q, [%1], %2;\n\t"
-                 "setp.ne.b32 l, %15, 0;\n\t"
+                 "elect.sync _|l, 0xffffffff;\n\t"
                  "setp.ne.b32 a0, %9, 0;\n\t"
-                 "setp.ne.b32 a1, %15, %10;\n\t"
+                 "setp.eq.b32 a1, %10, 0;\n\t"
                  "setp.gt.and.s32 g1, %11, 1, l;\n\t"
                  "setp.gt.and.s32 g2, %11, 2, l;\n\t"
                  "setp.gt.and.s32 g3, %11, 3, l;\n\t"
@@ -239,9 +246,33 @@ __device__ __forceinline__ uint32_t ummaBlockPeek(uint32_t leader, uint32_t tmem
                  "selp.u32 %0, 1, 0, q;\n\t}"
                  : "=r"(ready)
                  : "r"(smemAddr(peekBar)), "r"(peekParity), "r"(tmemD), "r"(a.low), "r"(a.high), "r"(b.low), "r"(b.high), "r"(idesc),
-                   "r"(accumulateFirst), "r"(0u), "r"(count), "r"(smemAddr(commitBar)), "r"(stepA), "r"(stepB), "r"(leader)
+                   "r"(accumulateFirst), "r"(0u), "r"(count), "r"(smemAddr(commitBar)), "r"(stepA), "r"(stepB)
                  : "memory");
     return ready;
+}
+// Up to four MMAs (`count` of them) in one statement, neither test nor commit.  (As statements of their own, each with its
+// election, they issue slower: one image of the ResNet-50 shape 226 us, in one statement 219.)
+__device__ __forceinline__ void ummaBlock(uint32_t tmemD, DescWords a, uint32_t stepA, DescWords b, uint32_t stepB, uint32_t idesc,
+                                          uint32_t accumulateFirst, int count) {
+    asm volatile("{\n\t.reg .pred l, a0, a1, g1, g2, g3;\n\t"
+                 ".reg .b32 la, lb;\n\t.reg .b64 da, db;\n\t"
+                 "elect.sync _|l, 0xffffffff;\n\t"
+                 "setp.ne.b32 a0, %6, 0;\n\t"
+                 "setp.eq.b32 a1, %7, 0;\n\t"
+                 "setp.gt.and.s32 g1, %8, 1, l;\n\t"
+                 "setp.gt.and.s32 g2, %8, 2, l;\n\t"
+                 "setp.gt.and.s32 g3, %8, 3, l;\n\t"
+                 "mov.b64 da, {%1, %2};\n\tmov.b64 db, {%3, %4};\n\t"
+                 "@l tcgen05.mma.cta_group::1.kind::i8 [%0], da, db, %5, {%7, %7, %7, %7}, a0;\n\t"
+                 "add.u32 la, %1, %9;\n\tadd.u32 lb, %3, %10;\n\tmov.b64 da, {la, %2};\n\tmov.b64 db, {lb, %4};\n\t"
+                 "@g1 tcgen05.mma.cta_group::1.kind::i8 [%0], da, db, %5, {%7, %7, %7, %7}, a1;\n\t"
+                 "add.u32 la, la, %9;\n\tadd.u32 lb, lb, %10;\n\tmov.b64 da, {la, %2};\n\tmov.b64 db, {lb, %4};\n\t"
+                 "@g2 tcgen05.mma.cta_group::1.kind::i8 [%0], da, db, %5, {%7, %7, %7, %7}, a1;\n\t"
+                 "add.u32 la, la, %9;\n\tadd.u32 lb, lb, %10;\n\tmov.b64 da, {la, %2};\n\tmov.b64 db, {lb, %4};\n\t"
+                 "@g3 tcgen05.mma.cta_group::1.kind::i8 [%0], da, db, %5, {%7, %7, %7, %7}, a1;\n\t}"
+                 ::"r"(tmemD), "r"(a.low), "r"(a.high), "r"(b.low), "r"(b.high), "r"(idesc), "r"(accumulateFirst), "r"(0u), "r"(count),
+                   "r"(stepA), "r"(stepB)
+                 : "memory");
 }
 // How many of a K block's four MMAs have anything but zero fill to multiply: `valid` = bytes of K in the block.
 __device__ __forceinline__ int ummaCountFor(int valid) { return valid >= BK ? BK / UMMA_K : (valid + UMMA_K - 1) / UMMA_K; }
