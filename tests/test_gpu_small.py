@@ -71,6 +71,24 @@ def test_every_tile_and_split_with_residual_tail(mlel, tile, hw, ic, oc):
         assert lib.mlel_set_tuning(b"small_kernel", 1) == 0
 
 
+@pytest.mark.parametrize("tile,oc,relu", [(101, 70, True), (204, 130, False), (102, 16, False)])
+def test_residual_tail_without_a_table(mlel, tile, oc, relu):
+    """Behind a convolution over padded channels the tail has no table: its RESCALEs are evaluated."""
+    r = np.random.Generator(np.random.PCG64(tile + oc))
+    g = GraphBuilder()
+    x, short = g.input(np.int8, (1, 9, 11, 20)), g.input(np.int8, (1, 9, 11, oc))
+    y = conv(g, r, x, oc, 3, 1, 1, -3, relu)
+    a = g.rescale(y, [int(r.integers(1 << 30, 1 << 31))], [23], 4, 0, np.int32)
+    b = g.rescale(short, [int(r.integers(1 << 30, 1 << 31))], [23], -3, 0, np.int32)
+    g.output(g.rescale(g.add(a, b), [int(r.integers(1 << 30, 1 << 31))], [40], 0, -20, np.int8, double_round=True))
+    lib = mlel.lib()
+    try:
+        assert lib.mlel_set_tuning(b"small_kernel", tile) == 0
+        run(mlel, g, [r.integers(-128, 128, v.shape, dtype=np.int8) for v in (x, short)])
+    finally:
+        assert lib.mlel_set_tuning(b"small_kernel", 1) == 0
+
+
 @pytest.mark.parametrize("rows,k,n", [(1, 2048, 1000), (64, 768, 768), (33, 80, 10), (1, 16, 1), (130, 3072, 768)])
 def test_products_with_constant_weights(mlel, rows, k, n):
     r = np.random.Generator(np.random.PCG64(rows + n))
