@@ -78,6 +78,31 @@ def test_result_scale_with_any_zero_point(mlel, in_zp, mult, shift):
     check_fused(mlel, g, [full_range(r, np.int8, shape), full_range(r, np.int8, shape)], [NORM])
 
 
+@pytest.mark.parametrize("length", [4, 124, 768, 1028])
+@pytest.mark.parametrize("up,norm_shift,out_shift,in_zp,out_zp,double_round,table", [
+    ((24, 24), 12, 45, 0, 0, True, "any"),       # both products of the last step in one, table values of either sign and zero
+    ((26, 21), 12, 42, -5, 100, True, "small"),  # factors below the MUL's rounding term; shifts that add up to 24
+    ((24, 22), 9, 53, 3, -128, True, "any"),     # ... to 32
+    ((24, 24), 9, 54, 0, 0, True, "any"),        # ... to 33: not in this form
+    ((25, 24), 12, 31, 0, 7, False, "any"),      # no double rounding, a small shift: not in this form
+    ((24, 24), 12, 46, 0, 0, False, "small"),
+])
+def test_whole_input_scales_and_a_power_of_two_on_the_result(mlel, length, up, norm_shift, out_shift, in_zp, out_zp, double_round, table):
+    r = rng(length + out_shift)
+    shape = (1, 11, length)
+    g = GraphBuilder()
+    a, b = g.input(np.int8, shape), g.input(np.int8, shape)
+    t = g.add(g.rescale(a, [3 << 28], [up[0]], in_zp, 0, np.int32), g.rescale(b, [1 << 30], [up[1]], 0, 2, np.int32))
+    inv = g.inline(np.asarray([(1 << 20) // length], np.int32).reshape(1, 1, 1))
+    cen = g.sub(t, g.mul(g.reduce("REDUCE_SUM", t, 2), inv, 20))
+    var = g.mul(g.reduce("REDUCE_SUM", g.mul(cen, cen, 8), 2), inv, 20)
+    bound = 32768 if table == "any" else 8
+    lut = r.integers(-bound, bound, (513,)).astype(np.int16)
+    y = g.mul(cen, g.table(g.rescale(var, [1 << 30], [34], 0, -32768, np.int16), lut), norm_shift)
+    g.output(g.rescale(y, [1 << 30], [out_shift], 0, out_zp, np.int8, double_round=double_round))
+    check_fused(mlel, g, [full_range(r, np.int8, shape), full_range(r, np.int8, shape)], [NORM])
+
+
 @pytest.mark.parametrize("length", [64, 132])
 def test_layer_norm_with_gain_and_bias(mlel, length):
     """Per-channel gain and bias behind the normalisation: not the register kernel's program, the operators' results."""

@@ -76,7 +76,7 @@ def test_residual_tail_without_a_table(mlel, tile, oc, relu):
     """Behind a convolution over padded channels the tail has no table: its RESCALEs are evaluated."""
     r = np.random.Generator(np.random.PCG64(tile + oc))
     g = GraphBuilder()
-    x, short = g.input(np.int8, (1, 9, 11, 20)), g.input(np.int8, (1, 9, 11, oc))
+    x, short = g.input(np.int8, (1, 9, 11, 40)), g.input(np.int8, (1, 9, 11, oc))
     y = conv(g, r, x, oc, 3, 1, 1, -3, relu)
     a = g.rescale(y, [int(r.integers(1 << 30, 1 << 31))], [23], 4, 0, np.int32)
     b = g.rescale(short, [int(r.integers(1 << 30, 1 << 31))], [23], -3, 0, np.int32)
