@@ -35,6 +35,7 @@
 //                             i[13] weightZeroPoint i[14] accType      in = {input, weights, biases}
 #include "graph_pipeline.hpp"
 #include "kernels/attention_i8.hpp"
+#include "kernels/depthwise_i8.hpp"
 #include "kernels/device_common.cuh"
 #include "kernels/gemm_i8_tcgen05.hpp"
 
@@ -2096,6 +2097,40 @@ void GraphPipeline::prepareTensorCore() {
     }
 }
 
+// Per-channel constants of a fused 3x3 depthwise convolution, for the kernel that reads them as a table.
+void GraphPipeline::prepareDepthwise() {
+    for (auto &op : exec_) {
+        if (op.kind != OP_FUSED_DEPTHWISE || op.epi.hasResidual || !op.epi.hasMain) {
+            continue;
+        }
+        const TensorDescriptor &in = tensor(op.in[0]), &w = tensor(op.in[1]), &b = tensor(op.in[2]), &out = tensor(op.out[0]);
+        const TensorDescriptor &mult = tensor(op.epi.main.multTensor), &shift = tensor(op.epi.main.shiftTensor);
+        const auto constant = [](const TensorDescriptor &t, int32_t dtype, int64_t count) {
+            return t.cls == TensorClass::Constant && t.packed() && t.dtype == dtype && t.numel() >= count;
+        };
+        if (in.dtype != MLEL_I8 || out.dtype != MLEL_I8 || in.rank() != 4 || out.rank() != 4 || w.rank() != 4 || !in.packed() || !out.packed()) {
+            continue;
+        }
+        const int64_t channels = in.dims[3], scales = op.epi.main.attr.perChannel ? channels : 1;
+        if (w.dims[0] != 3 || w.dims[1] != 3 || w.dims[2] != channels || w.dims[3] != 1 || out.dims[3] != channels || in.dims[0] != out.dims[0] ||
+            channels > (1 << 20) || (b.numel() != channels && b.numel() != 1) || !constant(w, MLEL_I8, 9 * channels) || !constant(b, MLEL_I32, 1) ||
+            !constant(mult, MLEL_I32, scales) || !constant(shift, MLEL_I8, scales)) {
+            continue;
+        }
+        const FusedRescale &f = op.epi.main;
+        DepthwiseConstants d{};
+        d.weights = reinterpret_cast<const int8_t *>(w.hostData.data()), d.bias = reinterpret_cast<const int32_t *>(b.hostData.data());
+        d.mult = reinterpret_cast<const int32_t *>(mult.hostData.data()), d.shift = reinterpret_cast<const int8_t *>(shift.hostData.data());
+        d.channels = int32_t(channels), d.biasCount = int32_t(b.numel()), d.perChannel = f.attr.perChannel;
+        d.doubleRound = f.attr.scale32 && f.attr.doubleRound;
+        d.inputZp = op.i[8], d.rescaleZp = int32_t(wrapTo(f.inDtype, f.attr.inZp)), d.outZp = int32_t(wrapTo(f.outDtype, f.attr.outZp)), d.lo = f.lo;
+        std::vector<DepthwiseChannel> table;
+        if (op.i[9] == 0 && makeDepthwiseChannels(d, &table)) {
+            op.aux[0] = addDerivedConstant(MLEL_U8, {int64_t(table.size() * sizeof(DepthwiseChannel))}, table.data());
+        }
+    }
+}
+
 const std::vector<OpDesc> &GraphPipeline::getExecList() {
     finalize();
     return exec_;
@@ -2109,6 +2144,7 @@ void GraphPipeline::finalize() {
     if (!(flags_ & MLEL_PIPELINE_NO_TENSOR_CORE)) {
         prepareTensorCore();
     }
+    prepareDepthwise();
     // Lay constants out in one slab, each on a 256-byte boundary.
     uint64_t offset = 0;
     for (auto &t : tensors_) {

@@ -162,6 +162,7 @@ class GraphPipeline {
                      const std::function<void(OpDesc, const std::vector<int> &)> &emit);
     void prepareTensorCore();
     void buildResidualTable(OpDesc &op);
+    void prepareDepthwise();
     int32_t addDerivedConstant(int32_t dtype, const std::vector<int64_t> &dims, const void *data);
     int32_t addScratchTensor(int32_t dtype, const std::vector<int64_t> &dims);
 

@@ -8,6 +8,7 @@
 #include <string>
 
 #include "kernels/attention_i8.hpp"
+#include "kernels/depthwise_i8.hpp"
 #include "kernels/device_common.cuh"
 #include "kernels/gemm_i8_tcgen05.hpp"
 #include "kernels/kernels.hpp"
@@ -561,6 +562,9 @@ int launchOp(const OpDesc &op, const TView *T, cudaStream_t s, LaunchChain *chai
         return fusedConv2dGeneric(in(0), in(1), in(2), out, convAttr(op), devEpilogue(op.epi, T), s);
     case OP_FUSED_DEPTHWISE: {
         const DevEpilogue epi = devEpilogue(op.epi, T);
+        if (op.aux[0] >= 0 && depthwiseTableTakes(in(0), out, convAttr(op))) {
+            return depthwiseFromTable(in(0), T[op.aux[0]], out, convAttr(op), epi.main, s);
+        }
         if (!epi.hasResidual && depthwise3x3Eligible(in(0), in(1), in(2), out, convAttr(op), true)) {
             return depthwise3x3(in(0), in(1), in(2), out, convAttr(op), &epi, s);
         }

@@ -259,6 +259,7 @@ struct OpDesc {
     //                 pixels; aux[3] weights per unit [units][OC][16]
     int32_t tc{0};
     int32_t scratch{-1};
+    //   FUSED_DEPTHWISE 3x3: aux[0] constants per channel (DepthwiseChannel), where a table describes the node
     int32_t aux[5]{-1, -1, -1, -1, -1};
     int32_t auxi[5]{0, 0, 0, 0, 0};
 };
