@@ -396,6 +396,10 @@ bool gemmI8OcMajorApplies(const GemmI8Problem &q) {
             p.epi.main.lo >= -128 && p.epi.main.hi <= 127 && (reinterpret_cast<uintptr_t>(p.epi.shortcut) & 15u) == 0);
 }
 
+bool gemmI8OcMajorMayTake(int64_t pixels, int64_t channels) {
+    return channels > 64 && (tensorCoreTuning().smallKernel.load(std::memory_order_relaxed) != 1 || !smallKernelWants(pixels, channels));
+}
+
 // Tile-level hand-over between consecutive launches (GemmI8Params::progressOut / progressIn, LaunchChain).
 //
 // Why it is safe.  Launch C follows launch B in the stream, both with programmatic dependent launch, and C's pixel

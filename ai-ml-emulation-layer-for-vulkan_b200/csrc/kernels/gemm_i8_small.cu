@@ -390,6 +390,10 @@ int launchSmallSplit(const CUtensorMap &mapX, const CUtensorMap &mapW, const Gem
 
 } // namespace
 
+bool smallKernelWants(int64_t pixels, int64_t channels) {
+    return (pixels + 127) / 128 * ((channels + kSmallChannels - 1) / kSmallChannels) * 3 <= smCount();
+}
+
 bool gemmI8SmallApplies(const GemmI8Problem &q, int *pixels, int *split) {
     const GemmI8Params &p = q.params;
     const int mode = tensorCoreTuning().smallKernel.load(std::memory_order_relaxed);
@@ -404,7 +408,7 @@ bool gemmI8SmallApplies(const GemmI8Problem &q, int *pixels, int *split) {
     // most one CTA per SM 267; narrow tiles always 249, but 16 images 487 against 478 us).
     const int sms = smCount();
     const int64_t cTiles = (p.N + kSmallChannels - 1) / kSmallChannels;
-    if (mode == 1 && int64_t((p.M + 127) / 128) * cTiles * 3 > sms) {
+    if (mode == 1 && !smallKernelWants(p.M, p.N)) {
         return false;
     }
     const int numKb = q.aMatrix != nullptr ? (p.K + BK - 1) / BK : p.KH * p.KW * ((p.IC + 127) / 128);

@@ -130,6 +130,8 @@ int gemmI8Launch(const GemmI8Problem &problem, cudaStream_t stream);
 // Channel-major variant (gemm_i8_ocmajor.cu) for fused int8 convolutions with more than 64 output channels:
 // same problem description, weights as the tensor-core A operand.  `Applies` tells whether it can take q.
 bool gemmI8OcMajorApplies(const GemmI8Problem &problem);
+// Whether a convolution of these sizes may run on it (false: another kernel takes it under the present selection).
+bool gemmI8OcMajorMayTake(int64_t pixels, int64_t channels);
 // `chain` (may be null): where the launch records what it publishes; `consumed` (may be null): what the launch before it
 // in the stream published.
 int gemmI8OcMajorLaunch(const GemmI8Problem &problem, cudaStream_t stream, LaunchChain *chain = nullptr,
@@ -146,6 +148,7 @@ int pairErrorWord();
 // Small-problem variant (gemm_i8_small.cu): narrow tiles whose K blocks are shared by a cluster.  `Applies` chooses the
 // pixels per tile and the CTAs per tile; Launch sets *taken as the paired variant does.
 bool gemmI8SmallApplies(const GemmI8Problem &problem, int *pixels, int *split);
+bool smallKernelWants(int64_t pixels, int64_t channels); // the rule on sizes in it
 int gemmI8SmallLaunch(const GemmI8Problem &problem, int pixels, int split, cudaStream_t stream, bool *taken);
 int smallErrorWord();
 

@@ -20,17 +20,21 @@ Session::Session(GraphPipeline *pipeline) : pipeline_(pipeline) {
     // Made here and not at the first dispatch, which may run inside a stream capture.  Without them (no
     // device, no memory) the dispatch simply does without the hand-over.
     const auto &exec = pipeline_->getExecList();
-    // one counter per 128 output pixels (the narrowest tile) of every convolution whose output the next one reads
+    // one counter per 128 output pixels (the narrowest tile) of every convolution whose output the next one reads, where both
+    // are the channel-major kernel's: zeroing the counters is a node of its own at the head of a replayed graph, 2 to 5 us of
+    // a pass that does not use them
     size_t words = 0;
+    const auto pixelsOf = [&](const OpDesc &op) {
+        const TensorDescriptor &out = pipeline_->tensor(op.out[0]);
+        return out.dims.back() == 0 ? int64_t(0) : out.numel() / out.dims.back();
+    };
+    const auto channelMajor = [&](const OpDesc &op) {
+        return op.tc != 0 && (op.kind == OP_CONV2D || op.kind == OP_FUSED_CONV2D) && !op.out.empty() && !op.in.empty() &&
+               gemmI8OcMajorMayTake(pixelsOf(op), pipeline_->tensor(op.out[0]).dims.back());
+    };
     for (size_t k = 0; k + 1 < exec.size(); ++k) {
-        if (exec[k].tc != 0 && exec[k + 1].tc != 0 && !exec[k].out.empty() && !exec[k + 1].in.empty() &&
-            exec[k + 1].in[0] == exec[k].out[0]) {
-            const TensorDescriptor &out = pipeline_->tensor(exec[k].out[0]);
-            int64_t pixels = 1;
-            for (int i = 0; i + 1 < out.rank(); ++i) {
-                pixels *= out.dims[size_t(i)];
-            }
-            words += size_t((pixels + 127) / 128);
+        if (channelMajor(exec[k]) && channelMajor(exec[k + 1]) && exec[k + 1].in[0] == exec[k].out[0]) {
+            words += size_t((pixelsOf(exec[k]) + 127) / 128);
         }
     }
     if (words != 0 && (cudaMalloc(&progressWords_, words * sizeof(uint32_t)) != cudaSuccess ||
