@@ -12,12 +12,13 @@ namespace tc {
 
 // Constants of the main RESCALE stage for one output column, two shared-memory reads per element in the general form (see
 // FastRescale): {mult, corr0, rnLo, rnHi, s2, bump} with the rounding constant for v < zpIn (input zero point folded in).
-// Where wordsScaleApplies to every column and the corrections are small, one read: the WordsScale {mult, low, high, shift}
-// with the correction folded in.
+// Where wordsScaleApplies to every column and the corrections are small, one read: the WordsScale {low, high, mult, shift}
+// with the correction folded in.  (The 64-bit addend first: as the middle of a 16-byte load, where no register pair starts, it
+// was moved for every result.)
 struct __align__(16) ColConst {
-    int32_t mult;
-    int32_t corr;        // general: correction of the most common border class; else WordsScale's low
-    uint32_t rnLo, rnHi; // general: rounding constant; else WordsScale's high and shift
+    int32_t mult;        // else WordsScale's low
+    int32_t corr;        // correction of the most common border class; else WordsScale's high
+    uint32_t rnLo, rnHi; // rounding constant; else WordsScale's mult and shift
     int32_t s2;          // max(shift - 32, 0)
     uint32_t bump;       // what the constant for v >= zpIn adds: 2^31 with double rounding and shift > 31, else 0
     int32_t s1;          // min(shift, 32)
@@ -31,15 +32,15 @@ __device__ __forceinline__ int wordsForm(const DevRescale &m) { return wordsScal
 
 __device__ __forceinline__ ColConst makeColConst(const FastRescale &f, int32_t corr0, const DevRescale &m, int form) {
     ColConst c;
-    c.mult = f.mult, c.s1 = f.s1, c.s2 = f.s2, c.corr0 = corr0;
+    c.s1 = f.s1, c.s2 = f.s2, c.corr0 = corr0;
     c.bump = f.rpLo - f.rnLo; // (rp - rn) mod 2^32: 0 or 2^31
     if (form != kGeneralForm) {
         const int32_t x0 = int32_t(uint32_t(corr0) - uint32_t(f.zpIn));
         const WordsScale w = form == kWords ? makeWordsScale<false>(f.mult, f.s1 + f.s2, m.doubleRound != 0, x0, m.outZp)
                                             : makeWordsScale<true>(f.mult, f.s1 + f.s2, m.doubleRound != 0, x0, 0);
-        c.corr = int32_t(w.low), c.rnLo = w.high, c.rnHi = uint32_t(w.shift);
+        c.mult = int32_t(w.low), c.corr = int32_t(w.high), c.rnLo = uint32_t(w.mult), c.rnHi = uint32_t(w.shift);
     } else {
-        c.corr = corr0, c.rnLo = f.rnLo, c.rnHi = f.rnHi;
+        c.mult = f.mult, c.corr = corr0, c.rnLo = f.rnLo, c.rnHi = f.rnHi;
     }
     return c;
 }
@@ -67,7 +68,7 @@ __device__ __forceinline__ void rescale16Words(const uint32_t (&acc)[16], uint32
         for (int e = 0; e < 4; ++e) {
             const int j = 4 * q + e;
             uint32_t mult, low, high, shift;
-            ldsV4(tabAddr + uint32_t(j) * 32u, mult, low, high, shift);
+            ldsV4(tabAddr + uint32_t(j) * 32u, low, high, mult, shift);
             const int32_t v = wordsScale<SIGNED>(WordsScale{int32_t(mult), int32_t(shift), low, high}, int32_t(acc[j]));
             y[e] = min(SIGNED ? __viaddmax_s32(v, outZp, lo) : max(v, lo), hi);
         }
