@@ -483,7 +483,7 @@ int gemmI8OcMajorLaunch(const GemmI8Problem &q, cudaStream_t s, LaunchChain *cha
     }
     const int progressMode = tensorCoreTuning().tileProgress.load(std::memory_order_relaxed);
     const bool handOver = chain != nullptr && xMode != kXGather && progressMode != 0 &&
-                          tensorCoreTuning().dependentLaunch.load(std::memory_order_relaxed) != 0;
+                          dependentLaunches();
     if (handOver && before.prevCounters != nullptr && (progressMode & 1)) {
         // read by tiles when the launch before this one wrote exactly this launch's pixel operand
         const void *input = q.aMatrix != nullptr ? q.aMatrix : static_cast<const void *>(p.in);

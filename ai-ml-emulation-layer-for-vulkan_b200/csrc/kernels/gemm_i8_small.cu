@@ -351,7 +351,7 @@ int launchSmall(const CUtensorMap &mapX, const CUtensorMap &mapW, const GemmI8Pa
     attrs[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attrs[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attrs;
-    cfg.numAttrs = tensorCoreTuning().dependentLaunch.load(std::memory_order_relaxed) != 0 ? 2 : 1;
+    cfg.numAttrs = dependentLaunches() ? 2 : 1;
     const cudaError_t err = cudaLaunchKernelEx(&cfg, kernel, mapX, mapW, p);
     if (err != cudaSuccess) {
         setLastError(std::string("small int8 GEMM launch: ") + cudaGetErrorString(err));

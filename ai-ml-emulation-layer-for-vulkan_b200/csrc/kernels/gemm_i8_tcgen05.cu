@@ -810,6 +810,13 @@ TensorCoreTuning &tensorCoreTuning() {
     return t;
 }
 
+namespace {
+thread_local bool t_plainLaunches = false;
+}
+bool dependentLaunches() { return !t_plainLaunches && tensorCoreTuning().dependentLaunch.load(std::memory_order_relaxed) != 0; }
+PlainLaunches::PlainLaunches(bool on) : before_(t_plainLaunches) { t_plainLaunches = t_plainLaunches || on; }
+PlainLaunches::~PlainLaunches() { t_plainLaunches = before_; }
+
 int gemmI8Launch(const GemmI8Problem &q, cudaStream_t s) {
     g_tensorCoreLaunches[0].fetch_add(1, std::memory_order_relaxed);
     GemmI8Params p = q.params;

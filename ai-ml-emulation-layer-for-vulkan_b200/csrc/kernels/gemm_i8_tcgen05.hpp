@@ -182,6 +182,19 @@ struct TensorCoreTuning {
 };
 TensorCoreTuning &tensorCoreTuning();
 
+// Whether launches of this thread ask for programmatic dependent launch: the tuning's choice, but not while a PlainLaunches
+// exists (launches that are captured with dependencies of their own, Session::capture).
+bool dependentLaunches();
+class PlainLaunches {
+  public:
+    explicit PlainLaunches(bool on);
+    ~PlainLaunches();
+    PlainLaunches(const PlainLaunches &) = delete;
+
+  private:
+    bool before_;
+};
+
 // Launches of the five tensor-core kernels since the library was loaded: 0 pixel-major (gemm_i8_tcgen05.cu),
 // 1 channel-major (gemm_i8_ocmajor.cu), 2 paired (gemm_i8_pair.cu), 3 small (gemm_i8_small.cu), 4 window
 // (gemm_i8_window.cu).  Tests use them to see which kernel took a case.

@@ -36,7 +36,7 @@ inline cudaError_t launchOverlapped(void (*kernel)(Params...), dim3 grid, unsign
     attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr.val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = &attr;
-    cfg.numAttrs = tensorCoreTuning().dependentLaunch.load(std::memory_order_relaxed) != 0 ? 1 : 0;
+    cfg.numAttrs = dependentLaunches() ? 1 : 0;
     return cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
 }
 

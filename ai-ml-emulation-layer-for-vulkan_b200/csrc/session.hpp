@@ -31,6 +31,8 @@ struct PlannedTensor {
     bool seen; // false: no launched operator touches it (only kept when fusion is off)
 };
 
+struct LaunchChain; // kernels/gemm_i8_tcgen05.hpp
+
 class Session {
   public:
     explicit Session(GraphPipeline *pipeline);
@@ -57,6 +59,11 @@ class Session {
     void planInterval();
     void planLinear();
     void planBestFit();
+    // Enqueues the operators on a stream that this session captures: as dispatch() does, except that operators between two
+    // tensor-core launches depend on what they touch, not on their order.
+    int capture(cudaStream_t stream);
+    int enqueueOp(size_t k, LaunchChain *chain, cudaStream_t stream);
+    std::vector<std::vector<size_t>> branches(size_t first, size_t end) const;
     int resolve(); // fills views_ with device addresses; fails if something is unbound
 
     GraphPipeline *pipeline_;

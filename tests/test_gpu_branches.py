@@ -1,0 +1,88 @@
+"""Replayed graphs whose operators do not form a chain: element-wise operators, pools, reductions and movement that depend on one
+another, on tensors which share memory, and on the contractions before and behind them.  Bit-exact against the CPU oracle, as
+replayed and as enqueued."""
+import random
+
+import numpy as np
+import pytest
+
+from mlel_b200.graph_builder import GraphBuilder
+from tests.graph_eval import evaluate
+
+pytestmark = pytest.mark.gpu
+
+
+def random_graph(seed, size, count):
+    """`count` operators on int8 tensors of one shape, each reading earlier results at random."""
+    choice = random.Random(seed)
+    r = np.random.Generator(np.random.PCG64(seed))
+    g = GraphBuilder()
+    values = [g.input(np.int8, size), g.input(np.int8, size)]
+    for _ in range(count):
+        x, y = (values[choice.randrange(max(0, len(values) - 6), len(values))] for _ in range(2))
+        kind = choice.choice(["clamp", "table", "add", "pool", "slice", "reverse", "conv"])
+        if kind == "clamp":
+            v = g.clamp(x, -int(r.integers(20, 120)), int(r.integers(20, 120)))
+        elif kind == "table":
+            v = g.table(x, r.integers(-128, 128, (256,), dtype=np.int8))
+        elif kind == "add":
+            a, b = (g.rescale(t, [1 << 30], [25], 0, 0, np.int32) for t in (x, y))
+            v = g.rescale(g.add(a, b), [1 << 30], [36], 0, 0, np.int8)
+        elif kind == "pool":
+            v = g.max_pool2d(x, [3, 3], [1, 1], [1, 1, 1, 1])
+        elif kind == "slice":
+            v = g.concat([g.slice(x, [0, 0, 0, 0], [size[0], size[1], size[2], 3]),
+                          g.slice(y, [0, 0, 0, 3], [size[0], size[1], size[2], size[3] - 3])], 3)
+        elif kind == "reverse":
+            v = g.reverse(x, 1)
+        else:
+            w = g.constant(r.integers(-128, 128, (size[3], 1, 1, size[3]), dtype=np.int8))
+            bias = g.constant(np.zeros((size[3],), np.int32))
+            v = g.rescale(g.conv2d(x, w, bias, [0] * 4, [1, 1], [1, 1], 0, 0), [1 << 30], [40], 0, 0, np.int8)
+        values.append(v)
+    for v in values[2:]:
+        if choice.random() < 0.4 or v is values[-1]:
+            g.output(v)
+    return g
+
+
+@pytest.mark.parametrize("seed", range(12))
+@pytest.mark.parametrize("size", [(1, 6, 7, 16), (2, 60, 60, 48)])
+def test_random_dependencies(mlel, seed, size):
+    from mlel_b200.runtime import GraphRunner
+    g = random_graph(seed, size, 14)
+    r = np.random.Generator(np.random.PCG64(seed + 100))
+    runner = GraphRunner(g)
+    for repeat in range(3):
+        data = [r.integers(-128, 128, size, dtype=np.int8) for _ in range(2)]
+        want = evaluate(g, data)
+        for use_cuda_graph in (True, False):
+            for a, b in zip(runner.run(data, use_cuda_graph=use_cuda_graph), want):
+                np.testing.assert_array_equal(a, b)
+
+
+def test_application_tensors_that_share_memory(mlel):
+    """The second operator's input lies where the first one's output does, and the third overwrites what the second reads."""
+    import torch
+    from mlel_b200.runtime import GraphRunner
+    shape = (1, 64, 64, 64)
+    r = np.random.Generator(np.random.PCG64(3))
+    g = GraphBuilder()
+    a, b, c = (g.input(np.int8, shape) for _ in range(3))
+    lut = r.integers(-128, 128, (256,), dtype=np.int8)
+    g.output(g.clamp(a, -30, 40))
+    g.output(g.table(b, lut))
+    g.output(g.clamp(c, -5, 90))
+    runner = GraphRunner(g)
+    shared = runner.outputs[0]
+    runner.session.set_external(*runner._in_keys[1][:2], shared.data_ptr())
+    runner.session.set_external(*runner._out_keys[2][:2], shared.data_ptr())
+    for _ in range(20):
+        data = [r.integers(-128, 128, shape, dtype=np.int8) for _ in range(3)]
+        runner.set_inputs(data)
+        runner.dispatch(use_cuda_graph=True)
+        torch.cuda.synchronize()
+        first = np.clip(data[0], -30, 40)
+        got = [t.cpu().numpy().view(np.int8).reshape(shape) for t in (runner.outputs[1], shared)]
+        np.testing.assert_array_equal(got[0], lut[first.astype(np.int32) + 128])
+        np.testing.assert_array_equal(got[1], np.clip(data[2], -5, 90))
