@@ -210,6 +210,12 @@ gemmI8Window(const __grid_constant__ CUtensorMap mapX, const __grid_constant__ C
                             umma(tmemD, {stage + pairX[m], pairHigh}, {w + uint32_t(2 * m * BN), weightHigh}, idesc, m == 0 ? 0u : 1u);
                         }
                     }
+                } else if (kThree && kSlices == 1) { // (a window row to a statement)
+#pragma unroll
+                    for (int ky = 0; ky < 3; ++ky) {
+                        ummaBlock(tmemD, {stageX + uint32_t(ky) * rowStep, highX}, tapStep, {lowW + uint32_t(3 * ky) * weightStep, highW},
+                                  weightStep, idesc, ky == 0 ? 0u : 1u, 3);
+                    }
                 } else if (kThree) {
 #pragma unroll
                     for (int t = 0; t < 9; ++t) {
