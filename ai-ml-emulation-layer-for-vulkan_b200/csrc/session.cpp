@@ -471,13 +471,13 @@ bool isPaced(const OpDesc &op) {
 
 } // namespace
 
-// For every operator of [first, end) the earlier ones in it (as offsets) whose bytes it reads or overwrites, or that read what
-// it overwrites.  By address, so that tensors which the session or the application placed over one another count.
-std::vector<std::vector<size_t>> Session::branches(size_t first, size_t end) const {
+// For every one of these operators the earlier ones (as positions in the list) whose bytes it reads or overwrites, or that read
+// what it overwrites.  By address, so that tensors which the session or the application placed over one another count.
+std::vector<std::vector<size_t>> Session::branches(const std::vector<size_t> &ops) const {
     const auto &exec = pipeline_->getExecList();
-    std::vector<std::vector<ByteRange>> reads(end - first), writes(end - first);
-    for (size_t k = first; k < end; ++k) {
-        const OpDesc &op = exec[k];
+    std::vector<std::vector<ByteRange>> reads(ops.size()), writes(ops.size());
+    for (size_t k = 0; k < ops.size(); ++k) {
+        const OpDesc &op = exec[ops[k]];
         const auto add = [&](std::vector<ByteRange> &list, int32_t t) {
             if (t >= 0 && pipeline_->tensor(t).cls != TensorClass::Constant) {
                 const ByteRange r = bytesOf(views_[size_t(t)], elemSize(views_[size_t(t)].dtype));
@@ -487,16 +487,16 @@ std::vector<std::vector<size_t>> Session::branches(size_t first, size_t end) con
             }
         };
         for (const int32_t t : op.in) {
-            add(reads[k - first], t);
+            add(reads[k], t);
         }
-        add(reads[k - first], op.epi.shortcutTensor);
+        add(reads[k], op.epi.shortcutTensor);
         for (const int32_t t : op.out) {
-            add(writes[k - first], t);
+            add(writes[k], t);
         }
-        add(writes[k - first], op.scratch);
+        add(writes[k], op.scratch);
     }
-    std::vector<std::vector<size_t>> before(end - first);
-    for (size_t k = 0; k < end - first; ++k) {
+    std::vector<std::vector<size_t>> before(ops.size());
+    for (size_t k = 0; k < ops.size(); ++k) {
         for (size_t j = 0; j < k; ++j) {
             if (meet(reads[k], writes[j]) || meet(writes[k], writes[j]) || meet(writes[k], reads[j])) {
                 before[k].push_back(j);
@@ -540,16 +540,23 @@ int Session::capture(cudaStream_t stream) {
     const auto follow = [&](std::vector<cudaGraphNode_t> &nodes) {
         return cudaStreamUpdateCaptureDependencies(stream, nodes.data(), nodes.size(), cudaStreamSetCaptureDependencies) == cudaSuccess;
     };
+    // (a RESHAPE within one storage launches nothing)
+    const auto launches = [&](const OpDesc &op) {
+        return op.kind != OP_RESHAPE || views_[size_t(op.in[0])].ptr != views_[size_t(op.out[0])].ptr;
+    };
     bool joined = false; // several nodes precede the next launch
     for (size_t k = 0; k < exec.size();) {
         size_t end = k;
-        while (end < exec.size() && !isPaced(exec[end])) {
-            ++end;
+        std::vector<size_t> ops;
+        for (; end < exec.size() && !isPaced(exec[end]); ++end) {
+            if (launches(exec[end])) {
+                ops.push_back(end);
+            }
         }
         std::vector<std::vector<size_t>> before;
-        bool chainOnly = end - k < 2;
+        bool chainOnly = ops.size() < 2;
         if (!chainOnly) {
-            before = branches(k, end);
+            before = branches(ops);
             chainOnly = true;
             for (size_t j = 1; j < before.size(); ++j) {
                 chainOnly = chainOnly && !before[j].empty() && before[j].back() == j - 1;
@@ -562,7 +569,7 @@ int Session::capture(cudaStream_t stream) {
                 if (r != MLEL_SUCCESS) {
                     return r;
                 }
-                joined = false;
+                joined = joined && !launches(exec[k]);
             }
             continue;
         }
@@ -594,7 +601,7 @@ int Session::capture(cudaStream_t stream) {
             }
             tail[lane] = j;
             load[lane] += uint64_t(12) << 20;
-            for (const auto *list : {&exec[k + j].in, &exec[k + j].out}) {
+            for (const auto *list : {&exec[ops[j]].in, &exec[ops[j]].out}) {
                 for (const int32_t t : *list) {
                     load[lane] += t >= 0 ? pipeline_->tensor(t).sizeBytes() : 0;
                 }
@@ -609,11 +616,11 @@ int Session::capture(cudaStream_t stream) {
             if (!follow(from)) {
                 return failed();
             }
-            const int r = enqueueOp(k + j, chainOrNull, stream);
+            const int r = enqueueOp(ops[j], chainOrNull, stream);
             if (r != MLEL_SUCCESS) {
                 return r;
             }
-            if (!leaves(&exits[j])) { // (an operator that launches nothing leaves what it follows)
+            if (!leaves(&exits[j])) {
                 return failed();
             }
         }

@@ -63,7 +63,7 @@ class Session {
     // tensor-core launches depend on what they touch, not on their order.
     int capture(cudaStream_t stream);
     int enqueueOp(size_t k, LaunchChain *chain, cudaStream_t stream);
-    std::vector<std::vector<size_t>> branches(size_t first, size_t end) const;
+    std::vector<std::vector<size_t>> branches(const std::vector<size_t> &ops) const;
     int resolve(); // fills views_ with device addresses; fails if something is unbound
 
     GraphPipeline *pipeline_;
