@@ -61,10 +61,14 @@ __device__ __forceinline__ void prefetchMap(const CUtensorMap *map) {
     asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(map)) : "memory");
 }
 
+// A residual tail: looked up in its table, or (where it has none) evaluated.
+enum : int { kNoTail = 0, kTailTable = 1, kTailArithmetic = 2 };
+
 // IM2COL: mapX is an im2col map of the NHWC input and mapW a {IC, taps, OC} map; else mapX is a plain pixel matrix.
-template <int BNP, int SPLIT, bool IM2COL, bool RESIDUAL, bool TABLE = false>
+template <int BNP, int SPLIT, bool IM2COL, int TAIL, bool TABLE = false>
 __global__ void __launch_bounds__(kSmallThreads, 2)
 gemmI8Small(const __grid_constant__ CUtensorMap mapX, const __grid_constant__ CUtensorMap mapW, const __grid_constant__ GemmI8Params p) {
+    constexpr bool RESIDUAL = TAIL != kNoTail;
     constexpr int kStages = smallStages(BNP);
     constexpr int kTileW = kSmallChannels * BK, kTileX = BNP * BK;
     constexpr int kPixels = BNP / SPLIT; // pixels that this CTA finishes
@@ -298,8 +302,7 @@ gemmI8Small(const __grid_constant__ CUtensorMap mapX, const __grid_constant__ CU
             }
         }
         FastRescale fa{}, fb{}, fo{};
-        const uint8_t *tail = RESIDUAL ? p.residualTable : nullptr;
-        if (RESIDUAL && tail == nullptr) {
+        if (TAIL == kTailArithmetic) {
             fa = makeFastRescale(__ldg(p.epi.a.mult), int32_t(__ldg(p.epi.a.shift)), p.epi.a.inZp, p.epi.a.doubleRound != 0);
             fb = makeFastRescale(__ldg(p.epi.b.mult), int32_t(__ldg(p.epi.b.shift)), p.epi.b.inZp, p.epi.b.doubleRound != 0);
             fo = makeFastRescale(__ldg(p.epi.out.mult), int32_t(__ldg(p.epi.out.shift)), p.epi.out.inZp, p.epi.out.doubleRound != 0);
@@ -308,11 +311,11 @@ gemmI8Small(const __grid_constant__ CUtensorMap mapX, const __grid_constant__ CU
 #pragma unroll
         for (int j = 0; j < kMine; ++j) {
             int32_t v = fastRescale(main, int32_t(acc[j] + uint32_t(corr[j])), p.epi.main.outZp, p.epi.main.lo, p.epi.main.hi);
-            if (RESIDUAL && tail != nullptr) {
+            if (TAIL == kTailTable) {
                 // The whole tail is a byte of this table, a load from cache where the three RESCALEs took 0.8 us of a layer's 4
                 // (one image of the ResNet-50 shape 222.1 -> 219.4 us, 32 of the MobileNetV2 shape 481 -> 473.5).
-                v = int32_t(__ldg(tail + (v + 128) * GemmI8Params::kResidualRowBytes + int32_t(uint8_t(shortcut[j]))));
-            } else if (RESIDUAL) {
+                v = int32_t(__ldg(p.residualTable + (v + 128) * GemmI8Params::kResidualRowBytes + int32_t(uint8_t(shortcut[j]))));
+            } else if (TAIL == kTailArithmetic) {
                 const int32_t ta = fastRescale(fa, v, p.epi.a.outZp, p.epi.a.lo, p.epi.a.hi);
                 const int32_t tb = fastRescale(fb, int32_t(shortcut[j]), p.epi.b.outZp, p.epi.b.lo, p.epi.b.hi);
                 v = fastRescale(fo, int32_t(uint32_t(ta) + uint32_t(tb)), p.epi.out.outZp, p.epi.out.lo, p.epi.out.hi);
@@ -332,11 +335,11 @@ gemmI8Small(const __grid_constant__ CUtensorMap mapX, const __grid_constant__ CU
     }
 }
 
-template <int BNP, int SPLIT, bool IM2COL, bool RESIDUAL, bool TABLE = false>
+template <int BNP, int SPLIT, bool IM2COL, int TAIL, bool TABLE = false>
 int launchSmall(const CUtensorMap &mapX, const CUtensorMap &mapW, const GemmI8Params &p, int tiles, cudaStream_t s) {
     constexpr size_t smem = size_t(smallStages(BNP)) * (kSmallChannels + BNP) * BK +
                             (SPLIT > 1 ? size_t(BNP) * kSmallChannels * 4 : 0) + sizeof(SmallBarriers) + 1024;
-    auto kernel = gemmI8Small<BNP, SPLIT, IM2COL, RESIDUAL, TABLE>;
+    auto kernel = gemmI8Small<BNP, SPLIT, IM2COL, TAIL, TABLE>;
     if (!allowDynamicSmem(reinterpret_cast<const void *>(kernel), smem)) {
         return MLEL_ERROR_DEVICE;
     }
@@ -362,15 +365,18 @@ int launchSmall(const CUtensorMap &mapX, const CUtensorMap &mapW, const GemmI8Pa
 
 template <int BNP, int SPLIT>
 int launchSmallMode(const CUtensorMap &mapX, const CUtensorMap &mapW, const GemmI8Params &p, int tiles, bool im2col, cudaStream_t s) {
+    const int tail = !p.epi.hasResidual ? kNoTail : (p.residualTable != nullptr ? kTailTable : kTailArithmetic);
     if (im2col) {
-        return p.epi.hasResidual ? launchSmall<BNP, SPLIT, true, true>(mapX, mapW, p, tiles, s)
-                                 : launchSmall<BNP, SPLIT, true, false>(mapX, mapW, p, tiles, s);
+        return tail == kNoTail      ? launchSmall<BNP, SPLIT, true, kNoTail>(mapX, mapW, p, tiles, s)
+               : tail == kTailTable ? launchSmall<BNP, SPLIT, true, kTailTable>(mapX, mapW, p, tiles, s)
+                                    : launchSmall<BNP, SPLIT, true, kTailArithmetic>(mapX, mapW, p, tiles, s);
     }
     if (p.epi.table != nullptr) {
-        return launchSmall<BNP, SPLIT, false, false, true>(mapX, mapW, p, tiles, s);
+        return launchSmall<BNP, SPLIT, false, kNoTail, true>(mapX, mapW, p, tiles, s);
     }
-    return p.epi.hasResidual ? launchSmall<BNP, SPLIT, false, true>(mapX, mapW, p, tiles, s)
-                             : launchSmall<BNP, SPLIT, false, false>(mapX, mapW, p, tiles, s);
+    return tail == kNoTail      ? launchSmall<BNP, SPLIT, false, kNoTail>(mapX, mapW, p, tiles, s)
+           : tail == kTailTable ? launchSmall<BNP, SPLIT, false, kTailTable>(mapX, mapW, p, tiles, s)
+                                : launchSmall<BNP, SPLIT, false, kTailArithmetic>(mapX, mapW, p, tiles, s);
 }
 
 template <int BNP>
