@@ -17,6 +17,7 @@ namespace {
 // of the copy: byte reads hit L1, writes are coalesced.
 __global__ void padImageKernel(const int8_t *__restrict__ in, int8_t *__restrict__ out, int64_t words, int H, int W, int C,
                                int Hp, int Wp, int Cp, int padTop, int padLeft) {
+    dependencySync();
     const int wordsPerPixel = Cp >> 2;
     for (int64_t e = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; e < words; e += int64_t(gridDim.x) * blockDim.x) {
         int64_t pix = e / wordsPerPixel;
@@ -65,6 +66,7 @@ template <bool BORDER>
 __global__ void __launch_bounds__(256) padPixels16Kernel(const int8_t *__restrict__ in, int4 *__restrict__ out, uint32_t units, int H,
                                                          int W, int C, FastDiv perPixel, FastDiv divWp, FastDiv divHp, int padTop,
                                                          int padLeft) {
+    dependencySync();
     for (uint32_t e = blockIdx.x * blockDim.x + threadIdx.x; e < units; e += gridDim.x * blockDim.x) {
         const uint32_t pix = fastDiv(e, perPixel);
         const int c0 = int(e - pix * perPixel.d) * 16;
@@ -111,6 +113,7 @@ __global__ void __launch_bounds__(256) gatherUnitsKernel(const int8_t *__restric
 // store) per thread, no divisions in the element loop.
 __global__ void __launch_bounds__(128) padImageRows4Kernel(const int8_t *__restrict__ in, int8_t *__restrict__ out, int H,
                                                           int W, int C, int Hp, int Wp, int padTop, int padLeft) {
+    dependencySync();
     const int row = blockIdx.x; // n * Hp + yp
     const int n = row / Hp;
     const int y = row - n * Hp - padTop;
@@ -145,6 +148,7 @@ __global__ void __launch_bounds__(128) padImageRows4Kernel(const int8_t *__restr
 template <bool ALIGNED>
 __global__ void __launch_bounds__(256) transposeColsumKernel(const int8_t *__restrict__ b, int8_t *__restrict__ bt,
                                                              int32_t *__restrict__ corr, int C, int W, int Cp, int32_t za, int split) {
+    dependencySync();
     __shared__ int8_t tile[64][64 + 16]; // [c][w], rows padded to spread the banks of the column reads
     __shared__ int32_t part[64];
     const int n = blockIdx.y;
@@ -425,6 +429,7 @@ struct PoolAcc {
 template <int KH, int KW>
 __global__ void maxPoolI8Kernel(const int8_t *__restrict__ in, int8_t *__restrict__ out, int64_t total, int H, int W,
                                 int C, int OH, int OW, PoolAttr a) {
+    dependencySync();
     const int groups = C >> 4;
     const int4 lowest = make_int4(int(0x80808080u), int(0x80808080u), int(0x80808080u), int(0x80808080u));
     for (int64_t e = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; e < total; e += int64_t(gridDim.x) * blockDim.x) {
@@ -470,6 +475,7 @@ template <int CH>
 __global__ void __launch_bounds__(256) maxPoolNarrowKernel(const int8_t *__restrict__ in, int8_t *__restrict__ out,
                                                            uint32_t total, int H, int W, int C, FastDiv groups, FastDiv divOW,
                                                            FastDiv divOH, PoolAttr a) {
+    dependencySync();
     const uint32_t step = gridDim.x * blockDim.x;
     for (uint64_t e64 = blockIdx.x * blockDim.x + threadIdx.x; e64 < total; e64 += step) {
         const uint32_t e = uint32_t(e64);
@@ -506,6 +512,7 @@ __global__ void __launch_bounds__(256) maxPoolNarrowKernel(const int8_t *__restr
 // adjacent outputs, whose windows share a column, from 15 loads instead of 18.  OW must be even.
 __global__ void maxPool3x3s2PairKernel(const int8_t *__restrict__ in, int8_t *__restrict__ out, int64_t total, int H,
                                        int W, int C, int OH, int OW, int padTop, int padLeft) {
+    dependencySync();
     const int groups = C >> 4, pairs = OW >> 1;
     const int4 lowest = make_int4(int(0x80808080u), int(0x80808080u), int(0x80808080u), int(0x80808080u));
     for (int64_t e = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; e < total; e += int64_t(gridDim.x) * blockDim.x) {
@@ -576,6 +583,7 @@ __device__ __forceinline__ int4 packLanes(const LaneWords &l) {
 
 __global__ void maxPool3x3s2QuadKernel(const int8_t *__restrict__ in, int8_t *__restrict__ out, int64_t total, int H,
                                        int W, int C, int OH, int OW, int padTop, int padLeft) {
+    dependencySync();
     const int groups = C >> 4, pairsX = OW >> 1, pairsY = OH >> 1;
     const int4 lowest = make_int4(int(0x80808080u), int(0x80808080u), int(0x80808080u), int(0x80808080u));
     for (int64_t e = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; e < total; e += int64_t(gridDim.x) * blockDim.x) {
@@ -624,19 +632,19 @@ int padImageI8(const int8_t *in, int8_t *out, int N, int H, int W, int C, int Hp
                cudaStream_t s) {
     if (Cp == 4 && C <= 4 && Wp % 2 == 0 && int64_t(N) * Hp < (int64_t(1) << 31) &&
         (reinterpret_cast<uintptr_t>(out) & 7u) == 0) {
-        padImageRows4Kernel<<<unsigned(N * Hp), 128, 0, s>>>(in, out, H, W, C, Hp, Wp, padTop, padLeft);
+        launchOverlapped(padImageRows4Kernel, dim3(unsigned(N * Hp)), 128, 0, s, in, out, H, W, C, Hp, Wp, padTop, padLeft);
         return finish("padded copy");
     }
     const int64_t pixels = int64_t(N) * Hp * Wp, units = pixels * (Cp >> 4);
     if (Cp % 16 == 0 && units < (int64_t(1) << 30) && (reinterpret_cast<uintptr_t>(out) & 15u) == 0) {
         const bool border = Hp != H || Wp != W || padTop != 0 || padLeft != 0;
-        (border ? padPixels16Kernel<true> : padPixels16Kernel<false>)<<<gridFor(units, 256, 8), 256, 0, s>>>(
+        launchOverlapped(border ? padPixels16Kernel<true> : padPixels16Kernel<false>, dim3(gridFor(units, 256, 8)), 256, 0, s,
             in, reinterpret_cast<int4 *>(out), uint32_t(units), H, W, C, makeFastDiv(Cp >> 4), makeFastDiv(Wp), makeFastDiv(Hp), padTop,
             padLeft);
         return finish("padded copy");
     }
     const int64_t words = int64_t(N) * Hp * Wp * (Cp >> 2);
-    padImageKernel<<<gridFor(words, kThreads, 8), kThreads, 0, s>>>(in, out, words, H, W, C, Hp, Wp, Cp, padTop, padLeft);
+    launchOverlapped(padImageKernel, dim3(gridFor(words, kThreads, 8)), kThreads, 0, s, in, out, words, H, W, C, Hp, Wp, Cp, padTop, padLeft);
     return finish("padded copy");
 }
 
@@ -659,12 +667,14 @@ int transposeForMatmul(const int8_t *b, int8_t *bt, int32_t *corr, int batches, 
     cfg.gridDim = dim3(unsigned(columns * split), unsigned(batches));
     cfg.blockDim = dim3(256);
     cfg.stream = s;
-    cudaLaunchAttribute attr{};
-    attr.id = cudaLaunchAttributeClusterDimension;
-    attr.val.clusterDim.x = unsigned(split);
-    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
-    cfg.attrs = &attr;
-    cfg.numAttrs = 1;
+    cudaLaunchAttribute attrs[2]{};
+    attrs[0].id = cudaLaunchAttributeClusterDimension;
+    attrs[0].val.clusterDim.x = unsigned(split);
+    attrs[0].val.clusterDim.y = attrs[0].val.clusterDim.z = 1;
+    attrs[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attrs[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attrs;
+    cfg.numAttrs = dependentLaunches() ? 2 : 1;
     cudaLaunchKernelEx(&cfg, W % 16 == 0 ? transposeColsumKernel<true> : transposeColsumKernel<false>, b, bt, corr, C, W,
                        (C + 15) / 16 * 16, za, split);
     return finish("MATMUL operand transpose");
@@ -757,7 +767,7 @@ int maxPoolI8(const TView &in, const TView &out, const PoolAttr &a, cudaStream_t
     if (const int unit = poolUnit(in, out); unit < 16) {
         const int64_t words = int64_t(out.dims[0]) * out.dims[1] * out.dims[2] * (out.dims[3] / unsigned(unit));
         const auto kernel = unit == 4 ? maxPoolNarrowKernel<4> : maxPoolNarrowKernel<1>;
-        kernel<<<gridFor(words, kThreads, 16), kThreads, 0, s>>>(
+        launchOverlapped(kernel, dim3(gridFor(words, kThreads, 16)), kThreads, 0, s, 
             reinterpret_cast<const int8_t *>(in.ptr), reinterpret_cast<int8_t *>(out.ptr), uint32_t(words), int(in.dims[1]),
             int(in.dims[2]), int(in.dims[3]), makeFastDiv(out.dims[3] / unsigned(unit)), makeFastDiv(out.dims[2]),
             makeFastDiv(out.dims[1]), a);
@@ -765,19 +775,19 @@ int maxPoolI8(const TView &in, const TView &out, const PoolAttr &a, cudaStream_t
     }
     const int64_t total = int64_t(out.dims[0]) * out.dims[1] * out.dims[2] * (out.dims[3] >> 4);
     const auto launch = [&](auto kernel) {
-        kernel<<<gridFor(total, kThreads, 16), kThreads, 0, s>>>(
+        launchOverlapped(kernel, dim3(gridFor(total, kThreads, 16)), kThreads, 0, s, 
             reinterpret_cast<const int8_t *>(in.ptr), reinterpret_cast<int8_t *>(out.ptr), total, int(in.dims[1]),
             int(in.dims[2]), int(in.dims[3]), int(out.dims[1]), int(out.dims[2]), a);
     };
     if (a.kernel[0] == 3 && a.kernel[1] == 3 && a.stride[0] == 2 && a.stride[1] == 2 && out.dims[2] % 2 == 0 &&
         out.dims[1] % 2 == 0) {
         const int64_t quads = total / 4;
-        maxPool3x3s2QuadKernel<<<gridFor(quads, 128, 16), 128, 0, s>>>(
+        launchOverlapped(maxPool3x3s2QuadKernel, dim3(gridFor(quads, 128, 16)), 128, 0, s, 
             reinterpret_cast<const int8_t *>(in.ptr), reinterpret_cast<int8_t *>(out.ptr), quads, int(in.dims[1]),
             int(in.dims[2]), int(in.dims[3]), int(out.dims[1]), int(out.dims[2]), a.pad[0], a.pad[2]);
     } else if (a.kernel[0] == 3 && a.kernel[1] == 3 && a.stride[0] == 2 && a.stride[1] == 2 && out.dims[2] % 2 == 0) {
         const int64_t pairs = total / 2;
-        maxPool3x3s2PairKernel<<<gridFor(pairs, kThreads, 16), kThreads, 0, s>>>(
+        launchOverlapped(maxPool3x3s2PairKernel, dim3(gridFor(pairs, kThreads, 16)), kThreads, 0, s, 
             reinterpret_cast<const int8_t *>(in.ptr), reinterpret_cast<int8_t *>(out.ptr), pairs, int(in.dims[1]),
             int(in.dims[2]), int(in.dims[3]), int(out.dims[1]), int(out.dims[2]), a.pad[0], a.pad[2]);
     } else if (a.kernel[0] == 3 && a.kernel[1] == 3) {

@@ -15,6 +15,7 @@
 #include "device_common.cuh"
 #include "gemm_i8_tcgen05.hpp"
 #include "kernels.hpp"
+#include "launch_overlapped.cuh"
 
 namespace mlel {
 
@@ -48,6 +49,7 @@ struct RunMoves {
 
 // Four units per thread and step, all loads before the first store; blockIdx.y selects the part.
 template <typename UNIT> __global__ void __launch_bounds__(256) runMoveKernel(const __grid_constant__ RunMoves moves) {
+    dependencySync();
     const RunMove &m = moves.part[blockIdx.y];
     const uint32_t step = gridDim.x * blockDim.x;
     for (uint64_t first = blockIdx.x * blockDim.x + threadIdx.x; first < m.units; first += uint64_t(step) * 4) {
@@ -163,19 +165,19 @@ bool launchRunMoves(RunMove *parts, const int64_t *runs, const int64_t *bytes, i
     const dim3 grid(unsigned(gridFor((most + 3) / 4, kThreads, 16)), unsigned(count));
     switch (unit) {
     case 16:
-        runMoveKernel<uint4><<<grid, kThreads, 0, s>>>(moves);
+        launchOverlapped(runMoveKernel<uint4>, dim3(grid), kThreads, 0, s, moves);
         break;
     case 8:
-        runMoveKernel<uint2><<<grid, kThreads, 0, s>>>(moves);
+        launchOverlapped(runMoveKernel<uint2>, dim3(grid), kThreads, 0, s, moves);
         break;
     case 4:
-        runMoveKernel<uint32_t><<<grid, kThreads, 0, s>>>(moves);
+        launchOverlapped(runMoveKernel<uint32_t>, dim3(grid), kThreads, 0, s, moves);
         break;
     case 2:
-        runMoveKernel<uint16_t><<<grid, kThreads, 0, s>>>(moves);
+        launchOverlapped(runMoveKernel<uint16_t>, dim3(grid), kThreads, 0, s, moves);
         break;
     default:
-        runMoveKernel<uint8_t><<<grid, kThreads, 0, s>>>(moves);
+        launchOverlapped(runMoveKernel<uint8_t>, dim3(grid), kThreads, 0, s, moves);
         break;
     }
     *rc = finish(what);
@@ -211,6 +213,7 @@ struct TileTranspose {
 template <typename T>
 __global__ void __launch_bounds__(256) tileTransposeKernel(const uint8_t *__restrict__ in, uint8_t *__restrict__ out,
                                                            uint32_t tiles, const __grid_constant__ TileTranspose p) {
+    dependencySync();
     constexpr int kPitch = 64 * int(sizeof(T)) + 4;
     __shared__ __align__(16) uint8_t tile[64 * kPitch];
     const int x = threadIdx.x & 63, y0 = threadIdx.x >> 6;
@@ -274,6 +277,7 @@ template <typename UNIT>
 __global__ void __launch_bounds__(256)
     resizeNearestKernel(const uint8_t *__restrict__ in, uint8_t *__restrict__ out, uint32_t units, FastDiv perPixel, FastDiv divOW,
                         FastDiv divOH, uint32_t H, uint32_t W, ResizeAttr a) {
+    dependencySync();
     const uint32_t step = gridDim.x * blockDim.x;
     for (uint32_t e = blockIdx.x * blockDim.x + threadIdx.x; e < units; e += step) {
         const uint32_t pixel = fastDiv(e, perPixel), u = e - pixel * perPixel.d;
@@ -301,6 +305,7 @@ constexpr int kArgmaxStage = 128;
 template <typename T>
 __global__ void __launch_bounds__(256)
     argmaxShortKernel(const T *__restrict__ in, int32_t *__restrict__ out, int64_t rows, int len, int32_t lowest) {
+    dependencySync();
     __shared__ __align__(16) uint8_t stage[256 * kArgmaxStage];
     const int64_t total = rows * len * int64_t(sizeof(T));
     for (int64_t row0 = int64_t(blockIdx.x) * 256; row0 < rows; row0 += int64_t(gridDim.x) * 256) {
@@ -333,6 +338,7 @@ __global__ void __launch_bounds__(256)
 template <typename T>
 __global__ void __launch_bounds__(256)
     argmaxLongKernel(const T *__restrict__ in, int32_t *__restrict__ out, int64_t rows, int len, int32_t lowest) {
+    dependencySync();
     const int lane = threadIdx.x & 31;
     const int64_t warps = (int64_t(gridDim.x) * blockDim.x) >> 5;
     for (int64_t row = (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5; row < rows; row += warps) {
@@ -365,9 +371,9 @@ int launchArgmax(const TView &in, const TView &out, int64_t rows, int len, cudaS
     int32_t *po = reinterpret_cast<int32_t *>(out.ptr);
     const int32_t lowest = int32_t(typeLowest(in.dtype));
     if (len * int(sizeof(T)) <= kArgmaxStage) {
-        argmaxShortKernel<T><<<gridFor(rows, 256, 16), 256, 0, s>>>(pi, po, rows, len, lowest);
+        launchOverlapped(argmaxShortKernel<T>, dim3(gridFor(rows, 256, 16)), 256, 0, s, pi, po, rows, len, lowest);
     } else {
-        argmaxLongKernel<T><<<gridFor(rows * 32, 256, 16), 256, 0, s>>>(pi, po, rows, len, lowest);
+        launchOverlapped(argmaxLongKernel<T>, dim3(gridFor(rows * 32, 256, 16)), 256, 0, s, pi, po, rows, len, lowest);
     }
     return finish("ARGMAX");
 }
@@ -438,11 +444,11 @@ bool moveTranspose(const TView &in, const TView &out, const uint32_t *perms, cud
             const auto *pi = reinterpret_cast<const uint8_t *>(in.ptr);
             auto *po = reinterpret_cast<uint8_t *>(out.ptr);
             if (elem == 1) {
-                tileTransposeKernel<uint8_t><<<grid, 256, 0, s>>>(pi, po, uint32_t(tiles), p);
+                launchOverlapped(tileTransposeKernel<uint8_t>, dim3(grid), 256, 0, s, pi, po, uint32_t(tiles), p);
             } else if (elem == 2) {
-                tileTransposeKernel<uint16_t><<<grid, 256, 0, s>>>(pi, po, uint32_t(tiles), p);
+                launchOverlapped(tileTransposeKernel<uint16_t>, dim3(grid), 256, 0, s, pi, po, uint32_t(tiles), p);
             } else {
-                tileTransposeKernel<uint32_t><<<grid, 256, 0, s>>>(pi, po, uint32_t(tiles), p);
+                launchOverlapped(tileTransposeKernel<uint32_t>, dim3(grid), 256, 0, s, pi, po, uint32_t(tiles), p);
             }
             *rc = finish("TRANSPOSE");
             return true;
@@ -561,9 +567,8 @@ bool moveResizeNearest(const TView &in, const TView &out, const ResizeAttr &a, c
     const int grid = gridFor(units, kThreads, 16);
     const FastDiv perPixel = makeFastDiv(pixelBytes / unit), divOW = makeFastDiv(out.dims[2]), divOH = makeFastDiv(out.dims[1]);
     const auto launch = [&](auto tag) {
-        resizeNearestKernel<decltype(tag)><<<grid, kThreads, 0, s>>>(reinterpret_cast<const uint8_t *>(in.ptr),
-                                                                    reinterpret_cast<uint8_t *>(out.ptr), uint32_t(units),
-                                                                    perPixel, divOW, divOH, in.dims[1], in.dims[2], a);
+        launchOverlapped(resizeNearestKernel<decltype(tag)>, dim3(grid), kThreads, 0, s, reinterpret_cast<const uint8_t *>(in.ptr),
+                         reinterpret_cast<uint8_t *>(out.ptr), uint32_t(units), perPixel, divOW, divOH, in.dims[1], in.dims[2], a);
     };
     switch (unit) {
     case 16:
