@@ -671,10 +671,13 @@ int transposeForMatmul(const int8_t *b, int8_t *bt, int32_t *corr, int batches, 
     attrs[0].id = cudaLaunchAttributeClusterDimension;
     attrs[0].val.clusterDim.x = unsigned(split);
     attrs[0].val.clusterDim.y = attrs[0].val.clusterDim.z = 1;
+    // A small operand's transpose as a dependent launch (5 x 128 x 160 x 48 8.2 -> 6.5 us a pass).  A large one's blocks would settle
+    // beside the product of the pass before, whose shared memory leaves them little of the cache that their loads in flight
+    // need (45 x 45 x 864 x 298 24.6 -> 37 us, 6 x 213 x 512 x 570 12.3 -> 16.3).
     attrs[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attrs[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attrs;
-    cfg.numAttrs = dependentLaunches() ? 2 : 1;
+    cfg.numAttrs = dependentLaunches() && int64_t(batches) * C * W <= int64_t(1) << 18 ? 2 : 1;
     cudaLaunchKernelEx(&cfg, W % 16 == 0 ? transposeColsumKernel<true> : transposeColsumKernel<false>, b, bt, corr, C, W,
                        (C + 15) / 16 * 16, za, split);
     return finish("MATMUL operand transpose");

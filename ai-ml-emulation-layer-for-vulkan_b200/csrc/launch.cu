@@ -362,9 +362,21 @@ int launchMatmul(const OpDesc &op, const TView *T, cudaStream_t s) {
 void setLastError(const std::string &msg) { g_lastError = msg; }
 const std::string &lastError() { return g_lastError; }
 
-bool overlappingProduct(const OpDesc &op, const TView *T) {
-    return op.kind == OP_FUSED_MATMUL && op.tc == 3 && op.epi.tableTensor < 0 && T[op.in[0]].dims[2] % 16 == 0 &&
-           matmulOnTensorCores(op, T) && pairTakesActivations(matmulProblem(op, T));
+int contractionLaunches(const OpDesc &op, const TView *T) {
+    switch (op.kind) {
+    case OP_CONV2D:
+    case OP_FUSED_CONV2D:
+        return op.tc == 2 || op.tc == 4 ? 2 : 1; // a copy of the input first
+    case OP_MATMUL:
+    case OP_FUSED_MATMUL:
+        if (!matmulOnTensorCores(op, T)) {
+            return op.epi.tableTensor >= 0 ? 2 : 1;
+        }
+        // copied rows, column sums or a transposed copy, the product, a table behind it
+        return 1 + (T[op.in[0]].dims[2] % 16 != 0 ? 1 : 0) + (op.tc == 3 ? 1 : 0) + (op.epi.tableTensor >= 0 ? 1 : 0);
+    default:
+        return 1;
+    }
 }
 
 int launchOp(const OpDesc &op, const TView *T, cudaStream_t s, LaunchChain *chain) {

@@ -269,9 +269,8 @@ struct OpDesc {
 struct LaunchChain; // kernels/gemm_i8_tcgen05.hpp: tile-level hand-over between consecutive tensor-core launches
 int launchOp(const OpDesc &op, const TView *tensors, cudaStream_t stream, LaunchChain *chain = nullptr);
 
-// Whether launchOp() enqueues `op` as the column sums and the paired kernel of a product of two activations, which overlap,
-// and nothing else.
-bool overlappingProduct(const OpDesc &op, const TView *tensors);
+// Kernels that launchOp() enqueues for a convolution or a product (at most).
+int contractionLaunches(const OpDesc &op, const TView *tensors);
 
 void setLastError(const std::string &msg);
 int elemSize(int32_t dtype);

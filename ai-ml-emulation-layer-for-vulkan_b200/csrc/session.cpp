@@ -682,18 +682,14 @@ int Session::dispatchGraph(cudaStream_t stream) {
     if (rc != MLEL_SUCCESS) {
         return rc;
     }
-    // One kernel is enqueued quicker than a graph of one node is launched: back to back 6.6 against 10.3 us for a small
-    // convolution, the host having 5.3 and 1.8 us to do.
-    // So are the two of a product of two activations on the paired kernel, which overlap (as a graph 10.3, enqueued 8.1 us
-    // for 4 x 512^3; 38.1 and 32.9 for 16 x 1024^3 out of memory), from 2^24 products on: below that the device would wait
-    // for the host.  Copies and transposes in front of a contraction do not overlap with it, and three launches (a TABLE
-    // behind the product is the third) cost the host more than a replay.
+    // One or two kernels are enqueued quicker than a graph of them is launched: back to back 5.4 against 8.2 us for a small
+    // convolution, 6.4 against 8.2 for one with a padded copy, 5.6 against 8.2 and 10.3 against 12.3 for products of two
+    // activations -- a replay begins on a whole number of 2.048 us (see launch_overlapped.cuh), launches behind one another do not.
+    // Three (copied rows or a TABLE besides) cost the host more than a replay: 7.7 against 6.2 us for a small product.
     const auto &exec = pipeline_->getExecList();
     if (exec.size() == 1) {
         const OpDesc &op = exec[0];
-        if (op.scratch < 0 ||
-            (overlappingProduct(op, views_.data()) &&
-             pipeline_->tensor(op.in[0]).numel() * pipeline_->tensor(op.in[1]).dims.back() >= int64_t(1) << 24)) {
+        if (op.scratch < 0 || contractionLaunches(op, views_.data()) <= 2) {
             return dispatch(stream);
         }
         // (a stream that is being captured takes kernels, not the launch of a graph)
