@@ -38,6 +38,7 @@
 #include "kernels/depthwise_i8.hpp"
 #include "kernels/device_common.cuh"
 #include "kernels/gemm_i8_tcgen05.hpp"
+#include "kernels/nearest_source.hpp"
 
 #include <cuda_runtime.h>
 
@@ -2131,6 +2132,119 @@ void GraphPipeline::prepareDepthwise() {
     }
 }
 
+// CONCAT along the channels with inputs that are RESIZE (NEAREST), or a SLICE of one, of a smaller tensor -> OP_FUSED_CONCAT.
+// The elided tensors are session memory, written once and read once.
+void GraphPipeline::fuseResizedConcats() {
+    std::map<int32_t, int> writer, readers;
+    for (size_t k = 0; k < exec_.size(); ++k) {
+        for (const int32_t t : exec_[k].out) {
+            writer[t] = writer.count(t) ? -1 : int(k); // (-1: written more than once)
+        }
+        for (const int32_t t : exec_[k].in) {
+            ++readers[t];
+        }
+        ++readers[exec_[k].epi.shortcutTensor];
+    }
+    for (const int32_t t : outputs_) {
+        ++readers[t];
+    }
+    std::vector<bool> gone(exec_.size(), false);
+    // the operator that makes t, if t is no more than a step on the way to its one reader
+    const auto stepOf = [&](int32_t t, OpKind kind) -> int {
+        const auto w = writer.find(t);
+        if (w == writer.end() || w->second < 0 || readers[t] != 1 || tensor(t).cls != TensorClass::Session || !tensor(t).packed()) {
+            return -1;
+        }
+        const OpDesc &op = exec_[size_t(w->second)];
+        return op.kind == kind && op.out.size() == 1 && !gone[size_t(w->second)] ? w->second : -1;
+    };
+    for (size_t c = 0; c < exec_.size(); ++c) {
+        OpDesc &op = exec_[c];
+        if (op.kind != OP_CONCAT || op.in.size() > size_t(kMaxResizedConcatInputs)) {
+            continue;
+        }
+        const TensorDescriptor &out = tensor(op.out[0]);
+        if (out.rank() != 4 || op.i[0] != 3 || !out.packed() || out.sizeBytes() == 0 || out.sizeBytes() >= (uint64_t(1) << 31)) {
+            continue;
+        }
+        auto plan = std::make_shared<ResizedConcat>();
+        std::vector<int32_t> sources, steps;
+        std::vector<std::vector<int32_t>> tables;
+        int64_t channels = 0;
+        bool fits = true;
+        for (size_t k = 0; k < op.in.size() && fits; ++k) {
+            const TensorDescriptor &in = tensor(op.in[k]);
+            fits = in.packed() && in.dtype == out.dtype && op.i[1 + k] == channels && in.dims[0] == out.dims[0] && in.dims[1] == out.dims[1] &&
+                   in.dims[2] == out.dims[2];
+            channels += in.dims[3];
+            plan->firstChannel.push_back(op.i[1 + k]);
+            int32_t source = op.in[k];
+            int64_t startY = 0, startX = 0;
+            const int slice = stepOf(source, OP_SLICE);
+            if (slice >= 0) {
+                const OpDesc &cut = exec_[size_t(slice)];
+                const TensorDescriptor &whole = tensor(cut.in[0]);
+                startY = cut.i[1], startX = cut.i[2];
+                if (cut.i[0] == 0 && cut.i[3] == 0 && whole.dims[0] == in.dims[0] && whole.dims[3] == in.dims[3] && startY >= 0 && startX >= 0 &&
+                    startY + in.dims[1] <= whole.dims[1] && startX + in.dims[2] <= whole.dims[2]) {
+                    source = cut.in[0];
+                }
+            }
+            const int resize = slice < 0 || source != op.in[k] ? stepOf(source, OP_RESIZE) : -1;
+            std::vector<int32_t> table;
+            if (resize >= 0) {
+                const OpDesc &r = exec_[size_t(resize)];
+                const TensorDescriptor &small = tensor(r.in[0]);
+                if (r.i[8] == 1 && small.dtype == in.dtype && small.packed() && small.dims[0] == in.dims[0] && small.dims[3] == in.dims[3] &&
+                    r.i[0] > 0 && r.i[2] > 0) {
+                    for (int64_t y = 0; y < in.dims[1]; ++y) {
+                        const uint32_t from = nearestSource(uint32_t(y + startY), r.i[0], r.i[1], r.i[4], uint32_t(small.dims[1]));
+                        table.push_back(from < uint32_t(small.dims[1]) ? int32_t(from) : -1);
+                    }
+                    for (int64_t x = 0; x < in.dims[2]; ++x) {
+                        const uint32_t from = nearestSource(uint32_t(x + startX), r.i[2], r.i[3], r.i[5], uint32_t(small.dims[2]));
+                        table.push_back(from < uint32_t(small.dims[2]) ? int32_t(from) : -1);
+                    }
+                    if (source != op.in[k]) {
+                        steps.push_back(slice);
+                    }
+                    steps.push_back(resize);
+                    source = r.in[0];
+                }
+            }
+            sources.push_back(table.empty() ? op.in[k] : source);
+            tables.push_back(std::move(table));
+        }
+        if (!fits || steps.empty() || channels != out.dims[3]) {
+            continue;
+        }
+        for (const auto &table : tables) {
+            plan->sources.push_back(table.empty() ? -1 : addDerivedConstant(MLEL_I32, {int64_t(table.size())}, table.data()));
+        }
+        std::string name;
+        for (const int32_t step : steps) {
+            gone[size_t(step)] = true;
+            name += exec_[size_t(step)].name + "+";
+            op.fusedOps.insert(op.fusedOps.end(), exec_[size_t(step)].fusedOps.begin(), exec_[size_t(step)].fusedOps.end());
+        }
+        std::sort(op.fusedOps.begin(), op.fusedOps.end());
+        op.kind = OP_FUSED_CONCAT;
+        op.name = name + op.name;
+        op.in = sources;
+        op.concat = plan;
+    }
+    size_t kept = 0;
+    for (size_t k = 0; k < exec_.size(); ++k) {
+        if (!gone[k]) {
+            if (kept != k) {
+                exec_[kept] = std::move(exec_[k]);
+            }
+            ++kept;
+        }
+    }
+    exec_.resize(kept);
+}
+
 const std::vector<OpDesc> &GraphPipeline::getExecList() {
     finalize();
     return exec_;
@@ -2141,6 +2255,9 @@ void GraphPipeline::finalize() {
         return;
     }
     fuse();
+    if (!(flags_ & MLEL_PIPELINE_NO_FUSION)) {
+        fuseResizedConcats();
+    }
     if (!(flags_ & MLEL_PIPELINE_NO_TENSOR_CORE)) {
         prepareTensorCore();
     }

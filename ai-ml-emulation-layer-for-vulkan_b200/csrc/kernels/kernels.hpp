@@ -96,6 +96,8 @@ bool moveSlice(const TView &in, const TView &out, const uint32_t *start, cudaStr
 bool moveTile(const TView &in, const TView &out, cudaStream_t s, int *rc);
 bool moveReverse(const TView &in, const TView &out, uint32_t axis, cudaStream_t s, int *rc);
 bool moveResizeNearest(const TView &in, const TView &out, const ResizeAttr &a, cudaStream_t s, int *rc);
+// OP_FUSED_CONCAT; `tensors`: where the plan's tables are.
+int concatResized(const ResizedConcat &plan, const TView *const *ins, int count, const TView *tensors, const TView &out, cudaStream_t s);
 bool moveArgmaxLast(const TView &in, const TView &out, uint32_t axis, cudaStream_t s, int *rc);
 
 // Joins column blocks of byte rows: out[row][first[g] + j] = staging[(g * rows + row) * pitch + j], j < count[g].

@@ -15,6 +15,7 @@
 #include "device_common.cuh"
 #include "gemm_i8_tcgen05.hpp"
 #include "kernels.hpp"
+#include "nearest_source.hpp"
 #include "launch_overlapped.cuh"
 
 namespace mlel {
@@ -254,25 +255,6 @@ __global__ void __launch_bounds__(256) tileTransposeKernel(const uint8_t *__rest
 }
 
 // ---- RESIZE, NEAREST (resize.comp:43-134): one source pixel per output pixel, its channels moved as units ---------
-__device__ inline int32_t floorDiv(int32_t n, int32_t d) {
-    int32_t r = n / d;
-    if (r * d > n) {
-        --r;
-    }
-    return r;
-}
-
-// Source coordinate along one axis with the shader's 16-bit positions; `pos` is the output coordinate.
-__device__ __forceinline__ uint32_t nearestSource(uint32_t pos, int32_t n, int32_t d, int32_t offset, uint32_t size) {
-    const int32_t y = int32_t(pos * uint32_t(d) + uint32_t(offset));
-    const int16_t i = int16_t(floorDiv(y, n));
-    const int16_t frac = int16_t(uint32_t(y) - uint32_t(int32_t(i)) * uint32_t(n));
-    const int16_t i0 = int16_t(i > 0 ? i : 0);
-    const uint32_t next = uint32_t(int32_t(i) + 1);
-    const int16_t i1 = int16_t(next < size - 1 ? next : size - 1);
-    return uint32_t(int32_t((2 * int32_t(frac) >= n) ? i1 : i0));
-}
-
 template <typename UNIT>
 __global__ void __launch_bounds__(256)
     resizeNearestKernel(const uint8_t *__restrict__ in, uint8_t *__restrict__ out, uint32_t units, FastDiv perPixel, FastDiv divOW,
@@ -292,6 +274,66 @@ __global__ void __launch_bounds__(256)
         reinterpret_cast<UNIT *>(out)[e] = v;
         if (units - e <= step) {
             break; // e + step could wrap
+        }
+    }
+}
+
+// ---- CONCAT along the channels of tensors that are enlarged on the way (OP_FUSED_CONCAT) -----------------------------
+// The joined tensor is written once and its sources are read where they lie; as RESIZE, SLICE and CONCAT the enlarged tensor went
+// to memory and back twice (270 x 480, 64 channels of 135 x 240 beside 32: three launches of 2.5 to 4.7 us).  Where a pixel comes
+// from is a table of rows and one of columns, made by the host: the shader's divisions per unit were most of RESIZE's time.
+struct ConcatPart {
+    const uint8_t *src;
+    const int32_t *rows, *columns; // or null: the pixel itself
+    uint32_t begin, units;         // units of a pixel of the result, first and count
+    uint32_t H, W;
+};
+struct ConcatParts {
+    ConcatPart part[kMaxResizedConcatInputs];
+    uint32_t units; // of the result
+    FastDiv perPixel, divOW, divOH;
+};
+
+template <typename UNIT>
+__global__ void __launch_bounds__(256) concatResizedKernel(uint8_t *__restrict__ out, const __grid_constant__ ConcatParts p) {
+    dependencySync();
+    const uint32_t step = gridDim.x * blockDim.x;
+    for (uint64_t first = blockIdx.x * blockDim.x + threadIdx.x; first < p.units; first += uint64_t(step) * 4) {
+        UNIT v[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const uint64_t at = first + uint64_t(j) * step;
+            v[j] = UNIT{};
+            if (at < p.units) {
+                const uint32_t e = uint32_t(at), pixel = fastDiv(e, p.perPixel), u = e - pixel * p.perPixel.d;
+                const uint8_t *src = p.part[0].src;
+                const int32_t *rows = p.part[0].rows, *columns = p.part[0].columns;
+                uint32_t begin = 0, units = p.part[0].units, H = p.part[0].H, W = p.part[0].W;
+#pragma unroll
+                for (int k = 1; k < kMaxResizedConcatInputs; ++k) {
+                    if (p.part[k].units != 0 && u >= p.part[k].begin) {
+                        src = p.part[k].src, rows = p.part[k].rows, columns = p.part[k].columns;
+                        begin = p.part[k].begin, units = p.part[k].units, H = p.part[k].H, W = p.part[k].W;
+                    }
+                }
+                int64_t from = pixel;
+                if (rows != nullptr) {
+                    const uint32_t line = fastDiv(pixel, p.divOW), ox = pixel - line * p.divOW.d;
+                    const uint32_t n = fastDiv(line, p.divOH), oy = line - n * p.divOH.d;
+                    const int32_t y = __ldg(rows + oy), x = __ldg(columns + ox);
+                    from = (y | x) < 0 ? -1 : (int64_t(n) * H + y) * W + x;
+                }
+                if (from >= 0) {
+                    v[j] = __ldg(reinterpret_cast<const UNIT *>(src) + from * units + (u - begin));
+                }
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const uint64_t at = first + uint64_t(j) * step;
+            if (at < p.units) {
+                reinterpret_cast<UNIT *>(out)[at] = v[j];
+            }
         }
     }
 }
@@ -546,6 +588,52 @@ bool moveReverse(const TView &in, const TView &out, uint32_t axis, cudaStream_t 
     }
     return moveOne(a, dtypeSize(out.dtype), in.ptr + int64_t(in.dims[axis] - 1) * in.strides[axis], out.ptr, numelOf(out),
                    "REVERSE", s, rc);
+}
+
+int concatResized(const ResizedConcat &plan, const TView *const *ins, int count, const TView *tensors, const TView &out, cudaStream_t s) {
+    const int64_t elem = dtypeSize(out.dtype), pixels = int64_t(out.dims[0]) * out.dims[1] * out.dims[2], pixelBytes = int64_t(out.dims[3]) * elem;
+    uint64_t bits = uint64_t(pixelBytes) | reinterpret_cast<uintptr_t>(out.ptr);
+    for (int k = 0; k < count; ++k) {
+        bits |= uint64_t(ins[k]->dims[3]) * uint64_t(elem) | reinterpret_cast<uintptr_t>(ins[k]->ptr);
+    }
+    int64_t unit = 16;
+    while ((bits & uint64_t(unit - 1)) != 0) {
+        unit >>= 1;
+    }
+    ConcatParts p{};
+    for (int k = 0; k < count; ++k) {
+        ConcatPart &part = p.part[k];
+        part.src = reinterpret_cast<const uint8_t *>(ins[k]->ptr);
+        part.begin = uint32_t(plan.firstChannel[size_t(k)] * elem / unit), part.units = uint32_t(ins[k]->dims[3] * elem / unit);
+        part.H = ins[k]->dims[1], part.W = ins[k]->dims[2];
+        if (plan.sources[size_t(k)] >= 0) {
+            part.rows = reinterpret_cast<const int32_t *>(tensors[plan.sources[size_t(k)]].ptr);
+            part.columns = part.rows + out.dims[1];
+        }
+    }
+    p.units = uint32_t(pixels * pixelBytes / unit); // (below 2^31: GraphPipeline::fuseResizedConcats)
+    p.perPixel = makeFastDiv(pixelBytes / unit), p.divOW = makeFastDiv(out.dims[2]), p.divOH = makeFastDiv(out.dims[1]);
+    const dim3 grid(unsigned(gridFor((int64_t(p.units) + 3) / 4, kThreads, 16)));
+    uint8_t *to = reinterpret_cast<uint8_t *>(out.ptr);
+    const auto launch = [&](auto tag) { launchOverlapped(concatResizedKernel<decltype(tag)>, grid, kThreads, 0, s, to, p); };
+    switch (unit) {
+    case 16:
+        launch(uint4{});
+        break;
+    case 8:
+        launch(uint2{});
+        break;
+    case 4:
+        launch(uint32_t{});
+        break;
+    case 2:
+        launch(uint16_t{});
+        break;
+    default:
+        launch(uint8_t{});
+        break;
+    }
+    return finish("RESIZE+CONCAT");
 }
 
 bool moveResizeNearest(const TView &in, const TView &out, const ResizeAttr &a, cudaStream_t s, int *rc) {

@@ -594,6 +594,13 @@ int launchOp(const OpDesc &op, const TView *T, cudaStream_t s, LaunchChain *chai
         return mulRescaleFused(in(0), in(1), out, uint32_t(op.i[0]), devRescale(op.epi.main, T), s);
     case OP_FUSED_ATTENTION:
         return attentionFused(*op.attention, in(0), in(1), in(2), in(3), in(4), out, s);
+    case OP_FUSED_CONCAT: {
+        const TView *ins[kMaxResizedConcatInputs];
+        for (size_t k = 0; k < op.in.size(); ++k) {
+            ins[k] = &in(k);
+        }
+        return concatResized(*op.concat, ins, int(op.in.size()), T, out, s);
+    }
     case OP_FUSED_ADD:
         return fusedAdd(reinterpret_cast<const int8_t *>(in(0).ptr), reinterpret_cast<const int8_t *>(in(1).ptr),
                         reinterpret_cast<int8_t *>(out.ptr), numelOf(out), devEpilogue(op.epi, T), s);

@@ -77,6 +77,9 @@ enum OpKind : int32_t {
     // Score MATMUL, row-wise softmax and context MATMUL of a quantised attention, head split and merge included.
     // in = {q, k, v, exponential table, reciprocal table}, out = {context}: see AttentionPlan.
     OP_FUSED_ATTENTION,
+    // CONCAT along the channels of NHWC tensors, some of which are a RESIZE (NEAREST) of another, cut by a SLICE or not: the
+    // enlarged tensors are read where their pixels come from.  in = the tensors read, out = {result}: see ResizedConcat.
+    OP_FUSED_CONCAT,
     OP_KIND_COUNT
 };
 
@@ -227,6 +230,12 @@ struct RowProgram {
     int64_t rows{0};
     int32_t len{0};
 };
+// OP_FUSED_CONCAT, per input: its first channel in the result, and the constant tensor of its source rows [OH] and columns [OW]
+// (int32, -1: outside the image, reads zero), or -1 for an input that has the result's own size.
+constexpr int kMaxResizedConcatInputs = 4;
+struct ResizedConcat {
+    std::vector<int32_t> firstChannel, sources;
+};
 struct AttentionPlan; // kernels/attention_i8.hpp
 constexpr int kMaxConcatPasses = 16; // consecutive CONCAT passes into one tensor that a node can hold
 constexpr int kMaxRowInsts = 40, kMaxRowValues = 16;
@@ -243,6 +252,7 @@ struct OpDesc {
     std::vector<int32_t> fusedOps;  // indices of the logical ops an exec node stands for
     std::shared_ptr<RowProgram> rows; // OP_FUSED_ROWS only
     std::shared_ptr<AttentionPlan> attention; // OP_FUSED_ATTENTION only
+    std::shared_ptr<ResizedConcat> concat; // OP_FUSED_CONCAT only
     // Tensor-core path (set by GraphPipeline::prepareTensorCore when the node qualifies):
     //   CONV2D kinds: aux[0] correction table int32 [classes][OC], aux[1] row classes u8 [OH],
     //                 aux[2] column classes u8 [OW]; auxi[0] = number of column classes, auxi[1] = classes,
