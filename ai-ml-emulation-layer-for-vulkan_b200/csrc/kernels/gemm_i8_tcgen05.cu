@@ -66,6 +66,12 @@ struct __align__(8) PipeBarriers {
 constexpr int kAGather = 0, kATiled = 1, kAIm2col = 2;
 constexpr int kMaxGatherPieces = 1024; // entries of the shared-memory copy of GemmI8Params::gatherTable
 
+// A residual tail's input RESCALEs, of every main-stage value (index value + 128) and of every shortcut byte: made once by each CTA,
+// so that an element takes two look-ups and one RESCALE instead of three.
+struct TailInputs {
+    int32_t main[256], shortcut[256];
+};
+
 struct TileCoord {
     int m0, n0, batch;
 };
@@ -109,7 +115,7 @@ __device__ __forceinline__ void storeRun(int8_t *to, const uint32_t *words, int 
 template <int BN, int NSTAGE, bool RESIDUAL, bool ROWS16, bool GATHER>
 __device__ __forceinline__ void epilogueInt8(const GemmI8Params &p, PipeBarriers *bars, ColConst *colTab,
                                              uint32_t tmemBase, int warp, int lane, int64_t numTiles, int mTiles,
-                                             int nTiles, uint32_t *rows8) {
+                                             int nTiles, uint32_t *rows8, const TailInputs *tail) {
     const int quarter = warp & 3; // TMEM lanes [32 * quarter, 32 * quarter + 32)
     const int half = warp >> 2;   // which half of the tile's columns
     constexpr int kColsPerWarp = BN / (kEpilogueWarps / 4);
@@ -117,10 +123,9 @@ __device__ __forceinline__ void epilogueInt8(const GemmI8Params &p, PipeBarriers
     const int row = quarter * 32 + lane;
     bool failed = false;
     uint32_t *rows = rows8 + quarter * (32 * kRowPitchWords<BN>); // !ROWS16: this quarter's rows
-    FastRescale fa{}, fb{}, fo{};
+    FastRescale fo{};
+    const uint32_t tailMain = smemAddr(tail->main) + 128u * 4u, tailShortcut = smemAddr(tail->shortcut);
     if (RESIDUAL) {
-        fa = makeFastRescale(__ldg(p.epi.a.mult), int32_t(__ldg(p.epi.a.shift)), p.epi.a.inZp, p.epi.a.doubleRound != 0);
-        fb = makeFastRescale(__ldg(p.epi.b.mult), int32_t(__ldg(p.epi.b.shift)), p.epi.b.inZp, p.epi.b.doubleRound != 0);
         fo = makeFastRescale(__ldg(p.epi.out.mult), int32_t(__ldg(p.epi.out.shift)), p.epi.out.inZp,
                              p.epi.out.doubleRound != 0);
     }
@@ -267,9 +272,8 @@ __device__ __forceinline__ void epilogueInt8(const GemmI8Params &p, PipeBarriers
                         }
                         int32_t r = min(__viaddmax_s32(q32 >> s2, outZpMain, loMain), hiMain);
                         if (RESIDUAL) {
-                            const int32_t ta = fastRescale(fa, r, p.epi.a.outZp, p.epi.a.lo, p.epi.a.hi);
-                            const int32_t sv = int32_t(int8_t(sc[q] >> (8 * e)));
-                            const int32_t tb = fastRescale(fb, sv, p.epi.b.outZp, p.epi.b.lo, p.epi.b.hi);
+                            const int32_t ta = ldsS32(tailMain + uint32_t(4 * int32_t(int8_t(r))));
+                            const int32_t tb = ldsS32(tailShortcut + 4u * ((sc[q] >> (8 * e)) & 0xffu));
                             r = fastRescale(fo, int32_t(uint32_t(ta) + uint32_t(tb)), p.epi.out.outZp, p.epi.out.lo,
                                             p.epi.out.hi);
                         }
@@ -433,20 +437,24 @@ __device__ __forceinline__ void epilogueInt32(const GemmI8Params &p, PipeBarrier
     }
 }
 
-template <int BN, int NSTAGE, bool ROWS16, bool GATHER>
+// What leaves the kernel: the raw sums, int8 results, int8 results with a residual tail (an instantiation each: together in one
+// kernel their registers spilled).
+enum : int { kOutInt32 = 0, kOutInt8 = 1, kOutTail = 2 };
+
+template <int BN, int NSTAGE, bool ROWS16, bool GATHER, int OUT>
 __device__ __forceinline__ void epilogueWarps(const GemmI8Params &p, PipeBarriers *bars, ColConst *colTab,
                                               uint32_t tmemBase, int warp, int lane, int64_t numTiles, int mTiles,
-                                              int nTiles, int32_t *staging, uint32_t *rows8) {
-    if (p.out32 != nullptr) {
+                                              int nTiles, int32_t *staging, uint32_t *rows8, const TailInputs *tail) {
+    if (OUT == kOutInt32) {
         // the staged stores need 16-byte aligned rows
         const bool staged = staging != nullptr && p.ldOut % 4 == 0 && (reinterpret_cast<uintptr_t>(p.out32) & 15u) == 0;
         epilogueInt32<BN, NSTAGE>(p, bars, tmemBase, warp, lane, numTiles, mTiles, nTiles, staged ? staging : nullptr);
         return;
     }
-    if (p.epi.hasResidual) {
-        epilogueInt8<BN, NSTAGE, true, ROWS16, GATHER>(p, bars, colTab, tmemBase, warp, lane, numTiles, mTiles, nTiles, rows8);
+    if (OUT == kOutTail) {
+        epilogueInt8<BN, NSTAGE, true, ROWS16, GATHER>(p, bars, colTab, tmemBase, warp, lane, numTiles, mTiles, nTiles, rows8, tail);
     } else {
-        epilogueInt8<BN, NSTAGE, false, ROWS16, GATHER>(p, bars, colTab, tmemBase, warp, lane, numTiles, mTiles, nTiles, rows8);
+        epilogueInt8<BN, NSTAGE, false, ROWS16, GATHER>(p, bars, colTab, tmemBase, warp, lane, numTiles, mTiles, nTiles, rows8, tail);
     }
 }
 
@@ -486,7 +494,7 @@ __device__ __forceinline__ void gatherPieces(const int8_t *origin, const int32_t
 // STAGE32: shared memory for the staged int32 stores of epilogueInt32 is set aside (see there).
 // ROWS16: see epilogueInt8 (a kernel of its own: in one kernel the two forms' registers spilled, 64 images of the
 // ResNet-50 shape 970 -> 1003 us).
-template <int BN, int NSTAGE, int A_MODE, bool B_MN, bool STAGE32 = false, bool ROWS16 = true>
+template <int BN, int NSTAGE, int A_MODE, bool B_MN, bool STAGE32, bool ROWS16, int OUT>
 __global__ void __launch_bounds__(A_MODE != kAGather ? kThreadsTma : kThreadsGather, 1)
 gemmI8Tcgen05(const __grid_constant__ CUtensorMap tmapA, const __grid_constant__ CUtensorMap tmapB, const GemmI8Params p) {
     constexpr bool A_TMA = A_MODE != kAGather;
@@ -508,6 +516,7 @@ gemmI8Tcgen05(const __grid_constant__ CUtensorMap tmapA, const __grid_constant__
     // the int8 epilogue's staging comes last
     uint32_t *rows8 = reinterpret_cast<uint32_t *>(gatherTab) +
                       (A_TMA ? (STAGE32 ? kEpilogueWarps * kStageBytesPerWarp / 4 : 0) : kMaxGatherPieces + kTapTabEntries);
+    TailInputs *tail = reinterpret_cast<TailInputs *>(reinterpret_cast<uint8_t *>(rows8) + (ROWS16 ? 0 : kStageBytesRows8<BN> + 16)); // kOutTail
     const bool fastGather = !A_TMA && fastGatherApplies(p);
 
     const int warp = threadIdx.x >> 5;
@@ -551,6 +560,13 @@ gemmI8Tcgen05(const __grid_constant__ CUtensorMap tmapA, const __grid_constant__
                      "r"(uint32_t(2 * BN))
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    if (OUT == kOutTail && threadIdx.x < 512) {
+        const bool forMain = threadIdx.x < 256;
+        const DevRescale &r = forMain ? p.epi.a : p.epi.b;
+        const FastRescale f = makeFastRescale(__ldg(r.mult), int32_t(__ldg(r.shift)), r.inZp, r.doubleRound != 0);
+        const int32_t byte = int32_t(threadIdx.x & 255u);
+        (forMain ? tail->main : tail->shortcut)[byte] = fastRescale(f, forMain ? byte - 128 : int32_t(int8_t(byte)), r.outZp, r.lo, r.hi);
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
@@ -758,7 +774,7 @@ gemmI8Tcgen05(const __grid_constant__ CUtensorMap tmapA, const __grid_constant__
         }
     } else {
         // ---------------- epilogue: warps 0-15 ----------------
-        epilogueWarps<BN, NSTAGE, ROWS16, !A_TMA>(p, bars, colTab, tmemBase, warp, lane, numTiles, mTiles, nTiles, staging, rows8);
+        epilogueWarps<BN, NSTAGE, ROWS16, !A_TMA, OUT>(p, bars, colTab, tmemBase, warp, lane, numTiles, mTiles, nTiles, staging, rows8, tail);
     }
 
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -772,8 +788,8 @@ gemmI8Tcgen05(const __grid_constant__ CUtensorMap tmapA, const __grid_constant__
 
 // ---- host side --------------------------------------------------------------------------------------------
 
-template <int BN, int NSTAGE, int A_MODE, bool B_MN, bool STAGE32 = false, bool ROWS16 = true>
-int launchVariant(const CUtensorMap &mapA, const CUtensorMap &mapB, const GemmI8Params &params, cudaStream_t s) {
+template <int BN, int NSTAGE, int A_MODE, bool B_MN, bool STAGE32, bool ROWS16, int OUT>
+int launchOut(const CUtensorMap &mapA, const CUtensorMap &mapB, const GemmI8Params &params, cudaStream_t s) {
     static_assert(!STAGE32 || A_MODE != kAGather, "the staging blocks take the place of the gather tables");
     GemmI8Params p = params;
     p.divPlane = makeFastDiv(int64_t(p.OH) * p.OW), p.divOW = makeFastDiv(p.OW);
@@ -781,9 +797,10 @@ int launchVariant(const CUtensorMap &mapA, const CUtensorMap &mapB, const GemmI8
     constexpr size_t smemBytes =
         size_t(NSTAGE) * (BM * BK + BN * BK) + BN * sizeof(ColConst) + sizeof(PipeBarriers) + 1024 +
         (A_MODE != kAGather ? 0 : (kMaxGatherPieces + kTapTabEntries) * sizeof(int32_t)) + 16 +
-        (STAGE32 ? size_t(kEpilogueWarps) * kStageBytesPerWarp : 0) + (ROWS16 ? 0 : kStageBytesRows8<BN>);
+        (STAGE32 ? size_t(kEpilogueWarps) * kStageBytesPerWarp : 0) + (ROWS16 ? 0 : kStageBytesRows8<BN> + 16) +
+        (OUT == kOutTail ? sizeof(TailInputs) : 0);
     static_assert(smemBytes <= 232448, "shared memory per CTA");
-    auto kernel = gemmI8Tcgen05<BN, NSTAGE, A_MODE, B_MN, STAGE32, ROWS16>;
+    auto kernel = gemmI8Tcgen05<BN, NSTAGE, A_MODE, B_MN, STAGE32, ROWS16, OUT>;
     if (!allowDynamicSmem(reinterpret_cast<const void *>(kernel), smemBytes)) {
         return MLEL_ERROR_DEVICE;
     }
@@ -799,6 +816,20 @@ int launchVariant(const CUtensorMap &mapA, const CUtensorMap &mapB, const GemmI8
         return MLEL_ERROR_DEVICE;
     }
     return MLEL_SUCCESS;
+}
+
+template <int BN, int NSTAGE, int A_MODE, bool B_MN, bool STAGE32 = false, bool ROWS16 = true>
+int launchVariant(const CUtensorMap &mapA, const CUtensorMap &mapB, const GemmI8Params &p, cudaStream_t s) {
+    if constexpr (ROWS16) {
+        if (p.out32 != nullptr) {
+            return launchOut<BN, NSTAGE, A_MODE, B_MN, STAGE32, ROWS16, kOutInt32>(mapA, mapB, p, s);
+        }
+    }
+    if constexpr (!STAGE32) {
+        return p.epi.hasResidual ? launchOut<BN, NSTAGE, A_MODE, B_MN, STAGE32, ROWS16, kOutTail>(mapA, mapB, p, s)
+                                 : launchOut<BN, NSTAGE, A_MODE, B_MN, STAGE32, ROWS16, kOutInt8>(mapA, mapB, p, s);
+    }
+    return MLEL_ERROR_UNKNOWN; // (staged stores are for int32 results)
 }
 
 } // namespace
