@@ -123,6 +123,8 @@ __device__ __forceinline__ void epilogueInt8(const GemmI8Params &p, PipeBarriers
     const int row = quarter * 32 + lane;
     bool failed = false;
     uint32_t *rows = rows8 + quarter * (32 * kRowPitchWords<BN>); // !ROWS16: this quarter's rows
+    // !ROWS16: rows of the output and of the shortcut are whole words
+    const bool words = p.N % 4 == 0 && p.ldOut % 4 == 0 && (!RESIDUAL || (reinterpret_cast<uintptr_t>(p.epi.shortcut) & 3u) == 0);
     FastRescale fo{};
     const uint32_t tailMain = smemAddr(tail->main) + 128u * 4u, tailShortcut = smemAddr(tail->shortcut);
     if (RESIDUAL) {
@@ -235,6 +237,13 @@ __device__ __forceinline__ void epilogueInt8(const GemmI8Params &p, PipeBarriers
                 if (ROWS16) {
                     const int4 s0 = __ldg(reinterpret_cast<const int4 *>(scp));
                     sc[0] = uint32_t(s0.x), sc[1] = uint32_t(s0.y), sc[2] = uint32_t(s0.z), sc[3] = uint32_t(s0.w);
+                } else if (words) {
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) {
+                        if (4 * q < ncols) {
+                            sc[q] = __ldg(reinterpret_cast<const uint32_t *>(scp) + q);
+                        }
+                    }
                 } else {
 #pragma unroll
                     for (int j = 0; j < 16; ++j) {
@@ -284,6 +293,13 @@ __device__ __forceinline__ void epilogueInt8(const GemmI8Params &p, PipeBarriers
             }
             if (ROWS16) {
                 *reinterpret_cast<int4 *>(dst) = make_int4(int(packed[0]), int(packed[1]), int(packed[2]), int(packed[3]));
+            } else if (nTiles == 1 && words) {
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    if (4 * q < ncols) {
+                        rows[uint32_t(lane * p.N + cl) / 4u + uint32_t(q)] = packed[q];
+                    }
+                }
             } else if (nTiles == 1) {
                 int8_t *mine = reinterpret_cast<int8_t *>(rows) + lane * p.N + cl;
 #pragma unroll
