@@ -164,6 +164,7 @@ class GraphPipeline {
     void buildResidualTable(OpDesc &op);
     void prepareDepthwise();
     void fuseResizedConcats();
+    void mergeProjections();
     int32_t addDerivedConstant(int32_t dtype, const std::vector<int64_t> &dims, const void *data);
     int32_t addScratchTensor(int32_t dtype, const std::vector<int64_t> &dims);
 

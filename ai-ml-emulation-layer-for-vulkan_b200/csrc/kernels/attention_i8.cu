@@ -539,9 +539,9 @@ int attentionFused(const AttentionPlan &plan, const TView &q, const TView &k, co
     }
     CUtensorMap maps[3];
     const int sequences = plan.batches / plan.heads;
-    if (!makeTokenMap(&maps[0], q.ptr, p.d, p.Sq, plan.heads, sequences, plan.qStride) ||
-        !makeTokenMap(&maps[1], k.ptr, p.d, p.Sk, plan.heads, sequences, plan.kStride) ||
-        !makeTokenMap(&maps[2], v.ptr, p.d, p.Sk, plan.heads, sequences, plan.vStride)) {
+    if (!makeTokenMap(&maps[0], q.ptr + plan.qOffset, p.d, p.Sq, plan.heads, sequences, plan.qStride) ||
+        !makeTokenMap(&maps[1], k.ptr + plan.kOffset, p.d, p.Sk, plan.heads, sequences, plan.kStride) ||
+        !makeTokenMap(&maps[2], v.ptr + plan.vOffset, p.d, p.Sk, plan.heads, sequences, plan.vStride)) {
         return MLEL_ERROR_DEVICE;
     }
     return p.keysPad <= kAttentionTwoBlockKeys ? launchAttention<8>(maps, p, s)

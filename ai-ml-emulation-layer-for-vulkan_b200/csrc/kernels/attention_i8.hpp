@@ -10,6 +10,7 @@ struct AttentionPlan {
     int32_t batches, heads; // batches = sequences x heads
     int32_t queries, keys, headDim;
     int64_t qStride[3], kStride[3], vStride[3], oStride[3]; // bytes: sequence, head, token (the head dimension is contiguous)
+    int64_t qOffset, kOffset, vOffset; // bytes, of the first element in the operand's tensor (a multiple of 16)
     // first RESCALE (score differences, int32 -> int16), its result 32768 higher: max((x * mult + addend) >> 32 + shift, 0)
     int32_t diffMult, diffShift;
     int64_t diffAddend;

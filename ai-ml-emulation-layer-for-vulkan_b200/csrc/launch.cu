@@ -346,7 +346,12 @@ int launchTable(const TView &in, const TView &out, const TView &table, cudaStrea
 }
 
 int launchMatmul(const OpDesc &op, const TView *T, cudaStream_t s) {
-    const TView &a = T[op.in[0]], &b = T[op.in[1]], &out = T[op.out[0]];
+    const TView &a = T[op.in[0]], &out = T[op.out[0]];
+    TView b = T[op.in[1]];
+    if (op.auxi[1] != 0) { // [1][W][C] is all there is: as [1][C][W]
+        std::swap(b.dims[1], b.dims[2]);
+        std::swap(b.strides[1], b.strides[2]);
+    }
     bool tableDone = false;
     const int rc = matmulOnTensorCores(op, T) ? launchMatmulTensorCore(op, T, s, &tableDone)
                    : op.kind == OP_MATMUL ? genericMatmul(a, b, out, op.i[0], op.i[1], s)

@@ -259,7 +259,8 @@ struct OpDesc {
     //                 auxi[3] = the most common class, auxi[4] = 1 when every correction is below 2^30 - 256 in size
     //                 with a fused residual tail and tc == 1: aux[3] = the tail as a table of 256 x 256 bytes
     //   MATMUL kinds with a constant second input: aux[0] correction int32 [batches][W],
-    //                 aux[3] the second input transposed to [batches][W][C]
+    //                 aux[3] the second input transposed to [batches][W][C]; auxi[1] = 1: in[1] is this tensor, too (several
+    //                 products as one, see GraphPipeline::mergeProjections)
     //   CONV2D kinds with tc == 2 (channel count not a multiple of 16): scratch = session tensor
     //                 [N][Hp][Wp][ICp], a copy of the input with zero-padded channels; aux[3] weights [OC][kPad]
     //                 padded alike.  With aux[4]: the copy has the borders, too, the weights are in the gather's K
