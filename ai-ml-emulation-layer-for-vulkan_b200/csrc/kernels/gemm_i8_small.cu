@@ -408,10 +408,13 @@ bool gemmI8SmallApplies(const GemmI8Problem &q, int *pixels, int *split) {
         return false;
     }
     // Rule.  The other kernels' 128-pixel tiles would leave two thirds of the SMs without work (a half or a quarter instead
-    // measured within 2 % on graphs of 1, 16 and 32 images).  Of the two tile widths the one that lets more CTAs share a
-    // tile's K blocks, two blocks each at least and at most two CTAs per SM -- neighbouring launches overlap, so a layer's
-    // own CTAs seldom meet --, and the narrow one where that is equal (one image of the ResNet-50-shaped graph: 248 us; at
-    // most one CTA per SM 267; narrow tiles always 249, but 16 images 487 against 478 us).
+    // measured within 2 % on graphs of 1, 16 and 32 images).  As many CTAs share a tile's K blocks as have two blocks each at
+    // least, with at most two CTAs per SM -- neighbouring launches overlap, so a layer's own CTAs seldom meet (one image of the
+    // ResNet-50-shaped graph: 248 us, at most one CTA per SM 267).  Tiles are 32 pixels wide.  With 64 a CTA of a larger split
+    // has half the blocks but a larger share of the reduction: worth it only from some 13 blocks on that the narrow tile
+    // would leave to a CTA (us a layer, narrow and wide: 2 x 33 x 33, 3x3, 160 <-> 128 channels, 4.5 blocks, 5.9 and 7.9; 14 x 14, 1x1,
+    // 2048 <-> 1024, 4, 4.9 and 6.2; 19 x 19, 3x3, 768 -> 768, 13.5, 12.7 and 12.5; 4 x 33 x 33, 128 <-> 768, 27, 10.5 and 9.8; 2 x 56 x 56,
+    // 2048 <-> 16, 144, 26.8 and 20.7).  While blocks took 0.3 us instead of 0.1 the wide one won wherever it allowed a larger split.
     const int sms = smCount();
     const int64_t cTiles = (p.N + kSmallChannels - 1) / kSmallChannels;
     if (mode == 1 && !smallKernelWants(p.M, p.N)) {
@@ -426,8 +429,9 @@ bool gemmI8SmallApplies(const GemmI8Problem &q, int *pixels, int *split) {
         return s;
     };
     const int split32 = splitFor(int64_t((p.M + 31) / 32) * cTiles), split64 = splitFor(int64_t((p.M + 63) / 64) * cTiles);
-    *pixels = split64 > split32 ? 64 : 32;
-    *split = std::max(split32, split64);
+    const bool wide = split64 > split32 && numKb > 13 * split32;
+    *pixels = wide ? 64 : 32;
+    *split = wide ? split64 : split32;
     if (mode >= 100) { // an experiment's choice: pixels and split
         *pixels = mode / 100 == 1 ? 32 : 64;
         *split = std::min(mode % 100, numKb >= 8 ? 8 : (numKb >= 4 ? 4 : (numKb >= 2 ? 2 : 1)));

@@ -113,3 +113,17 @@ def test_hand_over_between_channel_major_launches_without_the_small_kernel(mlel)
             _run(mlel, g, inputs, want, use_cuda_graph=True, times=3)
     finally:
         assert lib.mlel_set_tuning(b"small_kernel", 1) == 0
+
+
+@pytest.mark.parametrize("ic", [640, 736, 752, 768])  # 45 K blocks at 4 to a tile of 32 pixels; 54 at 8 to one of 64
+def test_tile_width_goes_by_the_blocks_of_a_cta(mlel, ic):
+    from mlel_b200.runtime import GraphRunner
+    r = np.random.Generator(np.random.PCG64(ic))
+    g = GraphBuilder()
+    x = g.input(np.int8, (2, 33, 33, ic))
+    g.output(conv(g, r, x, 16, 3, 1, 1, -5, False, base_shift=41))
+    data = [r.integers(-128, 128, x.shape, dtype=np.int8)]
+    before = mlel.lib().mlel_tensor_core_launches(3)
+    got = GraphRunner(g).run(data)[0]
+    assert mlel.lib().mlel_tensor_core_launches(3) == before + 1
+    np.testing.assert_array_equal(got, evaluate(g, data)[0])
