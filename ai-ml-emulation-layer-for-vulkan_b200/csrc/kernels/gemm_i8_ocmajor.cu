@@ -397,7 +397,7 @@ bool gemmI8OcMajorApplies(const GemmI8Problem &q) {
 }
 
 bool gemmI8OcMajorMayTake(int64_t pixels, int64_t channels) {
-    return channels > 64 && (tensorCoreTuning().smallKernel.load(std::memory_order_relaxed) != 1 || !smallKernelWants(pixels, channels));
+    return channels > 64 && (tensorCoreTuning().smallKernel.load(std::memory_order_relaxed) != 1 || !smallKernelWants(pixels, channels, kSmallKernelSurely));
 }
 
 // Tile-level hand-over between consecutive launches (GemmI8Params::progressOut / progressIn, LaunchChain).

@@ -396,8 +396,9 @@ int launchSmallSplit(const CUtensorMap &mapX, const CUtensorMap &mapW, const Gem
 
 } // namespace
 
-bool smallKernelWants(int64_t pixels, int64_t channels) {
-    return (pixels + 127) / 128 * ((channels + kSmallChannels - 1) / kSmallChannels) * 3 <= smCount();
+bool smallKernelWants(int64_t pixels, int64_t channels, int halves) {
+    const int64_t tiles = (pixels + 127) / 128 * ((channels + kSmallChannels - 1) / kSmallChannels);
+    return tiles * halves <= 2 * smCount();
 }
 
 bool gemmI8SmallApplies(const GemmI8Problem &q, int *pixels, int *split) {
@@ -407,8 +408,8 @@ bool gemmI8SmallApplies(const GemmI8Problem &q, int *pixels, int *split) {
         (q.aMatrix == nullptr && p.IC % 16 != 0)) {
         return false;
     }
-    // Rule.  The other kernels' 128-pixel tiles would leave two thirds of the SMs without work (a half or a quarter instead
-    // measured within 2 % on graphs of 1, 16 and 32 images).  As many CTAs share a tile's K blocks as have two blocks each at
+    // Rule.  The other kernels' 128-pixel tiles would leave two thirds of the SMs without work; for some forms below, half of
+    // them.  As many CTAs share a tile's K blocks as have two blocks each at
     // least, with at most two CTAs per SM -- neighbouring launches overlap, so a layer's own CTAs seldom meet (one image of the
     // ResNet-50-shaped graph: 248 us, at most one CTA per SM 267).  Tiles are 32 pixels wide.  With 64 a CTA of a larger split
     // has half the blocks but a larger share of the reduction: worth it only from some 13 blocks on that the narrow tile
@@ -417,7 +418,16 @@ bool gemmI8SmallApplies(const GemmI8Problem &q, int *pixels, int *split) {
     // 2048 <-> 16, 144, 26.8 and 20.7).  While blocks took 0.3 us instead of 0.1 the wide one won wherever it allowed a larger split.
     const int sms = smCount();
     const int64_t cTiles = (p.N + kSmallChannels - 1) / kSmallChannels;
-    if (mode == 1 && !smallKernelWants(p.M, p.N)) {
+    const bool matrix = q.aMatrix != nullptr, product = p.OH == 0; // (a product has no image)
+    // Beyond a third of the SMs, up to half for products of several blocks (of one block the gain is small: 3000 x 96 -> 384 4.4 and
+    // 3.9, and the paired kernel keeps them) and two fifths for the others (240 shapes of 50 to 74 tiles of 128 x 128,
+    // us a layer without and with): products of more than one channel tile and few blocks, which were the paired kernel's, 3201 x 256
+    // -> 256 5.1 and 3.9, 867 x 1024 -> 320 5.0 and 4.3 (942 x 2048 -> 1000 8.6 and 9.5, not taken); 1x1 of two blocks at most, 59 x 37,
+    // 160 -> 320 4.4 and 3.7 (102 x 17, 1024 -> 512 5.6 and 6.2, not taken; one channel tile, 36 x 93 x 2, 128 -> 128, 4.7 and 5.4); windows that
+    // the window kernel does not read, 4 x 42 x 44, 3x3, 256 -> 96 9.0 and 7.9 (56 x 61, 16 -> 256 7.8 and 9.9).
+    const bool further = matrix ? p.N > kSmallChannels && p.K <= (product ? 8 : 2) * BK : p.N > 64 && p.IC > 128;
+    const int halves = !further ? kSmallKernelSurely : (product && p.K > BK ? 4 : 5);
+    if (mode == 1 && !smallKernelWants(p.M, p.N, halves)) {
         return false;
     }
     const int numKb = q.aMatrix != nullptr ? (p.K + BK - 1) / BK : p.KH * p.KW * ((p.IC + 127) / 128);

@@ -148,7 +148,9 @@ int pairErrorWord();
 // Small-problem variant (gemm_i8_small.cu): narrow tiles whose K blocks are shared by a cluster.  `Applies` chooses the
 // pixels per tile and the CTAs per tile; Launch sets *taken as the paired variant does.
 bool gemmI8SmallApplies(const GemmI8Problem &problem, int *pixels, int *split);
-bool smallKernelWants(int64_t pixels, int64_t channels); // the rule on sizes in it
+// The rule on sizes in it: tiles of 128 x 128 times halves / 2 within the SMs.
+constexpr int kSmallKernelSurely = 6; // halves at which it takes every form
+bool smallKernelWants(int64_t pixels, int64_t channels, int halves);
 int gemmI8SmallLaunch(const GemmI8Problem &problem, int pixels, int split, cudaStream_t stream, bool *taken);
 int smallErrorWord();
 

@@ -127,3 +127,26 @@ def test_tile_width_goes_by_the_blocks_of_a_cta(mlel, ic):
     got = GraphRunner(g).run(data)[0]
     assert mlel.lib().mlel_tensor_core_launches(3) == before + 1
     np.testing.assert_array_equal(got, evaluate(g, data)[0])
+
+
+@pytest.mark.parametrize("rows,k,n,small", [
+    (1024, 256, 1152, True), (1025, 256, 1153, False), (2304, 1024, 512, True), (2304, 1040, 512, False), (1600, 64, 512, True),
+    (4736, 129, 129, True), (4737, 129, 129, False), (4736, 128, 129, False), (6400, 64, 128, False),
+])
+def test_products_on_either_side_of_the_rule(mlel, rows, k, n, small):
+    """Up to half as many tiles of 128 x 128 as SMs (148), with more than one channel tile and at most eight K blocks."""
+    import torch
+    from mlel_b200.runtime import GraphRunner
+    if torch.cuda.get_device_properties(0).multi_processor_count != 148:
+        pytest.skip("the sizes are for 148 SMs")
+    r = np.random.Generator(np.random.PCG64(rows + n))
+    g = GraphBuilder()
+    a = g.input(np.int8, (1, rows, k))
+    w = g.constant(r.integers(-128, 128, (1, k, n), dtype=np.int8))
+    mult = r.integers(1 << 30, (1 << 31) - 1, (n,), dtype=np.int64).astype(np.int32)
+    g.output(g.rescale(g.matmul(a, w, -20, 0), mult, np.full((n,), 38, np.int8), 0, 1, np.int8, double_round=True, per_channel=True))
+    data = [r.integers(-128, 128, a.shape, dtype=np.int8)]
+    before = mlel.lib().mlel_tensor_core_launches(3)
+    got = GraphRunner(g).run(data)[0]
+    assert mlel.lib().mlel_tensor_core_launches(3) - before == small
+    np.testing.assert_array_equal(got, evaluate(g, data)[0])
