@@ -25,8 +25,9 @@
 // every (CTAs / channel tiles)-th pixel tile.  Warps 0-15 epilogue, 16 TMA, 17 MMA; accumulators alternate.
 //
 // Measured (3x3, im2col kernels before): 64 x 56 x 56, 64 -> 64 channels 37.2 -> 19.1 us, 32 -> 64 37.8 -> 15.5; 270 x 480,
-// 96 -> 32 32.4 -> 11.9; 64 x 28 x 28, 128 -> 128 15.4 -> 13.8.  Bound now by the epilogue's RESCALEs and, with 128
-// channels, by the MMAs.
+// 96 -> 32 32.4 -> 11.9; 64 x 28 x 28, 128 -> 128 15.4 -> 13.8.  With the MMAs issued by a lane that their statement elects,
+// 270 x 480, 96 -> 32 8.6; where the epilogue is the longer part the denser MMAs slow it (16 x 56 x 56, 64 -> 64 7.5 -> 7.85).
+// Bound now by the epilogue's RESCALEs and, with 128 channels, by the MMAs.
 #include <cuda.h>
 #include <cuda_runtime.h>
 
