@@ -463,7 +463,7 @@ int launchPair(const PairMaps &maps, const GemmI8Params &params, cudaStream_t s)
     attrs[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attrs[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attrs;
-    cfg.numAttrs = 2;
+    cfg.numAttrs = dependentLaunches() ? 2 : 1;
     const cudaError_t err = cudaLaunchKernelEx(&cfg, kernel, maps.x, maps.w, maps.c, maps.d, p);
     if (err != cudaSuccess) {
         setLastError(std::string("tcgen05 paired convolution launch: ") + cudaGetErrorString(err));
