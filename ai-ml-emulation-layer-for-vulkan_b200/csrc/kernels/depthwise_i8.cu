@@ -56,7 +56,7 @@ __device__ __forceinline__ uint32_t loadBytes(const int8_t *p, int bytes) {
     const uintptr_t at = reinterpret_cast<uintptr_t>(p);
     const uint32_t skip = uint32_t(at & 3u);
     const uint32_t *words = reinterpret_cast<const uint32_t *>(at - skip);
-    const uint32_t first = __ldg(words), second = int(skip) + bytes > 4 ? __ldg(words + 1) : 0u;
+    const uint32_t first = words[0], second = int(skip) + bytes > 4 ? words[1] : 0u;
     return __funnelshift_r(first, second, 8 * skip);
 }
 
@@ -126,7 +126,7 @@ __global__ void __launch_bounds__(128, 4) depthwise3x3TableKernel(const __grid_c
 #pragma unroll
                 for (int i = 0; i < COLS; ++i) {
                     const bool ok = INSIDE || (rowOk && x0 + i >= 0 && x0 + i < p.W);
-                    cols[i] = !ok ? p.zeroWord : (ALIGNED ? __ldg(reinterpret_cast<const uint32_t *>(at)) : loadBytes(at, bytes));
+                    cols[i] = !ok ? p.zeroWord : (ALIGNED ? *reinterpret_cast<const uint32_t *>(at) : loadBytes(at, bytes));
                     at += p.C;
                 }
                 row += p.W * p.C;

@@ -15,7 +15,7 @@ namespace {
 // Copies an NHWC int8 tensor [N][H][W][C] into [N][Hp][Wp][Cp] (Cp >= C a multiple of 4) at row offset
 // padTop and column offset padLeft; the new channels and the border are zero.  One thread per 32-bit word
 // of the copy: byte reads hit L1, writes are coalesced.
-__global__ void padImageKernel(const int8_t *__restrict__ in, int8_t *__restrict__ out, int64_t words, int H, int W, int C,
+__global__ void padImageKernel(const int8_t *in, int8_t *out, int64_t words, int H, int W, int C,
                                int Hp, int Wp, int Cp, int padTop, int padLeft) {
     dependencySync();
     const int wordsPerPixel = Cp >> 2;
@@ -32,7 +32,7 @@ __global__ void padImageKernel(const int8_t *__restrict__ in, int8_t *__restrict
 #pragma unroll
             for (int b = 0; b < 4; ++b) {
                 if (c0 + b < C) {
-                    word |= uint32_t(uint8_t(__ldg(src + c0 + b))) << (8 * b);
+                    word |= uint32_t(uint8_t(src[c0 + b])) << (8 * b);
                 }
             }
         }
@@ -49,7 +49,7 @@ __device__ __forceinline__ int4 loadRagged16(const int8_t *p, int valid) {
     uint32_t w[5], v[4];
 #pragma unroll
     for (int k = 0; k < 5; ++k) {
-        w[k] = 4 * k < bytes ? __ldg(words + k) : 0u;
+        w[k] = 4 * k < bytes ? words[k] : 0u;
     }
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
@@ -63,7 +63,7 @@ __device__ __forceinline__ int4 loadRagged16(const int8_t *p, int valid) {
 // The same copy for channels padded to a multiple of 16: a thread makes 16 bytes of one pixel, from whole words.  BORDER:
 // the copy has pixels that the image has not (false: rows of C bytes become rows of Cp).  Bound by its bytes.
 template <bool BORDER>
-__global__ void __launch_bounds__(256) padPixels16Kernel(const int8_t *__restrict__ in, int4 *__restrict__ out, uint32_t units, int H,
+__global__ void __launch_bounds__(256) padPixels16Kernel(const int8_t *in, int4 *out, uint32_t units, int H,
                                                          int W, int C, FastDiv perPixel, FastDiv divWp, FastDiv divHp, int padTop,
                                                          int padLeft) {
     dependencySync();
@@ -87,7 +87,7 @@ __global__ void __launch_bounds__(256) padPixels16Kernel(const int8_t *__restric
 // of the rows 2 y - padTop + {0, 1} (there padLeft and padTop are the paddings' remainders); four channels each, the
 // missing ones and pixels outside the image zero.  Reads whole aligned words that hold a byte of the pixel.
 template <int STRIDE>
-__global__ void __launch_bounds__(256) gatherUnitsKernel(const int8_t *__restrict__ in, int4 *__restrict__ out, uint32_t units, int H,
+__global__ void __launch_bounds__(256) gatherUnitsKernel(const int8_t *in, int4 *out, uint32_t units, int H,
                                                          int W, int C, FastDiv divWu, FastDiv divHu, int padTop, int padLeft) {
     dependencySync();
     const uint32_t mask = C == 4 ? 0xffffffffu : (1u << (8 * C)) - 1u;
@@ -102,7 +102,7 @@ __global__ void __launch_bounds__(256) gatherUnitsKernel(const int8_t *__restric
             px[k] = 0;
             if (unsigned(x) < unsigned(W) && unsigned(y) < unsigned(H)) {
                 const int64_t at = ((int64_t(n) * H + y) * W + x) * C;
-                px[k] = __funnelshift_r(__ldg(words + (at >> 2)), __ldg(words + ((at + C - 1) >> 2)), 8 * (uint32_t(at) & 3u)) & mask;
+                px[k] = __funnelshift_r(words[at >> 2], words[(at + C - 1) >> 2], 8 * (uint32_t(at) & 3u)) & mask;
             }
         }
         out[e] = make_int4(int(px[0]), int(px[1]), int(px[2]), int(px[3]));
@@ -111,7 +111,7 @@ __global__ void __launch_bounds__(256) gatherUnitsKernel(const int8_t *__restric
 
 // The same copy for Cp == 4 and an even Wp (the RGB stem): one block per row of the copy, two pixels (one 8-byte
 // store) per thread, no divisions in the element loop.
-__global__ void __launch_bounds__(128) padImageRows4Kernel(const int8_t *__restrict__ in, int8_t *__restrict__ out, int H,
+__global__ void __launch_bounds__(128) padImageRows4Kernel(const int8_t *in, int8_t *out, int H,
                                                           int W, int C, int Hp, int Wp, int padTop, int padLeft) {
     dependencySync();
     const int row = blockIdx.x; // n * Hp + yp
@@ -129,7 +129,7 @@ __global__ void __launch_bounds__(128) padImageRows4Kernel(const int8_t *__restr
                 if (x >= 0 && x < W) {
                     const int8_t *px = src + x * C;
                     for (int b = 0; b < C; ++b) {
-                        w[j] |= uint32_t(uint8_t(__ldg(px + b))) << (8 * b);
+                        w[j] |= uint32_t(uint8_t(px[b])) << (8 * b);
                     }
                 }
             }
@@ -146,8 +146,8 @@ __global__ void __launch_bounds__(128) padImageRows4Kernel(const int8_t *__restr
 // Latency bounds it where there are few columns: a tile is a chain of load, turn and store.
 // ALIGNED: rows of B start on 16-byte boundaries.
 template <bool ALIGNED>
-__global__ void __launch_bounds__(256) transposeColsumKernel(const int8_t *__restrict__ b, int8_t *__restrict__ bt,
-                                                             int32_t *__restrict__ corr, int C, int W, int Cp, int32_t za, int split) {
+__global__ void __launch_bounds__(256) transposeColsumKernel(const int8_t *b, int8_t *bt,
+                                                             int32_t *corr, int C, int W, int Cp, int32_t za, int split) {
     dependencySync();
     __shared__ int8_t tile[64][64 + 16]; // [c][w], rows padded to spread the banks of the column reads
     __shared__ int32_t part[64];
@@ -165,7 +165,7 @@ __global__ void __launch_bounds__(256) transposeColsumKernel(const int8_t *__res
             return make_int4(0, 0, 0, 0);
         }
         const int8_t *p = src + int64_t(c0 + lr) * W + w0 + ls;
-        return ALIGNED ? __ldg(reinterpret_cast<const int4 *>(p)) : loadRagged16(p, min(16, W - (w0 + ls)));
+        return ALIGNED ? *reinterpret_cast<const int4 *>(p) : loadRagged16(p, min(16, W - (w0 + ls)));
     };
     int4 next = fetch(first);
     for (int c0 = first; c0 < last; c0 += 64) {
@@ -215,7 +215,7 @@ __global__ void __launch_bounds__(256) transposeColsumKernel(const int8_t *__res
 // flight per thread.  Each byte goes through one dp4a against a one-hot selector, which sign-extends and accumulates it.
 // A warp's eight slices join by shuffles, the eight warps in shared memory.
 // The product is let in at once and waits for the sums only before its epilogue (kLateCorrections): 1024^3 14.5 -> 12.4 us.
-__global__ void __launch_bounds__(256) columnSumKernel(const int8_t *__restrict__ b, int32_t *__restrict__ corr, int C, int W,
+__global__ void __launch_bounds__(256) columnSumKernel(const int8_t *b, int32_t *corr, int C, int W,
                                                        int32_t za) {
     __shared__ int32_t part[8][64];
     asm volatile("griddepcontrol.wait;" ::: "memory"); // first: the launch after this one relies on it
@@ -236,7 +236,7 @@ __global__ void __launch_bounds__(256) columnSumKernel(const int8_t *__restrict_
 #pragma unroll
             for (int u = 0; u < 8; ++u) {
                 const int c = c0 + 64 * u;
-                v[u] = c < C ? __ldg(reinterpret_cast<const int4 *>(src + int64_t(c) * W)) : make_int4(0, 0, 0, 0);
+                v[u] = c < C ? *reinterpret_cast<const int4 *>(src + int64_t(c) * W) : make_int4(0, 0, 0, 0);
             }
 #pragma unroll
             for (int u = 0; u < 8; ++u) {
@@ -427,7 +427,7 @@ struct PoolAcc {
 // KH, KW > 0: the window is known at compile time, all its loads are issued before the first maximum.
 // KH == 0: any window, two taps at a time.
 template <int KH, int KW>
-__global__ void maxPoolI8Kernel(const int8_t *__restrict__ in, int8_t *__restrict__ out, int64_t total, int H, int W,
+__global__ void maxPoolI8Kernel(const int8_t *in, int8_t *out, int64_t total, int H, int W,
                                 int C, int OH, int OW, PoolAttr a) {
     dependencySync();
     const int groups = C >> 4;
@@ -442,7 +442,7 @@ __global__ void maxPoolI8Kernel(const int8_t *__restrict__ in, int8_t *__restric
         const int iy0 = oy * max(a.stride[0], 1) - a.pad[0], ix0 = ox * max(a.stride[1], 1) - a.pad[2];
         const int4 *image = reinterpret_cast<const int4 *>(in + int64_t(n) * H * W * C) + g;
         const auto tap = [&](int y, int x) {
-            return (unsigned(y) < unsigned(H) && unsigned(x) < unsigned(W)) ? __ldg(image + (int64_t(y) * W + x) * groups)
+            return (unsigned(y) < unsigned(H) && unsigned(x) < unsigned(W)) ? image[(int64_t(y) * W + x) * groups]
                                                                             : lowest;
         };
         PoolAcc acc;
@@ -472,7 +472,7 @@ __global__ void maxPoolI8Kernel(const int8_t *__restrict__ in, int8_t *__restric
 
 // Channel counts that are no multiple of 16: a thread per output pixel and four channels (CH == 4, C % 4 == 0) or one.
 template <int CH>
-__global__ void __launch_bounds__(256) maxPoolNarrowKernel(const int8_t *__restrict__ in, int8_t *__restrict__ out,
+__global__ void __launch_bounds__(256) maxPoolNarrowKernel(const int8_t *in, int8_t *out,
                                                            uint32_t total, int H, int W, int C, FastDiv groups, FastDiv divOW,
                                                            FastDiv divOH, PoolAttr a) {
     dependencySync();
@@ -492,11 +492,11 @@ __global__ void __launch_bounds__(256) maxPoolNarrowKernel(const int8_t *__restr
             for (int x = x0; x < x1; ++x) {
                 const int8_t *p = image + (int64_t(y) * W + x) * C;
                 if (CH == 4) {
-                    const uint32_t w = __ldg(reinterpret_cast<const uint32_t *>(p));
+                    const uint32_t w = *reinterpret_cast<const uint32_t *>(p);
                     even = max3Lanes(even, evenBytesHigh(w), even);
                     odd = max3Lanes(odd, oddBytesHigh(w), odd);
                 } else {
-                    top = max(top, int32_t(__ldg(p)));
+                    top = max(top, int32_t(*p));
                 }
             }
         }
@@ -510,7 +510,7 @@ __global__ void __launch_bounds__(256) maxPoolNarrowKernel(const int8_t *__restr
 
 // The 3x3 window with stride 2 (the stem pool of the residual networks): one thread makes two horizontally
 // adjacent outputs, whose windows share a column, from 15 loads instead of 18.  OW must be even.
-__global__ void maxPool3x3s2PairKernel(const int8_t *__restrict__ in, int8_t *__restrict__ out, int64_t total, int H,
+__global__ void maxPool3x3s2PairKernel(const int8_t *in, int8_t *out, int64_t total, int H,
                                        int W, int C, int OH, int OW, int padTop, int padLeft) {
     dependencySync();
     const int groups = C >> 4, pairs = OW >> 1;
@@ -531,7 +531,7 @@ __global__ void maxPool3x3s2PairKernel(const int8_t *__restrict__ in, int8_t *__
             for (int kx = 0; kx < 5; ++kx) {
                 const int y = iy0 + ky, x = ix0 + kx;
                 v[ky][kx] = (unsigned(y) < unsigned(H) && unsigned(x) < unsigned(W))
-                                ? __ldg(image + (int64_t(y) * W + x) * groups)
+                                ? image[(int64_t(y) * W + x) * groups]
                                 : lowest;
             }
         }
@@ -581,7 +581,7 @@ __device__ __forceinline__ int4 packLanes(const LaneWords &l) {
                      int(__byte_perm(l.even[2], l.odd[2], 0x7351)), int(__byte_perm(l.even[3], l.odd[3], 0x7351)));
 }
 
-__global__ void maxPool3x3s2QuadKernel(const int8_t *__restrict__ in, int8_t *__restrict__ out, int64_t total, int H,
+__global__ void maxPool3x3s2QuadKernel(const int8_t *in, int8_t *out, int64_t total, int H,
                                        int W, int C, int OH, int OW, int padTop, int padLeft) {
     dependencySync();
     const int groups = C >> 4, pairsX = OW >> 1, pairsY = OH >> 1;
@@ -602,7 +602,7 @@ __global__ void maxPool3x3s2QuadKernel(const int8_t *__restrict__ in, int8_t *__
 #pragma unroll
             for (int kx = 0; kx < 5; ++kx) {
                 const int y = iy0 + ky, x = ix0 + kx;
-                v[kx] = (unsigned(y) < unsigned(H) && unsigned(x) < unsigned(W)) ? __ldg(image + (int64_t(y) * W + x) * groups)
+                v[kx] = (unsigned(y) < unsigned(H) && unsigned(x) < unsigned(W)) ? image[(int64_t(y) * W + x) * groups]
                                                                                  : lowest;
             }
             const LaneWords mid = toLanes(v[2]);

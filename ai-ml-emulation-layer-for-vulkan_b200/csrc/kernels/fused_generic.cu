@@ -227,9 +227,9 @@ __device__ __forceinline__ void transpose4x4Bytes(uint32_t a, uint32_t b, uint32
 }
 
 template <int R, int SX, bool OUT8>
-__global__ void __launch_bounds__(128, 4) depthwise3x3RowsKernel(const int8_t *__restrict__ in, const int8_t *__restrict__ w,
-                                                              const int32_t *__restrict__ bias, int biasCount,
-                                                              void *__restrict__ out, int N, int H, int W, int C, int OH,
+__global__ void __launch_bounds__(128, 4) depthwise3x3RowsKernel(const int8_t *in, const int8_t *w,
+                                                              const int32_t *bias, int biasCount,
+                                                              void *out, int N, int H, int W, int C, int OH,
                                                               int OW, FastDiv divC, FastDiv divX, FastDiv divY, ConvAttr a,
                                                               DevEpilogue epi) {
     constexpr int PX = 4;
@@ -253,9 +253,9 @@ __global__ void __launch_bounds__(128, 4) depthwise3x3RowsKernel(const int8_t *_
         int32_t wsum[4] = {0, 0, 0, 0};
 #pragma unroll
         for (int ky = 0; ky < 3; ++ky) {
-            const uint32_t w0 = __ldg(reinterpret_cast<const uint32_t *>(w + (ky * 3 + 0) * C + c0));
-            const uint32_t w1 = __ldg(reinterpret_cast<const uint32_t *>(w + (ky * 3 + 1) * C + c0));
-            const uint32_t w2 = __ldg(reinterpret_cast<const uint32_t *>(w + (ky * 3 + 2) * C + c0));
+            const uint32_t w0 = *reinterpret_cast<const uint32_t *>(w + (ky * 3 + 0) * C + c0);
+            const uint32_t w1 = *reinterpret_cast<const uint32_t *>(w + (ky * 3 + 1) * C + c0);
+            const uint32_t w2 = *reinterpret_cast<const uint32_t *>(w + (ky * 3 + 2) * C + c0);
             uint32_t tw[4];
             transpose4x4Bytes(w0, w1, w2, 0u, tw); // tw[k] = [w(kx=0) w(kx=1) w(kx=2) 0] of channel k
 #pragma unroll
@@ -292,7 +292,7 @@ __global__ void __launch_bounds__(128, 4) depthwise3x3RowsKernel(const int8_t *_
 #pragma unroll
                 for (int i = 0; i < COLS; ++i) {
                     const bool ok = INSIDE || (rowOk && x0 + i >= 0 && x0 + i < W);
-                    cols[i] = ok ? __ldg(reinterpret_cast<const uint32_t *>(in + offset)) : zword;
+                    cols[i] = ok ? *reinterpret_cast<const uint32_t *>(in + offset) : zword;
                     offset += uint32_t(C);
                 }
                 rowOffset += W * C;
@@ -334,7 +334,7 @@ __global__ void __launch_bounds__(128, 4) depthwise3x3RowsKernel(const int8_t *_
         bool words = OUT8 && (uint32_t(epi.main.inZp) + 256u) <= 512u;
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
-            const int32_t b = __ldg(bias + (biasCount == 1 ? 0 : c0 + k));
+            const int32_t b = bias[biasCount == 1 ? 0 : c0 + k];
             add[k] = int32_t(uint32_t(b) - uint32_t(a.inZp) * uint32_t(wsum[k]));
             if (OUT8) {
                 const int ci = epi.main.perChannel ? c0 + k : 0;

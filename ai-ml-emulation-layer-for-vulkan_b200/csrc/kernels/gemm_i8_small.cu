@@ -233,7 +233,7 @@ gemmI8Small(const __grid_constant__ CUtensorMap mapX, const __grid_constant__ CU
                 const uint32_t oy = fastDiv(rem, p.divOW);
                 cls = int(__ldg(p.rowClass + oy)) * p.numColClasses + int(__ldg(p.colClass + (rem - oy * uint32_t(p.OW))));
             }
-            corr[j] = ocValid ? __ldg(p.corr + int64_t(cls) * p.N + oc) : 0;
+            corr[j] = ocValid ? p.corr[int64_t(cls) * p.N + oc] : 0;
         }
         asm volatile("griddepcontrol.wait;" ::: "memory"); // from here on activations are read and written
     }
@@ -248,7 +248,7 @@ gemmI8Small(const __grid_constant__ CUtensorMap mapX, const __grid_constant__ CU
             const int8_t *row = p.epi.shortcut + int64_t(firstPixel) * p.ldOut + oc;
 #pragma unroll
             for (int j = 0; j < kMine; ++j) {
-                shortcut[j] = ocValid && firstPixel + j < p.M ? __ldg(row + int64_t(j) * p.ldOut) : int8_t(0);
+                shortcut[j] = ocValid && firstPixel + j < p.M ? row[int64_t(j) * p.ldOut] : int8_t(0);
             }
         }
         mbarWait(&bars->accFull, 0, 83);

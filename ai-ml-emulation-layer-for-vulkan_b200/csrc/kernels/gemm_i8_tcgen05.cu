@@ -169,7 +169,7 @@ __device__ __forceinline__ void epilogueInt8(const GemmI8Params &p, PipeBarriers
                 if (fails != 0) {
                     atomicAnd(const_cast<uint32_t *>(fastFlag), ~fails);
                 }
-                corr0 = col < p.N ? __ldg(corrBatch + int64_t(p.baseClass) * p.N + col) : 0;
+                corr0 = col < p.N ? corrBatch[int64_t(p.baseClass) * p.N + col] : 0;
             }
             epilogueSync();
             const uint32_t holds = *fastFlag;
@@ -227,7 +227,7 @@ __device__ __forceinline__ void epilogueInt8(const GemmI8Params &p, PipeBarriers
 #pragma unroll
                 for (int j = 0; j < 16; ++j) {
                     if (j < ncols) {
-                        acc[j] += uint32_t(__ldg(own + j)) - uint32_t(colTab[cl + j].corr0);
+                        acc[j] += uint32_t(own[j]) - uint32_t(colTab[cl + j].corr0);
                     }
                 }
             }
@@ -235,13 +235,13 @@ __device__ __forceinline__ void epilogueInt8(const GemmI8Params &p, PipeBarriers
             if (RESIDUAL) {
                 const int8_t *scp = p.epi.shortcut + outRow + col0;
                 if (ROWS16) {
-                    const int4 s0 = __ldg(reinterpret_cast<const int4 *>(scp));
+                    const int4 s0 = *reinterpret_cast<const int4 *>(scp);
                     sc[0] = uint32_t(s0.x), sc[1] = uint32_t(s0.y), sc[2] = uint32_t(s0.z), sc[3] = uint32_t(s0.w);
                 } else if (words) {
 #pragma unroll
                     for (int q = 0; q < 4; ++q) {
                         if (4 * q < ncols) {
-                            sc[q] = __ldg(reinterpret_cast<const uint32_t *>(scp) + q);
+                            sc[q] = reinterpret_cast<const uint32_t *>(scp)[q];
                         }
                     }
                 } else {
@@ -402,7 +402,7 @@ __device__ __forceinline__ void epilogueInt32(const GemmI8Params &p, PipeBarrier
                 if (corr != nullptr && rowValid) {
 #pragma unroll
                     for (int j = 0; j < 16; ++j) {
-                        acc[j] += uint32_t(__ldg(corr + col0 + j));
+                        acc[j] += uint32_t(corr[col0 + j]);
                     }
                 }
                 int32_t *mine = staging + warp * (32 * kStageInts);
@@ -432,7 +432,7 @@ __device__ __forceinline__ void epilogueInt32(const GemmI8Params &p, PipeBarrier
 #pragma unroll
             for (int j = 0; j < 16; ++j) {
                 if (corr != nullptr && j < ncols) {
-                    acc[j] += uint32_t(__ldg(corr + col0 + j));
+                    acc[j] += uint32_t(corr[col0 + j]);
                 }
             }
             if (ncols == 16 && (reinterpret_cast<uintptr_t>(dst) & 15u) == 0) {

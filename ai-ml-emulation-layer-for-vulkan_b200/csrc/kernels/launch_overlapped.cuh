@@ -5,6 +5,10 @@
 // later.  The trigger lets the successor start as early as it finds room.  Both are no-ops in a kernel launched the
 // ordinary way.
 //
+// Such a kernel reads activations by plain loads.  The read-only path (__ldg, or a const parameter with __restrict__) is for
+// memory that nothing writes while the kernel runs, and this one runs beside the kernel that writes its input; for a pointer
+// that is __restrict__ the compiler may also move an access across the wait.  __ldg is for graph constants.
+//
 // Beside the tensor-core kernels it is worth it between two of their launches (the layer norms and the GELU of a
 // BERT-shaped encoder: 2.495 -> 2.451 ms per dispatch of 12 layers), and for the copies, transposes, windows and moves in
 // front of and between them: an ordinary boundary between two kernels costs a whole number of 2.048 us on this machine, the

@@ -71,7 +71,7 @@ template <typename UNIT> __global__ void __launch_bounds__(256) runMoveKernel(co
                     to += i * m.dstStride[k];
                     row = q;
                 }
-                v[u] = __ldg(reinterpret_cast<const UNIT *>(m.src + so));
+                v[u] = *reinterpret_cast<const UNIT *>(m.src + so);
                 dst[u] = to;
             }
         }
@@ -212,7 +212,7 @@ struct TileTranspose {
 };
 
 template <typename T>
-__global__ void __launch_bounds__(256) tileTransposeKernel(const uint8_t *__restrict__ in, uint8_t *__restrict__ out,
+__global__ void __launch_bounds__(256) tileTransposeKernel(const uint8_t *in, uint8_t *out,
                                                            uint32_t tiles, const __grid_constant__ TileTranspose p) {
     dependencySync();
     constexpr int kPitch = 64 * int(sizeof(T)) + 4;
@@ -235,7 +235,7 @@ __global__ void __launch_bounds__(256) tileTransposeKernel(const uint8_t *__rest
 #pragma unroll
         for (int i = 0; i < 16; ++i) {
             const int r = r0 + y0 + 4 * i, c = c0 + x;
-            v[i] = r < p.R && c < p.C ? __ldg(reinterpret_cast<const T *>(in + so + int64_t(r) * p.srcRow) + c) : T(0);
+            v[i] = r < p.R && c < p.C ? *(reinterpret_cast<const T *>(in + so + int64_t(r) * p.srcRow) + c) : T(0);
         }
         __syncthreads(); // the previous tile has been read
 #pragma unroll
@@ -257,7 +257,7 @@ __global__ void __launch_bounds__(256) tileTransposeKernel(const uint8_t *__rest
 // ---- RESIZE, NEAREST (resize.comp:43-134): one source pixel per output pixel, its channels moved as units ---------
 template <typename UNIT>
 __global__ void __launch_bounds__(256)
-    resizeNearestKernel(const uint8_t *__restrict__ in, uint8_t *__restrict__ out, uint32_t units, FastDiv perPixel, FastDiv divOW,
+    resizeNearestKernel(const uint8_t *in, uint8_t *out, uint32_t units, FastDiv perPixel, FastDiv divOW,
                         FastDiv divOH, uint32_t H, uint32_t W, ResizeAttr a) {
     dependencySync();
     const uint32_t step = gridDim.x * blockDim.x;
@@ -269,7 +269,7 @@ __global__ void __launch_bounds__(256)
         const uint32_t x = nearestSource(ox, a.scale[2], a.scale[3], a.offset[1], W);
         UNIT v{}; // a position outside the image reads zero
         if (y < H && x < W) {
-            v = __ldg(reinterpret_cast<const UNIT *>(in) + (int64_t(n) * H + y) * W * perPixel.d + int64_t(x) * perPixel.d + u);
+            v = reinterpret_cast<const UNIT *>(in)[(int64_t(n) * H + y) * W * perPixel.d + int64_t(x) * perPixel.d + u];
         }
         reinterpret_cast<UNIT *>(out)[e] = v;
         if (units - e <= step) {
@@ -295,7 +295,7 @@ struct ConcatParts {
 };
 
 template <typename UNIT>
-__global__ void __launch_bounds__(256) concatResizedKernel(uint8_t *__restrict__ out, const __grid_constant__ ConcatParts p) {
+__global__ void __launch_bounds__(256) concatResizedKernel(uint8_t *out, const __grid_constant__ ConcatParts p) {
     dependencySync();
     const uint32_t step = gridDim.x * blockDim.x;
     for (uint64_t first = blockIdx.x * blockDim.x + threadIdx.x; first < p.units; first += uint64_t(step) * 4) {
@@ -324,7 +324,7 @@ __global__ void __launch_bounds__(256) concatResizedKernel(uint8_t *__restrict__
                     from = (y | x) < 0 ? -1 : (int64_t(n) * H + y) * W + x;
                 }
                 if (from >= 0) {
-                    v[j] = __ldg(reinterpret_cast<const UNIT *>(src) + from * units + (u - begin));
+                    v[j] = reinterpret_cast<const UNIT *>(src)[from * units + (u - begin)];
                 }
             }
         }
@@ -346,7 +346,7 @@ constexpr int kArgmaxStage = 128;
 
 template <typename T>
 __global__ void __launch_bounds__(256)
-    argmaxShortKernel(const T *__restrict__ in, int32_t *__restrict__ out, int64_t rows, int len, int32_t lowest) {
+    argmaxShortKernel(const T *in, int32_t *out, int64_t rows, int len, int32_t lowest) {
     dependencySync();
     __shared__ __align__(16) uint8_t stage[256 * kArgmaxStage];
     const int64_t total = rows * len * int64_t(sizeof(T));
@@ -356,7 +356,7 @@ __global__ void __launch_bounds__(256)
         const uint8_t *src = reinterpret_cast<const uint8_t *>(in) + base;
         __syncthreads();
         for (int i = threadIdx.x * 16; i + 16 <= bytes; i += 256 * 16) {
-            *reinterpret_cast<uint4 *>(stage + i) = __ldg(reinterpret_cast<const uint4 *>(src + i));
+            *reinterpret_cast<uint4 *>(stage + i) = *reinterpret_cast<const uint4 *>(src + i);
         }
         if (int(threadIdx.x) < (bytes & 15)) {
             stage[(bytes & ~15) + threadIdx.x] = src[(bytes & ~15) + threadIdx.x];
@@ -379,7 +379,7 @@ __global__ void __launch_bounds__(256)
 
 template <typename T>
 __global__ void __launch_bounds__(256)
-    argmaxLongKernel(const T *__restrict__ in, int32_t *__restrict__ out, int64_t rows, int len, int32_t lowest) {
+    argmaxLongKernel(const T *in, int32_t *out, int64_t rows, int len, int32_t lowest) {
     dependencySync();
     const int lane = threadIdx.x & 31;
     const int64_t warps = (int64_t(gridDim.x) * blockDim.x) >> 5;
@@ -387,7 +387,7 @@ __global__ void __launch_bounds__(256)
         const T *src = in + row * len;
         int32_t best = lowest, bestIndex = 0x7fffffff; // a lane that saw nothing above the start loses every tie
         for (int k = lane; k < len; k += 32) {
-            const int32_t v = int32_t(__ldg(src + k));
+            const int32_t v = int32_t(src[k]);
             if (v > best) {
                 best = v;
                 bestIndex = k;

@@ -290,7 +290,7 @@ __device__ __forceinline__ void epilogueOcMajor(const CUtensorMap *tmapD, const 
             const int ci = (p.epi.main.perChannel && ocValid) ? oc : 0;
             k.fm = makeFastRescale(__ldg(p.epi.main.mult + ci), int32_t(__ldg(p.epi.main.shift + ci)), p.epi.main.inZp,
                                    p.epi.main.doubleRound != 0);
-            k.corr0 = ocValid ? __ldg(corrBatch + int64_t(baseClass) * p.N + oc) : 0;
+            k.corr0 = ocValid ? corrBatch[int64_t(baseClass) * p.N + oc] : 0;
             const int32_t x0 = int32_t(uint32_t(k.corr0) - uint32_t(k.fm.zpIn));
             const bool twoRounds = p.epi.main.doubleRound != 0;
             const int shiftM = k.fm.s1 + k.fm.s2;
@@ -362,7 +362,7 @@ __device__ __forceinline__ void epilogueOcMajor(const CUtensorMap *tmapD, const 
                     if ((borderMask >> j) & 1u) {
                         const int c = __shfl_sync(0xffffffffu, mine, (col & 31) + j);
                         if (ocValid) {
-                            acc[j] += uint32_t(__ldg(corrBatch + int64_t(c) * p.N + oc)) - uint32_t(k.corr0);
+                            acc[j] += uint32_t(corrBatch[int64_t(c) * p.N + oc]) - uint32_t(k.corr0);
                         }
                     }
                 }

@@ -243,8 +243,7 @@ void launchRescale(const TView &in, const TView &out, const TView &mult, const T
 }
 
 // ---- TABLE (table.comp:17-52) -------------------------------------------------------------------------------
-__global__ void tableI8Kernel(const int8_t *__restrict__ in, int8_t *__restrict__ out, int64_t groups, int rest,
-                              const int8_t *__restrict__ table) {
+__global__ void tableI8Kernel(const int8_t *in, int8_t *out, int64_t groups, int rest, const int8_t *table) {
     dependencySync();
     __shared__ int8_t lut[256];
     for (int i = threadIdx.x; i < 256; i += blockDim.x) {
