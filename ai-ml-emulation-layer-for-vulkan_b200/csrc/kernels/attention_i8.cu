@@ -211,7 +211,7 @@ attentionI8Kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constan
                 }
                 __syncwarp();
             };
-            const auto wait = [&](uint64_t *bar, uint32_t parity, int code) { return __all_sync(0xffffffffu, mbarWait(bar, parity, code)) != 0; };
+            const auto wait = [&](uint64_t *bar, uint32_t parity, int code) { return mbarWaitWarp(bar, parity, code); };
             const DescWords descQ = descWords(smemDesc(smemAddr(tileQ), 16, 1024)), descK = descWords(smemDesc(smemAddr(tileK), 16, 1024));
             const DescWords descP = descWords(smemDesc(smemAddr(tileP), 16, 1024)), descV = descWords(smemDesc(smemAddr(tileV), BK * 128, 1024));
             const auto scoreProduct = [&] {
@@ -315,7 +315,7 @@ attentionI8Kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constan
 
     // Waits as a warp.  After a wait that ran out the warp keeps to the barriers of its quarter and does nothing else.
     const auto waitAll = [](uint64_t *bar, uint32_t phase, int code) {
-        const bool done = __all_sync(0xffffffffu, mbarWait(bar, phase, code));
+        const bool done = mbarWaitWarp(bar, phase, code);
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         return done;
     };

@@ -66,15 +66,15 @@ __global__ void __launch_bounds__(128, 1) int8MmaPeakKernel(int batches) {
         constexpr uint32_t idesc = instrDesc(kPeakN, false);
         const uint32_t aAddr = smemAddr(tileA), bAddr = smemAddr(tileB);
         bool ok = true;
-        for (int b = 0; b < batches && ok; ++b) {
+        int issued = 0;
+        for (int b = 0; b < batches; ++b, ++issued) {
             const uint32_t buf = uint32_t(b) & 1u;
             if (b >= 2) {
                 // the batch that last used this accumulator (and this barrier) has left the pipe
-                ok = mbarWait(&bars->done[buf], (uint32_t(b - 2) >> 1) & 1u, 21);
+                ok = mbarWaitWarp(&bars->done[buf], (uint32_t(b - 2) >> 1) & 1u, 21);
                 if (!ok) {
                     break;
                 }
-                __syncwarp();
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             }
             const uint32_t tmemD = tmemBase + buf * uint32_t(kPeakN);
@@ -86,9 +86,9 @@ __global__ void __launch_bounds__(128, 1) int8MmaPeakKernel(int batches) {
             }
             ummaCommit(&bars->done[buf]);
         }
-        // drain: the last two batches
-        for (int b = (batches > 2 ? batches - 2 : 0); b < batches && ok; ++b) {
-            ok = mbarWait(&bars->done[uint32_t(b) & 1u], (uint32_t(b) >> 1) & 1u, 22);
+        // drain: the last two batches, also behind a wait that ran out (the accumulators are given back below)
+        for (int b = max(issued - 2, 0); b < issued; ++b) {
+            mbarWaitWarp(&bars->done[uint32_t(b) & 1u], (uint32_t(b) >> 1) & 1u, 22);
         }
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");

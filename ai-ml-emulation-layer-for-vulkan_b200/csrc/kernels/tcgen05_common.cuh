@@ -104,6 +104,13 @@ __device__ __forceinline__ bool mbarWaitLimit(uint64_t *bar, uint32_t parity, in
 __device__ __forceinline__ bool mbarWait(uint64_t *bar, uint32_t parity, int code) {
     return mbarWaitLimit(bar, parity, code, kWaitLimitCycles);
 }
+// The same for a warp that then goes one way or the other as a whole, to warp-wide instructions (elect.sync): lanes leave a wait
+// that runs out by clocks of their own, so they agree by vote.  (Issuing warps that go on in any case, without waiting, need no
+// vote.  The epilogues' warps leave their loops by the thread: with a vote at each tile 64 images of the ResNet-50 shape take 858
+// instead of 851 us, with one in the waiting loop 855 and a 12-layer encoder 2066 instead of 2024.)
+__device__ __forceinline__ bool mbarWaitWarp(uint64_t *bar, uint32_t parity, int code) {
+    return __all_sync(0xffffffffu, mbarWait(bar, parity, code)) != 0;
+}
 
 __device__ __forceinline__ void tmaLoad3d(const CUtensorMap *map, void *dst, uint64_t *bar, int c0, int c1, int c2) {
     asm volatile(

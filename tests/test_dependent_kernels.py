@@ -49,3 +49,16 @@ def test_no_read_only_access_to_activations(path):
     text = open(path).read()
     if "launchOverlapped(" in text.replace("inline cudaError_t launchOverlapped(", ""):
         assert waiting > 0, "no kernel with a wait was recognised in a file that launches some"
+
+
+def test_issuing_warp_of_the_peak_loop_waits_as_a_whole():
+    """Its lanes go on to elect.sync together or leave together: no wait decides by the lane."""
+    text = open(next(p for p in KERNELS if p.endswith("int8_mma_peak.cu"))).read()
+    assert len(re.findall(r"\bmbarWaitWarp\(", text)) == 2 and not re.search(r"\bmbarWait\(", text)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("batches", [1, 2, 3, 4, 65])
+def test_peak_loop_of_few_batches(mlel, batches):
+    """Batches that need no wait before the drain, one, and several; no wait runs out (checked behind every test)."""
+    assert mlel.measure_int8_mma_peak(batches) > 0
