@@ -2125,9 +2125,9 @@ void GraphPipeline::prepareDepthwise() {
         d.channels = int32_t(channels), d.biasCount = int32_t(b.numel()), d.perChannel = f.attr.perChannel;
         d.doubleRound = f.attr.scale32 && f.attr.doubleRound;
         d.inputZp = op.i[8], d.rescaleZp = int32_t(wrapTo(f.inDtype, f.attr.inZp)), d.outZp = int32_t(wrapTo(f.outDtype, f.attr.outZp)), d.lo = f.lo;
-        std::vector<DepthwiseChannel> table;
+        std::vector<DepthwiseWord> table;
         if (op.i[9] == 0 && makeDepthwiseChannels(d, &table)) {
-            op.aux[0] = addDerivedConstant(MLEL_U8, {int64_t(table.size() * sizeof(DepthwiseChannel))}, table.data());
+            op.aux[0] = addDerivedConstant(MLEL_U8, {int64_t(table.size() * sizeof(DepthwiseWord))}, table.data());
         }
     }
 }

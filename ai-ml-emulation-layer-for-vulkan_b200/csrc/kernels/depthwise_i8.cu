@@ -18,11 +18,16 @@
 // Channel counts that are no multiple of four: the words start at any byte and are joined from two aligned ones, results leave
 // byte by byte.
 //
-// Measured (us, before -> now): 64 x 112 x 112 x 64 59.7 -> 48.7, with a ReLU 53.7 -> 47.7; one image of the MobileNetV2 shape
-// 186.7 -> 173.3; 63 channels (one thread per output before) 2244 -> 91, 16 x 57 x 57 x 35 86 -> 10.7.  Of 16 instructions an
-// output four address its loads: a copy of the tile in shared memory would save those.
+// The table stands word by word for all groups of channels, not channel by channel: neighbouring threads have neighbouring groups, and
+// with 128 bytes between their words each of a thread's eight loads of it took a warp 32 lines, 2 us of an SM with 16 warps.  (32 x 28 x
+// 28 x 192 7.9 us without the table, 8.7 so, 5.6 now; 32 x 14 x 14 x 576 7.1, 8.7 and 5.0; 32 images of the MobileNetV2 shape 450 -> 418.)
+//
+// Measured (us, without the table -> now): 64 x 112 x 112 x 64 59.8 -> 43.1, with a ReLU 53.7 -> 41.4; 32 x 56 x 56 x 144 17.2 -> 13.1;
+// 63 channels (one thread per output before) 2244 -> 76.5, 16 x 57 x 57 x 35 86 -> 9.3.  Of 16 instructions an output four address its
+// loads: a copy of the tile in shared memory would save those.
 #include <cstdint>
 #include <cstdlib>
+#include <cstring>
 #include <type_traits>
 
 #include "depthwise_i8.hpp"
@@ -36,7 +41,7 @@ namespace {
 struct DepthwiseParams {
     const int8_t *in;
     int8_t *out;
-    const DepthwiseChannel *table; // channels rounded up to four
+    const int4 *table; // [8][groups of four channels]
     int32_t N, H, W, C, OH, OW;
     FastDiv divC, divX, divY; // groups of channels, pixels and rows
     int32_t padTop, padLeft;
@@ -88,19 +93,20 @@ __global__ void __launch_bounds__(128, 4) depthwise3x3TableKernel(const __grid_c
     constexpr int COLS = (PX - 1) * SX + 3; // input pixels under the four windows of a row: 6 or 9
     constexpr int NT = SX == 1 ? 2 : 4;     // transposed groups of four pixels per input row
     constexpr int ROWS = (R - 1) * SX + 3;  // input rows under the R windows of a column
-    // Scheduled while the launch before drains, and lets the one after do the same: no activation before the wait.
+    // Scheduled while the launch before drains, and lets the one after do the same: no activation before the wait.  (Some thread has
+    // work and waits: a dimension of 0 is refused when a tensor is declared.)
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const int64_t total = int64_t(p.N) * p.divY.d * p.divX.d * p.divC.d;
     for (int64_t e = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; e < total; e += int64_t(gridDim.x) * blockDim.x) {
         const uint32_t tx = fastDiv(uint32_t(e), p.divC), ty = fastDiv(tx, p.divX), tn = fastDiv(ty, p.divY);
         const int c0 = int(uint32_t(e) - tx * p.divC.d) * 4, ox0 = int(tx - ty * p.divX.d) * PX, oy0 = int(ty - tn * p.divY.d) * R;
         const int n = int(tn), bytes = ALIGNED ? 4 : min(4, p.C - c0);
-        const int4 *channel = reinterpret_cast<const int4 *>(p.table + c0);
+        const int4 *channel = p.table + (uint32_t(e) - tx * p.divC.d); // word 2 k + h: channel[(2 k + h) * groups]
         uint32_t wa[3][4], wb[3][4]; // a window row's three weights at byte offsets 0 and 1
         int32_t acc[R][PX][4];
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
-            const int4 v = __ldg(channel + 2 * k);
+            const int4 v = __ldg(channel + 2 * k * p.divC.d);
             wa[0][k] = uint32_t(v.x), wa[1][k] = uint32_t(v.y), wa[2][k] = uint32_t(v.z);
 #pragma unroll
             for (int ky = 0; ky < 3; ++ky) {
@@ -181,7 +187,7 @@ __global__ void __launch_bounds__(128, 4) depthwise3x3TableKernel(const __grid_c
         int4 scale[4];
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
-            scale[k] = __ldg(channel + 2 * k + 1);
+            scale[k] = __ldg(channel + (2 * k + 1) * p.divC.d);
         }
         const bool full = oy0 + R <= p.OH && ox0 + PX <= p.OW;
         const auto finish = [&](auto signedTag, auto boundedTag) {
@@ -218,12 +224,12 @@ __global__ void __launch_bounds__(128, 4) depthwise3x3TableKernel(const __grid_c
 
 } // namespace
 
-bool makeDepthwiseChannels(const DepthwiseConstants &d, std::vector<DepthwiseChannel> *out) {
-    const int padded = (d.channels + 3) / 4 * 4;
+bool makeDepthwiseChannels(const DepthwiseConstants &d, std::vector<DepthwiseWord> *out) {
+    const size_t groups = size_t(d.channels + 3) / 4;
     const bool signFree = !d.doubleRound || d.lo >= d.outZp;
-    out->assign(size_t(padded), DepthwiseChannel{});
+    out->assign(8 * groups, DepthwiseWord{});
     for (int c = 0; c < d.channels; ++c) {
-        DepthwiseChannel &k = (*out)[size_t(c)];
+        DepthwiseChannel k{};
         const int32_t mult = d.mult[d.perChannel ? c : 0], shift = d.shift[d.perChannel ? c : 0];
         int64_t sum = 0;
         for (int ky = 0; ky < 3; ++ky) {
@@ -245,6 +251,10 @@ bool makeDepthwiseChannels(const DepthwiseConstants &d, std::vector<DepthwiseCha
         const int64_t addend = (int64_t(1) << (shift - 1)) + (d.doubleRound ? int64_t(1) << 30 : 0) + int64_t(d.outZp) * (int64_t(1) << shift);
         k.start = int32_t(start), k.mult = mult, k.shift = shift - 32;
         k.low = uint32_t(uint64_t(addend)), k.high = uint32_t(uint64_t(addend) >> 32);
+        for (size_t half = 0; half < 2; ++half) {
+            std::memcpy(&(*out)[(2 * size_t(c % 4) + half) * groups + size_t(c / 4)], reinterpret_cast<const DepthwiseWord *>(&k) + half,
+                        sizeof(DepthwiseWord));
+        }
     }
     return true;
 }
@@ -258,7 +268,7 @@ bool depthwiseTableTakes(const TView &in, const TView &out, const ConvAttr &a) {
 int depthwiseFromTable(const TView &in, const TView &table, const TView &out, const ConvAttr &a, const DevRescale &r, cudaStream_t s) {
     DepthwiseParams p{};
     p.in = reinterpret_cast<const int8_t *>(in.ptr), p.out = reinterpret_cast<int8_t *>(out.ptr);
-    p.table = reinterpret_cast<const DepthwiseChannel *>(table.ptr);
+    p.table = reinterpret_cast<const int4 *>(table.ptr);
     p.N = int(in.dims[0]), p.H = int(in.dims[1]), p.W = int(in.dims[2]), p.C = int(in.dims[3]), p.OH = int(out.dims[1]), p.OW = int(out.dims[2]);
     p.padTop = a.pad[0], p.padLeft = a.pad[2];
     p.zeroWord = uint32_t(uint8_t(a.inZp)) * 0x01010101u;

@@ -228,3 +228,13 @@ def test_replicated_pattern_rejects_non_divisible_counts(mlel):
     with pytest.raises(mlel.MlelError) as e:
         lower(mlel, text, [(0, 0, 0, mlel.I32, shape), (0, 1, 0, mlel.I32, shape)])
     assert "replicated constant element count" in str(e.value)
+
+
+@pytest.mark.parametrize("shape", [(0, 8, 8, 16), (1, 0, 8, 16), (1, 8, 8, 0)])
+def test_dimension_of_zero_is_refused(mlel, shape):
+    """No kernel meets an empty tensor (a launch whose threads all lack work would not wait for the one before it)."""
+    from mlel_b200.runtime import make_pipeline
+    g = GraphBuilder()
+    g.output(g.clamp(g.input(np.int8, shape), -5, 5))
+    with pytest.raises(mlel.MlelError, match="greater than zero"):
+        make_pipeline(g)
