@@ -26,7 +26,7 @@
 //
 // Measured (3x3, im2col kernels before): 64 x 56 x 56, 64 -> 64 channels 37.2 -> 19.1 us, 32 -> 64 37.8 -> 15.5; 270 x 480,
 // 96 -> 32 32.4 -> 11.9; 64 x 28 x 28, 128 -> 128 15.4 -> 13.8.  With the MMAs issued by a lane that their statement elects,
-// 270 x 480, 96 -> 32 8.6; where the epilogue is the longer part the denser MMAs slow it (16 x 56 x 56, 64 -> 64 7.5 -> 7.85).
+// 270 x 480, 96 -> 32 8.6 (not with two MMAs a tap and a long epilogue, see ummaLed).
 // Bound now by the epilogue's RESCALEs and, with 128 channels, by the MMAs.
 #include <cuda.h>
 #include <cuda_runtime.h>
@@ -78,6 +78,22 @@ __device__ __forceinline__ uint64_t rowDesc(uint32_t addr, uint32_t rowBytes, ui
 // Descriptor of a K-major operand without a swizzle: groups of eight 16-byte rows.
 __device__ __forceinline__ uint64_t smemDescPlain(uint32_t addr, uint32_t leadingBytes, uint32_t groupBytes) {
     return smemDesc(addr, leadingBytes, groupBytes) & ~(uint64_t(7) << 61);
+}
+
+// One MMA by lane 0, named by a predicate and not elected: it takes 62 cycles to issue where an elected one takes 21 (see umma).
+// That is the better pace for two MMAs a tap beside a tile of 64 channels and more, whose epilogue is the longer part in any case:
+// MMAs that arrive no faster than the pipe takes them (50 cycles) leave the epilogue warps of that scheduler their issue slots.
+// (us, elected and so: 16 x 56 x 56, 64 -> 64 7.8 and 7.4, 32 images 11.5 and 11.0, 64 -> 128 11.8 and 11.0, 8 x 61 x 19, 64 -> 464 9.9
+// and 9.5.  Elsewhere the pace is the MMAs': 16 x 56 x 56, 64 -> 32 5.6 and 6.0, 96 -> 64 7.6 and 9.4, 270 x 480, 96 -> 32 8.6 and 11.4.)
+__device__ __forceinline__ void ummaLed(uint32_t leader, uint32_t tmemD, DescWords a, DescWords b, uint32_t idesc, uint32_t accumulate) {
+    asm volatile("{\n\t.reg .pred p, l;\n\t.reg .b64 a, b;\n\t"
+                 "setp.ne.b32 l, %8, 0;\n\t"
+                 "setp.ne.b32 p, %6, 0;\n\t"
+                 "mov.b64 a, {%1, %2};\n\t"
+                 "mov.b64 b, {%3, %4};\n\t"
+                 "@l tcgen05.mma.cta_group::1.kind::i8 [%0], a, b, %5, {%7, %7, %7, %7}, p;\n\t}"
+                 ::"r"(tmemD), "r"(a.low), "r"(a.high), "r"(b.low), "r"(b.high), "r"(idesc), "r"(accumulate), "r"(0u), "r"(leader)
+                 : "memory");
 }
 
 // ODD: output rows start at any address.  The warps that share 32 rows of the accumulator put them together in shared memory
@@ -169,7 +185,7 @@ gemmI8Window(const __grid_constant__ CUtensorMap mapX, const __grid_constant__ C
         // the later MMAs read old bytes, the recorded error tells.
         dependencySync();
         constexpr uint32_t idesc = instrDesc(BN, false);
-        const uint32_t groupBytes = uint32_t((g.blocks ? g.boxW : 8) * g.pixelBytes);
+        const uint32_t groupBytes = uint32_t((g.blocks ? g.boxW : 8) * g.pixelBytes), leader = lane == 0 ? 1u : 0u;
         const uint64_t descX = rowDesc(smemAddr(stages), uint32_t(g.pixelBytes), groupBytes);
         const uint64_t descW = rowDesc(smemAddr(weights), uint32_t(g.pixelBytes), uint32_t(8 * g.pixelBytes));
         const uint32_t lowX = uint32_t(descX), highX = uint32_t(descX >> 32), lowW = uint32_t(descW), highW = uint32_t(descW >> 32);
@@ -201,7 +217,12 @@ gemmI8Window(const __grid_constant__ CUtensorMap mapX, const __grid_constant__ C
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const uint32_t tmemD = tmemBase + buf * uint32_t(BN);
                 const auto tap = [&](uint32_t x, uint32_t w, bool first) {
-                    ummaBlock(tmemD, {x, highX}, 2, {w, highW}, 2, idesc, first ? 0u : 1u, kSlices);
+                    if constexpr (kSlices == 2 && kThree && BN >= 64 && !ODD) {
+                        ummaLed(leader, tmemD, {x, highX}, {w, highW}, idesc, first ? 0u : 1u);
+                        ummaLed(leader, tmemD, {x + 2u, highX}, {w + 2u, highW}, idesc, 1u);
+                    } else {
+                        ummaBlock(tmemD, {x, highX}, 2, {w, highW}, 2, idesc, first ? 0u : 1u, kSlices);
+                    }
                 };
                 if (UNITS) {
                     const uint32_t stage = smemAddr(stages + s * g.stageBytes) >> 4, w = (smemAddr(weights) >> 4) + (uint32_t(BN) << 16);
