@@ -65,6 +65,19 @@ bool tryWindowKernel(const GemmI8Problem &q, cudaStream_t s, int *rc) {
     return taken || *rc != MLEL_SUCCESS;
 }
 
+// Windows of nine taps and more that both of them read, over at most 64 channels: above a quarter of the SMs' tiles of 128 x 128 the window kernel's.  Up to
+// a third they were the small kernel's, whose narrow tiles there are one round of CTAs that fetch all the weights again (us a layer,
+// small and window: 2 x 56 x 56, 64 -> 64 8.4 and 6.3, 32 -> 32 9.4 and 4.0; 80 x 64, 48 -> 64 8.7 and 4.3; 75 x 75, 64 -> 64 8.0 and
+// 4.2; 98 x 7 x 7, 64 -> 60 7.2 and 5.2; the first 7.7, the third 8.1 with the small kernel's wide tiles).  Over 128 channels the small
+// kernel has no more blocks, the window kernel twice the MMAs: 98 x 7 x 7, 128 -> 128 5.1 and 5.8; of few taps it has few blocks: 57 x
+// 109, 2x2, 64 -> 64 6.3 and 6.9, 64 -> 128 4.1 and 4.9.
+// A forced small kernel stays one.
+bool windowBeforeSmall(const GemmI8Problem &q) {
+    constexpr int kQuarter = 8; // (halves of the SMs, see smallKernelWants)
+    return tensorCoreTuning().smallKernel.load(std::memory_order_relaxed) == 1 && q.params.IC <= 64 && q.params.KH * q.params.KW >= 9 &&
+           !smallKernelWants(q.params.M, q.params.N, kQuarter);
+}
+
 PoolAttr poolAttr(const OpDesc &op) {
     PoolAttr a{};
     a.kernel[0] = op.i[0], a.kernel[1] = op.i[1], a.stride[0] = op.i[2], a.stride[1] = op.i[3];
@@ -224,7 +237,8 @@ int launchConvTensorCore(const OpDesc &op, const TView *T, cudaStream_t s, Launc
     q.bBatchBytes = 0;
     q.bMnMajor = false;
     int rc = MLEL_SUCCESS;
-    if (tryPairKernel(q, true, s, &rc) || trySmallKernel(q, s, &rc) || tryWindowKernel(q, s, &rc)) {
+    if (tryPairKernel(q, true, s, &rc) || (windowBeforeSmall(q) && tryWindowKernel(q, s, &rc)) || trySmallKernel(q, s, &rc) ||
+        tryWindowKernel(q, s, &rc)) {
         return rc;
     }
     return gemmI8OcMajorApplies(q) ? gemmI8OcMajorLaunch(q, s, chain, consumed) : gemmI8Launch(q, s);

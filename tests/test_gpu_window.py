@@ -69,3 +69,28 @@ def test_windows_of_few_channels(mlel, n, h, w, ic, oc, k, stride, pad, shift):
             bad = np.argwhere(a != b)
             assert len(bad) == 0, (len(bad), a.size, bad[0].tolist(), bad[-1].tolist())
     assert lib.mlel_tensor_core_launches(4) > before
+
+
+@pytest.mark.parametrize("n,h,w,ic,oc,k,expected", [
+    (1, 64, 74, 64, 64, 3, 3), (1, 64, 75, 64, 64, 3, 4),      # 37 and 38 tiles of 128 pixels
+    (3, 28, 28, 16, 129, 3, 4), (2, 56, 56, 32, 32, 5, 4),     # channel tiles count; another window
+    (1, 70, 90, 48, 63, 3, 4), (1, 56, 108, 64, 64, 2, 3),     # rows at any address; too few taps
+    (1, 64, 75, 80, 64, 3, 3), (1, 64, 75, 144, 64, 3, 3),     # more channels than the rule takes, than a pixel row holds
+    (1, 64, 75, 64, 64, 31, 3),                                # weights that do not fit beside the input
+])
+def test_window_kernel_before_the_small_one(mlel, n, h, w, ic, oc, k, expected):
+    """From a quarter of the SMs on (148: 37 tiles), below half of which the small kernel would take them too."""
+    from mlel_b200.runtime import GraphRunner
+    r = np.random.Generator(np.random.PCG64(h * 1000 + w))
+    g = GraphBuilder()
+    x = g.input(np.int8, (n, h, w, ic))
+    g.output(conv(g, r, x, oc, k, 1, k // 2, -7, True, 38))
+    data = r.integers(-128, 128, x.shape, dtype=np.int8)
+    want = evaluate(g, [data])[0]
+    lib = mlel.lib()
+    lib.mlel_tensor_core_launches.restype = ctypes.c_longlong
+    runner = GraphRunner(g)
+    before = [lib.mlel_tensor_core_launches(kernel) for kernel in range(5)]
+    got = runner.run([data])[0]
+    assert [lib.mlel_tensor_core_launches(kernel) - before[kernel] for kernel in range(5)] == [int(kernel == expected) for kernel in range(5)]
+    np.testing.assert_array_equal(got, want)
