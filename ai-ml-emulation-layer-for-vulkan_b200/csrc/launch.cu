@@ -398,6 +398,11 @@ int contractionLaunches(const OpDesc &op, const TView *T) {
     }
 }
 
+bool launchesAllDepend(const OpDesc &op, const TView *T) {
+    return (op.kind == OP_MATMUL || op.kind == OP_FUSED_MATMUL) && op.tc == 3 && op.epi.tableTensor < 0 && matmulOnTensorCores(op, T) &&
+           pairTakesActivations(matmulProblem(op, T));
+}
+
 int launchOp(const OpDesc &op, const TView *T, cudaStream_t s, LaunchChain *chain) {
     const auto in = [&](size_t k) -> const TView & { return T[op.in[k]]; };
     const TView &out = T[op.out[0]];

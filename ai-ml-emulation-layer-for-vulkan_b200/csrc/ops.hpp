@@ -282,6 +282,9 @@ int launchOp(const OpDesc &op, const TView *tensors, cudaStream_t stream, Launch
 
 // Kernels that launchOp() enqueues for a convolution or a product (at most).
 int contractionLaunches(const OpDesc &op, const TView *tensors);
+// A product of two activations whose second operand is read where it lies: copied rows, column sums and product are dependent
+// launches all (a transposed copy is one only where it is small).
+bool launchesAllDepend(const OpDesc &op, const TView *tensors);
 
 void setLastError(const std::string &msg);
 int elemSize(int32_t dtype);

@@ -685,11 +685,15 @@ int Session::dispatchGraph(cudaStream_t stream) {
     // One or two kernels are enqueued quicker than a graph of them is launched: back to back 5.4 against 8.2 us for a small
     // convolution, 6.4 against 8.2 for one with a padded copy, 5.6 against 8.2 and 10.3 against 12.3 for products of two
     // activations -- a replay begins on a whole number of 2.048 us (see launch_overlapped.cuh), launches behind one another do not.
-    // Three (copied rows or a TABLE besides) cost the host more than a replay: 7.7 against 6.2 us for a small product.
+    // Three (copied rows besides) keep the host 8 us, and a replay takes 6.2, 8.2 or 10.3: enqueued where all three depend on one
+    // another, 15 of 15 products 1.03 to 1.3 times as fast (4 x 17 x 55 x 384 7.95 and 9.3, 4 x 43 x 18 x 224 8.0 and 8.2, 5 x 189 x 99 x 640
+    // 8.6 and 10.3); replayed where the second operand is transposed first (2 x 40 x 30 x 64 7.7 and 6.2, 3 x 138 x 253 x 438 12.3 and
+    // 10.4; of 42 products 21 the one way, 21 the other) or a TABLE follows.
     const auto &exec = pipeline_->getExecList();
     if (exec.size() == 1) {
         const OpDesc &op = exec[0];
-        if (op.scratch < 0 || contractionLaunches(op, views_.data()) <= 2) {
+        const int launches = op.scratch < 0 ? 1 : contractionLaunches(op, views_.data());
+        if (launches <= 2 || (launches == 3 && launchesAllDepend(op, views_.data()))) {
             return dispatch(stream);
         }
         // (a stream that is being captured takes kernels, not the launch of a graph)

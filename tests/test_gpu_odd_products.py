@@ -89,3 +89,19 @@ def test_products_with_rows_at_odd_addresses_where_the_paired_kernel_begins(mlel
     before = lib.mlel_tensor_core_launches(2)
     check_fused(mlel, g, [a8] if constant else [a8, b8], ["MATMUL+RESCALE"])
     assert (lib.mlel_tensor_core_launches(2) > before) == paired
+
+
+@pytest.mark.parametrize("batch,rows,k,n", [(4, 17, 55, 384), (1, 9, 14, 272), (2, 300, 129, 640), (1, 1, 1, 144), (3, 40, 100, 128)])
+def test_product_of_activations_with_copied_rows_as_a_session(mlel, batch, rows, k, n):
+    """Three launches: enqueued where the second operand is read where it lies, replayed where it is transposed (the last).
+    New inputs at every pass, both ways in turn."""
+    from mlel_b200.runtime import GraphRunner
+    from tests.graph_eval import evaluate
+    r = np.random.Generator(np.random.PCG64(rows + n))
+    g = GraphBuilder()
+    a, b = g.input(np.int8, (batch, rows, k)), g.input(np.int8, (batch, k, n))
+    g.output(g.rescale(g.matmul(a, b, 3, 0), [1 << 30 | 12345], [37], 0, 1, np.int8, double_round=True))
+    runner = GraphRunner(g)
+    for use_cuda_graph in (True, False, True, True):
+        data = [r.integers(-128, 128, t.shape, dtype=np.int8) for t in (a, b)]
+        np.testing.assert_array_equal(runner.run(data, use_cuda_graph=use_cuda_graph)[0], evaluate(g, data)[0])
