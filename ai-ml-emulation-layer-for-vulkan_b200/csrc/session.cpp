@@ -51,8 +51,16 @@ Session::Session(GraphPipeline *pipeline) : pipeline_(pipeline) {
     progressCapacity_ = progressWords_ != nullptr ? words : 0;
 }
 
+void Session::dropCaptureStream() {
+    if (captureStream_ != nullptr) {
+        cudaStreamDestroy(captureStream_);
+        captureStream_ = nullptr;
+    }
+}
+
 Session::~Session() {
     dropGraphs();
+    dropCaptureStream();
     if (progressWords_ != nullptr) {
         cudaFree(progressWords_);
     }
@@ -556,16 +564,77 @@ std::vector<std::vector<size_t>> Session::branches(const std::vector<size_t> &op
     return before;
 }
 
+// Four lanes for a stretch of operators: which earlier ones each follows by an edge, and whether that is quicker than one after the
+// other by enough.
+//
+// Times are counted in bytes, a launch as 12 MB (2 us).  In a row they add up; on lanes the longest path through the edges counts, but
+// no less than all bytes take together.  Lanes are taken from a sixteenth less on: of 56 stretches of 2 to 12 operators with that much
+// (tensors of 4 KB to 17 MB, 2 to 4 chains) none was slower on lanes, most took 0.45 to 0.85 of the time; but they add 0.04 (two
+// lanes) to 0.14 ms (four) to the capture, once per set of addresses, which 50 operators that mostly follow one another (57.4 us
+// in a row, 56.6 on lanes) would not earn.
+Session::LanePlan Session::planLanes(const std::vector<size_t> &ops) const {
+    constexpr uint64_t kLaunch = uint64_t(12) << 20;
+    const auto &exec = pipeline_->getExecList();
+    const std::vector<std::vector<size_t>> before = branches(ops);
+    LanePlan plan;
+    plan.after.resize(ops.size());
+    std::vector<size_t> laneOf(ops.size());
+    std::array<size_t, kLanes> tail;
+    std::array<uint64_t, kLanes> load{};
+    tail.fill(SIZE_MAX);
+    // of every operator the last one of each lane that precedes it (or is it), plus one: an edge is laid only from operators
+    // that no other edge implies (with all of them 400 operators on four chains replayed in 1730 us instead of 430)
+    std::vector<std::array<size_t, kLanes>> known(ops.size());
+    std::vector<uint64_t> finish(ops.size());
+    uint64_t inARow = 0, bytes = 0, longest = 0;
+    for (size_t j = 0; j < ops.size(); ++j) {
+        // An operator goes on where the last one that it follows ended, or else on the lane with the least to do.
+        size_t lane = size_t(std::min_element(load.begin(), load.end()) - load.begin());
+        for (size_t l = 0; l < kLanes; ++l) {
+            if (!before[j].empty() && tail[l] == before[j].back()) {
+                lane = l;
+            }
+        }
+        std::array<size_t, kLanes> &mine = known[j];
+        mine.fill(0);
+        uint64_t start = 0;
+        const auto edgeFrom = [&](size_t b) {
+            if (mine[laneOf[b]] <= b) {
+                plan.after[j].push_back(b);
+                start = std::max(start, finish[b]);
+                for (size_t l = 0; l < kLanes; ++l) {
+                    mine[l] = std::max(mine[l], known[b][l]);
+                }
+            }
+        };
+        if (tail[lane] != SIZE_MAX) {
+            edgeFrom(tail[lane]);
+        }
+        std::for_each(before[j].rbegin(), before[j].rend(), edgeFrom); // (the last ones imply most)
+        tail[lane] = j, laneOf[j] = lane, mine[lane] = j + 1;
+        uint64_t moved = 0;
+        for (const auto *list : {&exec[ops[j]].in, &exec[ops[j]].out}) {
+            for (const int32_t t : *list) {
+                moved += t >= 0 ? pipeline_->tensor(t).sizeBytes() : 0;
+            }
+        }
+        bytes += moved, inARow += kLaunch + moved, load[lane] += kLaunch + moved;
+        finish[j] = start + kLaunch + moved;
+        longest = std::max(longest, finish[j]);
+    }
+    plan.pays = 16 * std::max(longest, bytes) <= 15 * inARow;
+    return plan;
+}
+
 int Session::capture(cudaStream_t stream) {
     // Operators that neither run on the tensor cores nor belong to the row kernels -- element-wise ones, pools, reductions,
     // movement -- are short or bound by memory, and one after the other each waits for the last block of the one before it
-    // and starts anew.  Where a stretch of them is no single chain, it is laid on four lanes, and an operator follows those
+    // and starts anew.  Where it pays (planLanes) a stretch of them is laid on four lanes, and an operator follows those
     // whose bytes it touches and the one before it on its lane (stream order is a full barrier like the one that the
     // reference records, graph/compute_graph_op.cpp:251-299; what it guarantees to the results are the former edges).
     // Twelve operators without dependencies, small and large tensors, on 1, 2, 3, 4, 6 and 12 lanes: 30.7, 19.9, 18.4, 17.2,
     // 17.8, 34.4 and 228, 203, 205, 202, 207, 216 us: a replayed graph pays for every root and every join.
     // Elsewhere consecutive launches overlap by dependent launches, which beat edges of this kind.
-    constexpr size_t kLanes = 4;
     const auto &exec = pipeline_->getExecList();
     LaunchChain chain{};
     if (progressWords_ != nullptr) {
@@ -603,16 +672,8 @@ int Session::capture(cudaStream_t stream) {
                 ops.push_back(end);
             }
         }
-        std::vector<std::vector<size_t>> before;
-        bool chainOnly = ops.size() < 2;
-        if (!chainOnly) {
-            before = branches(ops);
-            chainOnly = true;
-            for (size_t j = 1; j < before.size(); ++j) {
-                chainOnly = chainOnly && !before[j].empty() && before[j].back() == j - 1;
-            }
-        }
-        if (chainOnly) {
+        const LanePlan plan = ops.size() < 2 ? LanePlan{} : planLanes(ops);
+        if (!plan.pays) {
             for (const size_t last = std::max(end, k + 1); k < last; ++k) {
                 const PlainLaunches plain(joined);
                 const int r = enqueueOp(k, chainOrNull, stream);
@@ -624,8 +685,8 @@ int Session::capture(cudaStream_t stream) {
             continue;
         }
         std::vector<cudaGraphNode_t> entry;
-        std::vector<std::vector<cudaGraphNode_t>> exits(before.size());
-        std::vector<bool> followed(before.size(), false);
+        std::vector<std::vector<cudaGraphNode_t>> exits(ops.size());
+        std::vector<bool> followed(ops.size(), false);
         const auto failed = [&] {
             setLastError("CUDA graph capture: dependencies refused");
             return MLEL_ERROR_DEVICE;
@@ -634,42 +695,8 @@ int Session::capture(cudaStream_t stream) {
             return failed();
         }
         const PlainLaunches plain(true);
-        // An operator goes on where the last one that it follows ended, or else on the lane with the least to do: bytes, and
-        // what a launch costs (2 us) as bytes.
-        std::vector<size_t> tail(kLanes, SIZE_MAX), laneOf(before.size());
-        std::vector<uint64_t> load(kLanes, 0);
-        // of every operator the last one of each lane that precedes it (or is it), plus one: an edge is laid only from operators
-        // that no other edge implies (with all of them 400 operators on four chains replayed in 1730 us, see below)
-        std::vector<std::array<size_t, kLanes>> known(before.size());
-        for (size_t j = 0; j < before.size(); ++j) {
-            size_t lane = size_t(std::min_element(load.begin(), load.end()) - load.begin());
-            for (size_t l = 0; l < kLanes; ++l) {
-                if (!before[j].empty() && tail[l] == before[j].back()) {
-                    lane = l;
-                }
-            }
-            std::vector<size_t> after;
-            std::array<size_t, kLanes> &mine = known[j];
-            mine.fill(0);
-            const auto edgeFrom = [&](size_t b) {
-                if (mine[laneOf[b]] <= b) {
-                    after.push_back(b);
-                    for (size_t l = 0; l < kLanes; ++l) {
-                        mine[l] = std::max(mine[l], known[b][l]);
-                    }
-                }
-            };
-            if (tail[lane] != SIZE_MAX) {
-                edgeFrom(tail[lane]);
-            }
-            std::for_each(before[j].rbegin(), before[j].rend(), edgeFrom); // (the last ones imply most)
-            tail[lane] = j, laneOf[j] = lane, mine[lane] = j + 1;
-            load[lane] += uint64_t(12) << 20;
-            for (const auto *list : {&exec[ops[j]].in, &exec[ops[j]].out}) {
-                for (const int32_t t : *list) {
-                    load[lane] += t >= 0 ? pipeline_->tensor(t).sizeBytes() : 0;
-                }
-            }
+        for (size_t j = 0; j < ops.size(); ++j) {
+            const std::vector<size_t> &after = plan.after[j];
             std::vector<cudaGraphNode_t> from = after.empty() ? entry : std::vector<cudaGraphNode_t>{};
             for (const size_t b : after) {
                 from.insert(from.end(), exits[b].begin(), exits[b].end());
@@ -689,7 +716,7 @@ int Session::capture(cudaStream_t stream) {
             }
         }
         std::vector<cudaGraphNode_t> last;
-        for (size_t j = 0; j < before.size(); ++j) {
+        for (size_t j = 0; j < ops.size(); ++j) {
             if (!followed[j]) {
                 last.insert(last.end(), exits[j].begin(), exits[j].end());
             }
@@ -789,21 +816,29 @@ int Session::dispatchGraph(cudaStream_t stream) {
             }
             graphs_.erase(oldest);
         }
-        CapturedGraph captured;
-        cudaStream_t capture = nullptr;
-        if (cudaStreamCreateWithFlags(&capture, cudaStreamNonBlocking) != cudaSuccess) {
-            setLastError("cudaStreamCreate failed");
-            return MLEL_ERROR_DEVICE;
+        // The stream that takes the capture stays with the session: to make and to destroy one costs 0.11 ms, as much as a third of
+        // a first dispatch.
+        int device = 0;
+        if (cudaGetDevice(&device) != cudaSuccess || (captureStream_ != nullptr && device != captureDevice_)) {
+            dropCaptureStream();
         }
-        cudaError_t err = cudaStreamBeginCapture(capture, cudaStreamCaptureModeThreadLocal);
+        if (captureStream_ == nullptr) {
+            if (cudaStreamCreateWithFlags(&captureStream_, cudaStreamNonBlocking) != cudaSuccess) {
+                captureStream_ = nullptr;
+                setLastError("cudaStreamCreate failed");
+                return MLEL_ERROR_DEVICE;
+            }
+            captureDevice_ = device;
+        }
+        CapturedGraph captured;
+        cudaError_t err = cudaStreamBeginCapture(captureStream_, cudaStreamCaptureModeThreadLocal);
         if (err == cudaSuccess) {
-            rc = this->capture(capture);
-            err = cudaStreamEndCapture(capture, &captured.graph);
+            rc = capture(captureStream_);
+            err = cudaStreamEndCapture(captureStream_, &captured.graph);
         }
         if (err == cudaSuccess && rc == MLEL_SUCCESS) {
             err = cudaGraphInstantiate(&captured.exec, captured.graph, 0);
         }
-        cudaStreamDestroy(capture);
         if (rc != MLEL_SUCCESS || err != cudaSuccess) {
             if (captured.exec != nullptr) {
                 cudaGraphExecDestroy(captured.exec);

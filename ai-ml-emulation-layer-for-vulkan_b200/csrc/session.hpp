@@ -64,6 +64,12 @@ class Session {
     int capture(cudaStream_t stream);
     int enqueueOp(size_t k, LaunchChain *chain, cudaStream_t stream);
     std::vector<std::vector<size_t>> branches(const std::vector<size_t> &ops) const;
+    static constexpr size_t kLanes = 4;
+    struct LanePlan {
+        std::vector<std::vector<size_t>> after; // by operator, as positions in the list
+        bool pays = false;
+    };
+    LanePlan planLanes(const std::vector<size_t> &ops) const;
     int resolve(); // fills views_ with device addresses; fails if something is unbound
 
     GraphPipeline *pipeline_;
@@ -90,6 +96,9 @@ class Session {
     std::map<std::vector<const void *>, CapturedGraph> graphs_;
     std::vector<const void *> bindingKey() const;
     void dropGraphs();
+    cudaStream_t captureStream_{nullptr}; // takes the captures (nothing ever runs on it); made at the first one
+    int captureDevice_{0};
+    void dropCaptureStream();
 };
 
 const std::string &lastError();
