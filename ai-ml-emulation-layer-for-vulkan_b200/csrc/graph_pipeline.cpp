@@ -2132,31 +2132,55 @@ void GraphPipeline::prepareDepthwise() {
     }
 }
 
+GraphPipeline::TensorUses GraphPipeline::tensorUses() const {
+    TensorUses uses;
+    for (size_t k = 0; k < exec_.size(); ++k) {
+        for (const int32_t t : exec_[k].out) {
+            uses.writer[t] = uses.writer.count(t) ? -1 : int(k);
+        }
+        for (const int32_t t : exec_[k].in) {
+            ++uses.readers[t];
+        }
+        ++uses.readers[exec_[k].epi.shortcutTensor];
+    }
+    for (const int32_t t : outputs_) {
+        ++uses.readers[t];
+    }
+    return uses;
+}
+
+int GraphPipeline::stepTo(const TensorUses &uses, int32_t t, OpKind kind) const {
+    const auto w = uses.writer.find(t);
+    const auto r = uses.readers.find(t);
+    if (w == uses.writer.end() || w->second < 0 || r == uses.readers.end() || r->second != 1 || tensor(t).cls != TensorClass::Session ||
+        !tensor(t).packed()) {
+        return -1;
+    }
+    const OpDesc &op = exec_[size_t(w->second)];
+    return op.kind == kind && op.out.size() == 1 ? w->second : -1;
+}
+
+void GraphPipeline::dropOperators(const std::vector<bool> &gone) {
+    size_t kept = 0;
+    for (size_t k = 0; k < exec_.size(); ++k) {
+        if (!gone[k]) {
+            if (kept != k) {
+                exec_[kept] = std::move(exec_[k]);
+            }
+            ++kept;
+        }
+    }
+    exec_.resize(kept);
+}
+
 // CONCAT along the channels with inputs that are RESIZE (NEAREST), or a SLICE of one, of a smaller tensor -> OP_FUSED_CONCAT.
 // The elided tensors are session memory, written once and read once.
 void GraphPipeline::fuseResizedConcats() {
-    std::map<int32_t, int> writer, readers;
-    for (size_t k = 0; k < exec_.size(); ++k) {
-        for (const int32_t t : exec_[k].out) {
-            writer[t] = writer.count(t) ? -1 : int(k); // (-1: written more than once)
-        }
-        for (const int32_t t : exec_[k].in) {
-            ++readers[t];
-        }
-        ++readers[exec_[k].epi.shortcutTensor];
-    }
-    for (const int32_t t : outputs_) {
-        ++readers[t];
-    }
+    const TensorUses uses = tensorUses();
     std::vector<bool> gone(exec_.size(), false);
-    // the operator that makes t, if t is no more than a step on the way to its one reader
-    const auto stepOf = [&](int32_t t, OpKind kind) -> int {
-        const auto w = writer.find(t);
-        if (w == writer.end() || w->second < 0 || readers[t] != 1 || tensor(t).cls != TensorClass::Session || !tensor(t).packed()) {
-            return -1;
-        }
-        const OpDesc &op = exec_[size_t(w->second)];
-        return op.kind == kind && op.out.size() == 1 && !gone[size_t(w->second)] ? w->second : -1;
+    const auto stepOf = [&](int32_t t, OpKind kind) {
+        const int writer = stepTo(uses, t, kind);
+        return writer >= 0 && !gone[size_t(writer)] ? writer : -1;
     };
     for (size_t c = 0; c < exec_.size(); ++c) {
         OpDesc &op = exec_[c];
@@ -2233,16 +2257,7 @@ void GraphPipeline::fuseResizedConcats() {
         op.in = sources;
         op.concat = plan;
     }
-    size_t kept = 0;
-    for (size_t k = 0; k < exec_.size(); ++k) {
-        if (!gone[k]) {
-            if (kept != k) {
-                exec_[kept] = std::move(exec_[k]);
-            }
-            ++kept;
-        }
-    }
-    exec_.resize(kept);
+    dropOperators(gone);
 }
 
 // Products of one activation with constants whose results only an attention node reads (Q, K and V, or K and V) -> one product
@@ -2251,27 +2266,7 @@ void GraphPipeline::fuseResizedConcats() {
 // Three launches' ramps and partly filled rounds of tiles become one's: thirteen encoder shapes of 16 to 9216 tokens and 256 to
 // 1024 channels are all faster, four layers of 3 x 197 tokens 188 -> 163 us, twelve of 32 x 384 2123 -> 2035.
 void GraphPipeline::mergeProjections() {
-    std::map<int32_t, int> writer, readers;
-    for (size_t k = 0; k < exec_.size(); ++k) {
-        for (const int32_t t : exec_[k].out) {
-            writer[t] = writer.count(t) ? -1 : int(k); // (-1: written more than once)
-        }
-        for (const int32_t t : exec_[k].in) {
-            ++readers[t];
-        }
-        ++readers[exec_[k].epi.shortcutTensor];
-    }
-    for (const int32_t t : outputs_) {
-        ++readers[t];
-    }
-    const auto writerOf = [&](int32_t t, OpKind kind) -> int {
-        const auto w = writer.find(t);
-        if (w == writer.end() || w->second < 0 || readers[t] != 1 || tensor(t).cls != TensorClass::Session || !tensor(t).packed()) {
-            return -1;
-        }
-        const OpDesc &op = exec_[size_t(w->second)];
-        return op.kind == kind && op.out.size() == 1 ? w->second : -1;
-    };
+    const TensorUses uses = tensorUses();
     struct Part {
         int operand, product, reshape; // of the attention node; in exec_
     };
@@ -2290,8 +2285,8 @@ void GraphPipeline::mergeProjections() {
         }
         std::vector<Part> candidates;
         for (int operand = 0; operand < 3; ++operand) {
-            const int reshape = writerOf(exec_[a].in[size_t(operand)], OP_RESHAPE);
-            const int product = reshape < 0 ? -1 : writerOf(exec_[size_t(reshape)].in[0], OP_FUSED_MATMUL);
+            const int reshape = stepTo(uses, exec_[a].in[size_t(operand)], OP_RESHAPE);
+            const int product = reshape < 0 ? -1 : stepTo(uses, exec_[size_t(reshape)].in[0], OP_FUSED_MATMUL);
             if (product < 0) {
                 continue;
             }
@@ -2378,16 +2373,7 @@ void GraphPipeline::mergeProjections() {
         exec_[size_t(firstProduct)] = std::move(merged);
         exec_[a].attention = plan;
     }
-    size_t kept = 0;
-    for (size_t k = 0; k < exec_.size(); ++k) {
-        if (!gone[k]) {
-            if (kept != k) {
-                exec_[kept] = std::move(exec_[k]);
-            }
-            ++kept;
-        }
-    }
-    exec_.resize(kept);
+    dropOperators(gone);
 }
 
 const std::vector<OpDesc> &GraphPipeline::getExecList() {

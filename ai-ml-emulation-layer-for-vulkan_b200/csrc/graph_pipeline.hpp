@@ -165,6 +165,14 @@ class GraphPipeline {
     void prepareDepthwise();
     void fuseResizedConcats();
     void mergeProjections();
+    // Who makes and who reads the tensors of exec_ (graph outputs count as read); writer -1: written more than once.
+    struct TensorUses {
+        std::map<int32_t, int> writer, readers;
+    };
+    TensorUses tensorUses() const;
+    // The operator of that kind that makes t, if t is a session tensor between it and one reader; else -1.
+    int stepTo(const TensorUses &uses, int32_t t, OpKind kind) const;
+    void dropOperators(const std::vector<bool> &gone);
     int32_t addDerivedConstant(int32_t dtype, const std::vector<int64_t> &dims, const void *data);
     int32_t addScratchTensor(int32_t dtype, const std::vector<int64_t> &dims);
 

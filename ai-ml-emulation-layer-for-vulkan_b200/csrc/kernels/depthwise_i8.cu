@@ -49,13 +49,6 @@ struct DepthwiseParams {
     int32_t lo, hi, signedRounding;
 };
 
-__device__ __forceinline__ void transposeBytes(uint32_t a, uint32_t b, uint32_t c, uint32_t d, uint32_t (&o)[4]) {
-    const uint32_t t0 = __byte_perm(a, b, 0x5140), t1 = __byte_perm(c, d, 0x5140); // [a0 b0 a1 b1], [c0 d0 c1 d1]
-    const uint32_t t2 = __byte_perm(a, b, 0x7362), t3 = __byte_perm(c, d, 0x7362); // [a2 b2 a3 b3], [c2 d2 c3 d3]
-    o[0] = __byte_perm(t0, t1, 0x5410), o[1] = __byte_perm(t0, t1, 0x7632);
-    o[2] = __byte_perm(t2, t3, 0x5410), o[3] = __byte_perm(t2, t3, 0x7632);
-}
-
 // The first `bytes` bytes from any address (the others: anything).  Only aligned words that hold one of them are read.
 __device__ __forceinline__ uint32_t loadBytes(const int8_t *p, int bytes) {
     const uintptr_t at = reinterpret_cast<uintptr_t>(p);
@@ -154,11 +147,11 @@ __global__ void __launch_bounds__(128, 4) depthwise3x3TableKernel(const __grid_c
                 // tr[g][k]: four consecutive pixels of channel k.  Stride 1: pixels 0-3 and 2-5; window px starts at byte
                 // px & 1 of group px >> 1.  Stride 2: pixels 0-3, 2-5, 4-7, 5-8; windows start at bytes 0, 0, 0, 1.
                 uint32_t tr[NT][4];
-                transposeBytes(cols[0], cols[1], cols[2], cols[3], tr[0]);
-                transposeBytes(cols[2], cols[3], cols[4], cols[5], tr[1]);
+                transpose4x4Bytes(cols[0], cols[1], cols[2], cols[3], tr[0]);
+                transpose4x4Bytes(cols[2], cols[3], cols[4], cols[5], tr[1]);
                 if (SX == 2) {
-                    transposeBytes(cols[4], cols[5], cols[6], cols[7], tr[2]);
-                    transposeBytes(cols[5], cols[6], cols[7], cols[8], tr[3]);
+                    transpose4x4Bytes(cols[4], cols[5], cols[6], cols[7], tr[2]);
+                    transpose4x4Bytes(cols[5], cols[6], cols[7], cols[8], tr[3]);
                 }
 #pragma unroll
                 for (int r = 0; r < R; ++r) {

@@ -302,6 +302,13 @@ template <bool SIGNED> __device__ __forceinline__ int32_t wordsScale(const Words
     }
     return int32_t(high) >> w.shift;
 }
+// Four words of four bytes as a matrix, transposed: o[k] holds byte k of a, b, c and d.
+__device__ __forceinline__ void transpose4x4Bytes(uint32_t a, uint32_t b, uint32_t c, uint32_t d, uint32_t (&o)[4]) {
+    const uint32_t t0 = __byte_perm(a, b, 0x5140), t1 = __byte_perm(c, d, 0x5140); // [a0 b0 a1 b1], [c0 d0 c1 d1]
+    const uint32_t t2 = __byte_perm(a, b, 0x7362), t3 = __byte_perm(c, d, 0x7362); // [a2 b2 a3 b3], [c2 d2 c3 d3]
+    o[0] = __byte_perm(t0, t1, 0x5410), o[1] = __byte_perm(t0, t1, 0x7632);
+    o[2] = __byte_perm(t2, t3, 0x5410), o[3] = __byte_perm(t2, t3, 0x7632);
+}
 // Four results as bytes, saturated to int8 (value 0 in the lowest byte).
 __device__ __forceinline__ uint32_t packSatS8(int32_t y0, int32_t y1, int32_t y2, int32_t y3) {
     uint32_t r;

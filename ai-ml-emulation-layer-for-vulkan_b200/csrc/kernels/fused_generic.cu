@@ -219,13 +219,6 @@ __global__ void depthwise3x3Kernel(const int8_t *__restrict__ in, const int8_t *
 // the up to three output rows whose windows contain it, so the loads and transposes are shared vertically as
 // well.  Out-of-range taps read the input zero point, and bias - zp * (sum of weights) corrects for the raw sums,
 // as in depthwise3x3Kernel.  About 4.5 instructions per output for the convolution against 27 there.
-__device__ __forceinline__ void transpose4x4Bytes(uint32_t a, uint32_t b, uint32_t c, uint32_t d, uint32_t (&o)[4]) {
-    const uint32_t t0 = __byte_perm(a, b, 0x5140), t1 = __byte_perm(c, d, 0x5140); // [a0 b0 a1 b1], [c0 d0 c1 d1]
-    const uint32_t t2 = __byte_perm(a, b, 0x7362), t3 = __byte_perm(c, d, 0x7362); // [a2 b2 a3 b3], [c2 d2 c3 d3]
-    o[0] = __byte_perm(t0, t1, 0x5410), o[1] = __byte_perm(t0, t1, 0x7632);
-    o[2] = __byte_perm(t2, t3, 0x5410), o[3] = __byte_perm(t2, t3, 0x7632);
-}
-
 template <int R, int SX, bool OUT8>
 __global__ void __launch_bounds__(128, 4) depthwise3x3RowsKernel(const int8_t *in, const int8_t *w,
                                                               const int32_t *bias, int biasCount,
