@@ -26,7 +26,7 @@
 //
 // Measured (3x3, im2col kernels before): 64 x 56 x 56, 64 -> 64 channels 37.2 -> 19.1 us, 32 -> 64 37.8 -> 15.5; 270 x 480,
 // 96 -> 32 32.4 -> 11.9; 64 x 28 x 28, 128 -> 128 15.4 -> 13.8.  With the MMAs issued by a lane that their statement elects,
-// 270 x 480, 96 -> 32 8.6 (not with two MMAs a tap and a long epilogue, see ummaLed).
+// 270 x 480, 96 -> 32 8.6 (not with few MMAs a tap and a long epilogue, see ummaLed).
 // Bound now by the epilogue's RESCALEs and, with 128 channels, by the MMAs.
 #include <cuda.h>
 #include <cuda_runtime.h>
@@ -81,10 +81,12 @@ __device__ __forceinline__ uint64_t smemDescPlain(uint32_t addr, uint32_t leadin
 }
 
 // One MMA by lane 0, named by a predicate and not elected: it takes 62 cycles to issue where an elected one takes 21 (see umma).
-// That is the better pace for two MMAs a tap beside a tile of 64 channels and more, whose epilogue is the longer part in any case:
-// MMAs that arrive no faster than the pipe takes them (50 cycles) leave the epilogue warps of that scheduler their issue slots.
+// That is the better pace for one or two MMAs a tap beside tiles of 64 channels, where most CTAs have two: their epilogue is the longer
+// part, and MMAs that arrive no faster than the pipe takes them (50 cycles) leave the epilogue warps of that scheduler their issue slots.
 // (us, elected and so: 16 x 56 x 56, 64 -> 64 7.8 and 7.4, 32 images 11.5 and 11.0, 64 -> 128 11.8 and 11.0, 8 x 61 x 19, 64 -> 464 9.9
-// and 9.5.  Elsewhere the pace is the MMAs': 16 x 56 x 56, 64 -> 32 5.6 and 6.0, 96 -> 64 7.6 and 9.4, 270 x 480, 96 -> 32 8.6 and 11.4.)
+// and 9.5, 270 x 480, 32 -> 64 10.8 and 10.2, 8 x 112 x 112, 32 -> 64 9.2 and 8.8.  A CTA's first tile has to wait for its MMAs: with one
+// tile a CTA, 68 x 120, 64 -> 128, and with 1.8, 135 x 240, 32 -> 64, 0.1 us more.  Elsewhere the pace is the MMAs': 16 x 56 x 56, 64 -> 32
+// 5.6 and 6.0, 96 -> 64 7.6 and 9.4, 270 x 480, 96 -> 32 8.6 and 11.4; tiles of 128 channels the same either way.)
 __device__ __forceinline__ void ummaLed(uint32_t leader, uint32_t tmemD, DescWords a, DescWords b, uint32_t idesc, uint32_t accumulate) {
     asm volatile("{\n\t.reg .pred p, l;\n\t.reg .b64 a, b;\n\t"
                  "setp.ne.b32 l, %8, 0;\n\t"
@@ -103,7 +105,8 @@ template <int BN> constexpr int kOddPitch = BN + 4;                             
 template <int BN> constexpr int kOddBytes = 4 * 32 * kOddPitch<BN> * (BN == 32 ? 2 : 1) + 16; // quarters x rows x sets
 
 // BN: output channels of a tile (32, 64 or 128).  UNITS: the input is 16-byte units (see the head of the file).
-template <int BN, bool UNITS, bool ODD>
+// LED: for up to 64 input channels, 3x3 (see ummaLed).
+template <int BN, bool UNITS, bool ODD, bool LED>
 __global__ void __launch_bounds__(kThreadsTma, 1)
 gemmI8Window(const __grid_constant__ CUtensorMap mapX, const __grid_constant__ CUtensorMap mapW, const GemmI8Params p,
              const WindowTiling g) {
@@ -217,9 +220,11 @@ gemmI8Window(const __grid_constant__ CUtensorMap mapX, const __grid_constant__ C
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const uint32_t tmemD = tmemBase + buf * uint32_t(BN);
                 const auto tap = [&](uint32_t x, uint32_t w, bool first) {
-                    if constexpr (kSlices == 2 && kThree && BN >= 64 && !ODD) {
+                    if constexpr (LED) {
                         ummaLed(leader, tmemD, {x, highX}, {w, highW}, idesc, first ? 0u : 1u);
-                        ummaLed(leader, tmemD, {x + 2u, highX}, {w + 2u, highW}, idesc, 1u);
+                        if (kSlices == 2) {
+                            ummaLed(leader, tmemD, {x + 2u, highX}, {w + 2u, highW}, idesc, 1u);
+                        }
                     } else {
                         ummaBlock(tmemD, {x, highX}, 2, {w, highW}, 2, idesc, first ? 0u : 1u, kSlices);
                     }
@@ -232,7 +237,7 @@ gemmI8Window(const __grid_constant__ CUtensorMap mapX, const __grid_constant__ C
                             umma(tmemD, {stage + pairX[m], pairHigh}, {w + uint32_t(2 * m * BN), weightHigh}, idesc, m == 0 ? 0u : 1u);
                         }
                     }
-                } else if (kThree && kSlices == 1) { // (a window row to a statement)
+                } else if (kThree && kSlices == 1 && !LED) { // (a window row to a statement)
 #pragma unroll
                     for (int ky = 0; ky < 3; ++ky) {
                         ummaBlock(tmemD, {stageX + uint32_t(ky) * rowStep, highX}, tapStep, {lowW + uint32_t(3 * ky) * weightStep, highW},
@@ -263,8 +268,10 @@ gemmI8Window(const __grid_constant__ CUtensorMap mapX, const __grid_constant__ C
             }
         };
         const bool three = windowH == 3 && windowW == 3;
-        if (UNITS) {
+        if constexpr (UNITS) {
             tiles(std::integral_constant<int, 1>{}, std::false_type{});
+        } else if constexpr (LED) {
+            p.IC <= 32 ? tiles(std::integral_constant<int, 1>{}, std::true_type{}) : tiles(std::integral_constant<int, 2>{}, std::true_type{});
         } else {
             using Three = std::true_type;
             using Any = std::false_type;
@@ -413,14 +420,17 @@ gemmI8Window(const __grid_constant__ CUtensorMap mapX, const __grid_constant__ C
 
 // ---- host side --------------------------------------------------------------------------------------------
 
-template <int BN, bool UNITS, bool ODD>
+// CTAs of a channel tile.
+int windowCtas(const WindowTiling &g) { return std::max(1, std::min(smCount() / g.channelTiles, g.pixelTiles)); }
+
+template <int BN, bool UNITS, bool ODD, bool LED = false>
 int launchWindowRows(const CUtensorMap &mapX, const CUtensorMap &mapW, const GemmI8Params &p, const WindowTiling &g, size_t smem,
                  cudaStream_t s) {
-    auto kernel = gemmI8Window<BN, UNITS, ODD>;
+    auto kernel = gemmI8Window<BN, UNITS, ODD, LED>;
     if (!allowDynamicSmem(reinterpret_cast<const void *>(kernel), kWindowSmemLimit)) {
         return MLEL_ERROR_DEVICE;
     }
-    const int perChannelTile = std::max(1, std::min(smCount() / g.channelTiles, g.pixelTiles));
+    const int perChannelTile = windowCtas(g);
     const cudaError_t err = launchOverlapped(kernel, perChannelTile * g.channelTiles, kThreadsTma, smem, s, mapX, mapW, p, g);
     if (err != cudaSuccess) {
         setLastError(std::string("int8 window launch: ") + cudaGetErrorString(err));
@@ -435,8 +445,15 @@ bool windowOddRows(const GemmI8Params &p) { return p.ldOut % 16 != 0 || (reinter
 template <int BN, bool UNITS>
 int launchWindow(const CUtensorMap &mapX, const CUtensorMap &mapW, const GemmI8Params &p, const WindowTiling &g, size_t smem,
                  cudaStream_t s) {
-    return windowOddRows(p) ? launchWindowRows<BN, UNITS, true>(mapX, mapW, p, g, smem, s)
-                            : launchWindowRows<BN, UNITS, false>(mapX, mapW, p, g, smem, s);
+    if (windowOddRows(p)) {
+        return launchWindowRows<BN, UNITS, true>(mapX, mapW, p, g, smem, s);
+    }
+    if constexpr (BN == 64 && !UNITS) {
+        if (p.IC <= 64 && p.KH == 3 && p.KW == 3 && 15 * int64_t(windowCtas(g)) <= 8 * int64_t(g.pixelTiles)) {
+            return launchWindowRows<BN, UNITS, false, true>(mapX, mapW, p, g, smem, s);
+        }
+    }
+    return launchWindowRows<BN, UNITS, false>(mapX, mapW, p, g, smem, s);
 }
 
 size_t windowSmem(const WindowTiling &g, int bn, bool odd) {

@@ -94,3 +94,23 @@ def test_window_kernel_before_the_small_one(mlel, n, h, w, ic, oc, k, expected):
     got = runner.run([data])[0]
     assert [lib.mlel_tensor_core_launches(kernel) - before[kernel] for kernel in range(5)] == [int(kernel == expected) for kernel in range(5)]
     np.testing.assert_array_equal(got, want)
+
+
+@pytest.mark.parametrize("n,h,w,ic,oc", [
+    (5, 70, 110, 16, 64), (5, 70, 110, 32, 64), (5, 70, 110, 48, 64), (3, 75, 129, 64, 128),  # several tiles of 64 channels to a CTA
+    (1, 135, 240, 64, 64), (12, 56, 56, 64, 64),                                             # 1.7 and 2 tiles to a CTA
+    (3, 70, 110, 80, 64), (1, 70, 110, 64, 64), (3, 70, 110, 64, 63),                        # more channels, one tile, rows at any address
+])
+def test_both_forms_of_issue(mlel, n, h, w, ic, oc):
+    from mlel_b200.runtime import GraphRunner
+    r = np.random.Generator(np.random.PCG64(ic + oc))
+    g = GraphBuilder()
+    x = g.input(np.int8, (n, h, w, ic))
+    g.output(conv(g, r, x, oc, 3, 1, 1, -7, True, 37))
+    data = r.integers(-128, 128, x.shape, dtype=np.int8)
+    lib = mlel.lib()
+    lib.mlel_tensor_core_launches.restype = ctypes.c_longlong
+    runner = GraphRunner(g)
+    before = lib.mlel_tensor_core_launches(4)
+    np.testing.assert_array_equal(runner.run([data])[0], evaluate(g, [data])[0])
+    assert lib.mlel_tensor_core_launches(4) == before + 1
